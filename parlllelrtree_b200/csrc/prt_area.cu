@@ -25,10 +25,10 @@
 // even-odd test of each midpoint when a crossing is not clean; see
 // pair_boundary).  Contributions are scaled by the upstream gradient and
 // accumulated with atomicAdd, since a polygon may appear in many pairs.  Both
-// directions run in two stages: polygons of up to 64 vertices staged in
-// shared memory first, the pairs that do not fit listed for a 128-vertex
-// staging, larger ones on a global-memory path (backward) or the GPC clip
-// (forward).
+// directions run in stages: polygons of up to 64 vertices staged in shared
+// memory first, the pairs that do not fit listed for a 128-vertex staging,
+// then a 256-vertex one, and larger ones on a global-memory path (backward)
+// or the GPC clip (forward).
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -130,7 +130,7 @@ __device__ void pieces(const Poly &A, const Poly &B, double w, double *grad, int
   }
 }
 
-// ---- shared-memory adjoint (pairs up to kBwdMaxV vertices per polygon) ----
+// ---- shared-memory adjoint (pairs up to kBwdLargeV vertices per polygon) ----
 // The same boundary pieces with both polygons staged in shared memory, and
 // the candidate edges of the other polygon found through y slabs instead of
 // a scan over all of its edges.  The pair's common y range (float, rounded
@@ -151,10 +151,13 @@ __device__ void pieces(const Poly &A, const Poly &B, double w, double *grad, int
 // a vertex receives (as the end of one edge, as the start of the next) are
 // summed across neighbouring lanes before the atomics.  Edges with more than
 // kBwdMaxT crossings take the global-memory path (next_crossing).
-constexpr int kBwdMaxV = 128;
 constexpr int kBwdSmallV = 64;
+constexpr int kBwdMidV = 128;
+constexpr int kBwdLargeV = 256;  // BwdPoly's 8-bit vertex indices hold no more
 constexpr int kBwdMaxT = 16;
-constexpr int kBwdWarps = 4;
+// Warps (pairs) per block of the V-vertex stage: the 256-vertex staging takes
+// 22 KB a pair, so blocks of 2 warps fit 10 pairs an SM where blocks of 4 fit 8.
+constexpr int bwd_warps(int V) { return V > kBwdMidV ? 2 : 4; }
 constexpr int kSlabs = 32;
 constexpr unsigned kFullMask = 0xffffffffu;
 
@@ -431,26 +434,27 @@ __device__ __noinline__ void bwd_edge_exact(const BwdPoly<V> &Q, int nwq, const 
 // A (against B), e >= na edge e - na of B (against A); rounds of 32 edges.
 // ext[0], ext[1]: the float extents of A and B.
 //
-// Which intervals are inside: the midpoint of each interval (the
+// What is inside: by the midpoint of every interval between crossings (the
 // definition, bwd_edge_exact), or, while the pair's crossings are all clean,
-// by parity: a ring's first interval by its midpoint, every later interval of
-// the ring flips at each crossing (prefix XOR of the crossing counts over the
-// ring's edges, carried between rounds).  A crossing is clean when it is well
-// inside both edges (t and u at least 1e-9 from 0 and 1) and the edges are
-// not nearly parallel; collinear overlapping edges, two coinciding crossings
-// on an edge and an edge with more crossings than the list below holds are
-// not clean.
-// From the first round with an unclean edge on, the pair goes by the
-// definition.  Clean crossings flip the inside state exactly where the
-// midpoints change and pass next_crossing's test, so the two give the same
-// intervals.  The clean path keeps an edge's crossings sorted in registers.
-// Clean crossings kept per edge: 4 in gradient mode, 6 in area mode (1M
-// pairs of 16-64-vertex stars: 0.5% of the pairs have an edge with 5 or 6
-// crossings; in area mode they would go to the GPC clip, 3,670 pairs against
-// 119 with 6, while the gradient mode runs faster with the shorter list and
-// the definition for those pairs).
-constexpr int kBwdFast = 4;
-constexpr int kFwdFast = 6;
+// from the crossings alone: the state at an edge's start (the ring's first
+// edge by the midpoint of a piece of it, later ones flip with the number of
+// crossings before them on the ring: a prefix XOR carried between rounds) and
+// one signed term per crossing, +1 where the edge enters the other polygon
+// and -1 where it leaves it, by the side of the other edge that its ring's
+// orientation sign says is inside.  With the state s1 at the edge's end,
+//     sum (t1 - t0)         = s1 - sum sign t
+//     sum (t1^2 - t0^2) / 2 = (s1 - sum sign t^2) / 2
+// so no list of crossings is kept, sorted or bounded.  A crossing is clean
+// when it is well inside both edges (t and u at least 1e-9 from 0 and 1) and
+// the edges are not nearly parallel; collinear overlapping edges are not
+// clean, nor is an edge whose signed crossings do not add up to its change of
+// state (rings that cross, hole rings that are not flagged).  From the first
+// round with an unclean edge on, the pair goes by the definition.
+// (With a sorted register list per edge, of 4 crossings in gradient mode and 6
+// in area mode, 1M pairs of 16-64-vertex stars took 6.89 ms backward and 6.11
+// forward against 6.47 and 5.63 with the sums; of 50k pairs of 4-160 vertices,
+// whose long edges run along the other's spikes, 2.2 and 1.16 ms and a longer
+// GPC list against 1.09 and 1.05.)
 
 // Area mode of the same pass (the forward): per edge, the inside length
 // L = sum (t1 - t0) over its inside intervals contributes
@@ -495,12 +499,10 @@ __device__ inline bool pair_boundary(const BwdPoly<V> *M, const float4 *ext, int
       pb = P.bb[i];
     }
     const double rx = qx - px, ry = qy - py;
-    // clean crossings, ascending (2.0 = empty)
-    constexpr int kFast = kArea ? kFwdFast : kBwdFast;
-    double tc[kFast];
-#pragma unroll
-    for (int q = 0; q < kFast; q++) tc[q] = 2.0;
-    int m = 0;
+    double c1 = 0.0, c2 = 0.0;  // sums of sign t and sign t^2 over the edge's clean crossings
+    int c0 = 0;                 // and of the signs
+    int m = 0;                  // their number
+    double tfirst = 1.0;        // the first one
     bool unclean = false;
     if (valid && !exact) {
       const double rl = fabs(rx) + fabs(ry);
@@ -527,8 +529,7 @@ __device__ inline bool pair_boundary(const BwdPoly<V> *M, const float4 *ext, int
           const double d = fabs(den), tol = 1e-9 * d;
           const double tt = den > 0.0 ? tn : -tn, uu = den > 0.0 ? un : -un;
           if (tt < -tol || tt > d + tol || uu < -tol || uu > d + tol) continue;  // next_crossing rejects it
-          if (!(tt > tol && tt < d - tol && uu > tol && uu < d - tol && d > 1e-6 * rl * (fabs(sx) + fabs(sy))) ||
-              m == kFast) {
+          if (!(tt > tol && tt < d - tol && uu > tol && uu < d - tol && d > 1e-6 * rl * (fabs(sx) + fabs(sy)))) {
             unclean = true;
             continue;
           }
@@ -536,37 +537,32 @@ __device__ inline bool pair_boundary(const BwdPoly<V> *M, const float4 *ext, int
             const double sl = fabs(sx) + fabs(sy);
             err += (rl + sl) * rl * sl / d;
           }
-          double v = (apx * sy - apy * sx) / den;  // next_crossing's t
-          // sorted insert into the register list
-#pragma unroll
-          for (int q = 0; q < kFast; q++)
-            if (v < tc[q]) {
-              const double x = tc[q];
-              tc[q] = v;
-              v = x;
-            }
+          const double t = tn / den;  // next_crossing's t
+          // den > 0: the edge goes from the left of Q's edge to its right,
+          // out of Q where Q's material is on the left
+          const bool leaves = (den > 0.0) == (Q.sgn[k] > 0);
+          const double st = leaves ? -t : t;
+          c0 += leaves ? -1 : 1;
+          c1 += st;
+          c2 += st * t;
+          tfirst = fmin(tfirst, t);
           m++;
         }
       }
-#pragma unroll
-      for (int q = 1; q < kFast; q++) unclean |= m > q && tc[q - 1] == tc[q];
     }
     exact = __any_sync(kFullMask, unclean) || exact;
     if constexpr (kArea) {
       if (exact) return false;
     }
     double it = 0.0, i1 = 0.0;
-    if (exact) {
-      if (valid)
-        bwd_edge_exact(Q, nwq, ext[1 - side], g, gx, pb, px, py, rx, ry, side ? Ag : Bg, &it, &i1);
-    } else {
+    if (!exact) {
       const int rs = valid ? (side ? na : 0) + P.rst[i] : e;  // this edge's ring starts at edge rs
       // the first interval of each ring starting in this round, by its
       // midpoint: the whole warp tests it against all edges of the other polygon
       const bool rstart = valid && rs == e;
       double mx0 = 0.0, my0 = 0.0;
       if (rstart) {
-        const double tm = 0.5 * (m > 0 ? tc[0] : 1.0);
+        const double tm = 0.5 * tfirst;
         mx0 = px + tm * rx;
         my0 = py + tm * ry;
       }
@@ -595,26 +591,20 @@ __device__ inline bool pair_boundary(const BwdPoly<V> *M, const float4 *ext, int
       const int par = __popc(odd & lt & ~((1u << from) - 1u)) & 1;
       const bool sf = __shfl_sync(kFullMask, first, from);
       const bool st = (rs >= e0 ? sf : carry) != (par != 0);  // inside state at the edge's start
-      carry = __shfl_sync(kFullMask, st != ((m & 1) != 0), 31);
-      // intervals [0, tc[0]], [tc[0], tc[1]], ..., [tc[m-1], 1], alternately inside
+      const bool end = st != ((m & 1) != 0);
+      carry = __shfl_sync(kFullMask, end, 31);
+      if (__any_sync(kFullMask, valid && (int)st + c0 != (int)end)) {
+        exact = true;
+        if constexpr (kArea) return false;
+      }
       if (valid) {
-        bool in = st;
-        double a0 = 0.0;
-#pragma unroll
-        for (int a = 0; a <= kFast; a++) {
-          if (a <= m) {
-            const double a1 = a < m ? tc[a < kFast ? a : kFast - 1] : 1.0;
-            if (in) {
-              const double aa = 0.5 * (a1 * a1 - a0 * a0);
-              it += aa;
-              i1 += (a1 - a0) - aa;
-            }
-            a0 = a1;
-            in = !in;
-          }
-        }
+        const double s1 = end ? 1.0 : 0.0;
+        it = 0.5 * (s1 - c2);
+        i1 = (s1 - c1) - it;
       }
     }
+    if (exact && valid)
+      bwd_edge_exact(Q, nwq, ext[1 - side], g, gx, pb, px, py, rx, ry, side ? Ag : Bg, &it, &i1);
     if constexpr (kArea) {
       // it + i1 = sum (t1 - t0) over the inside intervals
       if (valid) area2 += P.sgn[i] * (it + i1) * ((px - ox) * ry - (py - oy) * rx);
@@ -668,10 +658,10 @@ __device__ __noinline__ void bwd_pair_global(const Poly &A, const Poly &B, doubl
   pieces(B, A, w, gb, lane);
 }
 
-// Pair lists of the two-stage launches: the first stage (V = kBwdSmallV)
-// takes every pair and lists those with a polygon above V vertices (or 31
-// rings) in `defer`; the second stage (V = kBwdMaxV) takes only the listed
-// pairs (`sel`, *sel_count of them).
+// Pair lists of the staged launches: the first stage (V = kBwdSmallV) takes
+// every pair and lists those with a polygon above V vertices (or 31 rings) in
+// `defer`; the next stages (V = kBwdMidV, kBwdLargeV) take only the pairs the
+// one before listed (`sel`, *sel_count of them).
 struct PairList {
   const int32_t *sel;                   // items of this launch (nullptr: pairs 0 .. n-1)
   const unsigned long long *sel_count;  // how many (device)
@@ -683,14 +673,17 @@ __device__ __forceinline__ int64_t list_items(const PairList &L, int64_t n) {
   return L.sel ? (int64_t)min((unsigned long long)n, *L.sel_count) : n;
 }
 
-// 4 blocks of 4 warps per SM (120 registers, no spills; measured at 1M
+// 4 blocks of 4 warps per SM (118-120 registers, no spills; measured at 1M
 // pairs of 16-64-vertex stars, 5 blocks of the V = 64 kernel spill and run
-// 10% slower).
+// 10% slower).  The 256-vertex stage is bound by its shared memory: 5 blocks
+// of 2 warps.  Before it, 50k pairs of 4-160 vertices (a third of them above
+// 128) took 10.8 ms here on the global-memory path and 11.5 ms in the
+// forward's GPC clip.
 template <int V>
-__global__ void __launch_bounds__(32 * kBwdWarps, 4) area_bwd_kernel(
+__global__ void __launch_bounds__(32 * bwd_warps(V), V > kBwdMidV ? 5 : 4) area_bwd_kernel(
     const int32_t *__restrict__ pa, const int32_t *__restrict__ pb, int64_t n, LayerDev base, LayerDev over,
     const double *__restrict__ upstream, double *grad_base, double *grad_over, PairList PL) {
-  __shared__ BwdPoly<V> sm[kBwdWarps][2];
+  __shared__ BwdPoly<V> sm[bwd_warps(V)][2];
   BwdPoly<V> *M = sm[threadIdx.x >> 5];
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -790,10 +783,10 @@ std::atomic<int64_t> g_fwd_fallbacks{0};
 // V = 64: 5 blocks of 4 warps per SM (96 registers: a few spills, 10% faster
 // than 4 blocks at 1M pairs of 16-64-vertex stars).
 template <int V>
-__global__ void __launch_bounds__(32 * kBwdWarps, V <= kBwdSmallV ? 5 : 4) area_fwd_kernel(
+__global__ void __launch_bounds__(32 * bwd_warps(V), V <= kBwdSmallV || V > kBwdMidV ? 5 : 4) area_fwd_kernel(
     const int32_t *__restrict__ pa, const int32_t *__restrict__ pb, int64_t n, LayerDev base, LayerDev over,
     double *__restrict__ area, int32_t *__restrict__ fb, unsigned long long *__restrict__ fb_count, PairList PL) {
-  __shared__ BwdPoly<V> sm[kBwdWarps][2];
+  __shared__ BwdPoly<V> sm[bwd_warps(V)][2];
   BwdPoly<V> *M = sm[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
@@ -878,14 +871,30 @@ __global__ void scatter_area_kernel(const int32_t *__restrict__ fb, int64_t m, c
     area[fb[k]] = src[k];
 }
 
-int area_blocks(int64_t n_pairs, const void *kernel) {
+int area_blocks(int64_t n_pairs, int threads, const void *kernel) {
   int b = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, 32 * kBwdWarps, 0) != cudaSuccess || b < 1) {
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, threads, 0) != cudaSuccess || b < 1) {
     cudaGetLastError();
     b = 4;
   }
   // exactly the resident blocks (each warp loops over pairs): no tail wave
-  return grid_for(n_pairs * 32, 32 * kBwdWarps, b);
+  return grid_for(n_pairs * 32, threads, b);
+}
+
+template <int V>
+void launch_area_fwd(const int32_t *pa, const int32_t *pb, int64_t n, const LayerDev &base, const LayerDev &over,
+                     double *area, int32_t *fb, unsigned long long *fb_count, const PairList &PL, cudaStream_t s) {
+  const int threads = 32 * bwd_warps(V);
+  area_fwd_kernel<V><<<area_blocks(n, threads, (const void *)area_fwd_kernel<V>), threads, 0, s>>>(
+      pa, pb, n, base, over, area, fb, fb_count, PL);
+}
+
+template <int V>
+void launch_area_bwd(const int32_t *pa, const int32_t *pb, int64_t n, const LayerDev &base, const LayerDev &over,
+                     const double *up, double *gb, double *go, const PairList &PL, cudaStream_t s) {
+  const int threads = 32 * bwd_warps(V);
+  area_bwd_kernel<V><<<area_blocks(n, threads, (const void *)area_bwd_kernel<V>), threads, 0, s>>>(pa, pb, n, base,
+                                                                                                  over, up, gb, go, PL);
 }
 
 }  // namespace
@@ -903,23 +912,23 @@ int prt_area_fwd(const int32_t *d_pair_a, const int32_t *d_pair_b, int64_t n_pai
   if (n_pairs == 0) return PRT_OK;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   // boundary integral for the clean pairs, the list of the others; pairs
-  // with a polygon above kBwdSmallV vertices go through the second stage
+  // with a polygon too large for one stage's staging go to the next
   unsigned char *scr = nullptr;
-  int rc = dmalloc(reinterpret_cast<void **>(&scr), 64 + 8 * (size_t)n_pairs, s);
+  int rc = dmalloc(reinterpret_cast<void **>(&scr), 64 + 12 * (size_t)n_pairs, s);
   if (rc) return rc;
-  unsigned long long *cnt = reinterpret_cast<unsigned long long *>(scr);
-  unsigned long long *dcnt = cnt + 1;
+  unsigned long long *cnt = reinterpret_cast<unsigned long long *>(scr);  // fallbacks, then the two stage lists
   int32_t *fb = reinterpret_cast<int32_t *>(scr + 64);
-  int32_t *defer = fb + n_pairs;
-  cudaError_t e = cudaMemsetAsync(cnt, 0, 16, s);
+  int32_t *mid = fb + n_pairs, *large = mid + n_pairs;
+  cudaError_t e = cudaMemsetAsync(cnt, 0, 24, s);
   if (e == cudaSuccess) {
     PRT_PROF("area_fwd", s);
-    area_fwd_kernel<kBwdSmallV><<<area_blocks(n_pairs, (const void *)area_fwd_kernel<kBwdSmallV>), 32 * kBwdWarps,
-                                  0, s>>>(d_pair_a, d_pair_b, n_pairs, layer_dev(base), layer_dev(overlay), d_area, fb,
-                                          cnt, PairList{nullptr, nullptr, defer, dcnt});
-    area_fwd_kernel<kBwdMaxV><<<area_blocks(n_pairs, (const void *)area_fwd_kernel<kBwdMaxV>), 32 * kBwdWarps, 0,
-                                s>>>(d_pair_a, d_pair_b, n_pairs, layer_dev(base), layer_dev(overlay), d_area, fb,
-                                     cnt, PairList{defer, dcnt, nullptr, nullptr});
+    const LayerDev A = layer_dev(base), B = layer_dev(overlay);
+    launch_area_fwd<kBwdSmallV>(d_pair_a, d_pair_b, n_pairs, A, B, d_area, fb, cnt,
+                                PairList{nullptr, nullptr, mid, cnt + 1}, s);
+    launch_area_fwd<kBwdMidV>(d_pair_a, d_pair_b, n_pairs, A, B, d_area, fb, cnt,
+                              PairList{mid, cnt + 1, large, cnt + 2}, s);
+    launch_area_fwd<kBwdLargeV>(d_pair_a, d_pair_b, n_pairs, A, B, d_area, fb, cnt,
+                                PairList{large, cnt + 2, nullptr, nullptr}, s);
     e = cudaGetLastError();
   }
   unsigned long long m = 0;
@@ -977,23 +986,23 @@ int prt_area_bwd(const int32_t *d_pair_a, const int32_t *d_pair_b, int64_t n_pai
             PRT_ERR_INVALID, "NULL argument");
   if (n_pairs == 0) return PRT_OK;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  // pairs with a polygon above kBwdSmallV vertices: listed by the first
-  // stage, taken by the second
+  // pairs with a polygon too large for one stage's staging: listed by it,
+  // taken by the next
   unsigned char *scr = nullptr;
-  int rc = dmalloc(reinterpret_cast<void **>(&scr), 64 + 4 * (size_t)n_pairs, s);
+  int rc = dmalloc(reinterpret_cast<void **>(&scr), 64 + 8 * (size_t)n_pairs, s);
   if (rc) return rc;
-  unsigned long long *dcnt = reinterpret_cast<unsigned long long *>(scr);
-  int32_t *defer = reinterpret_cast<int32_t *>(scr + 64);
-  cudaError_t e = cudaMemsetAsync(dcnt, 0, 8, s);
+  unsigned long long *cnt = reinterpret_cast<unsigned long long *>(scr);  // the two stage lists
+  int32_t *mid = reinterpret_cast<int32_t *>(scr + 64), *large = mid + n_pairs;
+  cudaError_t e = cudaMemsetAsync(cnt, 0, 16, s);
   if (e == cudaSuccess) {
     PRT_PROF("area_bwd", s);
-    area_bwd_kernel<kBwdSmallV><<<area_blocks(n_pairs, (const void *)area_bwd_kernel<kBwdSmallV>), 32 * kBwdWarps,
-                                  0, s>>>(d_pair_a, d_pair_b, n_pairs, layer_dev(base), layer_dev(overlay),
-                                          d_upstream, d_grad_base, d_grad_overlay,
-                                          PairList{nullptr, nullptr, defer, dcnt});
-    area_bwd_kernel<kBwdMaxV><<<area_blocks(n_pairs, (const void *)area_bwd_kernel<kBwdMaxV>), 32 * kBwdWarps, 0,
-                                s>>>(d_pair_a, d_pair_b, n_pairs, layer_dev(base), layer_dev(overlay), d_upstream,
-                                     d_grad_base, d_grad_overlay, PairList{defer, dcnt, nullptr, nullptr});
+    const LayerDev A = layer_dev(base), B = layer_dev(overlay);
+    launch_area_bwd<kBwdSmallV>(d_pair_a, d_pair_b, n_pairs, A, B, d_upstream, d_grad_base, d_grad_overlay,
+                                PairList{nullptr, nullptr, mid, cnt}, s);
+    launch_area_bwd<kBwdMidV>(d_pair_a, d_pair_b, n_pairs, A, B, d_upstream, d_grad_base, d_grad_overlay,
+                              PairList{mid, cnt, large, cnt + 1}, s);
+    launch_area_bwd<kBwdLargeV>(d_pair_a, d_pair_b, n_pairs, A, B, d_upstream, d_grad_base, d_grad_overlay,
+                                PairList{large, cnt + 1, nullptr, nullptr}, s);
     e = cudaGetLastError();
   }
   dfree(scr, s);

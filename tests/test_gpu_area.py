@@ -211,3 +211,31 @@ def test_forward_differentiable_configuration(cuda):
     for i in range(n):
         ref = oracle.result_area(oracle.gpc_clip(rings_of(A, i), rings_of(B, i), 1))
         assert abs(area[i] - ref) <= 1e-9 * abs(ref) + 1e-22, (i, area[i], ref)
+
+
+@pytest.mark.parametrize("nv", [64, 65, 128, 129, 255, 256, 257])
+def test_staging_edges(cuda, nv):
+    """A 64-vertex B against A of nv vertices: the last size of each staging
+    stage and the first of the next, against the oracle's area and gradient
+    (the tolerances of test_forward_and_adjoint_match_oracle)."""
+    import parlllelrtree_b200 as prt
+
+    n = 40
+    rng = np.random.default_rng(nv)
+    c, r = rng.random((n, 2)), np.full(n, 0.01)
+    A = dg.star_layer(n, seed=nv, nv_lo=nv, nv_hi=nv, centre_xy=c, radii=r)
+    B = dg.star_layer(n, seed=nv + 1, nv_lo=64, nv_hi=64, centre_xy=c + 0.003, radii=r)
+    LA, LB = prt.Layer.from_dict(A), prt.Layer.from_dict(B)
+    idx = torch.arange(n, dtype=torch.int32, device="cuda")
+    xa, xb = LA.xy.clone().requires_grad_(True), LB.xy.clone().requires_grad_(True)
+    area = prt.intersection_area(LA, LB, idx, idx, xa, xb)
+    area.sum().backward()
+    ga, gb = xa.grad.cpu().numpy().reshape(n, nv, 2), xb.grad.cpu().numpy().reshape(n, 64, 2)
+    for i in range(n):
+        s, c2 = rings_of(A, i), rings_of(B, i)
+        ref = oracle.result_area(oracle.gpc_clip(s, c2, 1))
+        assert abs(area[i].item() - ref) <= 1e-9 * abs(ref) + 1e-22, i
+        _, rs, rc = oracle.area_grad(s, c2, np.zeros(1, np.int32), np.zeros(1, np.int32))
+        scale = max(np.abs(rs).max(), np.abs(rc).max())
+        assert np.abs(ga[i] - rs).max() <= 1e-9 * scale, i
+        assert np.abs(gb[i] - rc).max() <= 1e-9 * scale, i
