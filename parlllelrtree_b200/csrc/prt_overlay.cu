@@ -153,16 +153,25 @@ __device__ __noinline__ void process_pair_warp(const PairSrc &S, const ClipOut &
 
 namespace {
 
-__global__ void nv_kernel(PairSrc S, int64_t n, const int64_t *__restrict__ idx, int scale, int64_t *__restrict__ nv,
-                          int64_t *__restrict__ demand) {
+// Adds v over the block to *total (one atomic per warp).
+__device__ __forceinline__ void add_total(unsigned long long v, unsigned long long *total) {
+  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0 && v) atomicAdd(total, v);
+}
+
+// Arena bytes of each item's pair, and the vertices of all of them.
+__global__ void demand_kernel(PairSrc S, int64_t n, const int64_t *__restrict__ idx, int scale,
+                              int64_t *__restrict__ demand, unsigned long long *__restrict__ total) {
+  unsigned long long sum = 0;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
     int64_t i = idx ? idx[t] : t;
     gpc::PolyView a, b;
     int64_t v = 0;
     if (!resolve(S, i, a, b, v)) v = 0;
-    if (nv) nv[t] = v;
-    if (demand) demand[t] = (int64_t)gpc::arena_bytes(gpc::caps_for(v, scale));
+    sum += (unsigned long long)v;
+    demand[t] = (int64_t)gpc::arena_bytes(gpc::caps_for(v, scale));
   }
+  add_total(sum, total);
 }
 
 __global__ void __launch_bounds__(128) clip_plain_kernel(PairSrc S, ClipOut O, const int64_t *__restrict__ idx,
@@ -251,20 +260,30 @@ __global__ void __launch_bounds__(32, kLptThreadWarpsPerSM)
   lpt_body<false>(S, O, order, plan, tickets, arena, scale, nullptr);
 }
 
-// Sort keys: larger vertex counts first.
-__global__ void size_key_kernel(const int64_t *__restrict__ nv, int64_t n, uint32_t *__restrict__ key,
-                                uint32_t *__restrict__ val) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    int64_t v = nv[i];
-    key[i] = 0xFFFFFFFFu - (uint32_t)(v > 0xFFFFFFFFll ? 0xFFFFFFFFll : v);
-    val[i] = (uint32_t)i;
+// Sort keys of the items' pairs, larger vertex counts first, and the vertices
+// of all of them.
+__global__ void size_key_kernel(PairSrc S, int64_t n, const int64_t *__restrict__ idx, uint32_t *__restrict__ key,
+                                uint32_t *__restrict__ val, unsigned long long *__restrict__ total) {
+  unsigned long long sum = 0;
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
+    gpc::PolyView a, b;
+    int64_t v = 0;
+    if (!resolve(S, idx ? idx[t] : t, a, b, v)) v = 0;
+    sum += (unsigned long long)v;
+    key[t] = 0xFFFFFFFFu - (uint32_t)(v > 0xFFFFFFFFll ? 0xFFFFFFFFll : v);
+    val[t] = (uint32_t)t;
   }
+  add_total(sum, total);
 }
+
+struct BinThresholds {
+  int64_t thr[PRT_MAX_BINS];
+};
 
 // bounds[b] = first sorted position whose vertex count is <= thr[b]
 // (counts descend along the sorted order); maxnv[b] = count at that position.
 __global__ void bin_bounds_kernel(const uint32_t *__restrict__ k0, const uint32_t *__restrict__ k1,
-                                  const int *__restrict__ sel, int64_t n, const int64_t *__restrict__ thr, int nbins,
+                                  const int *__restrict__ sel, int64_t n, BinThresholds T, int nbins,
                                   int64_t *__restrict__ bounds, int64_t *__restrict__ maxnv) {
   const uint32_t *k = *sel ? k1 : k0;
   int b = threadIdx.x;
@@ -273,7 +292,7 @@ __global__ void bin_bounds_kernel(const uint32_t *__restrict__ k0, const uint32_
   while (lo < hi) {
     int64_t mid = (lo + hi) / 2;
     int64_t v = (int64_t)(0xFFFFFFFFu - k[mid]);
-    if (v > thr[b]) lo = mid + 1;
+    if (v > T.thr[b]) lo = mid + 1;
     else hi = mid;
   }
   bounds[b] = lo;
@@ -316,28 +335,32 @@ __global__ void area_from_results_kernel(const int64_t *__restrict__ pair_cstart
   }
 }
 
-// contours, vertices and non-empty pairs over the live results
-__global__ void result_totals_kernel(const int64_t *__restrict__ pair_cstart, const int32_t *__restrict__ pair_ncont,
-                                     const int32_t *__restrict__ cont_nverts, int64_t n,
-                                     unsigned long long *__restrict__ tot) {
-  unsigned long long c = 0, v = 0, ne = 0;
+// Contours, vertices, non-empty pairs and pairs to retry over the results
+// (area-only mode, pair_ncont nullptr: the pairs to retry alone).
+__global__ void result_totals_kernel(const int32_t *__restrict__ status, const int64_t *__restrict__ pair_cstart,
+                                     const int32_t *__restrict__ pair_ncont, const int32_t *__restrict__ cont_nverts,
+                                     int64_t n, unsigned long long *__restrict__ tot) {
+  unsigned long long c = 0, v = 0, ne = 0, bad = 0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    int k = pair_ncont[i];
-    c += k;
-    ne += k > 0;
-    for (int j = 0; j < k; j++) v += cont_nverts[pair_cstart[i] + j];
+    if (status[i] != kPairOk) {
+      bad++;
+    } else if (pair_ncont) {
+      const int k = pair_ncont[i];
+      c += k;
+      ne += k > 0;
+      for (int j = 0; j < k; j++) v += cont_nverts[pair_cstart[i] + j];
+    }
   }
-  for (int o = 16; o; o >>= 1) {
-    c += __shfl_xor_sync(0xffffffffu, c, o);
-    v += __shfl_xor_sync(0xffffffffu, v, o);
-    ne += __shfl_xor_sync(0xffffffffu, ne, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    atomicAdd(&tot[0], c);
-    atomicAdd(&tot[1], v);
-    atomicAdd(&tot[2], ne);
-  }
+  add_total(c, &tot[0]);
+  add_total(v, &tot[1]);
+  add_total(ne, &tot[2]);
+  add_total(bad, &tot[3]);
 }
+
+// Arena bytes of one launch: a third of the free memory within these bounds.
+// The query is a driver call of 100-300 us (milliseconds on a shared host), so
+// a launch that needs no more than the lower bound goes without it.
+constexpr size_t kArenaBudgetLeast = (size_t)64 << 20, kArenaBudgetMost = (size_t)48 << 30;
 
 size_t arena_budget() {
   size_t fr = 0, tot = 0;
@@ -346,8 +369,7 @@ size_t arena_budget() {
     return (size_t)1 << 30;
   }
   size_t b = fr / 3;
-  const size_t cap = (size_t)48 << 30;
-  return std::max<size_t>(std::min(b, cap), (size_t)64 << 20);
+  return std::max<size_t>(std::min(b, kArenaBudgetMost), kArenaBudgetLeast);
 }
 
 }  // namespace
@@ -444,7 +466,28 @@ struct OverlayState {
   int64_t n;
   int sched = PRT_SCHED_PLAIN;
   int64_t retried = 0;
+  unsigned long long *words = nullptr;  // the block the pool counters are in: [2..5] result totals, [6] vertices in
 };
+
+// Result pools for a first guess at the result size from the vertices that
+// went in (grown on demand): one contour per pair and one per 64 vertices;
+// half of the vertices for an intersection, up to all of them and some
+// crossings for the other operations while that stays within kPoolGenerous
+// bytes (a pair the pool has no room for is clipped again).
+constexpr int64_t kPoolGenerous = 1ll << 30;
+
+static int first_pools(OverlayState &st, int64_t total_nv, cudaStream_t s) {
+  if (st.O.area || st.O.xy) return PRT_OK;
+  st.O.cap_c = total_nv / 64 + st.n + st.n / 4 + 1024;
+  st.O.cap_v = total_nv / 2 + 4096;
+  const int64_t wide = total_nv + total_nv / (st.S.op == PRT_GPC_XOR ? 2 : 8) + 4096;
+  if (st.S.op != PRT_GPC_INT && 16 * wide <= kPoolGenerous) st.O.cap_v = wide;
+  int rc = dalloc(&st.O.cont_vstart, st.O.cap_c, s);
+  if (!rc) rc = dalloc(&st.O.cont_nverts, st.O.cap_c, s);
+  if (!rc) rc = dalloc(&st.O.cont_hole, st.O.cap_c, s);
+  if (!rc) rc = dalloc(&st.O.xy, 2 * st.O.cap_v, s);
+  return rc;
+}
 
 static int grow_pools(OverlayState &st, cudaStream_t s, int64_t need_c, int64_t need_v) {
   unsigned long long used[2];
@@ -497,18 +540,21 @@ static int run_plain(OverlayState &st, const int64_t *d_idx, int64_t count, int 
     dfree(demand, s);
     return rc;
   }
+  cudaMemsetAsync(st.words + 6, 0, 8, s);
   {
     PRT_PROF("nv", s);
-    nv_kernel<<<grid_for(count, 256, 16), 256, 0, s>>>(st.S, count, d_idx, scale, nullptr, demand);
+    demand_kernel<<<grid_for(count, 256, 16), 256, 0, s>>>(st.S, count, d_idx, scale, demand, st.words + 6);
   }
   rc = exclusive_scan<int64_t>(demand, count, off, off + count, s);
   std::vector<int64_t> h_off(count + 1);
   if (!rc) {
+    unsigned long long total_nv = 0;
     cudaError_t e = cudaMemcpyAsync(h_off.data(), off, 8 * (count + 1), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&total_nv, st.words + 6, 8, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) rc = cuda_status(e, "overlay plain");
+    rc = e == cudaSuccess ? first_pools(st, (int64_t)total_nv, s) : cuda_status(e, "overlay plain");
   }
-  const int64_t budget = (int64_t)arena_budget();
+  const int64_t budget = (int64_t)(h_off[count] <= (int64_t)kArenaBudgetLeast ? kArenaBudgetLeast : arena_budget());
   unsigned char *arena = nullptr;
   int64_t arena_cap = 0;
   int64_t b = 0;
@@ -563,53 +609,51 @@ static int run_batched(OverlayState &st, const int64_t *d_idx, int64_t count, in
   const int64_t n = count;
   const prt_schedule sc = current_schedule();
   const int nb = sc.nbins;
-  int64_t *nv = nullptr;
+  // the words the host reads back after the size sort, in one copy
+  struct Head {
+    unsigned err;
+    int sel;
+    unsigned long long total_nv;
+    int64_t bnd[PRT_MAX_BINS], mx[PRT_MAX_BINS];
+    unsigned long long tickets[PRT_MAX_BINS + 1];  // bins + fallbacks
+  } h;
+  static_assert(sizeof(Head) <= 512, "head block");
   unsigned char *scr = nullptr;
-  int rc = dalloc(&nv, n, s);
-  if (!rc) rc = dmalloc(reinterpret_cast<void **>(&scr), 512 + 16 * n + 4 * n, s);
-  if (rc) {
-    dfree(nv, s);
-    return rc;
-  }
-  unsigned *err = reinterpret_cast<unsigned *>(scr);
-  int *sel = reinterpret_cast<int *>(scr + 8);
-  int64_t *thr = reinterpret_cast<int64_t *>(scr + 16);                            // PRT_MAX_BINS
-  int64_t *bnd = thr + PRT_MAX_BINS;                                               // PRT_MAX_BINS
-  int64_t *mx = bnd + PRT_MAX_BINS;                                                // PRT_MAX_BINS
-  unsigned long long *tickets = reinterpret_cast<unsigned long long *>(mx + PRT_MAX_BINS);  // bins + fallbacks
+  int rc = dmalloc(reinterpret_cast<void **>(&scr), 512 + 16 * n + 4 * n, s);
+  if (rc) return rc;
+  Head *d = reinterpret_cast<Head *>(scr);
   uint32_t *k0 = reinterpret_cast<uint32_t *>(scr + 512);
   uint32_t *k1 = k0 + n, *v0 = k1 + n, *v1 = v0 + n, *order = v1 + n;
   cudaMemsetAsync(scr, 0, 512, s);
-  cudaMemcpyAsync(thr, sc.bin_thresholds, sizeof(int64_t) * nb, cudaMemcpyHostToDevice, s);
+  BinThresholds T;
+  for (int b = 0; b < PRT_MAX_BINS; b++) T.thr[b] = b < nb ? sc.bin_thresholds[b] : 0;
   const int g = grid_for(n, 256, 16);
   {
-    PRT_PROF("nv", s);
-    nv_kernel<<<g, 256, 0, s>>>(st.S, n, d_idx, 1, nv, nullptr);
-  }
-  {
     PRT_PROF("size_key", s);
-    size_key_kernel<<<g, 256, 0, s>>>(nv, n, k0, v0);
+    size_key_kernel<<<g, 256, 0, s>>>(st.S, n, d_idx, k0, v0, &d->total_nv);
   }
-  rc = radix_sort_pairs<uint32_t>(k0, v0, k1, v1, n, 32, sel, err, s);
+  rc = radix_sort_pairs<uint32_t>(k0, v0, k1, v1, n, 32, &d->sel, &d->err, s);
   int64_t hb[PRT_MAX_BINS + 1] = {0}, hm[PRT_MAX_BINS] = {0};
   if (!rc) {
     {
       PRT_PROF("select_u32", s);
-      select_u32_kernel<<<g, 256, 0, s>>>(v0, v1, sel, n, order, d_idx);
+      select_u32_kernel<<<g, 256, 0, s>>>(v0, v1, &d->sel, n, order, d_idx);
     }
     {
       PRT_PROF("bin_bounds", s);
-      bin_bounds_kernel<<<1, 32, 0, s>>>(k0, k1, sel, n, thr, nb, bnd, mx);
+      bin_bounds_kernel<<<1, 32, 0, s>>>(k0, k1, &d->sel, n, T, nb, d->bnd, d->mx);
     }
-    unsigned herr = 0;
-    cudaMemcpyAsync(hb, bnd, sizeof(int64_t) * nb, cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(hm, mx, sizeof(int64_t) * nb, cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(&herr, err, sizeof herr, cudaMemcpyDeviceToHost, s);
-    cudaError_t e = cudaStreamSynchronize(s);
+    cudaError_t e = cudaMemcpyAsync(&h, d, sizeof h, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) rc = cuda_status(e, "overlay batched");
-    if (!rc && (herr & kErrTimeout)) {
+    if (!rc && (h.err & kErrTimeout)) {
       set_error("overlay batched: size sort look-back wait timed out");
       rc = PRT_ERR_TIMEOUT;
+    }
+    if (!rc) {
+      memcpy(hb, h.bnd, sizeof(int64_t) * nb);
+      memcpy(hm, h.mx, sizeof(int64_t) * nb);
+      rc = first_pools(st, (int64_t)h.total_nv, s);
     }
   }
   // bin b covers sorted positions [bnd[b], bnd[b+1]) (bnd[nbins] = n)
@@ -630,7 +674,8 @@ static int run_batched(OverlayState &st, const int64_t *d_idx, int64_t count, in
       for (int b = 0; b < nb; b++) run_sc.bin_warp_mode[b] = 1;
   }
   size_t smem = 0;
-  const size_t bytes = plan_bins(run_sc, counts, hm, arena_budget(), plan, &smem, scale, true);
+  size_t bytes = plan_bins(run_sc, counts, hm, kArenaBudgetMost, plan, &smem, scale, true);
+  if (bytes > kArenaBudgetLeast) bytes = plan_bins(run_sc, counts, hm, arena_budget(), plan, &smem, scale, true);
   plan.n_pairs = st.n;
   for (int b = 0; b < nb; b++) {
     plan.begin[b] = hb[b];
@@ -643,16 +688,15 @@ static int run_batched(OverlayState &st, const int64_t *d_idx, int64_t count, in
   if (!rc && warps > 0) {
     PRT_PROF("clip_batched", s);
     if (plan.thread_only)
-      clip_lpt_thread_kernel<<<(unsigned)warps, 32, 0, s>>>(st.S, st.O, order, plan, tickets, arena, scale);
+      clip_lpt_thread_kernel<<<(unsigned)warps, 32, 0, s>>>(st.S, st.O, order, plan, d->tickets, arena, scale);
     else
-      clip_lpt_kernel<<<(unsigned)warps, 32, smem, s>>>(st.S, st.O, order, plan, tickets, arena, scale, nullptr);
+      clip_lpt_kernel<<<(unsigned)warps, 32, smem, s>>>(st.S, st.O, order, plan, d->tickets, arena, scale, nullptr);
   }
   if (!rc) {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) rc = cuda_status(e, "clip_batched_kernel");
   }
   dfree(arena, s);
-  dfree(nv, s);
   dfree(scr, s);
   return rc;
 }
@@ -875,51 +919,35 @@ int overlay_impl(const PairSrc &S, int64_t n, int sched, double *d_area, cudaStr
   memset(&st.O, 0, sizeof st.O);
   st.O.area = d_area;
   int rc = dalloc(&st.O.status, std::max<int64_t>(n, 1), s);
-  if (!rc) rc = dalloc(&st.O.pool, 2, s);
+  if (!rc) rc = dalloc(&st.words, 8, s);
+  st.O.pool = st.words;
   if (!rc && !d_area) rc = dalloc(&st.O.pair_cstart, std::max<int64_t>(n, 1), s);
   if (!rc && !d_area) rc = dalloc(&st.O.pair_ncont, std::max<int64_t>(n, 1), s);
-  int64_t total_nv = 0;
-  if (!rc && !d_area && n > 0) {
-    int64_t *nv = nullptr, *tmp = nullptr;
-    rc = dalloc(&nv, n, s);
-    if (!rc) rc = dalloc(&tmp, n + 1, s);
-    if (!rc) {
-      {
-        PRT_PROF("nv", s);
-        nv_kernel<<<grid_for(n, 256, 16), 256, 0, s>>>(S, n, nullptr, 1, nv, nullptr);
-      }
-      rc = exclusive_scan<int64_t>(nv, n, tmp, tmp + n, s);
-    }
-    if (!rc) {
-      cudaError_t e = cudaMemcpyAsync(&total_nv, tmp + n, 8, cudaMemcpyDeviceToHost, s);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-      if (e != cudaSuccess) rc = cuda_status(e, "overlay sizes");
-    }
-    dfree(nv, s);
-    dfree(tmp, s);
-  }
-  if (!rc && !d_area) {
-    // first guess at the result size (grown on demand): half of the input
-    // vertices, one contour per 64 of them
-    st.O.cap_c = total_nv / 64 + 1024;
-    st.O.cap_v = total_nv / 2 + 4096;
-    rc = dalloc(&st.O.cont_vstart, st.O.cap_c, s);
-    if (!rc) rc = dalloc(&st.O.cont_nverts, st.O.cap_c, s);
-    if (!rc) rc = dalloc(&st.O.cont_hole, st.O.cap_c, s);
-    if (!rc) rc = dalloc(&st.O.xy, 2 * st.O.cap_v, s);
-  }
   if (!rc) {
-    cudaError_t e = cudaMemsetAsync(st.O.pool, 0, 16, s);
+    cudaError_t e = cudaMemsetAsync(st.words, 0, 64, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(st.O.status, 0, 4 * std::max<int64_t>(n, 1), s);
     if (e != cudaSuccess) rc = cuda_status(e, "memset");
   }
+  if (!rc && n == 0) rc = first_pools(st, 0, s);
   if (!rc && n > 0) rc = sched == PRT_SCHED_PLAIN ? run_plain(st, nullptr, n, 1, s) : run_batched(st, nullptr, n, 1, s);
-  if (!rc && n > 0) rc = retry_failed(st, s);
-  if (rc || d_area) {
-    if (!rc) {
-      cudaError_t e = cudaStreamSynchronize(s);
-      if (e != cudaSuccess) rc = cuda_status(e, "overlay");
+  // totals of the live results (pools may hold abandoned reservations) and
+  // the pairs to retry, read back together
+  unsigned long long tot[4] = {0, 0, 0, 0};
+  for (int pass = 0; pass < 2 && !rc && n > 0; pass++) {
+    cudaError_t e = pass ? cudaMemsetAsync(st.words + 2, 0, sizeof tot, s) : cudaSuccess;
+    if (e == cudaSuccess) {
+      PRT_PROF("result_totals", s);
+      result_totals_kernel<<<grid_for(n, 256, 8), 256, 0, s>>>(st.O.status, st.O.pair_cstart, st.O.pair_ncont,
+                                                               st.O.cont_nverts, n, st.words + 2);
+      e = cudaGetLastError();
     }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(tot, st.words + 2, sizeof tot, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) rc = cuda_status(e, "overlay results");
+    if (rc || tot[3] == 0) break;
+    rc = retry_failed(st, s);
+  }
+  if (rc || d_area) {
     free_state(st, s);
     return rc;
   }
@@ -934,28 +962,9 @@ int overlay_impl(const PairSrc &S, int64_t n, int sched, double *d_area, cudaStr
   r->cont_hole = st.O.cont_hole;
   r->xy = st.O.xy;
   r->pool = st.O.pool;
-  // exact totals of the live results (pools may hold abandoned reservations)
-  {
-    unsigned long long *tot = nullptr;
-    int rc2 = dalloc(&tot, 3, s);
-    unsigned long long h[3] = {0, 0, 0};
-    cudaError_t e = rc2 ? cudaErrorMemoryAllocation : cudaMemsetAsync(tot, 0, 24, s);
-    if (e == cudaSuccess && n > 0) {
-      PRT_PROF("result_totals", s);
-      result_totals_kernel<<<grid_for(n, 256, 8), 256, 0, s>>>(r->pair_cstart, r->pair_ncont, r->cont_nverts, n, tot);
-      e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h, tot, sizeof h, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    dfree(tot, s);
-    if (e != cudaSuccess) {
-      prt_results_free(r);
-      return cuda_status(e, "overlay results");
-    }
-    r->n_cont = (int64_t)h[0];
-    r->n_vert = (int64_t)h[1];
-    r->nonempty = (int64_t)h[2];
-  }
+  r->n_cont = (int64_t)tot[0];
+  r->n_vert = (int64_t)tot[1];
+  r->nonempty = (int64_t)tot[2];
   *out = r;
   return PRT_OK;
 }
@@ -1107,8 +1116,33 @@ int prt_results_copy(const prt_results *r, int64_t *h_pair_cont_off, int32_t *h_
                      double *h_xy) {
   PRT_CHECK(r && h_pair_cont_off && h_cont_nverts && h_cont_hole && h_xy, PRT_ERR_INVALID, "NULL argument");
   const int64_t n = r->n_pairs;
-  unsigned long long used[2];
   PRT_CUDA(cudaDeviceSynchronize());
+  // put into pair order on the device, so that each array leaves it in one
+  // copy straight into the caller's memory
+  {
+    void *block = nullptr;
+    int64_t *off = nullptr;
+    int32_t *nv = nullptr, *hole = nullptr;
+    double *xy = nullptr;
+    int rc = results_compact(r, nullptr, &block, &off, &nv, &hole, &xy);
+    if (!rc) {
+      cudaError_t e = cudaMemcpyAsync(h_pair_cont_off, off, 8 * (size_t)(n + 1), cudaMemcpyDeviceToHost, nullptr);
+      if (e == cudaSuccess && r->n_cont > 0) {
+        e = cudaMemcpyAsync(h_cont_nverts, nv, 4 * (size_t)r->n_cont, cudaMemcpyDeviceToHost, nullptr);
+        if (e == cudaSuccess)
+          e = cudaMemcpyAsync(h_cont_hole, hole, 4 * (size_t)r->n_cont, cudaMemcpyDeviceToHost, nullptr);
+        if (e == cudaSuccess)
+          e = cudaMemcpyAsync(h_xy, xy, 16 * (size_t)r->n_vert, cudaMemcpyDeviceToHost, nullptr);
+      }
+      if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+      dfree(block, nullptr);
+      return e == cudaSuccess ? PRT_OK : cuda_status(e, "results copy");
+    }
+    if (rc != PRT_ERR_NOMEM) return rc;
+  }
+  // no room on the device for a second copy of the results: the pools as
+  // they are, put into pair order on the host
+  unsigned long long used[2];
   PRT_CUDA(cudaMemcpy(used, r->pool, sizeof used, cudaMemcpyDeviceToHost));
   std::vector<int64_t> cs(n), cvs(used[0]);
   std::vector<int32_t> nc(n), cnv(used[0]), ch(used[0]);

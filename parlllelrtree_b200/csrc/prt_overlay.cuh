@@ -134,3 +134,13 @@ struct prt_results {
   double *xy;
   unsigned long long *pool;
 };
+
+namespace prt {
+
+// Compacts a result set into pair order in device buffers allocated on s:
+// pair_off [n+1], nverts / hole [n_cont], xy [2 n_vert] (all in one block
+// returned in *block, to be released with dfree).
+int results_compact(const prt_results *r, cudaStream_t s, void **block, int64_t **pair_off, int32_t **nverts,
+                    int32_t **hole, double **xy);
+
+}  // namespace prt

@@ -67,9 +67,6 @@ __global__ void compact_vertices_kernel(const int64_t *__restrict__ src, const i
 
 }  // namespace
 
-// Compacts a result set into pair order in device buffers allocated on s:
-// pair_off [n+1], nverts / hole [n_cont], xy [2 n_vert] (all in one block
-// returned in *block, to be released with dfree).
 int results_compact(const prt_results *r, cudaStream_t s, void **block, int64_t **pair_off, int32_t **nverts,
                     int32_t **hole, double **xy) {
   const int64_t n = r->n_pairs, nc = r->n_cont, nv = r->n_vert;
