@@ -172,6 +172,16 @@ int prt_join_noalloc(const prt_tree *t, const void *d_queries, int coord_type, i
 int prt_join_sorted(const prt_tree *t, const void *d_queries, int coord_type, int64_t nq,
                     prt_pair *d_pairs, int64_t cap, int64_t *h_count, void *stream);
 
+/* The same join for a caller that sizes the pair buffer by the result:
+ * prt_join_begin runs the traversal and gives the pair count, prt_join_finish
+ * writes that many pairs, sorted by (queryid, nodeid), on the stream given to
+ * prt_join_begin and releases the state (d_pairs NULL: releases it only).
+ * prt_join_begin waits for the stream once; prt_join_finish does not wait. */
+typedef struct prt_join_state prt_join_state;
+int prt_join_begin(const prt_tree *t, const void *d_queries, int coord_type, int64_t nq,
+                   prt_join_state **out, int64_t *h_count, void *stream);
+int prt_join_finish(prt_join_state *state, prt_pair *d_pairs);
+
 /* Per-query counters of the reference's DFS search, d_counts nq x 3 int64:
  * entries examined (node fill, or fanout per node when td_slots != 0 as the
  * top-down program counts), sum over visited nodes of max(0, overlapping

@@ -129,11 +129,18 @@ class Tree:
     def join(self, queries, cap: int | None = None, sorted: bool = False) -> torch.Tensor:
         """All intersecting (leaf entry, query) pairs, int32 [P, 2] on the device."""
         q = self._queries(queries)
-        fn = lib().prt_join_sorted if sorted else lib().prt_join
         count = C.c_int64(0)
         if cap is None:
-            check(lib().prt_join(self._h, _ptr(q), self.coord, len(q), None, 0, C.byref(count), _stream()))
-            cap = max(int(count.value), 1)
+            state = C.c_void_p()
+            check(lib().prt_join_begin(self._h, _ptr(q), self.coord, len(q), C.byref(state), C.byref(count), _stream()))
+            try:
+                out = torch.empty((int(count.value), 2), dtype=torch.int32, device="cuda")
+            except BaseException:
+                lib().prt_join_finish(state, None)
+                raise
+            check(lib().prt_join_finish(state, _ptr(out) if len(out) else None))
+            return out
+        fn = lib().prt_join_sorted if sorted else lib().prt_join
         out = torch.empty((cap, 2), dtype=torch.int32, device="cuda")
         rc = fn(self._h, _ptr(q), self.coord, len(q), _ptr(out), cap, C.byref(count), _stream())
         if rc == _lib.PRT_ERR_CAPACITY:

@@ -179,7 +179,9 @@ __global__ void extent_f64_kernel(const Box<T> *__restrict__ b, int64_t n, unsig
   }
 }
 
-__global__ void extent_init_kernel(unsigned long long *ext) {
+// also clears the tree's flags, which the leaf packing sets
+__global__ void extent_init_kernel(unsigned long long *ext, unsigned *flags) {
+  *flags = 0u;
   ext[0] = ord_f64(__longlong_as_double(0x7FF0000000000000ll));
   ext[1] = ext[0];
   ext[2] = ord_f64(-__longlong_as_double(0x7FF0000000000000ll));
@@ -210,7 +212,8 @@ __global__ void extent_i64_kernel(const Box<int64_t> *__restrict__ b, int64_t n,
   }
 }
 
-__global__ void extent_i64_init_kernel(long long *ext) {
+__global__ void extent_i64_init_kernel(long long *ext, unsigned *flags) {
+  *flags = 0u;
   ext[0] = 100000000000000000ll;
   ext[1] = 100000000000000000ll;
   ext[2] = 0;
@@ -716,11 +719,12 @@ template <typename T, int F>
 __global__ void __launch_bounds__(256) pack_leaf_kernel(const Box<T> *__restrict__ b, const int32_t *__restrict__ ids,
                                  const uint32_t *__restrict__ perm_a, const uint32_t *__restrict__ perm_b,
                                  const int *__restrict__ sel, int64_t n, int64_t padded, Box<T> *__restrict__ lv0,
-                                 int32_t *__restrict__ leaf_id, Box<T> *__restrict__ lv1) {
+                                 int32_t *__restrict__ leaf_id, Box<T> *__restrict__ lv1, unsigned *flags) {
   const uint32_t *perm = (sel && *sel) ? perm_b : perm_a;
   const int lane = threadIdx.x & 31;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   constexpr int64_t kChunk = 32 * kLeafUnroll;
+  bool improper = false;
   for (int64_t c = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; c * kChunk < padded; c += nwarps) {
     uint32_t r[kLeafUnroll];
 #pragma unroll
@@ -734,6 +738,7 @@ __global__ void __launch_bounds__(256) pack_leaf_kernel(const Box<T> *__restrict
     for (int k = 0; k < kLeafUnroll; k++) {
       const int64_t j = c * kChunk + 32 * k + lane;
       x[k] = j < n ? load_box(b, r[k]) : empty_box<T>();
+      improper |= j < n && !(x[k].x1 <= x[k].x2 && x[k].y1 <= x[k].y2);
     }
 #pragma unroll
     for (int k = 0; k < kLeafUnroll; k++) {
@@ -754,6 +759,7 @@ __global__ void __launch_bounds__(256) pack_leaf_kernel(const Box<T> *__restrict
       }
     }
   }
+  if (__any_sync(0xffffffffu, improper) && lane == 0) atomicOr(flags, kTreeImproper);
 }
 
 // Upper level: entry j of level l+1 = union of node j of level l.
@@ -800,7 +806,7 @@ int pack_tree(prt_tree *t, const void *d_boxes, const int32_t *d_ids, const uint
   case F: {                                                                                              \
     PRT_PROF("pack_leaf", s);                                                                            \
     pack_leaf_kernel<T, F><<<g, block, 0, s>>>(b, d_ids, perm_a, perm_b, d_sel, t->n, L.padded[0], mbr, \
-                                               t->d_leaf_id, lv1 ? lv1 : mbr);                           \
+                                               t->d_leaf_id, lv1 ? lv1 : mbr, t->d_flags);              \
     fused = lv1 != nullptr;                                                                              \
     break;                                                                                               \
   }
@@ -814,7 +820,7 @@ int pack_tree(prt_tree *t, const void *d_boxes, const int32_t *d_ids, const uint
       {
         PRT_PROF("pack_leaf", s);
         pack_leaf_kernel<T, 0><<<g, block, 0, s>>>(b, d_ids, perm_a, perm_b, d_sel, t->n, L.padded[0], mbr,
-                                                 t->d_leaf_id, nullptr);
+                                                 t->d_leaf_id, nullptr, t->d_flags);
       }
   }
   for (int l = 1; l < L.levels; l++) {
@@ -856,13 +862,14 @@ int new_tree(const void *d_boxes, int coord, int64_t n, int fanout, int kind, in
   cudaGetDevice(&t->device);
   size_t bs = 4 * coord_size(coord);
   int rc = dmalloc(&t->d_mbr, bs * t->lv.total, s);
-  if (!rc) rc = dalloc(&t->d_leaf_id, t->lv.padded[0], s);
+  if (!rc) rc = dalloc(&t->d_leaf_id, t->lv.padded[0] + 1, s);
   if (rc) {
     dfree(t->d_mbr, s);
     dfree(t->d_leaf_id, s);
     delete t;
     return rc;
   }
+  t->d_flags = reinterpret_cast<unsigned *>(t->d_leaf_id + t->lv.padded[0]);
   *out = t;
   return PRT_OK;
 }
@@ -913,7 +920,7 @@ int bu_enqueue(prt_tree *t, const void *d_boxes, const int32_t *d_ids, unsigned 
       }
       {
         PRT_PROF("extent_init", s);
-        extent_init_kernel<<<1, 1, 0, s>>>(ext);
+        extent_init_kernel<<<1, 1, 0, s>>>(ext, t->d_flags);
       }
       rc = dispatch_coord(t->coord, [&](auto tag) {
         using T = decltype(tag);
@@ -937,7 +944,7 @@ int bu_enqueue(prt_tree *t, const void *d_boxes, const int32_t *d_ids, unsigned 
       const Box<int64_t> *b = reinterpret_cast<const Box<int64_t> *>(d_boxes);
       {
         PRT_PROF("extent_i64_init", s);
-        extent_i64_init_kernel<<<1, 1, 0, s>>>(ei);
+        extent_i64_init_kernel<<<1, 1, 0, s>>>(ei, t->d_flags);
       }
       {
         PRT_PROF("extent_i64", s);
@@ -1045,6 +1052,7 @@ int prt_build_topdown(const void *d_boxes, int coord_type, const int32_t *d_ids,
   const void *cxy = d_boxes;
   int cstride = 4;
   cudaError_t e = cudaMemsetAsync(err, 0, 8, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(t->d_flags, 0, sizeof(unsigned), s);
   if (e != cudaSuccess) rc = cuda_status(e, "memset");
   const int g = grid_for(n, 256, 16);
   // the current order: pa or pb as *psel says (psel nullptr: pa; pa nullptr:

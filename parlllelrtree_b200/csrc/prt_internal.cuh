@@ -215,6 +215,10 @@ template <typename InT>
 int exclusive_scan(const InT *d_in, int64_t n, int64_t *d_out, int64_t *d_total, cudaStream_t s);
 
 // ---- tree ----------------------------------------------------------------------
+// prt_tree::d_flags: some record's box is not proper (x1 <= x2 and y1 <= y2,
+// no NaN), so a box may hold records that intersect nothing.
+enum : unsigned { kTreeImproper = 1u };
+
 struct TreeLevels {
   int levels;                        // L: level 0 = records
   int64_t count[PRT_MAX_LEVELS];     // entries per level
@@ -254,5 +258,6 @@ struct prt_tree {
   prt::TreeLevels lv;
   void *d_mbr;          // Box<T>[lv.total], level after level
   int32_t *d_leaf_id;   // record id per leaf entry
+  unsigned *d_flags;    // kTreeImproper (in d_leaf_id's block)
   int device;
 };

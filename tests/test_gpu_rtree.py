@@ -193,3 +193,38 @@ def test_large_build_parity(cuda):
     perm = oracle.td_order(b, 32)
     t = prt.build_topdown(torch.from_numpy(b).cuda(), fanout=32)
     assert np.array_equal(t.leaf_order().cpu().numpy(), perm)
+
+
+@pytest.mark.parametrize("kind", ["f32", "f64", "i64", "i32"])
+@pytest.mark.parametrize("F", [2, 3, 10, 16, 32])
+@pytest.mark.parametrize("n", [1, 33, 4097, 30011])
+def test_windows_that_contain_nodes(cuda, kind, F, n):
+    """Windows from a point to more than the whole extent, so that nodes of
+    every level lie inside some: pairs (one call, and into a given capacity)
+    and counters against the oracle; then with records that intersect nothing
+    (an empty polygon's box) inside their parents' boxes."""
+    import parlllelrtree_b200 as prt
+
+    rng = np.random.default_rng(n + F)
+    scale = 1.0 if kind in ("f32", "f64") else 1e4
+    dt = {"f32": np.float32, "f64": np.float64, "i64": np.int64, "i32": np.int32}[kind]
+    c, h = rng.random((n, 2)), rng.random((n, 2)) * 0.01
+    b = (np.concatenate([c - h, c + h], 1) * scale).astype(dt)
+    m = 300
+    c, h = rng.random((m, 2)), rng.random((m, 1)) ** 3 * 1.2
+    q = (np.concatenate([c - h, c + h], 1) * scale).astype(dt)
+    for improper in (False, True):
+        if improper:
+            big = np.finfo(dt).max if dt in (np.float32, np.float64) else np.iinfo(dt).max
+            b[:: max(1, n // 5)] = np.array([big, big, -big, -big], dt)
+        t = prt.build_topdown(torch.from_numpy(b).cuda(), fanout=F)
+        lv = t.levels_mbr()
+        qd = torch.from_numpy(q).cuda()
+        ref = oracle.join_pairs(lv, F, q)
+        ref = ref[np.lexsort((ref[:, 0], ref[:, 1]))]
+        for got in (t.join(qd), t.join(qd, sorted=True), t.join(qd, cap=len(ref) + 7, sorted=True)):
+            assert np.array_equal(got.cpu().numpy().astype(np.int64).reshape(-1, 2), ref.reshape(-1, 2))
+        un = t.join(qd, cap=len(ref) + 7).cpu().numpy().astype(np.int64).reshape(-1, 2)
+        assert np.array_equal(un[np.lexsort((un[:, 0], un[:, 1]))], ref.reshape(-1, 2))
+        for td in (False, True):
+            assert np.array_equal(t.query_counts(qd, td_slots=td).cpu().numpy(), oracle.query_counts(lv, F, q, td_slots=td))
