@@ -312,17 +312,31 @@ __device__ __forceinline__ uint64_t ukey(double v) {
 }
 __device__ __forceinline__ uint64_t ukey(int64_t v) { return (uint64_t)v ^ 0x8000000000000000ull; }
 
-// Top-down level key for 32-bit coordinates: (pos / seg) << 32 | coordinate.
+// Smallest and largest order-preserving image of the boxes' x1 and y1:
+// ext = {min x1, min y1, ~max x1, ~max y1}, set to ~0 before.
 template <typename T>
-__global__ void td_key32_kernel(const Box<T> *__restrict__ b, const uint32_t *__restrict__ perm, int64_t n,
-                                int64_t seg, int use_y, uint64_t *__restrict__ keys, uint32_t *__restrict__ vals) {
+__global__ void __launch_bounds__(256) td_range_kernel(const Box<T> *__restrict__ b, int64_t n,
+                                                       unsigned long long *ext) {
+  unsigned long long m[4] = {~0ull, ~0ull, ~0ull, ~0ull};
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    uint32_t r = perm ? perm[i] : (uint32_t)i;
-    if ((int64_t)r >= n) r = 0;  // only after a timed-out sort (reported by the caller)
-    Box<T> x = load_box(b, r);
-    uint32_t c = ukey(use_y ? x.y1 : x.x1);
-    keys[i] = ((uint64_t)(i / seg) << 32) | c;
-    vals[i] = r;
+    const Box<T> x = load_box(b, i);
+    const unsigned long long kx = ukey(x.x1), ky = ukey(x.y1);
+    m[0] = min(m[0], kx);
+    m[1] = min(m[1], ky);
+    m[2] = min(m[2], ~kx);
+    m[3] = min(m[3], ~ky);
+  }
+  __shared__ unsigned long long red[4][8];
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    for (int o = 16; o; o >>= 1) m[k] = min(m[k], __shfl_xor_sync(0xffffffffu, m[k], o));
+    if ((threadIdx.x & 31) == 0) red[k][threadIdx.x >> 5] = m[k];
+  }
+  __syncthreads();
+  if (threadIdx.x < 4) {
+    unsigned long long v = red[threadIdx.x][0];
+    for (int w = 1; w < 8; w++) v = min(v, red[threadIdx.x][w]);
+    atomicMin(&ext[threadIdx.x], v);
   }
 }
 
@@ -332,101 +346,76 @@ __device__ __forceinline__ const uint32_t *cur_perm(const uint32_t *perm_a, cons
   return perm_a ? ((sel && *sel) ? perm_b : perm_a) : nullptr;
 }
 
-// Top-down level whose runs are sorted one by one (radix_sort_runs) or that
-// is one run: the key is the coordinate's order-preserving image alone.  One
-// block per 4096 positions (inside one run, since runs are whole tiles)
-// counts the digit histograms of every pass on the way, into its run's
-// histograms hist[(run * passes + p) * 256 + digit], so the sort does not
-// read the keys again to count them.  The order is read and the values
-// written at the same positions by the same thread: vals may be the buffer
-// the order is read from.  Record r's (x1, y1) is at c[stride * r] (the boxes,
-// stride 4, or the compact copy, stride 2); with the identity order the
-// kernel can write that compact copy (xy_out), so later levels gather from
-// an array a quarter (float) of the boxes' size, which stays in L2.
-template <typename T, typename K>
+// Top-down level: every run is sorted on its own (radix_sort_runs), so the key
+// is the coordinate's order-preserving image alone, less the smallest one of
+// the boxes.  One block per kKeyTile positions of one run counts the digit
+// histograms of every pass on the way, into its run's histograms
+// hist[(run * sizeof(K) + p) * 256 + digit], so the sort does not read the keys
+// again to count them.  The order is read and the values written at the same
+// positions by the same thread: vals may be the buffer the order is read from.
+// Record r's (x1, y1) is at c[stride * r] (the boxes, stride 4, or the compact
+// copy, stride 2); with the identity order the kernel can write that compact
+// copy (xy_out), so later levels gather from an array a quarter (float) of the
+// boxes' size, which stays in L2.
+constexpr int64_t kKeyTile = 4096;
+
+template <typename T, typename K, bool kAllPasses>
 __global__ void __launch_bounds__(256) td_keyrun_kernel(const T *__restrict__ cxy, int stride, const uint32_t *perm_a,
                                                         const uint32_t *perm_b, const int *sel, int64_t n, int use_y,
-                                                        int64_t tiles_per_run, K *__restrict__ keys, uint32_t *vals,
+                                                        int64_t run_len, int tiles_per_run, K low, int some_passes,
+                                                        K *__restrict__ keys, uint32_t *vals,
                                                         uint32_t *__restrict__ hist, T *__restrict__ xy_out) {
   constexpr int kPasses = (int)sizeof(K);
-  constexpr int kPer = (int)(kSortRunTile / 256);
+  constexpr int kPer = (int)(kKeyTile / 256);
+  const int passes = kAllPasses ? kPasses : some_passes;
   __shared__ uint32_t sh[kPasses * 256];
-  for (int i = threadIdx.x; i < kPasses * 256; i += 256) sh[i] = 0;
+  for (int i = threadIdx.x; i < passes * 256; i += 256) sh[i] = 0;
   __syncthreads();
   const uint32_t *perm = cur_perm(perm_a, perm_b, sel);
   const T *c = cxy + (use_y ? 1 : 0);
-  const int64_t base = (int64_t)blockIdx.x * kSortRunTile + threadIdx.x;
+  const int run = (int)blockIdx.x / tiles_per_run;
+  const int64_t base = run * run_len + (int64_t)((int)blockIdx.x - run * tiles_per_run) * kKeyTile;
+  const int cnt = (int)min(kKeyTile, min(n, (run + 1) * run_len) - base);  // positions of this block
+  if (perm) perm += base;
+  keys += base;
+  vals += base;
   // all loads of the order first, then all coordinate loads, then the stores
   uint32_t r[kPer];
 #pragma unroll
   for (int j = 0; j < kPer; j++) {
-    const int64_t i = base + 256 * j;
-    r[j] = i < n ? (perm ? perm[i] : (uint32_t)i) : 0u;
+    const int i = (int)threadIdx.x + 256 * j;
+    r[j] = i < cnt ? (perm ? perm[i] : (uint32_t)base + (uint32_t)i) : 0u;
     if ((int64_t)r[j] >= n) r[j] = 0;  // only after a timed-out sort (reported by the caller)
   }
   K k[kPer];
 #pragma unroll
-  for (int j = 0; j < kPer; j++) k[j] = base + 256 * j < n ? (K)ukey(__ldg(&c[stride * (int64_t)r[j]])) : K(0);
-  if (xy_out) {  // identity order: record i's (x1, y1), read in order
+  for (int j = 0; j < kPer; j++)
+    k[j] = (int)threadIdx.x + 256 * j < cnt ? (K)ukey(__ldg(&c[stride * (int64_t)r[j]])) - low : K(0);
+  if (xy_out) {  // identity order: record base + i's (x1, y1), read in order
 #pragma unroll
     for (int j = 0; j < kPer; j++) {
-      const int64_t i = base + 256 * j;
-      if (i < n) {
-        xy_out[2 * i] = cxy[stride * i];
-        xy_out[2 * i + 1] = cxy[stride * i + 1];
+      const int i = (int)threadIdx.x + 256 * j;
+      if (i < cnt) {
+        xy_out[2 * (base + i)] = cxy[stride * (base + i)];
+        xy_out[2 * (base + i) + 1] = cxy[stride * (base + i) + 1];
       }
     }
   }
 #pragma unroll
   for (int j = 0; j < kPer; j++) {
-    const int64_t i = base + 256 * j;
-    if (i < n) {
+    const int i = (int)threadIdx.x + 256 * j;
+    if (i < cnt) {
       keys[i] = k[j];
       vals[i] = r[j];
 #pragma unroll
-      for (int p = 0; p < kPasses; p++) atomicAdd(&sh[p * 256 + (int)((k[j] >> (8 * p)) & 0xFF)], 1u);
+      for (int p = 0; p < kPasses; p++)
+        if (p < passes) atomicAdd(&sh[p * 256 + (int)((k[j] >> (8 * p)) & 0xFF)], 1u);
     }
   }
   __syncthreads();
-  uint32_t *h = hist + (int64_t)(blockIdx.x / tiles_per_run) * kPasses * 256;
-  for (int i = threadIdx.x; i < kPasses * 256; i += 256)
+  uint32_t *h = hist + (int64_t)run * kPasses * 256;
+  for (int i = threadIdx.x; i < passes * 256; i += 256)
     if (sh[i]) atomicAdd(&h[i], sh[i]);
-}
-
-// Top-down level, 64-bit coordinates, first stage: key = coordinate, value = position.
-template <typename T>
-__global__ void td_key64_kernel(const Box<T> *__restrict__ b, const uint32_t *__restrict__ perm, int64_t n,
-                                int use_y, uint64_t *__restrict__ keys, uint32_t *__restrict__ vals) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    uint32_t r = perm ? perm[i] : (uint32_t)i;
-    if ((int64_t)r >= n) r = 0;  // only after a timed-out sort (reported by the caller)
-    Box<T> x = load_box(b, r);
-    keys[i] = ukey(use_y ? x.y1 : x.x1);
-    vals[i] = (uint32_t)i;
-  }
-}
-
-// second stage: key = segment of the original position
-__global__ void td_segkey_kernel(const uint32_t *__restrict__ pos, int64_t n, int64_t seg,
-                                 uint32_t *__restrict__ keys) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    keys[i] = (uint32_t)(pos[i] / seg);
-}
-
-__global__ void gather_u32_kernel(const uint32_t *__restrict__ src, const uint32_t *__restrict__ idx, int64_t n,
-                                  uint32_t *__restrict__ dst) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    uint32_t k = idx[i];
-    if ((int64_t)k >= n) k = 0;  // only after a timed-out sort (reported by the caller)
-    dst[i] = src ? src[k] : k;
-  }
-}
-
-__global__ void select_copy_u32_kernel(const uint32_t *a, const uint32_t *b, const int *sel, int64_t n,
-                                       uint32_t *dst) {
-  const uint32_t *src = *sel ? b : a;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    dst[i] = src[i];
 }
 
 // ------------------------------------------------------------------ top-down, short runs
@@ -482,6 +471,7 @@ struct TdLocalLevels {
   int64_t seg[kTdMaxLocal];
   int use_y[kTdMaxLocal];
   int count;
+  int64_t chunk;  // records per block: whole runs of the first local level
 };
 
 // The last level's runs (F records) are short: each record's new position in
@@ -507,9 +497,9 @@ __global__ void __launch_bounds__(kTdThreads, kTdThreads == 256 ? (sizeof(T) == 
   extern __shared__ __align__(16) unsigned char smem_raw[];
   TdLocalSmem<T> &S = *reinterpret_cast<TdLocalSmem<T> *>(smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t chunk = (kTdLocal / lv.seg[0]) * lv.seg[0];  // whole runs of the first local level
-  const int64_t base = blockIdx.x * chunk;
-  const int m = (int)min(chunk, n - base);
+  const int64_t base = blockIdx.x * lv.chunk;
+  const int m = (int)min(lv.chunk, n - base);
+  const int per = (m + kTdThreads - 1) / kTdThreads;  // items per thread
   const uint32_t *perm_in = cur_perm(perm_a, perm_b, sel);
   for (int i = tid; i < m; i += kTdThreads) {
     uint32_t r = perm_in ? perm_in[base + i] : (uint32_t)(base + i);
@@ -597,7 +587,8 @@ __global__ void __launch_bounds__(kTdThreads, kTdThreads == 256 ? (sizeof(T) == 
       uint32_t *wh = S.wh[warp];
 #pragma unroll
       for (int j = 0; j < kTdItems; j++) {
-        const int i = warp * (32 * kTdItems) + j * 32 + lane;
+        if (j >= per) break;
+        const int i = warp * (32 * per) + j * 32 + lane;
         const bool ok = i < m;
         int d = 256 + lane;
         it[j] = 0;
@@ -664,8 +655,8 @@ __global__ void __launch_bounds__(kTdThreads, kTdThreads == 256 ? (sizeof(T) == 
       __syncthreads();
 #pragma unroll
       for (int j = 0; j < kTdItems; j++) {
-        const int i = warp * (32 * kTdItems) + j * 32 + lane;
-        if (i < m) S.item[1 - cur][S.dstart[dg[j]] + S.wh[warp][dg[j]] + rk[j]] = it[j];
+        const int i = warp * (32 * per) + j * 32 + lane;
+        if (j < per && i < m) S.item[1 - cur][S.dstart[dg[j]] + S.wh[warp][dg[j]] + rk[j]] = it[j];
       }
       cur = 1 - cur;
     }
@@ -683,8 +674,13 @@ __global__ void __launch_bounds__(kTdThreads, kTdThreads == 256 ? (sizeof(T) == 
 // most kTdLocal, each next one dividing it).
 template <typename T>
 int td_local_levels(const T *cxy, int stride, const uint32_t *perm_a, const uint32_t *perm_b, const int *sel,
-                    int64_t n, const TdLocalLevels &lv, uint32_t *perm_out, cudaStream_t s) {
-  const int64_t chunk = (kTdLocal / lv.seg[0]) * lv.seg[0];
+                    int64_t n, TdLocalLevels lv, uint32_t *perm_out, cudaStream_t s) {
+  // as many whole runs per block as fit, fewer where one wave of blocks
+  // (one per SM with 64-bit coordinates, two with 32-bit) can still take
+  // them all: a block's time goes by its records per thread
+  const int64_t runs = (n + lv.seg[0] - 1) / lv.seg[0], wave = kSMs * (sizeof(T) == 4 ? 2 : 1);
+  lv.chunk = std::min<int64_t>(kTdLocal / lv.seg[0], (runs + wave - 1) / wave) * lv.seg[0];
+  const int64_t chunk = lv.chunk;
   const size_t smem = sizeof(TdLocalSmem<T>);
   static bool attr_done[256] = {false};
   int dev = 0;
@@ -1025,13 +1021,13 @@ int prt_build_topdown(const void *d_boxes, int coord_type, const int32_t *d_ids,
   int rc = new_tree(d_boxes, coord_type, n, fanout, PRT_TOP_DOWN, -1, s, &t);
   if (rc) return rc;
   const int H = t->lv.levels;
-  const bool wide = coord_size(coord_type) == 8;
   unsigned char *scr = nullptr;
-  // per-run digit histograms: at most one run per sort tile, 8 passes
-  const size_t hist_words = (size_t)((n + kSortRunTile - 1) / kSortRunTile) * 8 * 256;
-  // and the compact (x1, y1) copy the first level writes
   const size_t csize = (size_t)coord_size(coord_type);
-  size_t need = 64 + 2 * 8 * n + 4 * 4 * n + 4 * hist_words + 2 * csize * n + 64;
+  // per-run digit histograms of a level: its runs are longer than kTdLocal
+  const size_t hist_words = (size_t)(n / kTdLocal + 1) * csize * 256;
+  // keys, values and the compact (x1, y1) copy the first level writes, then
+  // two order buffers of the short levels
+  size_t need = 64 + 2 * csize * n + 4 * 4 * n + 4 * hist_words + 2 * csize * n + 64;
   rc = dmalloc(reinterpret_cast<void **>(&scr), need, s);
   if (rc) {
     prt_tree_free(t);
@@ -1039,14 +1035,13 @@ int prt_build_topdown(const void *d_boxes, int coord_type, const int32_t *d_ids,
   }
   unsigned *err = reinterpret_cast<unsigned *>(scr);
   int *sel = reinterpret_cast<int *>(scr + 8);
-  uint64_t *k0 = reinterpret_cast<uint64_t *>(scr + 64);
-  uint64_t *k1 = k0 + n;
-  uint32_t *v0 = reinterpret_cast<uint32_t *>(k1 + n);
+  unsigned long long *ext = reinterpret_cast<unsigned long long *>(scr + 16);
+  unsigned char *k0 = scr + 64, *k1 = k0 + csize * n;
+  void *xyc = k1 + csize * n;
+  uint32_t *v0 = reinterpret_cast<uint32_t *>(static_cast<unsigned char *>(xyc) + 2 * csize * n);
   uint32_t *v1 = v0 + n;
-  uint32_t *perm = v1 + n;  // current leaf order (when materialised)
-  uint32_t *tmp = perm + n;  // scratch
-  uint32_t *hist = tmp + n;
-  void *xyc = hist + hist_words;
+  uint32_t *order[2] = {v1 + n, v1 + 2 * n};
+  uint32_t *hist = order[1] + n;
   // where the levels read record r's (x1, y1): d_boxes[4 r], or the compact
   // copy at xyc[2 r] once a level has written it
   const void *cxy = d_boxes;
@@ -1054,23 +1049,43 @@ int prt_build_topdown(const void *d_boxes, int coord_type, const int32_t *d_ids,
   cudaError_t e = cudaMemsetAsync(err, 0, 8, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(t->d_flags, 0, sizeof(unsigned), s);
   if (e != cudaSuccess) rc = cuda_status(e, "memset");
-  const int g = grid_for(n, 256, 16);
+  // Integer coordinates of a map use few of their bits: with the smallest x1
+  // and y1 taken off, the keys need only the passes of the range (three of
+  // eight for 20-bit int64 coordinates), which the host has to know to launch
+  // no others: one short pass over the boxes and one wait.  Floating-point
+  // images spread over all their bits.
+  unsigned long long low[2] = {0, 0};
+  int bits[2] = {8 * (int)csize, 8 * (int)csize};
+  if (!rc && n > kTdLocal && (coord_type == PRT_COORD_I64 || coord_type == PRT_COORD_I32)) {
+    unsigned long long h[4];
+    e = cudaMemsetAsync(ext, 0xFF, 32, s);
+    if (e == cudaSuccess) {
+      rc = dispatch_coord(coord_type, [&](auto tag) {
+        using T = decltype(tag);
+        PRT_PROF("td_range", s);
+        td_range_kernel<T><<<grid_for(n, 256, 8), 256, 0, s>>>(reinterpret_cast<const Box<T> *>(d_boxes), n, ext);
+        return PRT_OK;
+      });
+      e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h, ext, sizeof h, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) rc = cuda_status(e, "coordinate range");
+    for (int a = 0; a < 2 && !rc; a++) {
+      low[a] = h[a];
+      const unsigned long long span = ~h[2 + a] - h[a];
+      bits[a] = 1;
+      while (bits[a] < 64 && (span >> bits[a]) != 0) bits[a]++;
+    }
+  }
   // the current order: pa or pb as *psel says (psel nullptr: pa; pa nullptr:
   // the identity).  A sort leaves it in (v0, v1, sel) and the next level
-  // reads it there; paths that need one array copy it into perm first.
+  // reads it there.
   const uint32_t *pa = nullptr, *pb = nullptr;
   const int *psel = nullptr;
-  auto materialise = [&]() -> const uint32_t * {
-    if (psel && !rc) {
-      PRT_PROF("select_copy_u32", s);
-      select_copy_u32_kernel<<<g, 256, 0, s>>>(pa, pb, psel, n, perm);
-      pa = pb = perm;
-      psel = nullptr;
-    }
-    return pa;
-  };
+  int flip = 0;
   for (int p = 0; p < H && !rc; p++) {
-    // segment size fanout^(H-p), saturated at n
+    // run length fanout^(H-p), saturated at n
     int64_t seg = 1;
     for (int k = 0; k < H - p; k++) {
       seg *= fanout;
@@ -1079,9 +1094,6 @@ int prt_build_topdown(const void *d_boxes, int coord_type, const int32_t *d_ids,
         break;
       }
     }
-    int64_t nseg = (n + seg - 1) / seg;
-    int seg_bits = 0;
-    while ((1ll << seg_bits) < nseg) seg_bits++;
     const int use_y = p & 1;
     if (seg <= kTdLocal) {
       // this and every later level have short runs: all of them sorted in
@@ -1098,7 +1110,8 @@ int prt_build_topdown(const void *d_boxes, int coord_type, const int32_t *d_ids,
         lv.use_y[lv.count] = q & 1;
         lv.count++;
       }
-      uint32_t *out = (pa == tmp || pb == tmp) ? perm : tmp;
+      uint32_t *out = order[flip];
+      flip ^= 1;
       rc = dispatch_coord(coord_type, [&](auto tag) {
         using T = decltype(tag);
         return td_local_levels<T>(reinterpret_cast<const T *>(cxy), cstride, pa, pb, psel, n, lv, out, s);
@@ -1106,95 +1119,36 @@ int prt_build_topdown(const void *d_boxes, int coord_type, const int32_t *d_ids,
       pa = pb = out;
       psel = nullptr;
       p += lv.count - 1;  // the loop's p++ moves past the last local level
-    } else if (seg % kSortRunTile == 0 || seg == n) {
-      // runs of whole sort tiles (or one run): every run sorted on its own by
-      // the coordinate alone, 4 (32-bit) or 8 (64-bit) passes; the key kernel
+    } else {
+      // every run sorted on its own by the coordinate alone; the key kernel
       // counts the digit histograms
       rc = dispatch_coord(coord_type, [&](auto tag) {
         using T = decltype(tag);
         using K = typename std::conditional<sizeof(T) == 8, uint64_t, uint32_t>::type;
         K *kk0 = reinterpret_cast<K *>(k0), *kk1 = reinterpret_cast<K *>(k1);
-        const int64_t tiles = (n + kSortRunTile - 1) / kSortRunTile;
-        const int64_t tpr = seg == n ? tiles : seg / kSortRunTile;
-        PRT_CUDA(cudaMemsetAsync(hist, 0, sizeof(uint32_t) * (size_t)((tiles + tpr - 1) / tpr) * sizeof(K) * 256, s));
+        const int64_t runs = (n + seg - 1) / seg, tpr = (seg + kKeyTile - 1) / kKeyTile;
+        const int64_t tiles = (runs - 1) * tpr + (n - (runs - 1) * seg + kKeyTile - 1) / kKeyTile;
+        PRT_CUDA(cudaMemsetAsync(hist, 0, sizeof(uint32_t) * (size_t)runs * sizeof(K) * 256, s));
         // the identity order reads the boxes in order: write the compact copy
         T *xy_out = (pa == nullptr && cstride == 4) ? reinterpret_cast<T *>(xyc) : nullptr;
         {
           PRT_PROF("td_key", s);
-          td_keyrun_kernel<T, K><<<(unsigned)tiles, 256, 0, s>>>(reinterpret_cast<const T *>(cxy), cstride, pa, pb,
-                                                                 psel, n, use_y, tpr, kk0, v0, hist, xy_out);
+          const int passes = (bits[use_y] + 7) / 8;
+          auto kernel = passes == (int)sizeof(K) ? td_keyrun_kernel<T, K, true> : td_keyrun_kernel<T, K, false>;
+          kernel<<<(unsigned)tiles, 256, 0, s>>>(reinterpret_cast<const T *>(cxy), cstride, pa, pb, psel, n, use_y, seg,
+                                                 (int)tpr, (K)low[use_y], passes, kk0, v0, hist, xy_out);
         }
         if (xy_out) {
           cxy = xy_out;
           cstride = 2;
         }
         PRT_CUDA(cudaGetLastError());
-        return seg == n ? radix_sort_pairs<K>(kk0, v0, kk1, v1, n, 8 * (int)sizeof(K), sel, err, s, hist)
-                        : radix_sort_runs<K>(kk0, v0, kk1, v1, n, seg, sel, err, s, hist);
+        return runs == 1 ? radix_sort_pairs<K>(kk0, v0, kk1, v1, n, bits[use_y], sel, err, s, hist)
+                         : radix_sort_runs<K>(kk0, v0, kk1, v1, n, seg, bits[use_y], sel, err, s, hist);
       });
       pa = v0;
       pb = v1;
       psel = sel;
-    } else if (!wide) {
-      const uint32_t *cur = materialise();
-      rc = dispatch_coord(coord_type, [&](auto tag) {
-        using T = decltype(tag);
-        if constexpr (sizeof(T) == 4) {
-          {
-            PRT_PROF("td_key32", s);
-            td_key32_kernel<T><<<g, 256, 0, s>>>(reinterpret_cast<const Box<T> *>(d_boxes), cur, n, seg, use_y, k0,
-                                               v0);
-          }
-        }
-        return PRT_OK;
-      });
-      if (!rc) rc = radix_sort_pairs<uint64_t>(k0, v0, k1, v1, n, 32 + seg_bits, sel, err, s);
-      pa = v0;
-      pb = v1;
-      psel = sel;
-    } else {
-      const uint32_t *cur = materialise();
-      rc = dispatch_coord(coord_type, [&](auto tag) {
-        using T = decltype(tag);
-        if constexpr (sizeof(T) == 8) {
-          {
-            PRT_PROF("td_key64", s);
-            td_key64_kernel<T><<<g, 256, 0, s>>>(reinterpret_cast<const Box<T> *>(d_boxes), cur, n, use_y, k0, v0);
-          }
-        }
-        return PRT_OK;
-      });
-      if (!rc) rc = radix_sort_pairs<uint64_t>(k0, v0, k1, v1, n, 64, sel, err, s);
-      if (!rc) {
-        // positions, in coordinate order
-        PRT_PROF("select_copy_u32", s);
-        select_copy_u32_kernel<<<g, 256, 0, s>>>(v0, v1, sel, n, tmp);
-      }
-      if (!rc && seg_bits > 0) {
-        uint32_t *sk0 = reinterpret_cast<uint32_t *>(k0), *sk1 = reinterpret_cast<uint32_t *>(k1);
-        {
-          PRT_PROF("td_segkey", s);
-          td_segkey_kernel<<<g, 256, 0, s>>>(tmp, n, seg, sk0);
-        }
-        rc = radix_sort_pairs<uint32_t>(sk0, tmp, sk1, v1, n, seg_bits, sel, err, s);
-        if (!rc) {
-          PRT_PROF("select_copy_u32", s);
-          select_copy_u32_kernel<<<g, 256, 0, s>>>(tmp, v1, sel, n, v0);
-        }
-        if (!rc) {
-          cudaMemcpyAsync(tmp, v0, 4 * n, cudaMemcpyDeviceToDevice, s);
-        }
-      }
-      // positions -> records (gathered into v0 first: cur may alias perm)
-      if (!rc) {
-        {
-          PRT_PROF("gather_u32", s);
-          gather_u32_kernel<<<g, 256, 0, s>>>(cur, tmp, n, v0);
-        }
-        cudaMemcpyAsync(perm, v0, 4 * n, cudaMemcpyDeviceToDevice, s);
-      }
-      pa = pb = perm;
-      psel = nullptr;
     }
   }
   if (!rc) rc = dispatch_coord(coord_type, [&](auto tag) {

@@ -1,8 +1,8 @@
 // Onesweep LSD radix sort of (key, uint32 value) pairs.
 //
 // One upsweep kernel histograms every 8-bit digit of every key at once; a
-// tiny plan kernel scans the histograms and marks passes whose digit is the
-// same for all keys (they are skipped without a host round trip, so the whole
+// tiny plan kernel scans the histograms and marks passes whose digit differs
+// between keys (the others are skipped without a host round trip, so the whole
 // sort can be captured in a CUDA graph).  Each remaining pass is ONE kernel:
 // a CTA takes the next tile in launch order (atomic ticket), ranks its keys
 // with a warp-level multisplit (lanes with the same digit found by one ballot
@@ -13,7 +13,9 @@
 // original order within a warp, then warp order, then tile order.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 #include "prt_internal.cuh"
 
@@ -23,9 +25,6 @@ namespace {
 constexpr int kRadix = 256;
 constexpr int kSortBlock = 256;
 constexpr int kSortWarps = kSortBlock / 32;
-#ifndef PRT_SORT_ITEMS
-#define PRT_SORT_ITEMS 16  // keys per thread of a tile
-#endif
 #ifndef PRT_SORT_MIN_BLOCKS
 // resident blocks per SM the 32-bit-key pass is compiled for: 4 (64
 // registers, a 56-byte spill) against 3 (80 registers): 0.0872 ->
@@ -33,16 +32,16 @@ constexpr int kSortWarps = kSortBlock / 32;
 // The 64-bit-key pass stays at 3: its 58 KB tile fits no more per SM.
 #define PRT_SORT_MIN_BLOCKS 4
 #endif
-constexpr int kItems = PRT_SORT_ITEMS;
-constexpr int kTile = kSortBlock * kItems;
-static_assert(kTile == kSortRunTile, "the run sort's tile");
+// Keys per thread of a tile, by the number of keys that are sorted.  A pass
+// over few keys takes as long as one tile's chain of rankings and the look-back
+// over the tiles: 16, 8, 4 keys per thread take 7.7, 5.7, 3.6 us for 4k
+// keys, 9.6, 7.7, 7.7 for 150k, 9.8, 9.1, 9.8 for 300k and 11.7, 11.9, 14.0 for
+// 600k (32-bit keys); at 10M, where the pass is bound by instruction issue, 84,
+// 107 and 163 us.
+inline int sort_items(int64_t n) { return n <= 200000 ? 4 : n <= 600000 ? 8 : 16; }
 constexpr uint32_t kFlagAgg = 1u << 30;
 constexpr uint32_t kFlagPrefix = 2u << 30;
 constexpr uint32_t kCountMask = (1u << 30) - 1;
-
-struct PassPlan {
-  int active, src, dst, pad;
-};
 
 __device__ __forceinline__ uint32_t lanemask_lt() {
   uint32_t m;
@@ -79,45 +78,45 @@ __global__ void __launch_bounds__(256) hist_kernel(const KeyT *__restrict__ keys
     if (sh[i]) atomicAdd(&ghist[i], sh[i]);
 }
 
-__global__ void plan_kernel(const uint32_t *__restrict__ ghist, uint32_t *__restrict__ goff, int passes, int64_t n,
-                            PassPlan *__restrict__ plan, int *__restrict__ d_sel) {
-  __shared__ uint32_t scan[kRadix];
-  __shared__ int trivial[PRT_MAX_LEVELS];
-  for (int p = 0; p < passes; p++) {
-    uint32_t c = ghist[p * kRadix + threadIdx.x];
-    scan[threadIdx.x] = c;
-    if (threadIdx.x == 0) trivial[p] = 0;
-    __syncthreads();
-    if ((int64_t)c == n) trivial[p] = 1;
-    // inclusive Hillis-Steele scan over 256 bins
-    for (int o = 1; o < kRadix; o <<= 1) {
-      uint32_t v = threadIdx.x >= o ? scan[threadIdx.x - o] : 0u;
-      __syncthreads();
-      scan[threadIdx.x] += v;
-      __syncthreads();
-    }
-    goff[p * kRadix + threadIdx.x] = scan[threadIdx.x] - c;
-    __syncthreads();
+// Exclusive scan of one value per thread over a block of kRadix threads.
+__device__ __forceinline__ uint32_t scan_digits(uint32_t v, uint32_t *s_warp) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t incl = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
   }
-  if (threadIdx.x == 0) {
-    int cur = 0;
-    for (int p = 0; p < passes; p++) {
-      PassPlan pp;
-      pp.active = !trivial[p];
-      pp.src = cur;
-      pp.dst = 1 - cur;
-      pp.pad = 0;
-      if (pp.active) cur = 1 - cur;
-      plan[p] = pp;
-    }
-    *d_sel = cur;
-  }
+  if (lane == 31) s_warp[warp] = incl;
+  __syncthreads();
+  uint32_t off = 0;
+#pragma unroll
+  for (int w = 0; w < kRadix / 32; w++) off += w < warp ? s_warp[w] : 0u;
+  return off + incl - v;
 }
 
-template <typename KeyT>
+// Digit offsets of pass p and whether it moves anything (a pass whose digit is
+// the same for all keys of every run is skipped), one block per run and pass:
+// goff[(p * runs + run) * 256 + d] = the run's first position + the run's
+// exclusive digit scan; bit p of *active (cleared before) is set when some run
+// has more than one digit in pass p.  hist holds hist_passes x 256 counts per run.
+__global__ void __launch_bounds__(kRadix) plan_kernel(const uint32_t *__restrict__ hist, int64_t n, int64_t run_len,
+                                                      int64_t runs, int hist_passes, int passes,
+                                                      uint32_t *__restrict__ goff, unsigned *active) {
+  __shared__ uint32_t s_warp[kRadix / 32];
+  const int64_t run = blockIdx.x / passes;
+  const int p = (int)(blockIdx.x % passes);
+  const int64_t start = run * run_len;
+  const int64_t len = min(run_len, n - start);
+  const uint32_t c = hist[(run * hist_passes + p) * kRadix + threadIdx.x];
+  if (__syncthreads_or((int64_t)c != len && c != 0) && threadIdx.x == 0) atomicOr(active, 1u << p);
+  goff[((int64_t)p * runs + run) * kRadix + threadIdx.x] = (uint32_t)start + scan_digits(c, s_warp);
+}
+
+template <typename KeyT, int kItems>
 struct PassSmem {
-  KeyT keys[kTile];
-  uint32_t vals[kTile];
+  KeyT keys[kSortBlock * kItems];
+  uint32_t vals[kSortBlock * kItems];
   uint32_t warp_hist[kSortWarps][kRadix];
   uint32_t digit_start[kRadix];  // tile-local exclusive start of each digit
   uint32_t global_start[kRadix];
@@ -133,21 +132,26 @@ struct PassSmem {
 #endif
 constexpr int kLookBatch = PRT_SORT_LOOKBATCH;  // predecessor statuses read per look-back step
 
-template <typename KeyT>
-__global__ void __launch_bounds__(kSortBlock, sizeof(KeyT) == 4 ? PRT_SORT_MIN_BLOCKS : 3) onesweep_pass(KeyT *keys0, uint32_t *vals0, KeyT *keys1,
-                                                           uint32_t *vals1, int64_t n, int shift,
-                                                           const PassPlan *__restrict__ plan,
-                                                           const uint32_t *__restrict__ goff,
-                                                           uint32_t *status, unsigned *tile_ticket,
-                                                           unsigned *err, WaitLimit wl, int64_t tiles_per_run) {
+template <typename KeyT, int kItems, bool kRuns>
+__global__ void __launch_bounds__(kSortBlock, sizeof(KeyT) == 4 ? PRT_SORT_MIN_BLOCKS : 3)
+    onesweep_pass(KeyT *keys0, uint32_t *vals0, KeyT *keys1, uint32_t *vals1, int64_t n, int shift,
+                  int passes, const unsigned *__restrict__ active, int *d_sel,
+                  const uint32_t *__restrict__ goff, uint32_t *status, unsigned *tile_ticket, unsigned *err, WaitLimit wl, int64_t run_len,
+                  int tiles_per_run) {
+  constexpr int kTile = kSortBlock * kItems;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  PassSmem<KeyT> &S = *reinterpret_cast<PassSmem<KeyT> *>(smem_raw);
-  const PassPlan pp = *plan;
-  if (!pp.active) return;
-  const KeyT *src_k = pp.src ? keys1 : keys0;
-  const uint32_t *src_v = pp.src ? vals1 : vals0;
-  KeyT *dst_k = pp.dst ? keys1 : keys0;
-  uint32_t *dst_v = pp.dst ? vals1 : vals0;
+  PassSmem<KeyT, kItems> &S = *reinterpret_cast<PassSmem<KeyT, kItems> *>(smem_raw);
+  // the buffers swap at every active pass
+  const int pass = shift / 8;
+  const unsigned act = *active;
+  const bool moves = act >> pass & 1u;
+  const bool from = __popc(act & ((1u << pass) - 1u)) & 1;
+  if (pass == passes - 1 && blockIdx.x == 0 && threadIdx.x == 0) *d_sel = from != moves;
+  if (!moves) return;
+  const KeyT *src_k = from ? keys1 : keys0;
+  const uint32_t *src_v = from ? vals1 : vals0;
+  KeyT *dst_k = from ? keys0 : keys1;
+  uint32_t *dst_v = from ? vals0 : vals1;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int d = tid;  // kSortBlock == kRadix: thread d owns digit d
@@ -155,13 +159,18 @@ __global__ void __launch_bounds__(kSortBlock, sizeof(KeyT) == 4 ? PRT_SORT_MIN_B
   for (int i = tid; i < kSortWarps * kRadix; i += kSortBlock) (&S.warp_hist[0][0])[i] = 0;
   __syncthreads();
   const int tile = S.tile;
-  const int64_t base = (int64_t)tile * kTile;
-  const int valid = (int)min((int64_t)kTile, n - base);
-  // runs sorted independently (tiles_per_run > 0): the tile's run, its first
-  // tile and its digit offsets; otherwise one run
-  const int64_t run = tiles_per_run > 0 ? tile / tiles_per_run : 0;
-  const int first = (int)(run * tiles_per_run);
-  goff += run * kRadix;
+  // the tile's run (kRuns: runs of run_len keys are sorted independently), its
+  // first tile, its place and its digit offsets
+  int first = 0;
+  int64_t base = (int64_t)tile * kTile, end = n;
+  if constexpr (kRuns) {
+    const int run = tile / tiles_per_run;
+    first = run * tiles_per_run;
+    base = run * run_len + (int64_t)(tile - first) * kTile;
+    end = min(n, (run + 1) * run_len);
+    goff += run * kRadix;
+  }
+  const int valid = (int)min((int64_t)kTile, end - base);
   const int wb = warp * 32 * kItems;  // this warp's first item in the tile
 
   KeyT k[kItems];
@@ -305,202 +314,109 @@ __global__ void __launch_bounds__(kSortBlock, sizeof(KeyT) == 4 ? PRT_SORT_MIN_B
   }
 }
 
-// Digit histograms of every pass per run (runs of tiles_per_run tiles): one
-// block per tile, block histograms in shared memory, one global add per
-// nonzero bin into hist[(run * passes + p) * 256 + digit].
+// The passes of one sort, with kItems keys per thread.
+template <typename KeyT, int kItems, bool kRuns>
+cudaError_t launch_passes(KeyT *keys0, uint32_t *vals0, KeyT *keys1, uint32_t *vals1, int64_t n, int64_t run_len,
+                          int tpr, int64_t tiles, int64_t runs, int passes, const unsigned *active, int *d_sel, const uint32_t *goff,
+                          uint32_t *status, unsigned *tick, unsigned *err, cudaStream_t s) {
+  const size_t smem = sizeof(PassSmem<KeyT, kItems>);
+  // the shared-memory opt-in is set once per device (not a stream operation,
+  // but kept out of graph captures after the first call)
+  static bool attr_done[256] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  cudaError_t e = cudaSuccess;
+  if (dev < 0 || dev >= 256 || !attr_done[dev]) {
+    e = cudaFuncSetAttribute(onesweep_pass<KeyT, kItems, kRuns>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess && dev >= 0 && dev < 256) attr_done[dev] = true;
+  }
+  const WaitLimit wl = wait_limit();
+  for (int p = 0; p < passes && e == cudaSuccess; p++) {
+    PRT_PROF("onesweep_pass", s);
+    onesweep_pass<KeyT, kItems, kRuns><<<(unsigned)tiles, kSortBlock, smem, s>>>(
+        keys0, vals0, keys1, vals1, n, 8 * p, passes, active, d_sel, goff + (size_t)p * runs * kRadix,
+        status + (size_t)p * tiles * kRadix, tick + p, err, wl, run_len, tpr);
+  }
+  if (e == cudaSuccess) e = cudaGetLastError();
+  return e;
+}
+
+// Sorts n keys in runs of run_len; d_hist (nullptr: counted here, one run
+// only) holds hist_passes digit histograms per run.
 template <typename KeyT>
-__global__ void __launch_bounds__(256) run_hist_kernel(const KeyT *__restrict__ keys, int64_t n, int passes,
-                                                       int64_t tiles_per_run, uint32_t *__restrict__ hist) {
-  extern __shared__ uint32_t sh[];  // passes * 256
-  for (int i = threadIdx.x; i < passes * kRadix; i += blockDim.x) sh[i] = 0;
-  __syncthreads();
-  const int64_t base = (int64_t)blockIdx.x * kTile;
-  const int64_t end = min(base + (int64_t)kTile, n);
-  for (int64_t i = base + threadIdx.x; i < end; i += blockDim.x) {
-    const KeyT k = keys[i];
-    for (int p = 0; p < passes; p++) atomicAdd(&sh[p * kRadix + (int)((k >> (8 * p)) & 0xFF)], 1u);
+int sort_impl(KeyT *keys0, uint32_t *vals0, KeyT *keys1, uint32_t *vals1, int64_t n, int64_t run_len, int key_bits,
+              int *d_sel, unsigned *d_err, cudaStream_t s, const uint32_t *d_hist, int hist_passes) {
+  PRT_CHECK(n >= 0 && n < (int64_t)kCountMask, PRT_ERR_INVALID, "radix sort: n=%lld out of range",
+            (long long)n);
+  const int passes = std::max(1, (key_bits + 7) / 8);
+  PRT_CHECK(passes <= (int)sizeof(KeyT), PRT_ERR_INVALID, "radix sort: %d key bits", key_bits);
+  if (n == 0) {
+    PRT_CUDA(cudaMemsetAsync(d_sel, 0, sizeof(int), s));
+    return PRT_OK;
   }
-  __syncthreads();
-  uint32_t *h = hist + (int64_t)(blockIdx.x / tiles_per_run) * passes * kRadix;
-  for (int i = threadIdx.x; i < passes * kRadix; i += blockDim.x)
-    if (sh[i]) atomicAdd(&h[i], sh[i]);
-}
-
-// Per run and pass: goff[(p * runs + run) * 256 + d] = the run's first
-// position + the run's exclusive digit scan; trivial[p] is cleared when some
-// run has more than one digit in pass p.  One block (256 threads) per run.
-__global__ void run_plan_kernel(const uint32_t *__restrict__ hist, int64_t n, int64_t run_len, int64_t runs,
-                                int passes, uint32_t *__restrict__ goff, int *__restrict__ trivial) {
-  __shared__ uint32_t scan[kRadix];
-  const int64_t run = blockIdx.x;
-  const int64_t start = run * run_len;
-  const int64_t len = min(run_len, n - start);
-  const int d = threadIdx.x;
-  for (int p = 0; p < passes; p++) {
-    const uint32_t c = hist[(run * passes + p) * kRadix + d];
-    scan[d] = c;
-    __syncthreads();
-    if ((int64_t)c != len && c != 0) trivial[p] = 0;
-    for (int o = 1; o < kRadix; o <<= 1) {
-      const uint32_t v = d >= o ? scan[d - o] : 0u;
-      __syncthreads();
-      scan[d] += v;
-      __syncthreads();
+  PRT_CHECK(run_len >= 1, PRT_ERR_INVALID, "radix sort: run length %lld", (long long)run_len);
+  const int64_t runs = (n + run_len - 1) / run_len;
+  // smaller tiles where the last tile of every run would be mostly empty
+  int items = sort_items(n);
+  auto tile_of = [](int k) { return (int64_t)kSortBlock * k; };
+  while (items > 4 && (run_len + tile_of(items) - 1) / tile_of(items) * tile_of(items) > run_len + run_len / 8) items /= 2;
+  const int tpr = (int)((run_len + tile_of(items) - 1) / tile_of(items));
+  const int64_t tiles = (runs - 1) * tpr + (n - (runs - 1) * run_len + tile_of(items) - 1) / tile_of(items);
+  // scratch: active passes, tickets, histograms and status (cleared), offsets
+  const size_t head = 128;
+  const size_t hist_b = d_hist ? 0 : sizeof(uint32_t) * (size_t)passes * kRadix;
+  const size_t stat_b = sizeof(uint32_t) * (size_t)tiles * kRadix * passes;
+  const size_t goff_b = sizeof(uint32_t) * (size_t)runs * passes * kRadix;
+  unsigned char *scratch = nullptr;
+  int rc = dmalloc(reinterpret_cast<void **>(&scratch), head + hist_b + stat_b + goff_b, s);
+  if (rc) return rc;
+  unsigned *active = reinterpret_cast<unsigned *>(scratch);
+  unsigned *tick = reinterpret_cast<unsigned *>(scratch + 64);
+  uint32_t *ghist = reinterpret_cast<uint32_t *>(scratch + head);
+  uint32_t *status = reinterpret_cast<uint32_t *>(scratch + head + hist_b);
+  uint32_t *goff = reinterpret_cast<uint32_t *>(scratch + head + hist_b + stat_b);
+  cudaError_t e = cudaMemsetAsync(scratch, 0, head + hist_b + stat_b, s);
+  if (e == cudaSuccess) {
+    if (!d_hist) {
+      PRT_PROF("hist", s);
+      hist_kernel<KeyT><<<grid_for(n, 256, 4), 256, sizeof(uint32_t) * passes * kRadix, s>>>(keys0, n, passes, ghist);
+      d_hist = ghist;
+      hist_passes = passes;
     }
-    goff[((int64_t)p * runs + run) * kRadix + d] = (uint32_t)start + scan[d] - c;
-    __syncthreads();
+    {
+      PRT_PROF("plan", s);
+      plan_kernel<<<(unsigned)(runs * passes), kRadix, 0, s>>>(d_hist, n, run_len, runs, hist_passes, passes, goff,
+                                                               active);
+    }
+    auto go = [&](auto k) {
+      constexpr int kItems = decltype(k)::value;
+      auto launch = runs > 1 ? launch_passes<KeyT, kItems, true> : launch_passes<KeyT, kItems, false>;
+      return launch(keys0, vals0, keys1, vals1, n, run_len, tpr, tiles, runs, passes, active, d_sel, goff, status,
+                    tick, d_err, s);
+    };
+    e = items == 4   ? go(std::integral_constant<int, 4>{})
+        : items == 8 ? go(std::integral_constant<int, 8>{})
+                     : go(std::integral_constant<int, 16>{});
   }
-}
-
-// Pass plans from the trivial flags (a pass whose digit is constant within
-// every run moves nothing and is skipped).
-__global__ void run_plan_final_kernel(const int *__restrict__ trivial, int passes, PassPlan *__restrict__ plan,
-                                      int *__restrict__ d_sel) {
-  int cur = 0;
-  for (int p = 0; p < passes; p++) {
-    PassPlan pp;
-    pp.active = !trivial[p];
-    pp.src = cur;
-    pp.dst = 1 - cur;
-    pp.pad = 0;
-    if (pp.active) cur = 1 - cur;
-    plan[p] = pp;
-  }
-  *d_sel = cur;
+  dfree(scratch, s);
+  if (e != cudaSuccess) return cuda_status(e, "radix sort");
+  return PRT_OK;
 }
 
 }  // namespace
 
 template <typename KeyT>
 int radix_sort_runs(KeyT *keys0, uint32_t *vals0, KeyT *keys1, uint32_t *vals1, int64_t n, int64_t run_len,
-                    int *d_sel, unsigned *d_err, cudaStream_t s, const uint32_t *d_hist) {
-  PRT_CHECK(n >= 0 && n < (int64_t)kCountMask, PRT_ERR_INVALID, "radix sort: n=%lld out of range",
-            (long long)n);
-  PRT_CHECK(run_len >= kTile && run_len % kTile == 0, PRT_ERR_INVALID,
-            "run sort: run length %lld is not a multiple of the %d-key tile", (long long)run_len, kTile);
-  if (n == 0) {
-    PRT_CUDA(cudaMemsetAsync(d_sel, 0, sizeof(int), s));
-    return PRT_OK;
-  }
-  const int passes = (int)sizeof(KeyT);
-  const int64_t tiles = (n + kTile - 1) / kTile;
-  const int64_t tpr = run_len / kTile;
-  const int64_t runs = (n + run_len - 1) / run_len;
-  // scratch: trivial flags, plan, tickets, per-run histograms, per-run offsets, status
-  const size_t triv_b = 64, plan_b = sizeof(PassPlan) * passes, tick_b = 64;
-  const size_t hist_b = sizeof(uint32_t) * (size_t)runs * passes * kRadix;
-  const size_t stat_b = sizeof(uint32_t) * (size_t)tiles * kRadix * passes;
-  unsigned char *scratch = nullptr;
-  const size_t head = 256;  // trivial (64) + plan (<= 128) + tickets (64)
-  size_t total = head + 2 * hist_b + stat_b;
-  int rc = dmalloc(reinterpret_cast<void **>(&scratch), total, s);
-  if (rc) return rc;
-  int *trivial = reinterpret_cast<int *>(scratch);
-  PassPlan *plan = reinterpret_cast<PassPlan *>(scratch + triv_b);
-  unsigned *tick = reinterpret_cast<unsigned *>(scratch + triv_b + 128);
-  uint32_t *hist = reinterpret_cast<uint32_t *>(scratch + head);
-  uint32_t *goff = hist + (size_t)runs * passes * kRadix;
-  uint32_t *status = goff + (size_t)runs * passes * kRadix;
-  (void)plan_b;
-  (void)tick_b;
-  cudaError_t e = cudaMemsetAsync(scratch, 0, total, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(trivial, 0xFF, sizeof(int) * passes, s);  // nonzero = trivial
-  if (e == cudaSuccess) {
-    if (!d_hist) {
-      PRT_PROF("run_hist", s);
-      run_hist_kernel<KeyT><<<(unsigned)tiles, 256, sizeof(uint32_t) * passes * kRadix, s>>>(keys0, n, passes, tpr,
-                                                                                            hist);
-    }
-    {
-      PRT_PROF("plan", s);
-      run_plan_kernel<<<(unsigned)runs, kRadix, 0, s>>>(d_hist ? d_hist : hist, n, run_len, runs, passes, goff,
-                                                        trivial);
-      run_plan_final_kernel<<<1, 1, 0, s>>>(trivial, passes, plan, d_sel);
-    }
-    size_t smem = sizeof(PassSmem<KeyT>);
-    static bool attr_done[256] = {false};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 256 || !attr_done[dev]) {
-      e = cudaFuncSetAttribute(onesweep_pass<KeyT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e == cudaSuccess && dev >= 0 && dev < 256) attr_done[dev] = true;
-    }
-    const WaitLimit wl = wait_limit();
-    for (int p = 0; p < passes && e == cudaSuccess; p++) {
-      PRT_PROF("onesweep_pass", s);
-      onesweep_pass<KeyT><<<(unsigned)tiles, kSortBlock, smem, s>>>(
-        keys0, vals0, keys1, vals1, n, 8 * p, plan + p, goff + (size_t)p * runs * kRadix,
-        status + (size_t)p * tiles * kRadix, tick + p, d_err, wl, tpr);
-    }
-    if (e == cudaSuccess) e = cudaGetLastError();
-  }
-  dfree(scratch, s);
-  if (e != cudaSuccess) return cuda_status(e, "radix_sort_runs");
-  return PRT_OK;
+                    int key_bits, int *d_sel, unsigned *d_err, cudaStream_t s, const uint32_t *d_hist) {
+  return sort_impl<KeyT>(keys0, vals0, keys1, vals1, n, run_len, key_bits, d_sel, d_err, s, d_hist,
+                         (int)sizeof(KeyT));
 }
 
 template <typename KeyT>
 int radix_sort_pairs(KeyT *keys0, uint32_t *vals0, KeyT *keys1, uint32_t *vals1, int64_t n, int key_bits,
                      int *d_sel, unsigned *d_err, cudaStream_t s, const uint32_t *d_hist) {
-  PRT_CHECK(n >= 0 && n < (int64_t)kCountMask, PRT_ERR_INVALID, "radix sort: n=%lld out of range",
-            (long long)n);
-  int passes = (key_bits + 7) / 8;
-  if (passes < 1) passes = 1;
-  PRT_CHECK(passes <= (int)sizeof(KeyT), PRT_ERR_INVALID, "radix sort: %d key bits", key_bits);
-  if (n == 0) {
-    PRT_CUDA(cudaMemsetAsync(d_sel, 0, sizeof(int), s));
-    return PRT_OK;
-  }
-  const int64_t tiles = (n + kTile - 1) / kTile;
-  // scratch: hist, offsets, plan, tickets, status
-  size_t hist_b = sizeof(uint32_t) * passes * kRadix;
-  size_t plan_b = sizeof(PassPlan) * passes;
-  size_t tick_b = sizeof(unsigned) * passes;
-  size_t stat_b = sizeof(uint32_t) * (size_t)tiles * kRadix * passes;
-  unsigned char *scratch = nullptr;
-  size_t total = 2 * hist_b + plan_b + tick_b + stat_b + 256;
-  int rc = dmalloc(reinterpret_cast<void **>(&scratch), total, s);
-  if (rc) return rc;
-  uint32_t *ghist = reinterpret_cast<uint32_t *>(scratch);
-  uint32_t *goff = ghist + passes * kRadix;
-  PassPlan *plan = reinterpret_cast<PassPlan *>(goff + passes * kRadix);
-  unsigned *tick = reinterpret_cast<unsigned *>(plan + passes);
-  uint32_t *status = reinterpret_cast<uint32_t *>(tick + passes);
-  cudaError_t e = cudaMemsetAsync(scratch, 0, total, s);
-  if (e == cudaSuccess) {
-    int g = grid_for(n, 256, 4);
-    if (!d_hist) {
-      PRT_PROF("hist", s);
-      hist_kernel<KeyT><<<g, 256, sizeof(uint32_t) * passes * kRadix, s>>>(keys0, n, passes, ghist);
-    }
-    {
-      PRT_PROF("plan", s);
-      plan_kernel<<<1, kRadix, 0, s>>>(d_hist ? d_hist : ghist, goff, passes, n, plan, d_sel);
-    }
-    size_t smem = sizeof(PassSmem<KeyT>);
-    // the shared-memory opt-in is set once per device (not a stream
-    // operation, but kept out of graph captures after the first call)
-    static bool attr_done[256] = {false};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 256 || !attr_done[dev]) {
-      e = cudaFuncSetAttribute(onesweep_pass<KeyT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e == cudaSuccess && dev >= 0 && dev < 256) attr_done[dev] = true;
-    }
-    const WaitLimit wl = wait_limit();
-    for (int p = 0; p < passes && e == cudaSuccess; p++) {
-      {
-        PRT_PROF("onesweep_pass", s);
-        onesweep_pass<KeyT><<<(unsigned)tiles, kSortBlock, smem, s>>>(
-          keys0, vals0, keys1, vals1, n, 8 * p, plan + p, goff + p * kRadix,
-          status + (size_t)p * tiles * kRadix, tick + p, d_err, wl, 0);
-      }
-    }
-    if (e == cudaSuccess) e = cudaGetLastError();
-  }
-  dfree(scratch, s);
-  if (e != cudaSuccess) return cuda_status(e, "radix_sort_pairs");
-  return PRT_OK;
+  return sort_impl<KeyT>(keys0, vals0, keys1, vals1, n, n, key_bits, d_sel, d_err, s, d_hist,
+                         std::max(1, (key_bits + 7) / 8));
 }
 
 namespace {
@@ -510,10 +426,10 @@ std::atomic<int> g_wait_blind{0};
 
 WaitLimit wait_limit() { return WaitLimit{g_wait_polls.load(), g_wait_blind.load()}; }
 
-template int radix_sort_runs<uint32_t>(uint32_t *, uint32_t *, uint32_t *, uint32_t *, int64_t, int64_t, int *,
-                                       unsigned *, cudaStream_t, const uint32_t *);
-template int radix_sort_runs<uint64_t>(uint64_t *, uint32_t *, uint64_t *, uint32_t *, int64_t, int64_t, int *,
-                                       unsigned *, cudaStream_t, const uint32_t *);
+template int radix_sort_runs<uint32_t>(uint32_t *, uint32_t *, uint32_t *, uint32_t *, int64_t, int64_t, int,
+                                       int *, unsigned *, cudaStream_t, const uint32_t *);
+template int radix_sort_runs<uint64_t>(uint64_t *, uint32_t *, uint64_t *, uint32_t *, int64_t, int64_t, int,
+                                       int *, unsigned *, cudaStream_t, const uint32_t *);
 template int radix_sort_pairs<uint32_t>(uint32_t *, uint32_t *, uint32_t *, uint32_t *, int64_t, int, int *,
                                         unsigned *, cudaStream_t, const uint32_t *);
 template int radix_sort_pairs<uint64_t>(uint64_t *, uint32_t *, uint64_t *, uint32_t *, int64_t, int, int *,

@@ -228,3 +228,28 @@ def test_windows_that_contain_nodes(cuda, kind, F, n):
         assert np.array_equal(un[np.lexsort((un[:, 0], un[:, 1]))], ref.reshape(-1, 2))
         for td in (False, True):
             assert np.array_equal(t.query_counts(qd, td_slots=td).cpu().numpy(), oracle.query_counts(lv, F, q, td_slots=td))
+
+
+@pytest.mark.parametrize("kind", ["f32", "f64", "i64", "i32"])
+@pytest.mark.parametrize("F,n", [(10, 4097), (10, 20001), (17, 4914), (17, 83522), (16, 65537), (3, 50000),
+                                 (10, 200001), (31, 30000)])
+def test_topdown_run_lengths(cuda, kind, F, n):
+    """Levels whose runs are no multiple of the sort's tiles, and sizes at the
+    edges of its tile sizes; integers below zero and with the range of the
+    whole type, so that the keys take every number of passes."""
+    import parlllelrtree_b200 as prt
+
+    rng = np.random.default_rng(F * n)
+    dt = {"f32": np.float32, "f64": np.float64, "i64": np.int64, "i32": np.int32}[kind]
+    c = rng.random((n, 2)) - 0.3
+    for scale in (1.0, 300.0, 1e6) if dt in (np.int64, np.int32) else (1.0,):
+        b = np.concatenate([c, c + 0.01], 1) * scale
+        b = np.floor(b).astype(dt) if dt in (np.int64, np.int32) else b.astype(dt)
+        if scale == 1e6:  # one record far away: 63 (31) significant bits
+            b[n // 2, :2] = np.iinfo(dt).min // 2
+            b[n // 3, 2:] = np.iinfo(dt).max // 2
+            b[n // 3, :2] = np.iinfo(dt).max // 2
+        perm = oracle.td_order(b, F)
+        t = prt.build_topdown(torch.from_numpy(b).cuda(), fanout=F)
+        assert np.array_equal(t.leaf_order().cpu().numpy(), perm)
+        check_levels(t, oracle.pack(b, F, perm))
