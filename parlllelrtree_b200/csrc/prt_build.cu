@@ -126,11 +126,13 @@ __device__ __forceinline__ T vmax(T a, T b) {
   else return b > a ? b : a;
 }
 
-// ext[0..3] = ordered encodings of min x1, min y1, max x2, max y2 (as double).
-// The per-thread min / max run in the coordinate type (the conversion to
-// double is monotone, so the result is the same as in double).
+// Smallest x1, y1 and largest x2, y2 of the boxes i0, i0 + step, .. of a
+// block, on thread 0 (as double).  The per-thread min / max run in the
+// coordinate type (the conversion to double is monotone, so the result is the
+// same as in double).
 template <typename T>
-__global__ void extent_f64_kernel(const Box<T> *__restrict__ b, int64_t n, unsigned long long *ext) {
+__device__ __forceinline__ void block_extent(const Box<T> *__restrict__ b, int64_t n, int64_t i0, int64_t step,
+                                             double (*red)[32], double *out) {
   T hi, lo;
   if constexpr (std::is_floating_point<T>::value) {
     hi = (T)__longlong_as_double(0x7FF0000000000000ll);
@@ -140,7 +142,7 @@ __global__ void extent_f64_kernel(const Box<T> *__restrict__ b, int64_t n, unsig
     lo = std::numeric_limits<T>::lowest();
   }
   T tnx = hi, tny = hi, txx = lo, txy = lo;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+  for (int64_t i = i0; i < n; i += step) {
     Box<T> x = load_box(b, i);
     tnx = vmin(tnx, x.x1);
     tny = vmin(tny, x.y1);
@@ -154,9 +156,6 @@ __global__ void extent_f64_kernel(const Box<T> *__restrict__ b, int64_t n, unsig
     mxx = fmax(mxx, __shfl_xor_sync(0xffffffffu, mxx, o));
     mxy = fmax(mxy, __shfl_xor_sync(0xffffffffu, mxy, o));
   }
-  // the block's warps, then one set of atomics per block (the four words
-  // are the same for every block, so fewer atomics means less contention)
-  __shared__ double red[4][32];
   const int w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
   if ((threadIdx.x & 31) == 0) {
     red[0][w] = mnx;
@@ -165,22 +164,48 @@ __global__ void extent_f64_kernel(const Box<T> *__restrict__ b, int64_t n, unsig
     red[3][w] = mxy;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int k = 1; k < nw; k++) {
-      mnx = fmin(mnx, red[0][k]);
-      mny = fmin(mny, red[1][k]);
-      mxx = fmax(mxx, red[2][k]);
-      mxy = fmax(mxy, red[3][k]);
+  if (threadIdx.x < 32) {
+    const int k = min((int)threadIdx.x, nw - 1);
+    mnx = red[0][k];
+    mny = red[1][k];
+    mxx = red[2][k];
+    mxy = red[3][k];
+    for (int o = 16; o; o >>= 1) {
+      mnx = fmin(mnx, __shfl_xor_sync(0xffffffffu, mnx, o));
+      mny = fmin(mny, __shfl_xor_sync(0xffffffffu, mny, o));
+      mxx = fmax(mxx, __shfl_xor_sync(0xffffffffu, mxx, o));
+      mxy = fmax(mxy, __shfl_xor_sync(0xffffffffu, mxy, o));
     }
-    atomicMin(&ext[0], ord_f64(mnx));
-    atomicMin(&ext[1], ord_f64(mny));
-    atomicMax(&ext[2], ord_f64(mxx));
-    atomicMax(&ext[3], ord_f64(mxy));
+    if (threadIdx.x == 0) {
+      out[0] = mnx;
+      out[1] = mny;
+      out[2] = mxx;
+      out[3] = mxy;
+    }
   }
 }
 
-// also clears the tree's flags, which the leaf packing sets
-__global__ void extent_init_kernel(unsigned long long *ext, unsigned *flags) {
+// ext[0..3] = ordered encodings of min x1, min y1, max x2, max y2 (as double):
+// one set of atomics per block (the four words are the same for every block,
+// so fewer atomics means less contention).
+template <typename T>
+__global__ void extent_f64_kernel(const Box<T> *__restrict__ b, int64_t n, unsigned long long *ext) {
+  __shared__ double red[4][32];
+  double m[4];
+  block_extent(b, n, blockIdx.x * (int64_t)blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x, red, m);
+  if (threadIdx.x == 0) {
+    atomicMin(&ext[0], ord_f64(m[0]));
+    atomicMin(&ext[1], ord_f64(m[1]));
+    atomicMax(&ext[2], ord_f64(m[2]));
+    atomicMax(&ext[3], ord_f64(m[3]));
+  }
+}
+
+// also clears the tree's flags, which the leaf packing sets, and the digit
+// histograms, which the key kernel counts
+__global__ void extent_init_kernel(unsigned long long *ext, unsigned *flags, uint32_t *hist) {
+  for (int i = threadIdx.x; i < 4 * 256; i += blockDim.x) hist[i] = 0u;
+  if (threadIdx.x) return;
   *flags = 0u;
   ext[0] = ord_f64(__longlong_as_double(0x7FF0000000000000ll));
   ext[1] = ext[0];
@@ -231,8 +256,26 @@ __device__ __forceinline__ uint32_t part1by1_16(uint32_t v) {
   return v;
 }
 
-// MORTON32: centre of each box on a 65536^2 grid over the data extent; the
+// MORTON32: centre of a box on a 65536^2 grid over the data extent; the
 // expression order matches the oracle exactly (no FMA: built with -fmad=false).
+struct MortonGrid {
+  double minX, minY, inv;
+  __device__ MortonGrid(double x0, double y0, double x1, double y1) : minX(x0), minY(y0) {
+    const double ex = (x1 - x0) > (y1 - y0) ? (x1 - x0) : (y1 - y0);
+    inv = ex > 0.0 ? 65535.0 / ex : 0.0;
+  }
+  template <typename T>
+  __device__ uint32_t operator()(const Box<T> &x) const {
+    double cx = 0.5 * ((double)x.x1 + (double)x.x2);
+    double cy = 0.5 * ((double)x.y1 + (double)x.y2);
+    double tx = (cx - minX) * inv;
+    double ty = (cy - minY) * inv;
+    uint32_t gx = tx >= 65535.0 ? 65535u : (tx > 0.0 ? (uint32_t)tx : 0u);
+    uint32_t gy = ty >= 65535.0 ? 65535u : (ty > 0.0 ? (uint32_t)ty : 0u);
+    return part1by1_16(gx) | (part1by1_16(gy) << 1);
+  }
+};
+
 // The four 8-bit digit histograms of the keys are counted on the way (block
 // histograms in shared memory, one global add per nonzero bin), so the sort
 // need not read the keys again to plan its passes.
@@ -244,19 +287,9 @@ __global__ void __launch_bounds__(256) morton32_kernel(const Box<T> *__restrict_
   __shared__ uint32_t h[4 * 256];
   for (int i = threadIdx.x; i < 4 * 256; i += blockDim.x) h[i] = 0;
   __syncthreads();
-  const double minX = unord_f64(ext[0]), minY = unord_f64(ext[1]);
-  const double maxX = unord_f64(ext[2]), maxY = unord_f64(ext[3]);
-  const double ex = (maxX - minX) > (maxY - minY) ? (maxX - minX) : (maxY - minY);
-  const double inv = ex > 0.0 ? 65535.0 / ex : 0.0;
+  const MortonGrid grid(unord_f64(ext[0]), unord_f64(ext[1]), unord_f64(ext[2]), unord_f64(ext[3]));
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    Box<T> x = load_box(b, i);
-    double cx = 0.5 * ((double)x.x1 + (double)x.x2);
-    double cy = 0.5 * ((double)x.y1 + (double)x.y2);
-    double tx = (cx - minX) * inv;
-    double ty = (cy - minY) * inv;
-    uint32_t gx = tx >= 65535.0 ? 65535u : (tx > 0.0 ? (uint32_t)tx : 0u);
-    uint32_t gy = ty >= 65535.0 ? 65535u : (ty > 0.0 ? (uint32_t)ty : 0u);
-    const uint32_t k = part1by1_16(gx) | (part1by1_16(gy) << 1);
+    const uint32_t k = grid(load_box(b, i));
     keys[i] = k;
     vals[i] = (uint32_t)i;
 #pragma unroll
@@ -758,33 +791,62 @@ __global__ void __launch_bounds__(256) pack_leaf_kernel(const Box<T> *__restrict
   if (__any_sync(0xffffffffu, improper) && lane == 0) atomicOr(flags, kTreeImproper);
 }
 
-// Upper level: entry j of level l+1 = union of node j of level l.
+// Union of entries [a, e) of a level, in order, several loads in flight at a
+// time.  The level may have been written by the calling kernel.
 template <typename T>
-__global__ void pack_level_kernel(const Box<T> *__restrict__ lo, int64_t n_lo, int fanout, Box<T> *__restrict__ hi,
-                                  int64_t n_hi, int64_t padded_hi) {
-  for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < padded_hi; j += (int64_t)gridDim.x * blockDim.x) {
-    if (j >= n_hi) {
-      store_box(hi, j, empty_box<T>());
-      continue;
-    }
-    int64_t a = j * fanout, e = min(a + fanout, n_lo);
-    Box<T> u = load_box(lo, a);
-    for (int64_t k = a + 1; k < e; k++) {
-      Box<T> x = load_box(lo, k);
-      u.x1 = tmin(u.x1, x.x1);
-      u.y1 = tmin(u.y1, x.y1);
-      u.x2 = tmax(u.x2, x.x2);
-      u.y2 = tmax(u.y2, x.y2);
-    }
-    store_box(hi, j, u);
+__device__ __forceinline__ Box<T> node_union(const Box<T> *lo, int64_t a, int64_t e) {
+  constexpr int kLoads = sizeof(T) == 4 ? 8 : 4;
+  Box<T> u = reload_box(lo, a);
+  for (int64_t k = a + 1; k < e; k += kLoads) {
+    Box<T> x[kLoads];
+#pragma unroll
+    for (int i = 0; i < kLoads; i++)
+      if (k + i < e) x[i] = reload_box(lo, k + i);
+#pragma unroll
+    for (int i = 0; i < kLoads; i++)
+      if (k + i < e) {
+        u.x1 = tmin(u.x1, x[i].x1);
+        u.y1 = tmin(u.y1, x[i].y1);
+        u.x2 = tmax(u.x2, x[i].x2);
+        u.y2 = tmax(u.y2, x[i].y2);
+      }
+  }
+  return u;
+}
+
+// Upper level: entry j of level l+1 = union of node j of level l.  Also fills
+// the padding of level l, [n_lo, pad_lo), where the leaf kernel wrote it.
+template <typename T>
+__global__ void pack_level_kernel(Box<T> *lo, int64_t n_lo, int64_t pad_lo, int fanout, Box<T> *hi, int64_t n_hi,
+                                  int64_t padded_hi) {
+  const int64_t first = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (n_lo + first < pad_lo) store_box(lo, n_lo + first, empty_box<T>());
+  for (int64_t j = first; j < padded_hi; j += (int64_t)gridDim.x * blockDim.x)
+    store_box(hi, j, j < n_hi ? node_union(lo, j * fanout, min((j + 1) * fanout, n_lo)) : empty_box<T>());
+}
+
+// The levels above a short one (kTailEntries entries at most), one after
+// another in one block: a launch for each would cost more than its work.
+constexpr int64_t kTailEntries = 4096;
+constexpr int kTailBlock = 1024;
+
+template <typename T>
+__device__ __forceinline__ void pack_tail(Box<T> *mbr, const TreeLevels &L, int from, int fanout) {
+  for (int l = from; l + 1 < L.levels; l++) {
+    const Box<T> *lo = mbr + L.offset[l];
+    Box<T> *hi = mbr + L.offset[l + 1];
+    for (int64_t j = threadIdx.x; j < L.padded[l + 1]; j += blockDim.x)
+      store_box(hi, j, j < L.count[l + 1] ? node_union(lo, j * fanout, min((j + 1) * fanout, L.count[l])) : empty_box<T>());
+    __syncthreads();
   }
 }
 
-// padding of level 1 when the leaf kernel wrote the unions
 template <typename T>
-__global__ void pad_level_kernel(Box<T> *__restrict__ lv, int64_t n, int64_t padded) {
-  int64_t j = n + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (j < padded) store_box(lv, j, empty_box<T>());
+__global__ void __launch_bounds__(kTailBlock) pack_tail_kernel(Box<T> *mbr, TreeLevels L, int from, int64_t pad_lo,
+                                                               int fanout) {
+  const int64_t k = L.count[from] + threadIdx.x;  // less than one node of padding
+  if (k < pad_lo) store_box(mbr + L.offset[from], k, empty_box<T>());
+  pack_tail(mbr, L, from, fanout);
 }
 
 template <typename T>
@@ -819,23 +881,218 @@ int pack_tree(prt_tree *t, const void *d_boxes, const int32_t *d_ids, const uint
                                                  t->d_leaf_id, nullptr, t->d_flags);
       }
   }
-  for (int l = 1; l < L.levels; l++) {
-    if (l == 1 && fused) {
-      int64_t pad = L.padded[1] - L.count[1];
-      if (pad > 0) {
-        PRT_PROF("pad_level", s);
-        pad_level_kernel<T><<<1, 64, 0, s>>>(lv1, L.count[1], L.padded[1]);
+  // the leaf kernel left level 1 without its padding when it wrote it
+  for (int l = fused ? 1 : 0; l < L.levels; l++) {
+    const int64_t pad = l == 1 && fused ? L.padded[1] : L.count[l];
+    if (L.count[l] <= kTailEntries) {
+      if (l + 1 < L.levels || pad > L.count[l]) {
+        PRT_PROF("pack_tail", s);
+        pack_tail_kernel<T><<<1, kTailBlock, 0, s>>>(mbr, L, l, pad, t->fanout);
       }
-      continue;
+      break;
     }
-    {
-      PRT_PROF("pack_level", s);
-      pack_level_kernel<T><<<grid_for(L.padded[l], block, 16), block, 0, s>>>(
-        mbr + L.offset[l - 1], L.count[l - 1], t->fanout, mbr + L.offset[l], L.count[l], L.padded[l]);
-    }
+    PRT_PROF("pack_level", s);
+    pack_level_kernel<T><<<grid_for(L.padded[l + 1], block, 16), block, 0, s>>>(
+        mbr + L.offset[l], L.count[l], pad, t->fanout, mbr + L.offset[l + 1], L.count[l + 1], L.padded[l + 1]);
   }
   PRT_CUDA(cudaGetLastError());
   return PRT_OK;
+}
+
+// ------------------------------------------------------------------ small bottom-up build
+
+// The whole bottom-up build (MORTON32) of up to kSmallBuild records in one
+// block: extent, keys, an LSD sort in shared memory by the multisplit of the
+// big sort's passes (skipping digits that are the same for all keys), leaves
+// and levels.  Its time is a chain of latencies, but one launch's: a call with
+// 1,000, 4,001 and 8,192 float boxes takes 40, 53 and 71 us against 90, 92 and
+// 92 with the grid-wide kernels' 10 launches, with 6,000 double boxes 77 against
+// 93 and with 8,192 as long: from there one SM's throughput is the bound.
+constexpr int kSmallBuild = 8192;
+constexpr int kSmallBuildWide = 6144;  // 64-bit coordinates
+constexpr int kSmallBlock = 1024;
+constexpr int kSmallWarps = kSmallBlock / 32;
+constexpr int kSmallItems = kSmallBuild / kSmallBlock;
+
+struct SmallSmem {
+  uint32_t key[kSmallBuild];
+  uint16_t val[kSmallBuild];
+  uint32_t wh[kSmallWarps][256];
+  uint32_t dstart[256];
+  uint32_t wsum[8];
+  double red[4][32];
+  double ext[4];
+  uint32_t differ;
+  unsigned improper;
+};
+
+template <typename T>
+__global__ void __launch_bounds__(kSmallBlock) bu_small_kernel(const Box<T> *__restrict__ b,
+                                                               const int32_t *__restrict__ ids, int n, int fanout,
+                                                               TreeLevels L, Box<T> *mbr, int32_t *__restrict__ leaf_id,
+                                                               unsigned *flags) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  SmallSmem &S = *reinterpret_cast<SmallSmem *>(smem_raw);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) {
+    S.differ = 0;
+    S.improper = 0;
+  }
+  block_extent(b, (int64_t)n, tid, kSmallBlock, S.red, S.ext);
+  __syncthreads();
+  const MortonGrid grid(S.ext[0], S.ext[1], S.ext[2], S.ext[3]);
+  // items per thread, in tile order: item j of lane l of warp w is position
+  // w * 32 * per + 32 j + l
+  const int per = (n + kSmallBlock - 1) / kSmallBlock;
+  const int base = warp * 32 * per + lane;
+  uint32_t k[kSmallItems], v[kSmallItems];
+  uint32_t differ = 0;
+  const uint32_t k0 = grid(load_box(b, 0));
+#pragma unroll
+  for (int j = 0; j < kSmallItems; j++) {
+    const int i = base + 32 * j;
+    k[j] = 0;
+    v[j] = (uint32_t)i;
+    if (j < per && i < n) {
+      k[j] = grid(load_box(b, i));
+      differ |= k[j] ^ k0;
+    }
+  }
+  differ = __reduce_or_sync(0xffffffffu, differ);
+  if (lane == 0 && differ) atomicOr(&S.differ, differ);
+  __syncthreads();
+  differ = S.differ;
+  const uint32_t lt = lane_lt();
+  for (int shift = 0; shift < 32; shift += 8) {
+    if (!(differ >> shift & 0xFFu)) continue;
+    for (int i = tid; i < kSmallWarps * 256; i += kSmallBlock) (&S.wh[0][0])[i] = 0;
+    __syncthreads();
+    uint32_t *wh = S.wh[warp];
+    uint32_t rk[kSmallItems];
+#pragma unroll
+    for (int j = 0; j < kSmallItems; j++) {
+      if (j >= per) break;
+      const bool ok = base + 32 * j < n;
+      const uint32_t d = k[j] >> shift & 0xFFu;
+      uint32_t peers = __ballot_sync(0xffffffffu, ok);
+#pragma unroll
+      for (int bit = 0; bit < 8; bit++) {
+        const uint32_t bm = __ballot_sync(0xffffffffu, (d >> bit) & 1u);
+        peers &= ((d >> bit) & 1u) ? bm : ~bm;
+      }
+      if (!ok) peers = 1u << lane;
+      const int leader = __ffs(peers) - 1;
+      uint32_t cnt = 0;
+      if (lane == leader && ok) {
+        cnt = wh[d];
+        wh[d] = cnt + __popc(peers);
+      }
+      cnt = __shfl_sync(0xffffffffu, cnt, leader);
+      rk[j] = cnt + __popc(peers & lt);
+      __syncwarp();
+    }
+    __syncthreads();
+    // thread d < 256: exclusive prefix of digit d over the warps, then over digits
+    uint32_t tot = 0, incl = 0;
+    if (tid < 256) {
+#pragma unroll 8
+      for (int w = 0; w < kSmallWarps; w++) {
+        const uint32_t x = S.wh[w][tid];
+        S.wh[w][tid] = tot;
+        tot += x;
+      }
+      incl = tot;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      if (lane == 31) S.wsum[warp] = incl;
+    }
+    __syncthreads();
+    if (tid < 256) {
+      uint32_t woff = 0;
+#pragma unroll
+      for (int w = 0; w < 8; w++) woff += w < warp ? S.wsum[w] : 0u;
+      S.dstart[tid] = woff + incl - tot;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kSmallItems; j++)
+      if (j < per && base + 32 * j < n) {
+        const uint32_t d = k[j] >> shift & 0xFFu;
+        const uint32_t at = S.dstart[d] + wh[d] + rk[j];
+        S.key[at] = k[j];
+        S.val[at] = (uint16_t)v[j];
+      }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kSmallItems; j++)
+      if (j < per && base + 32 * j < n) {
+        k[j] = S.key[base + 32 * j];
+        v[j] = S.val[base + 32 * j];
+      }
+    __syncthreads();
+  }
+  // leaves, and for fanouts that divide 32 the unions of level 1 by shuffles,
+  // as in pack_leaf_kernel
+  const bool fused = L.levels > 1 && (fanout & (fanout - 1)) == 0;
+  Box<T> *lv1 = L.levels > 1 ? mbr + L.offset[1] : mbr;
+  bool improper = false;
+#pragma unroll
+  for (int j = 0; j < kSmallItems; j++) {
+    const int i = base + 32 * j;
+    if (j >= per) break;
+    Box<T> x = i < n ? load_box(b, v[j]) : empty_box<T>();
+    improper |= i < n && !(x.x1 <= x.x2 && x.y1 <= x.y2);
+    if (i < n) leaf_id[i] = ids ? ids[v[j]] : (int32_t)v[j];
+    else if (i < L.padded[0]) leaf_id[i] = -1;
+    if (i < L.padded[0]) store_box(mbr, i, x);
+    if (fused) {
+      for (int o = fanout / 2; o > 0; o >>= 1) {
+        x.x1 = tmin(x.x1, __shfl_xor_sync(0xffffffffu, x.x1, o));
+        x.y1 = tmin(x.y1, __shfl_xor_sync(0xffffffffu, x.y1, o));
+        x.x2 = tmax(x.x2, __shfl_xor_sync(0xffffffffu, x.x2, o));
+        x.y2 = tmax(x.y2, __shfl_xor_sync(0xffffffffu, x.y2, o));
+      }
+      if (i % fanout == 0 && i < n) store_box(lv1, i / fanout, x);
+    }
+  }
+  // padding beyond the last item row (less than one node)
+  const int row = kSmallBlock * per;
+  if (row + tid < L.padded[0]) {
+    leaf_id[row + tid] = -1;
+    store_box(mbr, row + tid, empty_box<T>());
+  }
+  if (fused && L.count[1] + tid < L.padded[1]) store_box(lv1, L.count[1] + tid, empty_box<T>());
+  if (__any_sync(0xffffffffu, improper) && lane == 0) atomicOr(&S.improper, kTreeImproper);
+  __syncthreads();
+  if (tid == 0) *flags = S.improper;
+  pack_tail(mbr, L, fused ? 1 : 0, fanout);
+}
+
+bool bu_is_small(const prt_tree *t) {
+  return t->key_mode == PRT_KEY_MORTON32 && t->n <= (coord_size(t->coord) == 4 ? kSmallBuild : kSmallBuildWide);
+}
+
+int bu_small(prt_tree *t, const void *d_boxes, const int32_t *d_ids, cudaStream_t s) {
+  return dispatch_coord(t->coord, [&](auto tag) {
+    using T = decltype(tag);
+    static bool attr_done[256] = {false};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 256 || !attr_done[dev]) {
+      PRT_CUDA(cudaFuncSetAttribute(bu_small_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)sizeof(SmallSmem)));
+      if (dev >= 0 && dev < 256) attr_done[dev] = true;
+    }
+    PRT_PROF("bu_small", s);
+    bu_small_kernel<T><<<1, kSmallBlock, sizeof(SmallSmem), s>>>(
+        reinterpret_cast<const Box<T> *>(d_boxes), d_ids, (int)t->n, t->fanout, t->lv,
+        reinterpret_cast<Box<T> *>(t->d_mbr), t->d_leaf_id, t->d_flags);
+    PRT_CUDA(cudaGetLastError());
+    return PRT_OK;
+  });
 }
 
 int new_tree(const void *d_boxes, int coord, int64_t n, int fanout, int kind, int key_mode, cudaStream_t s,
@@ -892,6 +1149,7 @@ int finish(unsigned *d_err, cudaStream_t s, int rc) {
 // look-back wait gives up.
 int bu_enqueue(prt_tree *t, const void *d_boxes, const int32_t *d_ids, unsigned *err, cudaStream_t s) {
   const int64_t n = t->n;
+  if (bu_is_small(t)) return bu_small(t, d_boxes, d_ids, s);
   // scratch: ext (4 x 8), err, sel, digit histograms (4 x 256), keys0/1, vals0/1
   unsigned char *scr = nullptr;
   size_t kb = t->key_mode == PRT_KEY_REF64 ? 8 : 4;
@@ -909,14 +1167,9 @@ int bu_enqueue(prt_tree *t, const void *d_boxes, const int32_t *d_ids, unsigned 
   int g = grid_for(n, 256, 16);
   if (e == cudaSuccess) {
     if (t->key_mode == PRT_KEY_MORTON32) {
-      e = cudaMemsetAsync(hist, 0, 4096, s);
-      if (e != cudaSuccess) {
-        dfree(scr, s);
-        return cuda_status(e, "memset");
-      }
       {
         PRT_PROF("extent_init", s);
-        extent_init_kernel<<<1, 1, 0, s>>>(ext, t->d_flags);
+        extent_init_kernel<<<1, 256, 0, s>>>(ext, t->d_flags, hist);
       }
       rc = dispatch_coord(t->coord, [&](auto tag) {
         using T = decltype(tag);
@@ -997,15 +1250,24 @@ int prt_build_bottomup(const void *d_boxes, int coord_type, const int32_t *d_ids
   prt_tree *t = nullptr;
   int rc = new_tree(d_boxes, coord_type, n, fanout, PRT_BOTTOM_UP, key_mode, s, &t);
   if (rc) return rc;
-  unsigned *err = nullptr;
-  rc = dalloc(&err, 2, s);
-  if (!rc) {
-    cudaError_t e = cudaMemsetAsync(err, 0, 8, s);
-    if (e != cudaSuccess) rc = cuda_status(e, "memset");
+  if (bu_is_small(t)) {
+    // nothing in it waits for another block: no error word to read back
+    rc = bu_small(t, d_boxes, d_ids, s);
+    if (!rc) {
+      cudaError_t e = cudaStreamSynchronize(s);
+      if (e != cudaSuccess) rc = cuda_status(e, "build");
+    }
+  } else {
+    unsigned *err = nullptr;
+    rc = dalloc(&err, 2, s);
+    if (!rc) {
+      cudaError_t e = cudaMemsetAsync(err, 0, 8, s);
+      if (e != cudaSuccess) rc = cuda_status(e, "memset");
+    }
+    if (!rc) rc = bu_enqueue(t, d_boxes, d_ids, err, s);
+    rc = finish(err, s, rc);
+    dfree(err, s);
   }
-  if (!rc) rc = bu_enqueue(t, d_boxes, d_ids, err, s);
-  rc = finish(err, s, rc);
-  dfree(err, s);
   if (rc) {
     prt_tree_free(t);
     return rc;

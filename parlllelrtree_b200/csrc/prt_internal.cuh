@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdio.h>
+#include <string.h>
 
 #include <string>
 
@@ -151,13 +152,34 @@ __device__ inline Box<int64_t> load_box(const Box<int64_t> *p, int64_t i) {
   return Box<int64_t>{a.x, a.y, b.x, b.y};
 }
 
+// A box as 16-byte words (a Box array is 16-byte aligned).
 template <typename T>
 __device__ inline void store_box(Box<T> *p, int64_t i, const Box<T> &b) {
-  p[i] = b;
+  if constexpr (sizeof(T) == 4) {
+    uint4 v;
+    memcpy(&v, &b, 16);
+    reinterpret_cast<uint4 *>(p)[i] = v;
+  } else {
+    ulonglong2 v[2];
+    memcpy(v, &b, 32);
+    reinterpret_cast<ulonglong2 *>(p)[2 * i] = v[0];
+    reinterpret_cast<ulonglong2 *>(p)[2 * i + 1] = v[1];
+  }
 }
-template <>
-__device__ inline void store_box(Box<float> *p, int64_t i, const Box<float> &b) {
-  reinterpret_cast<float4 *>(p)[i] = make_float4(b.x1, b.y1, b.x2, b.y2);
+
+// load_box for boxes that the same kernel may have written (no read-only cache)
+template <typename T>
+__device__ inline Box<T> reload_box(const Box<T> *p, int64_t i) {
+  Box<T> b;
+  if constexpr (sizeof(T) == 4) {
+    const uint4 v = reinterpret_cast<const uint4 *>(p)[i];
+    memcpy(&b, &v, 16);
+  } else {
+    const ulonglong2 v[2] = {reinterpret_cast<const ulonglong2 *>(p)[2 * i],
+                             reinterpret_cast<const ulonglong2 *>(p)[2 * i + 1]};
+    memcpy(&b, v, 32);
+  }
+  return b;
 }
 
 inline size_t coord_size(int coord) {

@@ -253,3 +253,21 @@ def test_topdown_run_lengths(cuda, kind, F, n):
         t = prt.build_topdown(torch.from_numpy(b).cuda(), fanout=F)
         assert np.array_equal(t.leaf_order().cpu().numpy(), perm)
         check_levels(t, oracle.pack(b, F, perm))
+
+
+@pytest.mark.parametrize("kind", ["f32", "f64", "i64", "i32"])
+@pytest.mark.parametrize("F", [2, 3, 16, 32])
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 1023, 1024, 1025, 4096, 6143, 6144, 6145, 8191, 8192, 8193])
+def test_one_block_build(cuda, kind, F, n):
+    """Sizes at the edges of the one-block build (rows of 1,024 records, its
+    largest sizes for 32- and 64-bit coordinates), with ties and given ids."""
+    import parlllelrtree_b200 as prt
+
+    b = boxes_of(kind, n, seed=n + F)
+    b[n // 3: n // 2] = b[n // 3]  # a run of equal boxes keeps its order
+    keys, _ = oracle.keys_morton32(b)
+    perm = oracle.stable_argsort(keys)
+    ids = np.arange(n, dtype=np.int32)[::-1].copy()
+    t = prt.build_bottomup(torch.from_numpy(b).cuda(), fanout=F, ids=ids)
+    assert np.array_equal(t.leaf_order().cpu().numpy(), ids[perm])
+    check_levels(t, oracle.pack(b, F, perm))
