@@ -780,6 +780,307 @@ constexpr double kFwdTol = 1e-10;
 // Pairs the last forward call listed for the GPC clip (prt_area_fwd_fallbacks).
 std::atomic<int64_t> g_fwd_fallbacks{0};
 
+// ---- pairs of tiny polygons: one thread each -----------------------------------
+// Two polygons of one ring and 3 to kTinyV vertices (parcels, map tiles) have too
+// few edges for a warp (4-6-vertex parcels filled 10 of its 32 lanes, and staging
+// them cost more than their crossings).  One thread takes such a pair and
+// intersects every pair of edges once, for both: with the edge p + t r of A
+// and a + u s of B, t and u are the crossing seen from A's and from B's side, bit
+// for bit what the two passes of pair_boundary compute.  B's vertices and
+// per-edge sums stay in registers, A's vertices (and in gradient mode its
+// gradient, until the pair is known to be clean) in shared memory.  The other
+// pairs are listed for the staged kernels, the unclean ones too in gradient
+// mode; in area mode those go to the GPC clip like theirs.
+constexpr int kTinyV = 8;
+constexpr int kTinyBlock = 128;
+
+// Appends i to a list for the threads of the block that ask (one atomic per
+// block: when no pair is tiny, every one of them is listed).
+__device__ __forceinline__ void append_pair(bool ask, int64_t i, int32_t *list, unsigned long long *count,
+                                            unsigned *s_count, unsigned long long *s_base) {
+  const unsigned who = __ballot_sync(kFullMask, ask);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (lane == 0) s_count[warp] = __popc(who);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned total = 0;
+    for (int w = 0; w < kTinyBlock / 32; w++) total += s_count[w];
+    *s_base = total ? atomicAdd(count, (unsigned long long)total) : 0ull;
+  }
+  __syncthreads();
+  unsigned long long at = *s_base;
+  for (int w = 0; w < warp; w++) at += s_count[w];
+  if (ask) list[at + __popc(who & ((1u << lane) - 1u))] = (int32_t)i;
+  __syncthreads();
+}
+
+// The ring of a polygon that a thread can take: first vertex, vertices and
+// orientation sign flip of a hole; false for the others.
+__device__ __forceinline__ bool tiny_ring(const LayerDev &L, int64_t poly, int64_t *v0, int *nv, bool *hole) {
+  const int64_t r = L.poly_ring[poly];
+  if (L.poly_ring[poly + 1] != r + 1) return false;
+  *v0 = L.ring_vert[r];
+  const int64_t n = L.ring_vert[r + 1] - *v0;
+  if (n < 3 || n > kTinyV) return false;
+  *nv = (int)n;
+  *hole = L.ring_hole && L.ring_hole[r];
+  return true;
+}
+
+template <bool kArea>
+struct TinySmem {
+  double x[kTinyV][kTinyBlock], y[kTinyV][kTinyBlock];  // A's vertices, a column per thread
+  double gx[kArea ? 1 : kTinyV][kTinyBlock], gy[kArea ? 1 : kTinyV][kTinyBlock];
+};
+
+// 200k parcels (471k pairs): forward 85 us, backward 105 against 535 and 604 with
+// a warp each; 3 blocks per SM for the gradients (120 us against 132 with 4, and
+// 186 with 5), 4 for the areas (103; 107 and 123 with 3 and 5).
+template <bool kArea>
+__global__ void __launch_bounds__(kTinyBlock, kArea ? 4 : 3) area_tiny_kernel(
+    const int32_t *__restrict__ pa, const int32_t *__restrict__ pb, int64_t n, LayerDev base, LayerDev over,
+    const double *__restrict__ upstream, double *grad_base, double *grad_over, double *__restrict__ area,
+    int32_t *__restrict__ fb, unsigned long long *__restrict__ fb_count, int32_t *__restrict__ defer,
+    unsigned long long *__restrict__ defer_count) {
+  __shared__ TinySmem<kArea> S;
+  __shared__ unsigned s_count[kTinyBlock / 32];
+  __shared__ unsigned long long s_base;
+  const int tid = threadIdx.x;
+  const int64_t i = blockIdx.x * (int64_t)kTinyBlock + tid;
+  int64_t va = 0, vb = 0;
+  int na = 0, nb = 0;
+  bool ha = false, hb = false;
+  bool mine = false;  // this thread takes the pair
+  if (i < n) {
+    const int64_t a = pa[i], b = pb[i];
+    if (a >= 0 && a < base.n_poly && b >= 0 && b < over.n_poly)
+      mine = tiny_ring(base, a, &va, &na, &ha) && tiny_ring(over, b, &vb, &nb, &hb);
+  }
+  bool clean = true;
+  double bound = 0.0, area2 = 0.0;
+  if (mine) {
+    double bx[kTinyV], by[kTinyV];
+    double cmax = 0.0, sa = 0.0, sb = 0.0;
+    double lox = 0.0, loy = 0.0, hix = 0.0, hiy = 0.0;  // A's box
+    for (int k = 0; k < na; k++) {
+      const double x = base.xy[2 * (va + k)], y = base.xy[2 * (va + k) + 1];
+      S.x[k][tid] = x;
+      S.y[k][tid] = y;
+      lox = k ? fmin(lox, x) : x;
+      loy = k ? fmin(loy, y) : y;
+      hix = k ? fmax(hix, x) : x;
+      hiy = k ? fmax(hiy, y) : y;
+    }
+    cmax = fmax(fmax(fabs(lox), fabs(loy)), fmax(fabs(hix), fabs(hiy)));
+    double blx = 0.0, bly = 0.0, bhx = 0.0, bhy = 0.0;
+#pragma unroll
+    for (int k = 0; k < kTinyV; k++) {
+      bx[k] = by[k] = 0.0;
+      if (k < nb) {
+        bx[k] = over.xy[2 * (vb + k)];
+        by[k] = over.xy[2 * (vb + k) + 1];
+        blx = k ? fmin(blx, bx[k]) : bx[k];
+        bly = k ? fmin(bly, by[k]) : by[k];
+        bhx = k ? fmax(bhx, bx[k]) : bx[k];
+        bhy = k ? fmax(bhy, by[k]) : by[k];
+      }
+    }
+    cmax = fmax(cmax, fmax(fmax(fabs(blx), fabs(bly)), fmax(fabs(bhx), fabs(bhy))));
+    // boxes apart: no crossing, no point of one inside the other (a NaN
+    // coordinate is not apart, and not clean below)
+    const bool apart = lox > bhx || hix < blx || loy > bhy || hiy < bly;
+    if (!apart) {
+      for (int k = 0; k < na; k++) {
+        const int l = k + 1 == na ? 0 : k + 1;
+        sa += S.x[k][tid] * S.y[l][tid] - S.x[l][tid] * S.y[k][tid];
+      }
+#pragma unroll
+      for (int k = 0; k < kTinyV; k++)
+        if (k < nb) {
+          const bool last = k + 1 == nb;
+          const double ex = last ? bx[0] : bx[k + 1 < kTinyV ? k + 1 : 0], ey = last ? by[0] : by[k + 1 < kTinyV ? k + 1 : 0];
+          sb += bx[k] * ey - ex * by[k];
+        }
+      // material on the left: CCW outer rings and CW holes
+      const bool la = (sa >= 0.0) != ha, lb = (sb >= 0.0) != hb;
+      const double sgna = la ? 1.0 : -1.0, sgnb = lb ? 1.0 : -1.0;
+      const double w = !kArea && upstream ? upstream[i] : 1.0;
+      const double ox = S.x[0][tid], oy = S.y[0][tid];  // the pair-local origin
+      // per edge of B: sums of sign u and sign u^2, and crossings (low half) and
+      // signs (high half) as 4-bit fields, biased by 8
+      double c1b[kTinyV], c2b[kTinyV];
+#pragma unroll
+      for (int k = 0; k < kTinyV; k++) c1b[k] = c2b[k] = 0.0;
+      uint32_t mb = 0, c0b = 0x88888888u;
+      double ufirst = 1.0;  // first crossing of B's edge 0
+      double err = 0.0;
+      bool st = false;  // inside state at the start of A's edge k
+      double cx = 0.0, cy = 0.0;  // what the edge before gives to A's vertex k
+      for (int k = 0; k < na; k++) {
+        const int l = k + 1 == na ? 0 : k + 1;
+        const double px = S.x[k][tid], py = S.y[k][tid], qx = S.x[l][tid], qy = S.y[l][tid];
+        const double rx = qx - px, ry = qy - py;
+        const double rl = fabs(rx) + fabs(ry);
+        double c1 = 0.0, c2 = 0.0, tfirst = 1.0;
+        int m = 0, c0 = 0;
+#pragma unroll
+        for (int e = 0; e < kTinyV; e++) {
+          if (e >= nb) break;
+          const bool last = e + 1 == nb;
+          const double ax = bx[e], ay = by[e];
+          const double sx = (last ? bx[0] : bx[e + 1 < kTinyV ? e + 1 : 0]) - ax;
+          const double sy = (last ? by[0] : by[e + 1 < kTinyV ? e + 1 : 0]) - ay;
+          const double den = rx * sy - ry * sx;
+          const double apx = ax - px, apy = ay - py;
+          const double tn = apx * sy - apy * sx;
+          const double un = apx * ry - apy * rx;
+          if (den == 0.0) {
+            // collinear edges whose boxes meet
+            if ((tn == 0.0 || un == 0.0) && fmin(ax, ax + sx) <= fmax(px, qx) && fmin(px, qx) <= fmax(ax, ax + sx) &&
+                fmin(ay, ay + sy) <= fmax(py, qy) && fmin(py, qy) <= fmax(ay, ay + sy))
+              clean = false;
+            continue;
+          }
+          // t = tn / den and u = un / den, with the signs of den folded in
+          const double d = fabs(den), tol = 1e-9 * d;
+          const double tt = den > 0.0 ? tn : -tn, uu = den > 0.0 ? un : -un;
+          if (tt < -tol || tt > d + tol || uu < -tol || uu > d + tol) continue;
+          const double sl = fabs(sx) + fabs(sy);
+          if (!(tt > tol && tt < d - tol && uu > tol && uu < d - tol && d > 1e-6 * rl * sl)) {
+            clean = false;
+            continue;
+          }
+          if constexpr (kArea) err += 2.0 * ((rl + sl) * rl * sl / d);  // seen from both edges
+          const double t = tn / den, u = un / den;
+          const bool out_b = (den > 0.0) == lb;  // A's edge leaves B here
+          const bool out_a = (den < 0.0) == la;  // B's edge leaves A
+          const double ts = out_b ? -t : t, us = out_a ? -u : u;
+          c0 += out_b ? -1 : 1;
+          c1 += ts;
+          if constexpr (!kArea) c2 += ts * t;
+          tfirst = fmin(tfirst, t);
+          m++;
+          c0b += out_a ? 0u - (1u << (4 * e)) : 1u << (4 * e);
+          mb ^= 1u << e;
+          c1b[e] += us;
+          if constexpr (!kArea) c2b[e] += us * u;
+          if (e == 0) ufirst = fmin(ufirst, u);
+        }
+        if (k == 0) {
+          // the ring's first piece by its midpoint
+          const double mx = px + 0.5 * tfirst * rx, my = py + 0.5 * tfirst * ry;
+          bool in = false;
+#pragma unroll
+          for (int e = 0; e < kTinyV; e++) {
+            if (e >= nb) break;
+            const bool last = e + 1 == nb;
+            const double ax = bx[e], ay = by[e];
+            const double ex = last ? bx[0] : bx[e + 1 < kTinyV ? e + 1 : 0], ey = last ? by[0] : by[e + 1 < kTinyV ? e + 1 : 0];
+            if ((ay > my) != (ey > my) && mx < ax + (my - ay) * (ex - ax) / (ey - ay)) in = !in;
+          }
+          st = in;
+        }
+        const bool end = st != ((m & 1) != 0);
+        if ((int)st + c0 != (int)end) clean = false;
+        st = end;
+        const double s1 = end ? 1.0 : 0.0;
+        if constexpr (kArea) {
+          area2 += sgna * (s1 - c1) * ((px - ox) * ry - (py - oy) * rx);
+        } else {
+          const double it = 0.5 * (s1 - c2), i1 = (s1 - c1) - it;
+          const double nx = w * sgna * ry, ny = -w * sgna * rx;
+          S.gx[k][tid] = cx + nx * i1;
+          S.gy[k][tid] = cy + ny * i1;
+          cx = nx * it;
+          cy = ny * it;
+        }
+      }
+      if constexpr (!kArea) {
+        S.gx[0][tid] += cx;
+        S.gy[0][tid] += cy;
+      }
+      // B's edges, from their sums
+      {
+        const double dx = bx[1] - bx[0], dy = by[1] - by[0];
+        const double mx = bx[0] + 0.5 * ufirst * dx, my = by[0] + 0.5 * ufirst * dy;
+        bool in = false;
+        for (int k = 0; k < na; k++) {
+          const int l = k + 1 == na ? 0 : k + 1;
+          const double ax = S.x[k][tid], ay = S.y[k][tid], ex = S.x[l][tid], ey = S.y[l][tid];
+          if ((ay > my) != (ey > my) && mx < ax + (my - ay) * (ex - ax) / (ey - ay)) in = !in;
+        }
+        st = in;
+      }
+      uint32_t ends = 0;  // inside state at the edges' ends
+#pragma unroll
+      for (int e = 0; e < kTinyV; e++) {
+        if (e >= nb) break;
+        const bool end = st != ((mb >> e & 1u) != 0);
+        if ((int)st + (int)(c0b >> (4 * e) & 15u) - 8 != (int)end) clean = false;
+        st = end;
+        ends |= (end ? 1u : 0u) << e;
+      }
+      if constexpr (kArea) {
+#pragma unroll
+        for (int e = 0; e < kTinyV; e++) {
+          if (e >= nb) break;
+          const bool last = e + 1 == nb;
+          const double rx = (last ? bx[0] : bx[e + 1 < kTinyV ? e + 1 : 0]) - bx[e];
+          const double ry = (last ? by[0] : by[e + 1 < kTinyV ? e + 1 : 0]) - by[e];
+          const double s1 = ends >> e & 1u ? 1.0 : 0.0;
+          area2 += sgnb * (s1 - c1b[e]) * ((bx[e] - ox) * ry - (by[e] - oy) * rx);
+        }
+        bound = 2.0 * 2.220446049250313e-16 * cmax * err;
+      } else if (clean) {
+        for (int k = 0; k < na; k++) {
+          const double x = S.gx[k][tid], y = S.gy[k][tid];
+          if (x != 0.0 || y != 0.0) {
+            atomicAdd(&grad_base[2 * (va + k)], x);
+            atomicAdd(&grad_base[2 * (va + k) + 1], y);
+          }
+        }
+        double fx = 0.0, fy = 0.0;  // vertex 0's own part
+        cx = cy = 0.0;
+#pragma unroll
+        for (int e = 0; e < kTinyV; e++) {
+          if (e >= nb) break;
+          const bool last = e + 1 == nb;
+          const double rx = (last ? bx[0] : bx[e + 1 < kTinyV ? e + 1 : 0]) - bx[e];
+          const double ry = (last ? by[0] : by[e + 1 < kTinyV ? e + 1 : 0]) - by[e];
+          const double s1 = ends >> e & 1u ? 1.0 : 0.0;
+          const double it = 0.5 * (s1 - c2b[e]), i1 = (s1 - c1b[e]) - it;
+          const double nx = w * sgnb * ry, ny = -w * sgnb * rx;
+          const double x = cx + nx * i1, y = cy + ny * i1;
+          if (e == 0) {
+            fx = x;
+            fy = y;
+          } else if (x != 0.0 || y != 0.0) {
+            atomicAdd(&grad_over[2 * (vb + e)], x);
+            atomicAdd(&grad_over[2 * (vb + e) + 1], y);
+          }
+          cx = nx * it;
+          cy = ny * it;
+        }
+        fx += cx;
+        fy += cy;
+        if (fx != 0.0 || fy != 0.0) {
+          atomicAdd(&grad_over[2 * vb], fx);
+          atomicAdd(&grad_over[2 * vb + 1], fy);
+        }
+      }
+    }
+  }
+  if constexpr (kArea) {
+    const double ar = 0.5 * area2;
+    const bool keep = mine && clean && bound <= kFwdTol * fabs(ar);
+    if (keep) area[i] = ar;
+    append_pair(mine && !keep, i, fb, fb_count, s_count, &s_base);
+    append_pair(i < n && !mine, i, defer, defer_count, s_count, &s_base);
+  } else {
+    append_pair(i < n && !(mine && clean), i, defer, defer_count, s_count, &s_base);
+  }
+}
+
 // V = 64: 5 blocks of 4 warps per SM (96 registers: a few spills, 10% faster
 // than 4 blocks at 1M pairs of 16-64-vertex stars).
 template <int V>
@@ -914,21 +1215,23 @@ int prt_area_fwd(const int32_t *d_pair_a, const int32_t *d_pair_b, int64_t n_pai
   // boundary integral for the clean pairs, the list of the others; pairs
   // with a polygon too large for one stage's staging go to the next
   unsigned char *scr = nullptr;
-  int rc = dmalloc(reinterpret_cast<void **>(&scr), 64 + 12 * (size_t)n_pairs, s);
+  int rc = dmalloc(reinterpret_cast<void **>(&scr), 64 + 16 * (size_t)n_pairs, s);
   if (rc) return rc;
-  unsigned long long *cnt = reinterpret_cast<unsigned long long *>(scr);  // fallbacks, then the two stage lists
+  unsigned long long *cnt = reinterpret_cast<unsigned long long *>(scr);  // fallbacks, then the three stage lists
   int32_t *fb = reinterpret_cast<int32_t *>(scr + 64);
-  int32_t *mid = fb + n_pairs, *large = mid + n_pairs;
-  cudaError_t e = cudaMemsetAsync(cnt, 0, 24, s);
+  int32_t *small = fb + n_pairs, *mid = small + n_pairs, *large = mid + n_pairs;
+  cudaError_t e = cudaMemsetAsync(cnt, 0, 32, s);
   if (e == cudaSuccess) {
     PRT_PROF("area_fwd", s);
     const LayerDev A = layer_dev(base), B = layer_dev(overlay);
+    area_tiny_kernel<true><<<(unsigned)((n_pairs + kTinyBlock - 1) / kTinyBlock), kTinyBlock, 0, s>>>(
+        d_pair_a, d_pair_b, n_pairs, A, B, nullptr, nullptr, nullptr, d_area, fb, cnt, small, cnt + 1);
     launch_area_fwd<kBwdSmallV>(d_pair_a, d_pair_b, n_pairs, A, B, d_area, fb, cnt,
-                                PairList{nullptr, nullptr, mid, cnt + 1}, s);
+                                PairList{small, cnt + 1, mid, cnt + 2}, s);
     launch_area_fwd<kBwdMidV>(d_pair_a, d_pair_b, n_pairs, A, B, d_area, fb, cnt,
-                              PairList{mid, cnt + 1, large, cnt + 2}, s);
+                              PairList{mid, cnt + 2, large, cnt + 3}, s);
     launch_area_fwd<kBwdLargeV>(d_pair_a, d_pair_b, n_pairs, A, B, d_area, fb, cnt,
-                                PairList{large, cnt + 2, nullptr, nullptr}, s);
+                                PairList{large, cnt + 3, nullptr, nullptr}, s);
     e = cudaGetLastError();
   }
   unsigned long long m = 0;
@@ -989,20 +1292,23 @@ int prt_area_bwd(const int32_t *d_pair_a, const int32_t *d_pair_b, int64_t n_pai
   // pairs with a polygon too large for one stage's staging: listed by it,
   // taken by the next
   unsigned char *scr = nullptr;
-  int rc = dmalloc(reinterpret_cast<void **>(&scr), 64 + 8 * (size_t)n_pairs, s);
+  int rc = dmalloc(reinterpret_cast<void **>(&scr), 64 + 12 * (size_t)n_pairs, s);
   if (rc) return rc;
-  unsigned long long *cnt = reinterpret_cast<unsigned long long *>(scr);  // the two stage lists
-  int32_t *mid = reinterpret_cast<int32_t *>(scr + 64), *large = mid + n_pairs;
-  cudaError_t e = cudaMemsetAsync(cnt, 0, 16, s);
+  unsigned long long *cnt = reinterpret_cast<unsigned long long *>(scr);  // the three stage lists
+  int32_t *small = reinterpret_cast<int32_t *>(scr + 64), *mid = small + n_pairs, *large = mid + n_pairs;
+  cudaError_t e = cudaMemsetAsync(cnt, 0, 24, s);
   if (e == cudaSuccess) {
     PRT_PROF("area_bwd", s);
     const LayerDev A = layer_dev(base), B = layer_dev(overlay);
+    area_tiny_kernel<false><<<(unsigned)((n_pairs + kTinyBlock - 1) / kTinyBlock), kTinyBlock, 0, s>>>(
+        d_pair_a, d_pair_b, n_pairs, A, B, d_upstream, d_grad_base, d_grad_overlay, nullptr, nullptr, nullptr, small,
+        cnt);
     launch_area_bwd<kBwdSmallV>(d_pair_a, d_pair_b, n_pairs, A, B, d_upstream, d_grad_base, d_grad_overlay,
-                                PairList{nullptr, nullptr, mid, cnt}, s);
+                                PairList{small, cnt, mid, cnt + 1}, s);
     launch_area_bwd<kBwdMidV>(d_pair_a, d_pair_b, n_pairs, A, B, d_upstream, d_grad_base, d_grad_overlay,
-                              PairList{mid, cnt, large, cnt + 1}, s);
+                              PairList{mid, cnt + 1, large, cnt + 2}, s);
     launch_area_bwd<kBwdLargeV>(d_pair_a, d_pair_b, n_pairs, A, B, d_upstream, d_grad_base, d_grad_overlay,
-                                PairList{large, cnt + 1, nullptr, nullptr}, s);
+                                PairList{large, cnt + 2, nullptr, nullptr}, s);
     e = cudaGetLastError();
   }
   dfree(scr, s);

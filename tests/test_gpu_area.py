@@ -239,3 +239,37 @@ def test_staging_edges(cuda, nv):
         scale = max(np.abs(rs).max(), np.abs(rc).max())
         assert np.abs(ga[i] - rs).max() <= 1e-9 * scale, i
         assert np.abs(gb[i] - rc).max() <= 1e-9 * scale, i
+
+
+@pytest.mark.parametrize("nv", [(3, 3), (4, 6), (8, 8), (8, 9), (9, 3)])
+def test_tiny_polygons(cuda, nv):
+    """Pairs at the edges of the one-thread-per-pair kernel (3 to 8 vertices in
+    both), rings in both directions, a few pairs apart or nested, weights:
+    against the oracle's area and gradient (the tolerances of
+    test_forward_and_adjoint_match_oracle)."""
+    import parlllelrtree_b200 as prt
+
+    n = 1000
+    rng = np.random.default_rng(nv[0] * 10 + nv[1])
+    c, r = rng.random((n, 2)), np.full(n, 0.01)
+    off = rng.uniform(-0.012, 0.012, (n, 2))
+    A = dg.star_layer(n, seed=1, nv_lo=nv[0], nv_hi=nv[0], centre_xy=c, radii=r)
+    B = dg.star_layer(n, seed=2, nv_lo=nv[1], nv_hi=nv[1], centre_xy=c + off, radii=r * rng.uniform(0.1, 1.5, n))
+    A["xy"] = np.ascontiguousarray(A["xy"].reshape(n, nv[0], 2)[:, ::-1].reshape(-1, 2))
+    LA, LB = prt.Layer.from_dict(A), prt.Layer.from_dict(B)
+    idx = torch.arange(n, dtype=torch.int32, device="cuda")
+    xa, xb = LA.xy.clone().requires_grad_(True), LB.xy.clone().requires_grad_(True)
+    w = torch.from_numpy(rng.uniform(0.5, 2.0, n)).cuda()
+    area = prt.intersection_area(LA, LB, idx, idx, xa, xb)
+    (area * w).sum().backward()
+    ga, gb = xa.grad.cpu().numpy().reshape(n, -1, 2), xb.grad.cpu().numpy().reshape(n, -1, 2)
+    wn = w.cpu().numpy()
+    zero = np.zeros(1, np.int32)
+    for i in range(n):
+        s, q = rings_of(A, i), rings_of(B, i)
+        ref = oracle.result_area(oracle.gpc_clip(s, q, 1))
+        assert abs(area[i].item() - ref) <= 1e-9 * abs(ref) + 1e-22, i
+        _, rs, rc = oracle.area_grad(s, q, zero, zero)
+        scale = wn[i] * max(np.abs(rs).max(), np.abs(rc).max(), 1e-30)
+        assert np.abs(ga[i] - wn[i] * rs).max() <= 1e-9 * scale, i
+        assert np.abs(gb[i] - wn[i] * rc).max() <= 1e-9 * scale, i
