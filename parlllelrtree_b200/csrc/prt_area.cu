@@ -165,12 +165,34 @@ template <int V>
 struct BwdPoly {  // one polygon in shared memory (up to V vertices)
   float4 bb[V];                    // edge k's box (x_lo, y_lo, x_hi, y_hi), rounded outwards
   double x[V], y[V];
-  uint32_t slab[V / 32][kSlabs];   // y slabs: word c of slab s, bit k = edge 32 c + k reaches slab s
-  uint32_t xslab[V / 32][kSlabs];  // the same for x slabs
   int16_t ringv[33];                      // first vertex of ring r; ringv[rings] = the vertex count
   int8_t sgn[V];                   // orientation sign of edge k (0: ring of < 2 vertices)
   uint8_t nxt[V];                  // end vertex of edge k
   uint8_t rst[V];                  // first vertex of edge k's ring
+};
+
+// Slab masks of one polygon's edges.
+template <int V>
+struct BwdSlabs {
+  uint32_t y[V / 32][kSlabs];  // word c of slab s, bit k = edge 32 c + k reaches slab s
+  uint32_t x[V / 32][kSlabs];
+};
+
+// Crossings of a pair, chained by the edge of the searched polygon.
+constexpr int bwd_crossings(int V) { return V > kBwdMidV ? 192 : 128; }
+template <int V>
+struct BwdCrossings {
+  double u[bwd_crossings(V)];       // parameter on that edge, negative where the edge leaves the other polygon
+  uint16_t next[bwd_crossings(V)];  // 1 + the next crossing of the same edge (0: none)
+  uint32_t head[V];                 // 1 + the edge's first crossing (0: none)
+  uint32_t count;                   // crossings found (beyond the room too)
+};
+
+template <int V>
+struct BwdPair {  // one warp's shared memory
+  BwdPoly<V> poly[2];
+  BwdSlabs<V> slab;  // of the polygon that is searched
+  BwdCrossings<V> cross;
 };
 
 // coordinate -> slab: monotone non-decreasing (round-to-nearest float steps
@@ -186,6 +208,14 @@ struct SlabGrid {
 __device__ inline SlabGrid slab_grid(float lo, float hi) {
   const float span = __fsub_rn(hi, lo);
   return SlabGrid{lo, span > 1e-30f ? __fdiv_rn((float)kSlabs, span) : 0.0f};
+}
+
+// Smallest value of the warp, by one integer reduction of the order-preserving
+// image.
+__device__ __forceinline__ float warp_fmin(float v) {
+  const int i = __float_as_int(v);
+  const int k = __reduce_min_sync(kFullMask, i >= 0 ? i : i ^ 0x7fffffff);
+  return __int_as_float(k >= 0 ? k : k ^ 0x7fffffff);
 }
 
 // Stages both polygons of a pair (A from rings [ra0, ra1) of LA, B from
@@ -263,13 +293,7 @@ __device__ inline bool bwd_load_pair(const LayerDev &LA, int64_t ra0, int64_t ra
       for (int t = 0; t < V / 32; t++)
         if (rix[p][t] == r) M[p].sgn[32 * t + lane] = sg;
     }
-    for (int o = 16; o; o >>= 1) {
-      e[p].x = fminf(e[p].x, __shfl_xor_sync(kFullMask, e[p].x, o));
-      e[p].y = fminf(e[p].y, __shfl_xor_sync(kFullMask, e[p].y, o));
-      e[p].z = fmaxf(e[p].z, __shfl_xor_sync(kFullMask, e[p].z, o));
-      e[p].w = fmaxf(e[p].w, __shfl_xor_sync(kFullMask, e[p].w, o));
-    }
-    ext[p] = e[p];
+    ext[p] = make_float4(warp_fmin(e[p].x), warp_fmin(e[p].y), -warp_fmin(-e[p].z), -warp_fmin(-e[p].w));
   }
   __syncwarp();
   return true;
@@ -288,29 +312,20 @@ __device__ inline uint32_t bit_transpose(uint32_t x) {
   return x;
 }
 
-// y and x slab masks of both staged polygons (four independent transposes
-// per word).
+// y and x slab masks of a staged polygon (two independent transposes per word).
 template <int V>
-__device__ inline void bwd_slabs(BwdPoly<V> *M, const int *nv, const SlabGrid &gy, const SlabGrid &gx) {
+__device__ inline void bwd_slabs(const BwdPoly<V> &Q, int nq, const SlabGrid &gy, const SlabGrid &gx, BwdSlabs<V> &S) {
   const int lane = threadIdx.x & 31;
-  const int nw = ((nv[0] > nv[1] ? nv[0] : nv[1]) + 31) / 32;
-  for (int c = 0; c < nw; c++) {
-    uint32_t ry[2], rx[2];
-#pragma unroll
-    for (int p = 0; p < 2; p++) {
-      const int k = 32 * c + lane;
-      ry[p] = rx[p] = 0;
-      if (k < nv[p]) {
-        const float4 b = M[p].bb[k];
-        ry[p] = (kFullMask >> (31 - gy(b.w))) & (kFullMask << gy(b.y));
-        rx[p] = (kFullMask >> (31 - gx(b.z))) & (kFullMask << gx(b.x));
-      }
+  for (int c = 0; 32 * c < nq; c++) {
+    const int k = 32 * c + lane;
+    uint32_t ry = 0, rx = 0;
+    if (k < nq) {
+      const float4 b = Q.bb[k];
+      ry = (kFullMask >> (31 - gy(b.w))) & (kFullMask << gy(b.y));
+      rx = (kFullMask >> (31 - gx(b.z))) & (kFullMask << gx(b.x));
     }
-#pragma unroll
-    for (int p = 0; p < 2; p++) {
-      M[p].slab[c][lane] = bit_transpose(ry[p]);
-      M[p].xslab[c][lane] = bit_transpose(rx[p]);
-    }
+    S.y[c][lane] = bit_transpose(ry);
+    S.x[c][lane] = bit_transpose(rx);
   }
   __syncwarp();
 }
@@ -335,14 +350,14 @@ __device__ __noinline__ void bwd_edge_global(const Poly &Qg, double px, double p
 // Even-odd test of (mx, my) against staged polygon Q through the slab of
 // my: inside_evenodd's expression over the edges that can straddle my.
 template <int V>
-__device__ inline bool bwd_inside(const BwdPoly<V> &Q, int nwq, const float4 &qe, const SlabGrid &g, double mx,
-                                  double my) {
+__device__ inline bool bwd_inside(const BwdPoly<V> &Q, const BwdSlabs<V> &S, int nwq, const float4 &qe,
+                                  const SlabGrid &g, double mx, double my) {
   const float fy = __double2float_rn(my);
   if (fy < qe.y || fy > qe.w) return false;  // no edge of Q straddles my
   const int s = g(fy);
   bool in = false;
   for (int c = 0; c < nwq; c++) {
-    uint32_t bits = Q.slab[c][s];
+    uint32_t bits = S.y[c][s];
     while (bits) {
       const int k = 32 * c + __ffs(bits) - 1;
       bits &= bits - 1;
@@ -361,10 +376,10 @@ __device__ inline bool bwd_inside(const BwdPoly<V> &Q, int nwq, const float4 &qe
 // Candidate edges of Q (mask word c) for an edge whose box covers y slabs
 // [s0, s1] and x slabs [x0, x1].
 template <int V>
-__device__ inline uint32_t bwd_cands(const BwdPoly<V> &Q, int c, int s0, int s1, int x0, int x1) {
+__device__ inline uint32_t bwd_cands(const BwdSlabs<V> &S, int c, int s0, int s1, int x0, int x1) {
   uint32_t ybits = 0, xbits = 0;
-  for (int s = s0; s <= s1; s++) ybits |= Q.slab[c][s];
-  for (int s = x0; s <= x1; s++) xbits |= Q.xslab[c][s];
+  for (int s = s0; s <= s1; s++) ybits |= S.y[c][s];
+  for (int s = x0; s <= x1; s++) xbits |= S.x[c][s];
   return ybits & xbits;
 }
 
@@ -372,7 +387,7 @@ __device__ inline uint32_t bwd_cands(const BwdPoly<V> &Q, int c, int s0, int s1,
 // crossing by next_crossing's test (kBwdMaxT at most, else the global-memory
 // path), sorted and deduplicated, and every interval by its midpoint.
 template <int V>
-__device__ __noinline__ void bwd_edge_exact(const BwdPoly<V> &Q, int nwq, const float4 &qe, const SlabGrid &g,
+__device__ __noinline__ void bwd_edge_exact(const BwdPoly<V> &Q, const BwdSlabs<V> &S, int nwq, const float4 &qe, const SlabGrid &g,
                                             const SlabGrid &gx, const float4 &pb, double px, double py, double rx,
                                             double ry, const Poly &Qg, double *it_out, double *i1_out) {
   double ts[kBwdMaxT];
@@ -380,7 +395,7 @@ __device__ __noinline__ void bwd_edge_exact(const BwdPoly<V> &Q, int nwq, const 
   bool over = false;
   const int s0 = g(pb.y), s1 = g(pb.w), x0 = gx(pb.x), x1 = gx(pb.z);
   for (int c = 0; c < nwq; c++) {
-    uint32_t bits = bwd_cands(Q, c, s0, s1, x0, x1);
+    uint32_t bits = bwd_cands(S, c, s0, s1, x0, x1);
     while (bits) {
       const int k = 32 * c + __ffs(bits) - 1;
       bits &= bits - 1;
@@ -419,7 +434,7 @@ __device__ __noinline__ void bwd_edge_exact(const BwdPoly<V> &Q, int nwq, const 
     for (int a = 0; a <= m; a++) {
       const double t0 = a == 0 ? 0.0 : ts[a - 1], t1 = a < m ? ts[a] : 1.0;
       const double tm = 0.5 * (t0 + t1);
-      if (bwd_inside(Q, nwq, qe, g, px + tm * rx, py + tm * ry)) {
+      if (bwd_inside(Q, S, nwq, qe, g, px + tm * rx, py + tm * ry)) {
         const double aa = 0.5 * (t1 * t1 - t0 * t0);
         it += aa;
         i1 += (t1 - t0) - aa;
@@ -430,9 +445,12 @@ __device__ __noinline__ void bwd_edge_exact(const BwdPoly<V> &Q, int nwq, const 
   *i1_out = i1;
 }
 
-// pieces() for both polygons of a staged pair: lane edge e < na is edge e of
-// A (against B), e >= na edge e - na of B (against A); rounds of 32 edges.
-// ext[0], ext[1]: the float extents of A and B.
+// pieces() for both polygons of a staged pair, in rounds of 32 edges (one per
+// lane): first the edges of the polygon with fewer, P, which search the other,
+// Q, for crossings; then Q's edges, which find theirs in chains that the
+// search left: a crossing of p + t r and a + u s has t = tn / den and u = un /
+// den from the same three products, whichever edge looks, so each is computed
+// once.  ext[0], ext[1]: the float extents of A and B.
 //
 // What is inside: by the midpoint of every interval between crossings (the
 // definition, bwd_edge_exact), or, while the pair's crossings are all clean,
@@ -473,21 +491,29 @@ struct AreaSum {
 // (the caller then clips the pair with GPC); in gradient mode it always runs
 // to the end, by the definition from the first unclean crossing on.
 template <bool kArea, int V>
-__device__ inline bool pair_boundary(const BwdPoly<V> *M, const float4 *ext, int na, int nb, const SlabGrid &g,
+__device__ inline bool pair_boundary(BwdPair<V> &W, const float4 *ext, int na, int nb, const SlabGrid &g,
                                      const SlabGrid &gx, double w, double *ga, double *gb, int64_t va, int64_t vb,
                                      const Poly &Ag, const Poly &Bg, double ox, double oy, AreaSum *acc) {
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
+  BwdCrossings<V> &X = W.cross;
+  const int searcher = nb < na ? 1 : 0;
+  int masks = 1 - searcher;  // the polygon W.slab belongs to
+  bwd_slabs(W.poly[masks], masks ? nb : na, g, gx, W.slab);
+  for (int k = lane; k < (masks ? nb : na); k += 32) X.head[k] = 0;
+  if (lane == 0) X.count = 0;
+  __syncwarp();
   bool exact = false;  // by the definition from here on (sticky)
-  bool carry = false;  // inside state after the last edge of the previous round
   double area2 = 0.0, err = 0.0;
-  for (int e0 = 0; e0 < na + nb; e0 += 32) {
-    const int e = e0 + lane;
-    const int side = e < na ? 0 : 1;
-    const int i = side ? e - na : e;
-    const BwdPoly<V> &P = M[side], &Q = M[1 - side];
-    const int nwq = ((side ? na : nb) + 31) >> 5;
-    const bool valid = e < na + nb && P.sgn[i] != 0;
+  for (int half = 0; half < 2; half++) {
+  const int side = half ? 1 - searcher : searcher;
+  const BwdPoly<V> &P = W.poly[side], &Q = W.poly[1 - side];
+  const int np = side ? nb : na, nq = side ? na : nb;
+  const int nwq = (nq + 31) >> 5;
+  bool carry = false;  // inside state after the last edge of the previous round
+  for (int e0 = 0; e0 < np; e0 += 32) {
+    const int i = e0 + lane;
+    const bool valid = i < np && P.sgn[i] != 0;
     const int j = valid ? P.nxt[i] : 0;
     double px = 0.0, py = 0.0, qx = 0.0, qy = 0.0;
     float4 pb = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -503,63 +529,82 @@ __device__ inline bool pair_boundary(const BwdPoly<V> *M, const float4 *ext, int
     int c0 = 0;                 // and of the signs
     int m = 0;                  // their number
     double tfirst = 1.0;        // the first one
-    bool unclean = false;
-    if (valid && !exact) {
-      const double rl = fabs(rx) + fabs(ry);
-      const int s0 = g(pb.y), s1 = g(pb.w), x0 = gx(pb.x), x1 = gx(pb.z);
-      for (int c = 0; c < nwq; c++) {
-        uint32_t bits = bwd_cands(Q, c, s0, s1, x0, x1);
-        while (bits) {
-          const int k = 32 * c + __ffs(bits) - 1;
-          bits &= bits - 1;
-          const float4 b = Q.bb[k];
-          if (b.w < pb.y || b.y > pb.w || b.z < pb.x || b.x > pb.z) continue;
-          const int l = Q.nxt[k];
-          const double ax = Q.x[k], ay = Q.y[k], bx = Q.x[l], by = Q.y[l];
-          const double sx = bx - ax, sy = by - ay;
-          const double den = rx * sy - ry * sx;
-          const double apx = ax - px, apy = ay - py;
-          const double tn = apx * sy - apy * sx;
-          if (den == 0.0) {
-            unclean |= tn == 0.0;  // collinear
-            continue;
-          }
-          const double un = apx * ry - apy * rx;
-          // t = tn / den and u = un / den, with the signs of den folded in
-          const double d = fabs(den), tol = 1e-9 * d;
-          const double tt = den > 0.0 ? tn : -tn, uu = den > 0.0 ? un : -un;
-          if (tt < -tol || tt > d + tol || uu < -tol || uu > d + tol) continue;  // next_crossing rejects it
-          if (!(tt > tol && tt < d - tol && uu > tol && uu < d - tol && d > 1e-6 * rl * (fabs(sx) + fabs(sy)))) {
-            unclean = true;
-            continue;
-          }
-          if constexpr (kArea) {
+    if (half == 0 && !exact) {
+      bool unclean = false;
+      if (valid) {
+        const bool material_left = P.sgn[i] > 0;
+        const double rl = fabs(rx) + fabs(ry);
+        const int s0 = g(pb.y), s1 = g(pb.w), x0 = gx(pb.x), x1 = gx(pb.z);
+        for (int c = 0; c < nwq; c++) {
+          uint32_t bits = bwd_cands(W.slab, c, s0, s1, x0, x1);
+          while (bits) {
+            const int k = 32 * c + __ffs(bits) - 1;
+            bits &= bits - 1;
+            const float4 b = Q.bb[k];
+            if (b.w < pb.y || b.y > pb.w || b.z < pb.x || b.x > pb.z) continue;
+            const int l = Q.nxt[k];
+            const double ax = Q.x[k], ay = Q.y[k], bx = Q.x[l], by = Q.y[l];
+            const double sx = bx - ax, sy = by - ay;
+            const double den = rx * sy - ry * sx;
+            const double apx = ax - px, apy = ay - py;
+            const double tn = apx * sy - apy * sx;
+            const double un = apx * ry - apy * rx;
+            if (den == 0.0) {
+              unclean |= tn == 0.0 || un == 0.0;  // collinear
+              continue;
+            }
+            // t = tn / den and u = un / den, with the signs of den folded in
+            const double d = fabs(den), tol = 1e-9 * d;
+            const double tt = den > 0.0 ? tn : -tn, uu = den > 0.0 ? un : -un;
+            if (tt < -tol || tt > d + tol || uu < -tol || uu > d + tol) continue;  // next_crossing rejects it
             const double sl = fabs(sx) + fabs(sy);
-            err += (rl + sl) * rl * sl / d;
+            if (!(tt > tol && tt < d - tol && uu > tol && uu < d - tol && d > 1e-6 * rl * sl)) {
+              unclean = true;
+              continue;
+            }
+            if constexpr (kArea) err += 2.0 * ((rl + sl) * rl * sl / d);  // seen from both edges
+            const double t = tn / den, u = un / den;  // next_crossing's t from either edge
+            // den > 0: P's edge goes from the left of Q's edge to its right,
+            // out of Q where Q's material is on the left, and Q's edge the
+            // other way
+            const bool leaves = (den > 0.0) == (Q.sgn[k] > 0);
+            const double st = leaves ? -t : t;
+            c0 += leaves ? -1 : 1;
+            c1 += st;
+            c2 += st * t;
+            tfirst = fmin(tfirst, t);
+            m++;
+            const uint32_t x = atomicAdd(&X.count, 1u);
+            if (x < (uint32_t)bwd_crossings(V)) {
+              X.u[x] = (den < 0.0) == material_left ? -u : u;
+              X.next[x] = (uint16_t)atomicExch(&X.head[k], x + 1);
+            } else {
+              unclean = true;
+            }
           }
-          const double t = tn / den;  // next_crossing's t
-          // den > 0: the edge goes from the left of Q's edge to its right,
-          // out of Q where Q's material is on the left
-          const bool leaves = (den > 0.0) == (Q.sgn[k] > 0);
-          const double st = leaves ? -t : t;
-          c0 += leaves ? -1 : 1;
-          c1 += st;
-          c2 += st * t;
-          tfirst = fmin(tfirst, t);
-          m++;
         }
       }
-    }
-    exact = __any_sync(kFullMask, unclean) || exact;
-    if constexpr (kArea) {
-      if (exact) return false;
+      exact = __any_sync(kFullMask, unclean);
+      if constexpr (kArea) {
+        if (exact) return false;
+      }
+    } else if (half == 1 && !exact && valid) {
+      for (uint32_t x = X.head[i]; x;) {
+        const double st = X.u[x - 1], t = fabs(st);
+        c0 += st < 0.0 ? -1 : 1;
+        c1 += st;
+        c2 += st * t;
+        tfirst = fmin(tfirst, t);
+        m++;
+        x = X.next[x - 1];
+      }
     }
     double it = 0.0, i1 = 0.0;
     if (!exact) {
-      const int rs = valid ? (side ? na : 0) + P.rst[i] : e;  // this edge's ring starts at edge rs
+      const int rs = valid ? P.rst[i] : i;  // this edge's ring starts at edge rs
       // the first interval of each ring starting in this round, by its
       // midpoint: the whole warp tests it against all edges of the other polygon
-      const bool rstart = valid && rs == e;
+      const bool rstart = valid && rs == i;
       double mx0 = 0.0, my0 = 0.0;
       if (rstart) {
         const double tm = 0.5 * tfirst;
@@ -570,15 +615,12 @@ __device__ inline bool pair_boundary(const BwdPoly<V> *M, const float4 *ext, int
       for (unsigned q = __ballot_sync(kFullMask, rstart); q; q &= q - 1) {
         const int L = __ffs(q) - 1;
         const double mxl = __shfl_sync(kFullMask, mx0, L), myl = __shfl_sync(kFullMask, my0, L);
-        const int sl = e0 + L < na ? 0 : 1;
-        const BwdPoly<V> &QL = M[1 - sl];
-        const int nql = sl ? na : nb;
         bool in = false;
-        for (int k = lane; k < nql; k += 32) {
-          const int l = QL.nxt[k];
-          const double ay = QL.y[k], by = QL.y[l];
+        for (int k = lane; k < nq; k += 32) {
+          const int l = Q.nxt[k];
+          const double ay = Q.y[k], by = Q.y[l];
           if ((ay > myl) != (by > myl)) {
-            const double ax = QL.x[k], bx = QL.x[l];
+            const double ax = Q.x[k], bx = Q.x[l];
             const double xi = ax + (myl - ay) * (bx - ax) / (by - ay);
             if (mxl < xi) in = !in;
           }
@@ -603,8 +645,17 @@ __device__ inline bool pair_boundary(const BwdPoly<V> *M, const float4 *ext, int
         i1 = (s1 - c1) - it;
       }
     }
-    if (exact && valid)
-      bwd_edge_exact(Q, nwq, ext[1 - side], g, gx, pb, px, py, rx, ry, side ? Ag : Bg, &it, &i1);
+    if constexpr (!kArea) {
+      if (exact) {
+        if (masks != 1 - side) {
+          masks = 1 - side;
+          __syncwarp();
+          bwd_slabs(Q, nq, g, gx, W.slab);
+        }
+        if (valid)
+          bwd_edge_exact(Q, W.slab, nwq, ext[1 - side], g, gx, pb, px, py, rx, ry, side ? Ag : Bg, &it, &i1);
+      }
+    }
     if constexpr (kArea) {
       // it + i1 = sum (t1 - t0) over the inside intervals
       if (valid) area2 += P.sgn[i] * (it + i1) * ((px - ox) * ry - (py - oy) * rx);
@@ -622,8 +673,8 @@ __device__ inline bool pair_boundary(const BwdPoly<V> *M, const float4 *ext, int
       gxi = nx * i1;
       gyi = ny * i1;
     }
-    const int key = valid ? (side << 8) | i : -1;           // this edge's start vertex
-    const int kend = valid ? (side << 8) | j : -2;          // its end vertex
+    const int key = valid ? i : -1;                         // this edge's start vertex
+    const int kend = valid ? j : -2;                        // its end vertex
     const int knext = __shfl_down_sync(kFullMask, key, 1);  // start vertex of the next lane's edge
     const int kprev = __shfl_up_sync(kFullMask, kend, 1);   // end vertex of the previous lane's edge
     const double hx = __shfl_down_sync(kFullMask, gxi, 1), hy = __shfl_down_sync(kFullMask, gyi, 1);
@@ -643,6 +694,8 @@ __device__ inline bool pair_boundary(const BwdPoly<V> *M, const float4 *ext, int
       atomicAdd(&gr[2 * (vbase + i)], gxi);
       atomicAdd(&gr[2 * (vbase + i) + 1], gyi);
     }
+  }
+  __syncwarp();  // the crossings of the first half, for the second
   }
   if constexpr (kArea) {
     acc->area = area2;
@@ -683,8 +736,9 @@ template <int V>
 __global__ void __launch_bounds__(32 * bwd_warps(V), V > kBwdMidV ? 5 : 4) area_bwd_kernel(
     const int32_t *__restrict__ pa, const int32_t *__restrict__ pb, int64_t n, LayerDev base, LayerDev over,
     const double *__restrict__ upstream, double *grad_base, double *grad_over, PairList PL) {
-  __shared__ BwdPoly<V> sm[bwd_warps(V)][2];
-  BwdPoly<V> *M = sm[threadIdx.x >> 5];
+  __shared__ BwdPair<V> sm[bwd_warps(V)];
+  BwdPair<V> &W = sm[threadIdx.x >> 5];
+  BwdPoly<V> *M = W.poly;
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const int64_t items = list_items(PL, n);
@@ -737,10 +791,9 @@ __global__ void __launch_bounds__(32 * bwd_warps(V), V > kBwdMidV ? 5 : 4) area_
         const float y0 = fmaxf(ext[0].y, ext[1].y), y1 = fminf(ext[0].w, ext[1].w);
         if (!(x0 > x1 || y0 > y1)) {
           const SlabGrid gy = slab_grid(y0, y1), gx = slab_grid(x0, x1);
-          bwd_slabs(M, nv, gy, gx);
           Poly A{base.ring_vert, base.ring_hole, base.xy, rr[0], rr[1]};
           Poly B{over.ring_vert, over.ring_hole, over.xy, rr[2], rr[3]};
-          pair_boundary<false>(M, ext, nv[0], nv[1], gy, gx, w, grad_base, grad_over, vb[0], vb[1], A, B, 0.0,
+          pair_boundary<false>(W, ext, nv[0], nv[1], gy, gx, w, grad_base, grad_over, vb[0], vb[1], A, B, 0.0,
                                0.0, nullptr);
         }
       } else if (PL.defer) {
@@ -1087,8 +1140,9 @@ template <int V>
 __global__ void __launch_bounds__(32 * bwd_warps(V), V <= kBwdSmallV || V > kBwdMidV ? 5 : 4) area_fwd_kernel(
     const int32_t *__restrict__ pa, const int32_t *__restrict__ pb, int64_t n, LayerDev base, LayerDev over,
     double *__restrict__ area, int32_t *__restrict__ fb, unsigned long long *__restrict__ fb_count, PairList PL) {
-  __shared__ BwdPoly<V> sm[bwd_warps(V)][2];
-  BwdPoly<V> *M = sm[threadIdx.x >> 5];
+  __shared__ BwdPair<V> sm[bwd_warps(V)];
+  BwdPair<V> &W = sm[threadIdx.x >> 5];
+  BwdPoly<V> *M = W.poly;
   const int lane = threadIdx.x & 31;
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -1128,12 +1182,11 @@ __global__ void __launch_bounds__(32 * bwd_warps(V), V <= kBwdSmallV || V > kBwd
       continue;
     }
     const SlabGrid gy = slab_grid(y0, y1), gx = slab_grid(x0, x1);
-    bwd_slabs(M, nv, gy, gx);
     Poly A{base.ring_vert, base.ring_hole, base.xy, ra0, ra1};
     Poly B{over.ring_vert, over.ring_hole, over.xy, rb0, rb1};
     AreaSum acc{0.0, 0.0};
     const double ox = M[0].x[0], oy = M[0].y[0];  // the pair-local origin
-    const bool ok = pair_boundary<true>(M, ext, nv[0], nv[1], gy, gx, 1.0, nullptr, nullptr, vb[0], vb[1], A, B,
+    const bool ok = pair_boundary<true>(W, ext, nv[0], nv[1], gy, gx, 1.0, nullptr, nullptr, vb[0], vb[1], A, B,
                                         ox, oy, &acc);
     if (ok) {
       double a2 = acc.area, er = acc.err;
