@@ -23,6 +23,7 @@
 #include "prt_gpc.cuh"
 #include "prt_internal.cuh"
 #include "prt_overlay.cuh"
+#include "prt_trace.cuh"
 #include "prt_wgpc.cuh"
 
 namespace prt {
@@ -153,6 +154,14 @@ __device__ __noinline__ void process_pair_warp(const PairSrc &S, const ClipOut &
 
 namespace {
 
+// Pairs per bin that tracing left (nullptr: nothing was traced), and the launch's
+// condition: their warps, one pair per thread, in [min_warps, max_warps).
+struct TraceRest {
+  const unsigned long long *left;
+  unsigned thread_bins;
+  int64_t min_warps, max_warps;
+};
+
 // Adds v over the block to *total (one atomic per warp).
 __device__ __forceinline__ void add_total(unsigned long long v, unsigned long long *total) {
   for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -192,22 +201,33 @@ __global__ void __launch_bounds__(128) clip_plain_kernel(PairSrc S, ClipOut O, c
 // shared memory holds the warp clipper's active-edge slots.
 // The body of the persistent launch; kWarp = false compiles the warp clipper
 // out (every bin in thread mode).
+// rest: the bins hold the pairs that the tracing kernels left, and the launch
+// runs only if their number is what it was planned for.
 template <bool kWarp>
 __device__ __forceinline__ void lpt_body(const PairSrc &S, const ClipOut &O, const uint32_t *__restrict__ order,
                                          const BinPlan &plan, unsigned long long *tickets, unsigned char *arena,
-                                         int scale, const int64_t *__restrict__ dyn_ranges) {
+                                         int scale, const int64_t *__restrict__ dyn_ranges, const TraceRest &rest) {
   __shared__ int64_t s_begin[PRT_MAX_BINS], s_end[PRT_MAX_BINS];
   __shared__ int32_t s_mode[PRT_MAX_BINS];
   const int lane = threadIdx.x & 31;
   const int64_t w = blockIdx.x;
   const int nbins = plan.nbins;
+  int64_t thread_warps = 0;
   if (lane < nbins) {
-    // bin ranges from the plan, or computed on the device (graph mode)
+    // bin ranges from the plan, or computed on the device (graph mode, and what
+    // the tracing kernels left)
     s_begin[lane] = dyn_ranges ? dyn_ranges[2 * lane] : plan.begin[lane];
-    s_end[lane] = dyn_ranges ? dyn_ranges[2 * lane + 1] : plan.end[lane];
+    s_end[lane] = dyn_ranges ? dyn_ranges[2 * lane + 1]
+                  : rest.left ? plan.begin[lane] + (int64_t)rest.left[lane]
+                              : plan.end[lane];
     s_mode[lane] = plan.warp_mode[lane];
+    if (rest.left && (rest.thread_bins >> lane & 1)) thread_warps = ((int64_t)rest.left[lane] + 31) / 32;
   }
   __syncwarp();
+  if (rest.left) {
+    for (int o = 16; o; o >>= 1) thread_warps += __shfl_xor_sync(0xffffffffu, thread_warps, o);
+    if (thread_warps < rest.min_warps || thread_warps >= rest.max_warps) return;
+  }
   gpc::WAet W = gpc::waet_carve(plan.wcap);
   int g = 0;
   while (g + 1 < nbins && w >= plan.warp0[g + 1]) g++;
@@ -247,8 +267,8 @@ __device__ __forceinline__ void lpt_body(const PairSrc &S, const ClipOut &O, con
 __global__ void __launch_bounds__(32, kLptWarpsPerSM)
     clip_lpt_kernel(PairSrc S, ClipOut O, const uint32_t *__restrict__ order, BinPlan plan,
                     unsigned long long *tickets, unsigned char *arena, int scale,
-                    const int64_t *__restrict__ dyn_ranges) {
-  lpt_body<true>(S, O, order, plan, tickets, arena, scale, dyn_ranges);
+                    const int64_t *__restrict__ dyn_ranges, TraceRest rest) {
+  lpt_body<true>(S, O, order, plan, tickets, arena, scale, dyn_ranges, rest);
 }
 
 // The same launch when no bin with pairs is in warp mode: without the warp
@@ -256,8 +276,64 @@ __global__ void __launch_bounds__(32, kLptWarpsPerSM)
 // which hide more of its list-walking latency.
 __global__ void __launch_bounds__(32, kLptThreadWarpsPerSM)
     clip_lpt_thread_kernel(PairSrc S, ClipOut O, const uint32_t *__restrict__ order, BinPlan plan,
-                           unsigned long long *tickets, unsigned char *arena, int scale) {
-  lpt_body<false>(S, O, order, plan, tickets, arena, scale, nullptr);
+                           unsigned long long *tickets, unsigned char *arena, int scale, TraceRest rest) {
+  lpt_body<false>(S, O, order, plan, tickets, arena, scale, nullptr, rest);
+}
+
+// Intersections by tracing (prt_trace.cuh): one block per pair of the sorted
+// positions [begin, end), largest pairs first, from one ticket.  A pair that is
+// not traced goes to its bin's part of left_order for the launch above.
+template <typename C>
+__global__ void __launch_bounds__(C::NT, C::kBlocks)
+    trace_kernel(PairSrc S, ClipOut O, const uint32_t *__restrict__ order, int64_t begin, int64_t end, BinPlan plan,
+                 unsigned long long *ticket, uint32_t *__restrict__ left_order, unsigned long long *left) {
+  extern __shared__ __align__(16) unsigned char trace_smem[];
+  trace::Smem<C> &M = *reinterpret_cast<trace::Smem<C> *>(trace_smem);
+  trace::Sink K;
+  K.status = O.status;
+  K.pair_cstart = O.pair_cstart;
+  K.pair_ncont = O.pair_ncont;
+  K.cont_vstart = O.cont_vstart;
+  K.cont_nverts = O.cont_nverts;
+  K.cont_hole = O.cont_hole;
+  K.xy = O.xy;
+  K.pool = O.pool;
+  K.cap_c = O.cap_c;
+  K.cap_v = O.cap_v;
+  K.area = O.area;
+  for (;;) {
+    trace::bsync<C::NT>();
+    if (threadIdx.x == 0) M.ticket = atomicAdd(ticket, 1ull);
+    trace::bsync<C::NT>();
+    const int64_t k = begin + (int64_t)M.ticket;
+    if (k >= end) break;
+    const int64_t i = (int64_t)order[k];
+    if (i >= plan.n_pairs) continue;
+    gpc::PolyView a, b;
+    int64_t nv = 0;
+    if (!resolve(S, i, a, b, nv)) {
+      if (threadIdx.x == 0) invalid_pair(O, i);
+      continue;
+    }
+    if (trace::trace_pair<C>(M, a, b, K, i, kPairPool) == trace::kLeft && threadIdx.x == 0) {
+      int g = 0;
+      while (g + 1 < plan.nbins && k >= plan.end[g]) g++;
+      left_order[plan.begin[g] + (int64_t)atomicAdd(&left[g], 1ull)] = (uint32_t)i;
+    }
+  }
+}
+
+template <typename C>
+int launch_trace(const PairSrc &S, const ClipOut &O, const uint32_t *order, int64_t begin, int64_t end,
+                 const BinPlan &plan, unsigned long long *ticket, uint32_t *left_order, unsigned long long *left,
+                 cudaStream_t s) {
+  if (begin >= end) return PRT_OK;
+  const size_t smem = sizeof(trace::Smem<C>);
+  PRT_CUDA(cudaFuncSetAttribute(trace_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int64_t grid = std::min<int64_t>(end - begin, (int64_t)kSMs * C::kBlocks);
+  trace_kernel<C><<<(unsigned)grid, C::NT, smem, s>>>(S, O, order, begin, end, plan, ticket, left_order, left);
+  PRT_CUDA(cudaGetLastError());
+  return PRT_OK;
 }
 
 // Sort keys of the items' pairs, larger vertex counts first, and the vertices
@@ -276,8 +352,10 @@ __global__ void size_key_kernel(PairSrc S, int64_t n, const int64_t *__restrict_
   add_total(sum, total);
 }
 
+// The schedule's bins, then the tracing kernels' classes.
+constexpr int kCuts = PRT_MAX_BINS + trace::kClasses;
 struct BinThresholds {
-  int64_t thr[PRT_MAX_BINS];
+  int64_t thr[kCuts];
 };
 
 // bounds[b] = first sorted position whose vertex count is <= thr[b]
@@ -614,19 +692,26 @@ static int run_batched(OverlayState &st, const int64_t *d_idx, int64_t count, in
     unsigned err;
     int sel;
     unsigned long long total_nv;
-    int64_t bnd[PRT_MAX_BINS], mx[PRT_MAX_BINS];
+    int64_t bnd[kCuts], mx[kCuts];
     unsigned long long tickets[PRT_MAX_BINS + 1];  // bins + fallbacks
+    unsigned long long rest_tickets[PRT_MAX_BINS + 1], trace_tickets[trace::kClasses];
+    unsigned long long left[PRT_MAX_BINS];  // pairs of each bin that were not traced
   } h;
   static_assert(sizeof(Head) <= 512, "head block");
+  const bool trace_pairs = st.S.op == PRT_GPC_INT;
   unsigned char *scr = nullptr;
-  int rc = dmalloc(reinterpret_cast<void **>(&scr), 512 + 16 * n + 4 * n, s);
+  int rc = dmalloc(reinterpret_cast<void **>(&scr), 512 + 20 * n + (trace_pairs ? 4 * n : 0), s);
   if (rc) return rc;
   Head *d = reinterpret_cast<Head *>(scr);
   uint32_t *k0 = reinterpret_cast<uint32_t *>(scr + 512);
-  uint32_t *k1 = k0 + n, *v0 = k1 + n, *v1 = v0 + n, *order = v1 + n;
+  uint32_t *k1 = k0 + n, *v0 = k1 + n, *v1 = v0 + n, *order = v1 + n, *left_order = order + n;
   cudaMemsetAsync(scr, 0, 512, s);
   BinThresholds T;
-  for (int b = 0; b < PRT_MAX_BINS; b++) T.thr[b] = b < nb ? sc.bin_thresholds[b] : 0;
+  for (int b = 0; b < nb; b++) T.thr[b] = sc.bin_thresholds[b];
+  const int64_t cls_verts[trace::kClasses] = {trace::Class3::kVerts, trace::Class2::kVerts, trace::Class1::kVerts,
+                                              trace::Class0::kVerts};
+  for (int c = 0; c < trace::kClasses; c++) T.thr[nb + c] = cls_verts[c];
+  const int cuts = nb + (trace_pairs ? trace::kClasses : 0);
   const int g = grid_for(n, 256, 16);
   {
     PRT_PROF("size_key", s);
@@ -641,7 +726,7 @@ static int run_batched(OverlayState &st, const int64_t *d_idx, int64_t count, in
     }
     {
       PRT_PROF("bin_bounds", s);
-      bin_bounds_kernel<<<1, 32, 0, s>>>(k0, k1, &d->sel, n, T, nb, d->bnd, d->mx);
+      bin_bounds_kernel<<<1, 32, 0, s>>>(k0, k1, &d->sel, n, T, cuts, d->bnd, d->mx);
     }
     cudaError_t e = cudaMemcpyAsync(&h, d, sizeof h, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -658,39 +743,72 @@ static int run_batched(OverlayState &st, const int64_t *d_idx, int64_t count, in
   }
   // bin b covers sorted positions [bnd[b], bnd[b+1]) (bnd[nbins] = n)
   hb[nb] = n;
-  BinPlan plan;
+  BinPlan plan, few;
   int64_t counts[PRT_MAX_BINS];
   for (int b = 0; b < nb; b++) counts[b] = hb[b + 1] - hb[b];
   // Too few pairs to keep the GPU busy one per thread (under half a wave of
   // the thread-only launch, e.g. the 2 x 10,000-star overlay's ~21k pairs in
   // ~650 warps): clip every pair with a whole warp instead, so there are as
   // many warps as pairs.  Both clippers give the same output.
-  prt_schedule run_sc = sc;
-  {
-    int64_t thread_warps = 0;
-    for (int b = 0; b < nb; b++)
-      if (!sc.bin_warp_mode[b]) thread_warps += (counts[b] + 31) / 32;
-    if (thread_warps > 0 && thread_warps < (int64_t)kSMs * kLptThreadWarpsPerSM / 2)
-      for (int b = 0; b < nb; b++) run_sc.bin_warp_mode[b] = 1;
+  constexpr int64_t kFewWarps = (int64_t)kSMs * kLptThreadWarpsPerSM / 2;
+  prt_schedule run_sc = sc, few_sc = sc;
+  unsigned thread_bins = 0;
+  int64_t thread_warps = 0;
+  for (int b = 0; b < nb; b++) {
+    if (!sc.bin_warp_mode[b]) {
+      thread_bins |= 1u << b;
+      thread_warps += (counts[b] + 31) / 32;
+    }
+    few_sc.bin_warp_mode[b] = 1;
   }
-  size_t smem = 0;
+  if (thread_warps > 0 && thread_warps < kFewWarps) run_sc = few_sc;
+  size_t smem = 0, few_smem = 0;
   size_t bytes = plan_bins(run_sc, counts, hm, kArenaBudgetMost, plan, &smem, scale, true);
   if (bytes > kArenaBudgetLeast) bytes = plan_bins(run_sc, counts, hm, arena_budget(), plan, &smem, scale, true);
-  plan.n_pairs = st.n;
-  for (int b = 0; b < nb; b++) {
-    plan.begin[b] = hb[b];
-    plan.end[b] = hb[b + 1];
+  // What tracing leaves may be few pairs out of many: that is known on the device
+  // alone, so both launches are made and one of them ends at once.
+  const bool both = trace_pairs && thread_warps >= kFewWarps;
+  if (both) bytes = std::max(bytes, plan_bins(few_sc, counts, hm, bytes, few, &few_smem, scale, true));
+  for (int p = 0; p < (both ? 2 : 1); p++) {
+    BinPlan &pl = p ? few : plan;
+    pl.n_pairs = st.n;
+    for (int b = 0; b < nb; b++) {
+      pl.begin[b] = hb[b];
+      pl.end[b] = hb[b + 1];
+    }
   }
   const int64_t warps = plan.warp0[nb];
   unsigned char *arena = nullptr;
-  if (!rc) rc = prepare_lpt_launch(smem);
+  if (!rc) rc = prepare_lpt_launch(std::max(smem, few_smem));
   if (!rc && warps > 0) rc = dmalloc(reinterpret_cast<void **>(&arena), bytes, s);
+  TraceRest rest = {nullptr, 0, 0, 0};
+  if (!rc && warps > 0 && trace_pairs) {
+    PRT_PROF("trace", s);
+    const int64_t *cut = h.bnd + nb;
+    rc = launch_trace<trace::Class3>(st.S, st.O, order, 0, cut[1], plan, &d->trace_tickets[0], left_order, d->left, s);
+    if (!rc)
+      rc = launch_trace<trace::Class2>(st.S, st.O, order, cut[1], cut[2], plan, &d->trace_tickets[1], left_order,
+                                       d->left, s);
+    if (!rc)
+      rc = launch_trace<trace::Class1>(st.S, st.O, order, cut[2], cut[3], plan, &d->trace_tickets[2], left_order,
+                                       d->left, s);
+    if (!rc)
+      rc = launch_trace<trace::Class0>(st.S, st.O, order, cut[3], n, plan, &d->trace_tickets[3], left_order, d->left, s);
+    rest = {d->left, thread_bins, both ? kFewWarps : 0, INT64_MAX};
+  }
   if (!rc && warps > 0) {
     PRT_PROF("clip_batched", s);
+    const uint32_t *todo = trace_pairs ? left_order : order;
     if (plan.thread_only)
-      clip_lpt_thread_kernel<<<(unsigned)warps, 32, 0, s>>>(st.S, st.O, order, plan, d->tickets, arena, scale);
+      clip_lpt_thread_kernel<<<(unsigned)warps, 32, 0, s>>>(st.S, st.O, todo, plan, d->tickets, arena, scale, rest);
     else
-      clip_lpt_kernel<<<(unsigned)warps, 32, smem, s>>>(st.S, st.O, order, plan, d->tickets, arena, scale, nullptr);
+      clip_lpt_kernel<<<(unsigned)warps, 32, smem, s>>>(st.S, st.O, todo, plan, d->tickets, arena, scale, nullptr, rest);
+    if (both) {
+      rest.min_warps = 0;
+      rest.max_warps = kFewWarps;
+      clip_lpt_kernel<<<(unsigned)few.warp0[nb], 32, few_smem, s>>>(st.S, st.O, todo, few, d->rest_tickets, arena, scale,
+                                                                   nullptr, rest);
+    }
   }
   if (!rc) {
     cudaError_t e = cudaGetLastError();
@@ -881,7 +999,8 @@ int overlay_graph_enqueue(const PairSrc &S, const unsigned long long *d_npairs, 
   const int64_t warps = G.plan.warp0[G.plan.nbins];
   if (warps > 0) {
     PRT_PROF("clip_batched", s);
-    clip_lpt_kernel<<<(unsigned)warps, 32, G.smem, s>>>(S, O, G.order, G.plan, G.tickets, G.arena, 1, G.ranges);
+    clip_lpt_kernel<<<(unsigned)warps, 32, G.smem, s>>>(S, O, G.order, G.plan, G.tickets, G.arena, 1, G.ranges,
+                                                        TraceRest{nullptr, 0, 0, 0});
   }
   {
     PRT_PROF("result_totals", s);

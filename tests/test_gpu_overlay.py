@@ -167,3 +167,109 @@ def test_results_area_matches_oracle(cuda):
         # same contours, same centred shoelace in the same order as the oracle
         ref = oracle.result_area(oracle.gpc_clip(rings_of(A, i), rings_of(B, j), 1))
         assert abs(area[k] - ref) <= 1e-12 * abs(ref) + 1e-24
+
+
+def layer_of(polys):
+    rings = [np.asarray(r, dtype=np.float64).reshape(-1, 2) for p in polys for r in p]
+    return {"poly_ring": np.cumsum([0] + [len(p) for p in polys]).astype(np.int64),
+            "ring_vert": np.cumsum([0] + [len(r) for r in rings]).astype(np.int64),
+            "ring_hole": np.zeros(len(rings), dtype=np.int32),
+            "xy": np.concatenate(rings)}
+
+
+def clip_all(A, B, n):
+    import parlllelrtree_b200 as prt
+
+    ids = np.arange(n, dtype=np.int32)
+    pairs = torch.from_numpy(np.stack([ids, ids], axis=1)).cuda()
+    return prt.overlay(pairs, prt.Layer.from_dict(A), prt.Layer.from_dict(B), op="int").contours()
+
+
+@pytest.mark.parametrize("na,nb,hole_frac", [
+    (3, 3, 0.0), (4, 5, 0.0), (16, 15, 0.9), (17, 16, 0.0), (63, 64, 0.0), (64, 64, 0.0), (64, 65, 0.0),
+    (124, 4, 0.0), (60, 50, 0.9), (511, 512, 0.0), (512, 512, 0.0), (512, 513, 0.9), (1020, 4, 0.0), (1025, 3, 0.0),
+    (2000, 2223, 0.0), (4096, 128, 0.0), (4096, 129, 0.9), (4096, 4096, 0.0), (4352, 4096, 0.0), (4353, 4096, 0.0)])
+def test_traced_intersections(cuda, na, nb, hole_frac):
+    """Stars around the edges of the tracing classes' sizes (128, 1,024, 4,224 and
+    8,448 vertices a pair), apart, overlapping in one and in several contours, and
+    one inside the other."""
+    n = 64 if na + nb < 200 else 12 if na + nb < 2000 else 5
+    rng = np.random.default_rng(na * 10007 + nb)
+    c = rng.random((n, 2))
+    r = np.full(n, 0.01)
+    A = dg.star_layer(n, seed=na, nv_lo=na, nv_hi=na, centre_xy=c, radii=r, hole_frac=hole_frac)
+    B = dg.star_layer(n, seed=nb + 1, nv_lo=nb, nv_hi=nb, centre_xy=c + rng.uniform(-0.012, 0.012, (n, 2)),
+                      radii=r * rng.uniform(0.2, 1.5, n), hole_frac=hole_frac)
+    got = clip_all(A, B, n)
+    for i in range(n):
+        assert same_contours(got[i], oracle.gpc_clip(rings_of(A, i), rings_of(B, i), 1)), f"pair {i}"
+
+
+def test_pairs_that_are_not_traced(cuda):
+    """Pairs outside general position: shared vertices and edges,
+    vertices on edges, polygons that cross or touch themselves, equal polygons,
+    crossings at one y, slivers of an ulp, rings of under three vertices, more rings
+    than are kept, coordinates of very different sizes."""
+    sq = [(0, 0), (4, 0), (4, 4), (0, 4)]
+    tri = [(0.0, 0.0), (4.0, 0.5), (1.0, 4.0)]
+    bow = [(0, 0.1), (4, 4), (4, 0), (0.3, 3.9)]
+    star = [tuple(p) for p in dg.star_layer(1, seed=5, nv_lo=21, nv_hi=21, centre_xy=np.array([[2.0, 2.0]]),
+                                            radii=np.array([2.0]))["xy"]]
+    ulp = [(x, float(np.nextafter(y, 9.0))) for x, y in star]
+    dots = [[(0.3 + 0.11 * k, 0.3 + 0.107 * k), (0.35 + 0.11 * k, 0.33 + 0.107 * k), (0.31 + 0.11 * k, 0.38 + 0.107 * k)]
+            for k in range(33)]
+    cases = [([sq], [sq]), ([sq], [[(2, 2), (6, 2), (6, 6), (2, 6)]]), ([tri], [tri]), ([tri], [sq]),
+             ([bow], [tri]), ([tri], [bow]), ([bow], [bow]), ([star], [star]), ([star], [ulp]), ([star], [sq]),
+             ([tri], [[(2.0, 0.25), (5.0, 1.0), (3.0, 3.0)]]),           # a vertex on an edge
+             ([tri], [[(4.0, 0.5), (6.0, 1.5), (5.0, 3.0)]]),            # a shared vertex
+             ([tri], [[(0.0, 0.0), (4.0, 0.5), (2.0, -3.0)]]),           # a shared edge
+             ([[(0, 0), (2, 3), (4, 0.5), (2, 1)]], [[(0, 0.25), (4, 0.25), (2, -1)]]),
+             ([[(-1, -3), (1, 3.5), (1.5, 3)]], [[(1, -3.25), (-1, 3.25), (-1.5, 2.75)]]),
+             ([tri, [(1.0, 1.0)]], [sq]), ([tri, [(1.0, 1.0), (2.0, 1.5)]], [star]),
+             (dots, [star]), ([star], dots + [sq]), (dots[:16], dots[16:32] + [star]),
+             ([[(1e12 * x, 1e12 * y) for x, y in star]], [tri]), ([tri], [[(1e-12 * x, 1e-12 * y) for x, y in star]]),
+             ([[(0.0, 0.0), (4.0, 0.5), (4.0, 0.5), (1.0, 4.0)]], [star])]
+    A, B = layer_of([a for a, _ in cases]), layer_of([b for _, b in cases])
+    got = clip_all(A, B, len(cases))
+    for i in range(len(cases)):
+        assert same_contours(got[i], oracle.gpc_clip(rings_of(A, i), rings_of(B, i), 1)), f"pair {i}"
+
+
+def test_traced_on_a_grid(cuda):
+    """Rectangles, Ls, combs and stars on whole numbers: equal ys, horizontal and
+    vertical edges, crossings on horizontal edges; many pairs share points too."""
+    rng = np.random.default_rng(12)
+
+    def rect():
+        x, y = np.sort(rng.integers(0, 40, 2)) + [0, 1], np.sort(rng.integers(0, 40, 2)) + [0, 1]
+        return np.array([(x[0], y[0]), (x[1], y[0]), (x[1], y[1]), (x[0], y[1])], float)[::rng.choice([1, -1])]
+
+    def ell():
+        a, b = np.sort(rng.choice(40, 3, replace=False)), np.sort(rng.choice(40, 3, replace=False))
+        r = np.array([(a[0], b[0]), (a[2], b[0]), (a[2], b[1]), (a[1], b[1]), (a[1], b[2]), (a[0], b[2])], float)
+        return np.roll(np.abs(40.0 * rng.integers(0, 2, 2) - r), rng.integers(6), 0)
+
+    def comb():
+        k = int(rng.integers(2, 6))
+        x = np.sort(rng.choice(60, 2 * k, replace=False)).astype(float)
+        p = [(x[0], 0.0)]
+        for t in range(k):
+            p += [(x[2 * t], h := float(rng.integers(10, 45))), (x[2 * t + 1], h)]
+            if t < k - 1:
+                p += [(x[2 * t + 1], g := float(rng.integers(1, 9))), (x[2 * t + 2], g)]
+        p = np.array(p + [(x[-1], 0.0)])
+        return np.abs([0.0, 45.0 * rng.integers(0, 2)] - p)[:, ::rng.choice([1, -1])]
+
+    def star():
+        t = np.sort(rng.random(int(rng.integers(4, 16)))) * 2 * np.pi
+        r = rng.uniform(5, 20, len(t))
+        return np.round(np.stack([20 + r * np.cos(t), 20 + r * np.sin(t)], 1) + rng.uniform(-5, 5, 2))
+
+    def polygon():
+        return [[rect, ell, comb, star][rng.integers(4)]() for _ in range(rng.choice([1, 1, 2]))]
+
+    n = 3000
+    A, B = layer_of([polygon() for _ in range(n)]), layer_of([polygon() for _ in range(n)])
+    got = clip_all(A, B, n)
+    for i in range(n):
+        assert same_contours(got[i], oracle.gpc_clip(rings_of(A, i), rings_of(B, i), 1)), f"pair {i}"
