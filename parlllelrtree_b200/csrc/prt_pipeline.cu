@@ -21,44 +21,94 @@
 namespace prt {
 namespace {
 
-// Bounding box (x1, y1, x2, y2) of every polygon over all its rings, one warp
-// per polygon: the lanes read the vertex array in coalesced 16-byte (x, y)
-// loads and reduce by shuffles.  A polygon without vertices gets the empty box
-// (DBL_MAX, DBL_MAX, -DBL_MAX, -DBL_MAX).  With Out = int32_t the box is
-// quantised as the reference's readData does, (int)(v * scale) truncated
-// toward zero (vector_map_overlay_gpc_kernel.cu:805-808, 845-848); values
-// outside the int32 range saturate.
+// Extent of the vertices v0 + first, + kStep, ... below v1.
+template <bool kAligned, int kStep>
+__device__ __forceinline__ void extend(const double *__restrict__ xy, int64_t v0, int64_t v1, int first, double *b) {
+  for (int64_t v = v0 + first; v < v1; v += kStep) {
+    double2 q;
+    if constexpr (kAligned) q = __ldg(reinterpret_cast<const double2 *>(xy) + v);
+    else q = make_double2(__ldg(xy + 2 * v), __ldg(xy + 2 * v + 1));
+    b[0] = fmin(b[0], q.x);
+    b[1] = fmin(b[1], q.y);
+    b[2] = fmax(b[2], q.x);
+    b[3] = fmax(b[3], q.y);
+  }
+}
+
+// Reduces an extent over the lanes that differ in the bits below `lanes`.
+__device__ __forceinline__ void reduce_extent(double *b, int lanes) {
+  for (int o = lanes / 2; o; o >>= 1) {
+    b[0] = fmin(b[0], __shfl_xor_sync(0xffffffffu, b[0], o));
+    b[1] = fmin(b[1], __shfl_xor_sync(0xffffffffu, b[1], o));
+    b[2] = fmax(b[2], __shfl_xor_sync(0xffffffffu, b[2], o));
+    b[3] = fmax(b[3], __shfl_xor_sync(0xffffffffu, b[3], o));
+  }
+}
+
 template <typename Out>
-__global__ void poly_mbr_kernel(LayerDev L, double scale, Out *__restrict__ out) {
-  const int lane = threadIdx.x & 31;
+__device__ __forceinline__ void store_extent(const double *b, double scale, int k, int64_t p, Out *out) {
+  const double v = k == 0 ? b[0] : k == 1 ? b[1] : k == 2 ? b[2] : b[3];
+  if constexpr (sizeof(Out) == 8) out[4 * p + k] = (Out)v;
+  else out[4 * p + k] = (Out)__double2int_rz(v * scale);
+}
+
+// Bounding box (x1, y1, x2, y2) of every polygon over all its rings: the lanes
+// read the vertex array in coalesced 16-byte (x, y) loads and reduce by shuffles.
+// A polygon without vertices gets the empty box (DBL_MAX, DBL_MAX, -DBL_MAX,
+// -DBL_MAX).  With Out = int32_t the box is quantised as the reference's readData
+// does, (int)(v * scale) truncated toward zero
+// (vector_map_overlay_gpc_kernel.cu:805-808, 845-848); values outside the int32
+// range saturate.
+// A warp takes kMbrGroup polygons, 8 lanes each while all of them are small, in
+// turn otherwise: for the usual 10 to 60 vertices a warp per polygon leaves lanes
+// idle and spends its time on the pointers (two dependent loads) and 20 shuffles of
+// doubles per polygon.  Layers of too few polygons to fill the GPU that way keep a
+// warp per polygon (kMbrGrouped).  200,000 polygons of 4 and 6 vertices: 93 -> 30 us;
+// 10,000 stars and 10,000 uneven polygons of up to 4,096 vertices stay at 13 and 85.
+constexpr int kMbrGroup = 4, kMbrSmall = 64;
+constexpr int64_t kMbrGrouped = (int64_t)kSMs * 64 * kMbrGroup;
+
+template <typename Out, bool kAligned>
+__device__ __forceinline__ void poly_mbr_body(const LayerDev &L, double scale, Out *__restrict__ out) {
+  const int lane = threadIdx.x & 31, g = lane >> 3;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t p = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; p < L.n_poly; p += nw) {
-    const int64_t v0 = L.ring_vert[L.poly_ring[p]], v1 = L.ring_vert[L.poly_ring[p + 1]];
-    double x1 = 1.7976931348623157e308, y1 = x1, x2 = -x1, y2 = -x1;
-    const bool aligned = (reinterpret_cast<uintptr_t>(L.xy) & 15) == 0;
-    const double2 *xy = reinterpret_cast<const double2 *>(L.xy);
-    for (int64_t v = v0 + lane; v < v1; v += 32) {
-      const double2 q = aligned ? __ldg(&xy[v]) : make_double2(__ldg(&L.xy[2 * v]), __ldg(&L.xy[2 * v + 1]));
-      x1 = fmin(x1, q.x);
-      y1 = fmin(y1, q.y);
-      x2 = fmax(x2, q.x);
-      y2 = fmax(y2, q.y);
+  const int64_t w0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  constexpr double kMax = 1.7976931348623157e308;
+  const int group = L.n_poly >= kMbrGrouped ? kMbrGroup : 1;
+  for (int64_t p0 = w0 * group; p0 < L.n_poly; p0 += nw * group) {
+    // lanes 8 g .. 8 g + 7: polygon p0 + g (one polygon: all lanes)
+    const int64_t p = group > 1 ? p0 + g : p0;
+    int64_t v0 = 0, v1 = 0;
+    if (p < L.n_poly) {
+      v0 = L.ring_vert[L.poly_ring[p]];
+      v1 = L.ring_vert[L.poly_ring[p + 1]];
     }
-    for (int o = 16; o; o >>= 1) {
-      x1 = fmin(x1, __shfl_xor_sync(0xffffffffu, x1, o));
-      y1 = fmin(y1, __shfl_xor_sync(0xffffffffu, y1, o));
-      x2 = fmax(x2, __shfl_xor_sync(0xffffffffu, x2, o));
-      y2 = fmax(y2, __shfl_xor_sync(0xffffffffu, y2, o));
+    if (group > 1 && !__any_sync(0xffffffffu, v1 - v0 > kMbrSmall)) {
+      double b[4] = {kMax, kMax, -kMax, -kMax};
+      extend<kAligned, 8>(L.xy, v0, v1, lane & 7, b);
+      reduce_extent(b, 8);
+      if (p < L.n_poly && (lane & 7) < 4) store_extent(b, scale, lane & 7, p, out);
+      continue;
     }
-    if (lane < 4) {
-      const double v = lane == 0 ? x1 : lane == 1 ? y1 : lane == 2 ? x2 : y2;
-      if constexpr (sizeof(Out) == 8) out[4 * p + lane] = (Out)v;
-      else out[4 * p + lane] = (Out)__double2int_rz(v * scale);
+    for (int k = 0; k < group && p0 + k < L.n_poly; k++) {
+      double b[4] = {kMax, kMax, -kMax, -kMax};
+      extend<kAligned, 32>(L.xy, __shfl_sync(0xffffffffu, v0, 8 * k), __shfl_sync(0xffffffffu, v1, 8 * k), lane, b);
+      reduce_extent(b, 32);
+      if (lane < 4) store_extent(b, scale, lane, p0 + k, out);
     }
   }
 }
 
-inline int poly_mbr_grid(int64_t n_poly) { return grid_for(n_poly * 32, 256, 8); }
+template <typename Out>
+__global__ void poly_mbr_kernel(LayerDev L, double scale, Out *__restrict__ out) {
+  if ((reinterpret_cast<uintptr_t>(L.xy) & 15) == 0) poly_mbr_body<Out, true>(L, scale, out);
+  else poly_mbr_body<Out, false>(L, scale, out);
+}
+
+inline int poly_mbr_grid(int64_t n_poly) {
+  const int64_t group = n_poly >= kMbrGrouped ? kMbrGroup : 1;
+  return grid_for((n_poly + group - 1) / group * 32, 256, 8);
+}
 
 // Largest vertex count of a polygon of the layer (sizes the biggest arenas).
 __global__ void max_poly_vertices_kernel(LayerDev L, unsigned long long *out) {

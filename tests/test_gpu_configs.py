@@ -140,3 +140,30 @@ def test_join_10m_1m_windows(boxes_10m):
     exp[:, 1] = sample[exp[:, 1]]
     exp = exp[np.lexsort((exp[:, 0], exp[:, 1]))]
     assert np.array_equal(got_s, exp)
+
+
+@pytest.mark.parametrize("n", [37887, 37888, 37889, 37891])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_mbr_grouped(cuda, n, shift):
+    """Polygon boxes around the number of polygons from which a warp takes four of
+    them, vertex counts around its 64, polygons without vertices, and vertices that
+    do not start on a 16-byte boundary."""
+    import parlllelrtree_b200 as prt
+
+    rng = np.random.default_rng(n)
+    nv = rng.integers(3, 12, n)
+    nv[rng.integers(0, n, 300)] = rng.choice([0, 1, 31, 32, 33, 63, 64, 65, 66, 200], 300)
+    nv[-1] = 65
+    off = np.cumsum(np.concatenate([[0], nv])).astype(np.int64)
+    xy = rng.normal(size=(int(off[-1]), 2))
+    big = np.finfo(np.float64).max
+    ref = np.tile([big, big, -big, -big], (n, 1))
+    some = nv > 0
+    ref[some, :2] = np.minimum.reduceat(xy, off[:-1][some])
+    ref[some, 2:] = np.maximum.reduceat(xy, off[:-1][some])
+    L = prt.Layer.from_dict({"poly_ring": np.arange(n + 1, dtype=np.int64), "ring_vert": off,
+                             "ring_hole": np.zeros(n, dtype=np.int32), "xy": xy})
+    flat = torch.zeros(2 * len(xy) + 1, dtype=torch.float64, device="cuda")
+    flat[shift:shift + 2 * len(xy)] = torch.from_numpy(xy.reshape(-1))
+    got = L.mbr(flat[shift:shift + 2 * len(xy)].view(-1, 2)).cpu().numpy()
+    assert np.array_equal(got, ref)
