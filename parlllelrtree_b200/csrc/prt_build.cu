@@ -462,8 +462,9 @@ __global__ void __launch_bounds__(256) td_keyrun_kernel(const T *__restrict__ cx
 // within the tile, key - the tile's smallest key) with an LSD radix sort in
 // shared memory over only the bits that needs, 8 bits per pass, each pass
 // ranked by the warp multisplit (lanes with the same digit from one ballot
-// per digit bit); the last level (runs of F <= 32) places each record by
-// counting the run's smaller keys.  The tile's index order is the current
+// per digit bit), or by buckets where the keys are spread evenly enough (10M
+// float boxes at F = 16, three local levels: 580 -> 444 us); the last level (runs
+// of F <= 32) places each record by counting the run's smaller keys.  The tile's index order is the current
 // order, so equal keys keep it, as each level's stable sort requires; each
 // item's run travels with it.  One read and one write of the order replace
 // 4-7 global passes per level.
@@ -493,7 +494,7 @@ template <typename T>
 struct TdLocalSmem {
   uint32_t item[2][kTdLocal];
   T xy[kTdLocal][2];
-  uint32_t wh[kTdWarps][256];
+  alignas(16) uint32_t wh[kTdWarps][256];
   uint32_t dstart[256];
   uint32_t wsum[8];
   unsigned long long red[2][kTdWarps];
@@ -512,6 +513,7 @@ struct TdLocalLevels {
 // key at an earlier position (a stable sort by counting), seg comparisons
 // per record instead of the radix passes.
 constexpr int kTdRankMax = 32;
+constexpr uint32_t kTdCrowd = 32;  // largest bucket that a level's buckets may have
 
 __device__ __forceinline__ int bit_length(uint32_t x) { return 32 - __clz(x); }
 __device__ __forceinline__ int bit_length(uint64_t x) { return 64 - __clzll((long long)x); }
@@ -605,10 +607,99 @@ __global__ void __launch_bounds__(kTdThreads, kTdThreads == 256 ? (sizeof(T) == 
       lo = a < lo ? a : lo;
       hi = z > hi ? z : hi;
     }
-    const int key_bits = hi > lo ? bit_length(hi - lo) : 0;
+    if (hi == lo) continue;  // all equal: the order stays
+    const int key_bits = bit_length(hi - lo);
     int run_bits = 0;
     while ((1 << run_bits) < (m + seg - 1) / seg) run_bits++;
     const int total_bits = key_bits + run_bits;
+    // By buckets: each run's keys are spread over its part of the counters in
+    // proportion to key - lo, about as many buckets as records, and a record's
+    // place in its bucket is counted like the last level's, instead of three radix
+    // passes or more; with 64-bit coordinates and one block of them per SM four or
+    // more (300k 64-bit boxes on a 1e6 grid, three passes: 37 us against 39).  The counting grows with the largest bucket: with one above kTdCrowd
+    // the passes below sort the level (tiles of equal keys; without the limit 720
+    // us where it takes 444 with one of 32, 453 with 12).
+    if (total_bits > (sizeof(T) == 4 ? 16 : 24)) {
+      constexpr int kPer = kTdWarps * 256 / kTdThreads;  // counters per thread
+      uint32_t *cnt = &S.wh[0][0];
+      const int nb = kTdWarps * 256 / ((m + seg - 1) / seg);
+      const float scale = (float)nb / (float)(hi - lo);
+      for (int i = tid; i < kTdWarps * 256; i += kTdThreads) cnt[i] = 0;
+      __syncthreads();
+      uint32_t bk[kTdItems];
+#pragma unroll
+      for (int q = 0; q < kTdItems; q++) {
+        const int i = tid + kTdThreads * q;
+        if (i < m) {
+          const uint32_t x = S.item[cur][i];
+          const K rel = (K)ukey(S.xy[x & 0xFFFFu][axis]) - lo;
+          bk[q] = (x >> 16) * nb + min(nb - 1, (int)((float)rel * scale));  // conversion and product keep the order
+          atomicAdd(&cnt[bk[q]], 1u);
+        }
+      }
+      __syncthreads();
+      static_assert(kPer % 4 == 0, "four counters per access");
+      uint4 c[kPer / 4];
+      uint32_t sum = 0, most = 0;
+#pragma unroll
+      for (int k = 0; k < kPer / 4; k++) {
+        c[k] = reinterpret_cast<uint4 *>(cnt)[tid * (kPer / 4) + k];
+        most = max(max(most, max(c[k].x, c[k].y)), max(c[k].z, c[k].w));
+        sum += c[k].x + c[k].y + c[k].z + c[k].w;
+      }
+      uint32_t incl = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      if (lane == 31) S.dstart[warp] = incl;
+      if (!__syncthreads_or(most > kTdCrowd)) {
+        uint32_t run0 = incl - sum;
+#pragma unroll
+        for (int w = 0; w < kTdWarps; w++) run0 += w < warp ? S.dstart[w] : 0u;
+#pragma unroll
+        for (int k = 0; k < kPer / 4; k++) {
+          const uint4 at = make_uint4(run0, run0 + c[k].x, run0 + c[k].x + c[k].y, run0 + c[k].x + c[k].y + c[k].z);
+          reinterpret_cast<uint4 *>(cnt)[tid * (kPer / 4) + k] = at;
+          run0 = at.w + c[k].w;
+        }
+        __syncthreads();
+        uint32_t *in_bucket = S.item[1 - cur];
+#pragma unroll
+        for (int q = 0; q < kTdItems; q++) {
+          const int i = tid + kTdThreads * q;
+          if (i < m) in_bucket[atomicAdd(&cnt[bk[q]], 1u)] = (uint32_t)i;
+        }
+        __syncthreads();
+        // cnt[b] is now the end of bucket b, the start of the next
+#pragma unroll
+        for (int q = 0; q < kTdItems; q++) {
+          const int i = tid + kTdThreads * q;
+          if (i < m) {
+            const uint32_t k0 = bk[q] ? cnt[bk[q] - 1] : 0u, k1 = cnt[bk[q]];
+            uint32_t rank = k0;
+            if (k1 - k0 > 1) {
+              const K ki = (K)ukey(S.xy[S.item[cur][i] & 0xFFFFu][axis]);
+              for (uint32_t k = k0; k < k1; k++) {
+                const int j = (int)in_bucket[k];
+                const K kj = (K)ukey(S.xy[S.item[cur][j] & 0xFFFFu][axis]);
+                rank += kj < ki || (kj == ki && j < i) ? 1u : 0u;
+              }
+            }
+            bk[q] = rank;
+          }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < kTdItems; q++) {
+          const int i = tid + kTdThreads * q;
+          if (i < m) S.item[1 - cur][bk[q]] = S.item[cur][i];
+        }
+        cur = 1 - cur;
+        continue;
+      }
+    }
     for (int shift = 0; shift < total_bits; shift += 8) {
       const int width = min(8, total_bits - shift);
       __syncthreads();

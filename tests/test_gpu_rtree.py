@@ -256,6 +256,34 @@ def test_topdown_run_lengths(cuda, kind, F, n):
 
 
 @pytest.mark.parametrize("kind", ["f32", "f64", "i64", "i32"])
+@pytest.mark.parametrize("F", [2, 10, 16, 31, 32])
+@pytest.mark.parametrize("shape", ["even", "32 equal", "33 equal", "skewed", "one value"])
+def test_topdown_buckets(cuda, kind, F, shape):
+    """Short runs whose keys fill the buckets evenly, with the largest bucket at the
+    limit and one above it, almost all in one bucket, and equal."""
+    import parlllelrtree_b200 as prt
+
+    rng = np.random.default_rng(F)
+    n = 9001
+    if shape == "even":
+        c = np.stack([rng.permutation(n), rng.permutation(n)], 1).astype(np.float64)
+    elif shape == "one value":
+        c = np.full((n, 2), 7.0)
+    elif shape == "skewed":
+        c = np.round(np.exp(rng.uniform(0, 20, (n, 2))))
+    else:
+        k = int(shape.split()[0])
+        c = np.stack([rng.permutation(n), rng.permutation(n)], 1).astype(np.float64)
+        c[rng.choice(n, k, replace=False)] = 4000.0
+    dt = {"f32": np.float32, "f64": np.float64, "i64": np.int64, "i32": np.int32}[kind]
+    b = np.concatenate([c, c + 1], 1).astype(dt)
+    perm = oracle.td_order(b, F)
+    t = prt.build_topdown(torch.from_numpy(b).cuda(), fanout=F)
+    assert np.array_equal(t.leaf_order().cpu().numpy(), perm)
+    check_levels(t, oracle.pack(b, F, perm))
+
+
+@pytest.mark.parametrize("kind", ["f32", "f64", "i64", "i32"])
 @pytest.mark.parametrize("F", [2, 3, 16, 32])
 @pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 1023, 1024, 1025, 4096, 6143, 6144, 6145, 8191, 8192, 8193])
 def test_one_block_build(cuda, kind, F, n):
