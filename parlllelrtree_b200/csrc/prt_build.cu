@@ -993,22 +993,26 @@ int pack_tree(prt_tree *t, const void *d_boxes, const int32_t *d_ids, const uint
 // ------------------------------------------------------------------ small bottom-up build
 
 // The whole bottom-up build (MORTON32) of up to kSmallBuild records in one
-// block: extent, keys, an LSD sort in shared memory by the multisplit of the
-// big sort's passes (skipping digits that are the same for all keys), leaves
-// and levels.  Its time is a chain of latencies, but one launch's: a call with
-// 1,000, 4,001 and 8,192 float boxes takes 40, 53 and 71 us against 90, 92 and
-// 92 with the grid-wide kernels' 10 launches, with 6,000 double boxes 77 against
-// 93 and with 8,192 as long: from there one SM's throughput is the bound.
+// block: extent, keys, a sort in shared memory by buckets (radix passes by the
+// multisplit of the big sort where a bucket is crowded, skipping digits that are
+// the same for all keys), leaves and levels.  Its time is a chain of latencies, but
+// one launch's: with radix passes alone a call with 1,000, 4,001 and 8,192 float
+// boxes took 40, 53 and 71 us against 90, 92 and 92 with the grid-wide kernels' 10
+// launches, with 6,000 double boxes 77 against 93 and with 8,192 as long: from
+// there one SM's throughput is the bound.  The buckets take another 7, 10, 13 and
+// 12 us off these four.
 constexpr int kSmallBuild = 8192;
 constexpr int kSmallBuildWide = 6144;  // 64-bit coordinates
 constexpr int kSmallBlock = 1024;
 constexpr int kSmallWarps = kSmallBlock / 32;
 constexpr int kSmallItems = kSmallBuild / kSmallBlock;
+constexpr int kSmallBucketBits = 13;
+static_assert(1 << kSmallBucketBits == kSmallWarps * 256 && kSmallItems == 8 && kSmallWarps == 32, "eight counters a thread");
 
 struct SmallSmem {
   uint32_t key[kSmallBuild];
   uint16_t val[kSmallBuild];
-  uint32_t wh[kSmallWarps][256];
+  alignas(16) uint32_t wh[kSmallWarps][256];
   uint32_t dstart[256];
   uint32_t wsum[8];
   double red[4][32];
@@ -1053,8 +1057,79 @@ __global__ void __launch_bounds__(kSmallBlock) bu_small_kernel(const Box<T> *__r
   if (lane == 0 && differ) atomicOr(&S.differ, differ);
   __syncthreads();
   differ = S.differ;
+  // By buckets of the highest bits that differ, a record's place in its bucket
+  // counted (equal keys in input order); with a bucket above kTdCrowd by the radix
+  // passes below.
+  bool crowded = differ != 0;
+  if (differ) {
+    uint32_t *cnt = &S.wh[0][0];
+    const int low = max(0, bit_length(differ) - kSmallBucketBits);
+    auto bucket = [&](uint32_t key) { return key >> low & ((1u << kSmallBucketBits) - 1u); };
+    for (int i = tid; i < kSmallBuild; i += kSmallBlock) cnt[i] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kSmallItems; j++)
+      if (j < per && base + 32 * j < n) atomicAdd(&cnt[bucket(k[j])], 1u);
+    __syncthreads();
+    uint4 c[2];
+    uint32_t sum = 0, most = 0;
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      c[q] = reinterpret_cast<uint4 *>(cnt)[2 * tid + q];
+      most = max(max(most, max(c[q].x, c[q].y)), max(c[q].z, c[q].w));
+      sum += c[q].x + c[q].y + c[q].z + c[q].w;
+    }
+    uint32_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (lane == 31) S.dstart[warp] = incl;
+    crowded = __syncthreads_or(most > kTdCrowd);
+    if (!crowded) {
+      uint32_t before = S.dstart[lane];
+      before = __reduce_add_sync(0xffffffffu, lane < warp ? before : 0u);
+      uint32_t run = before + incl - sum;
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        const uint4 at = make_uint4(run, run + c[q].x, run + c[q].x + c[q].y, run + c[q].x + c[q].y + c[q].z);
+        reinterpret_cast<uint4 *>(cnt)[2 * tid + q] = at;
+        run = at.w + c[q].w;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < kSmallItems; j++)
+        if (j < per && base + 32 * j < n) {
+          const uint32_t at = atomicAdd(&cnt[bucket(k[j])], 1u);
+          S.key[at] = k[j];
+          S.val[at] = (uint16_t)v[j];
+        }
+      __syncthreads();
+      // cnt[b] is now the end of bucket b, the start of the next
+#pragma unroll
+      for (int j = 0; j < kSmallItems; j++)
+        if (j < per && base + 32 * j < n) {
+          const uint32_t d = bucket(k[j]), begin = d ? cnt[d - 1] : 0u, end = cnt[d];
+          uint32_t rank = begin;
+          for (uint32_t i = begin; i < end; i++) {
+            const uint32_t ki = S.key[i];
+            rank += ki < k[j] || (ki == k[j] && S.val[i] < v[j]) ? 1u : 0u;
+          }
+          k[j] = rank;
+        }
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < kSmallItems; j++)
+        if (j < per && base + 32 * j < n) S.val[k[j]] = (uint16_t)v[j];
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < kSmallItems; j++)
+        if (j < per && base + 32 * j < n) v[j] = S.val[base + 32 * j];
+    }
+  }
   const uint32_t lt = lane_lt();
-  for (int shift = 0; shift < 32; shift += 8) {
+  for (int shift = 0; shift < 32 && crowded; shift += 8) {
     if (!(differ >> shift & 0xFFu)) continue;
     for (int i = tid; i < kSmallWarps * 256; i += kSmallBlock) (&S.wh[0][0])[i] = 0;
     __syncthreads();

@@ -299,3 +299,20 @@ def test_one_block_build(cuda, kind, F, n):
     t = prt.build_bottomup(torch.from_numpy(b).cuda(), fanout=F, ids=ids)
     assert np.array_equal(t.leaf_order().cpu().numpy(), ids[perm])
     check_levels(t, oracle.pack(b, F, perm))
+
+
+@pytest.mark.parametrize("kind", ["f32", "f64", "i64"])
+@pytest.mark.parametrize("equal", [32, 33, 5000])
+@pytest.mark.parametrize("n", [40, 5000, 6144, 8192])
+def test_one_block_buckets(cuda, kind, equal, n):
+    """One-block builds whose largest bucket is at the limit of the counting, one
+    above it, and almost all of the boxes."""
+    import parlllelrtree_b200 as prt
+
+    b = boxes_of(kind, n, seed=n + equal)
+    rng = np.random.default_rng(n * equal)
+    b[rng.choice(n, min(n, equal), replace=False)] = b[0]
+    t = prt.build_bottomup(torch.from_numpy(b).cuda(), fanout=16)
+    perm = oracle.stable_argsort(oracle.keys_morton32(b)[0])
+    assert np.array_equal(t.leaf_order().cpu().numpy(), perm)
+    check_levels(t, oracle.pack(b, 16, perm))
