@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(32, kLptThreadWarpsPerSM)
   lpt_body<false>(S, O, order, plan, tickets, arena, scale, nullptr, rest);
 }
 
-// Intersections by tracing (prt_trace.cuh): one block per pair of the sorted
+// All operations but XOR by tracing (prt_trace.cuh): one block per pair of the sorted
 // positions [begin, end), largest pairs first, from one ticket.  A pair that is
 // not traced goes to its bin's part of left_order for the launch above.
 template <typename C>
@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(C::NT, C::kBlocks)
       if (threadIdx.x == 0) invalid_pair(O, i);
       continue;
     }
-    if (trace::trace_pair<C>(M, a, b, K, i, kPairPool) == trace::kLeft && threadIdx.x == 0) {
+    if (trace::trace_pair<C>(M, S.op, a, b, K, i, kPairPool) == trace::kLeft && threadIdx.x == 0) {
       int g = 0;
       while (g + 1 < plan.nbins && k >= plan.end[g]) g++;
       left_order[plan.begin[g] + (int64_t)atomicAdd(&left[g], 1ull)] = (uint32_t)i;
@@ -698,7 +698,7 @@ static int run_batched(OverlayState &st, const int64_t *d_idx, int64_t count, in
     unsigned long long left[PRT_MAX_BINS];  // pairs of each bin that were not traced
   } h;
   static_assert(sizeof(Head) <= 512, "head block");
-  const bool trace_pairs = st.S.op == PRT_GPC_INT;
+  const bool trace_pairs = st.S.op != PRT_GPC_XOR;
   unsigned char *scr = nullptr;
   int rc = dmalloc(reinterpret_cast<void **>(&scr), 512 + 20 * n + (trace_pairs ? 4 * n : 0), s);
   if (rc) return rc;

@@ -1,5 +1,6 @@
-// Intersection of a pair in general position by tracing, with the result that
-// the scanbeam clippers (prt_gpc.cuh, prt_wgpc.cuh) give, bit for bit.
+// Intersection, difference and union of a pair in general position by tracing, with
+// the result that the scanbeam clippers (prt_gpc.cuh, prt_wgpc.cuh) give, bit for
+// bit.  (An exclusive or passes every crossing twice and stays with them.)
 //
 // GPC sweeps the pair beam by beam (a beam: two neighbouring vertex ys), a chain
 // of dependent steps per beam however little happens in it.  When nothing
@@ -9,8 +10,9 @@
 //    its two edges and the beam that it lies in (the edges' x at the beam's two
 //    ys, build_intersection_table, GPC:1309-1471);
 //  * the boundary runs along A where A is inside B and along B where B is inside
-//    A and changes over at every crossing, so the contours are cycles of runs of
-//    consecutive vertices between crossings;
+//    A (outside for a union, and of a difference along B backwards) and changes
+//    over at every crossing, so the contours are cycles of runs of consecutive
+//    vertices between crossings;
 //  * GPC's vertex lists grow to the left and right and are joined at maxima, so a
 //    contour comes out cut at its highest vertex: that vertex is the last one
 //    written of an outer contour and the first one of a hole;
@@ -111,6 +113,7 @@ struct Pair {
   Smem<C> &S;
   int n;
   double margin, least;
+  bool convex;
   __device__ __forceinline__ double x(int v) const { return S.vx[v]; }
   __device__ __forceinline__ double y(int v) const { return S.sy[S.rank[v]]; }
   __device__ __forceinline__ int nxt(int v) const {
@@ -257,7 +260,7 @@ __device__ __forceinline__ uint32_t node_key(const Smem<C> &S, int node) {
 // Whether the material lies below a contour's local maximum (node m).
 template <typename C>
 __device__ __forceinline__ bool max_is_outer(const Pair<C> &P, int m) {
-  if (m & 0x8000) return true;  // one quadrant at a crossing is in both polygons
+  if (m & 0x8000) return P.convex;  // one quadrant at a crossing belongs to the result, of a union three
   const TEdge e1 = edge_of(P, m), e0 = edge_of(P, P.prv(m));
   const bool fwd = P.S.mat[P.S.ring[m]];
   // material on the left: below when the boundary comes up the right edge (the
@@ -356,7 +359,7 @@ enum : int { kTraced = 0, kLeft = 1 };
 // scanbeam clippers (nothing written).  pool_full: the status to record when the
 // result pools are too small.
 template <typename C>
-__device__ int trace_pair(Smem<C> &S, const gpc::PolyView &A, const gpc::PolyView &B, const Sink &O, int64_t pair,
+__device__ int trace_pair(Smem<C> &S, int op, const gpc::PolyView &A, const gpc::PolyView &B, const Sink &O, int64_t pair,
                           int pool_full) {
   constexpr int NT = C::NT;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -371,7 +374,8 @@ __device__ int trace_pair(Smem<C> &S, const gpc::PolyView &A, const gpc::PolyVie
   bool bad = false;  // this thread found the pair not in general position, or too large
   if (na + nb > kMaxRings) return kLeft;
   // ---- rings whose boxes meet a ring of the other polygon (minimax_test,
-  // GPC:1656-1709); the others take no part
+  // GPC:1656-1709); the others take no part (a difference keeps the subject's, a
+  // union all)
   for (int r = 0; r < na + nb; r++) {
     const gpc::PolyView &p = r < na ? A : B;
     const int64_t g = r < na ? A.r0 + r : B.r0 + (r - na);
@@ -395,7 +399,7 @@ __device__ int trace_pair(Smem<C> &S, const gpc::PolyView &A, const gpc::PolyVie
   double most = 0.0, most_x = 0.0, wide = 0.0, ymin = gpc::kDblMax, ymax = -gpc::kDblMax;
   int n = 0, nr = 0;
   for (int r = 0; r < na + nb; r++) {
-    bool meets = false;
+    bool meets = op == PRT_GPC_UNION || (op == PRT_GPC_DIFF && r < na);
     for (int q = r < na ? na : 0; q < (r < na ? na + nb : na); q++)
       meets |= r < na ? gpc::bbox_overlap(S.rbb[r], S.rbb[q]) : gpc::bbox_overlap(S.rbb[q], S.rbb[r]);
     if (!meets) continue;
@@ -424,7 +428,8 @@ __device__ int trace_pair(Smem<C> &S, const gpc::PolyView &A, const gpc::PolyVie
   // the distance of two by eps(|x| + 6w).  Above twice that and GPC's own epsilon a
   // computed distance has the sign of the true one, and so it has, and is above the
   // epsilon, at every beam between two such ends.
-  Pair<C> P{S, n, gpc::kEps * (2.1 * most_x + 16.0 * wide + 1.1), gpc::kEps * (2.1 * most_x + 1.1)};
+  Pair<C> P{S, n, gpc::kEps * (2.1 * most_x + 16.0 * wide + 1.1), gpc::kEps * (2.1 * most_x + 1.1),
+            op != PRT_GPC_UNION};
   if (n > 0) {
     // ---- vertices, and their ys in order
     for (int r = 0; r < nr; r++) {
@@ -592,7 +597,8 @@ __device__ int trace_pair(Smem<C> &S, const gpc::PolyView &A, const gpc::PolyVie
       const int side = S.rside[r];
       left ^= inside_rings(P, m, [&](int q) { return q != r && S.rside[q] == side; });
     }
-    if (tid == 0) S.mat[r] = left;
+    // a difference is the intersection with the other polygon's outside
+    if (tid == 0) S.mat[r] = left != (op == PRT_GPC_DIFF && S.rside[r] == 1);
   }
   const int nx = n > 0 ? S.ncross : 0;
   bsync<NT>();
@@ -624,10 +630,10 @@ __device__ int trace_pair(Smem<C> &S, const gpc::PolyView &A, const gpc::PolyVie
       S.pos[s][c] = (uint16_t)at[s];
       S.seq[s][at[s]] = (uint16_t)c;
     }
-    // polygon 0's boundary enters polygon 1 here: the boundary of the result goes
-    // on along polygon 0, else along polygon 1
+    // polygon 0's boundary enters polygon 1 here: the boundary of an intersection
+    // goes on along polygon 0, else along polygon 1; of a union the other way round
     const bool same = (up[0] == (S.mat[ring[0]] != 0)) == (up[1] == (S.mat[ring[1]] != 0));
-    S.out[c] = (same != (S.aleft[c] != 0)) ? 0 : 1;
+    S.out[c] = ((same != (S.aleft[c] != 0)) != (op == PRT_GPC_UNION)) ? 0 : 1;
   }
   if (bany<NT>(bad)) return kLeft;
   // the run that starts at each crossing: its vertices and the crossing at its end
@@ -675,7 +681,8 @@ __device__ int trace_pair(Smem<C> &S, const gpc::PolyView &A, const gpc::PolyVie
   for (int r = 0; r < nr; r++) {
     if (S.hit[r]) continue;
     const int side = S.rside[r];
-    if (!inside_rings(P, S.rstart[r], [&](int q) { return S.rside[q] != side; })) continue;
+    const bool wanted = op != PRT_GPC_UNION && (op != PRT_GPC_DIFF || side == 1);  // inside, else outside
+    if (inside_rings(P, S.rstart[r], [&](int q) { return S.rside[q] != side; }) != wanted) continue;
     const int len = S.rstart[r + 1] - S.rstart[r];
     if (nc >= C::kContours || total + len > C::kList) return kLeft;
     if (tid == 0) {

@@ -273,3 +273,28 @@ def test_traced_on_a_grid(cuda):
     got = clip_all(A, B, n)
     for i in range(n):
         assert same_contours(got[i], oracle.gpc_clip(rings_of(A, i), rings_of(B, i), 1)), f"pair {i}"
+
+
+@pytest.mark.parametrize("op", [0, 3])
+@pytest.mark.parametrize("na,nb,hole_frac", [(3, 3, 0.0), (16, 15, 0.9), (64, 64, 0.9), (64, 65, 0.0), (512, 513, 0.9),
+                                             (4096, 129, 0.9), (4352, 4096, 0.0)])
+def test_traced_difference_and_union(cuda, op, na, nb, hole_frac):
+    """The same pairs' difference and union, and polygons on a grid."""
+    import parlllelrtree_b200 as prt
+
+    n = 64 if na + nb < 200 else 6
+    rng = np.random.default_rng(na + 7919 * nb)
+    c = rng.random((n, 2))
+    r = np.full(n, 0.01)
+    A = dg.star_layer(n, seed=na, nv_lo=na, nv_hi=na, centre_xy=c, radii=r, hole_frac=hole_frac)
+    B = dg.star_layer(n, seed=nb + 1, nv_lo=nb, nv_hi=nb, centre_xy=c + rng.uniform(-0.012, 0.012, (n, 2)),
+                      radii=r * rng.uniform(0.2, 1.5, n), hole_frac=hole_frac)
+    if na < 200:  # the second half on a grid that a few of their points share
+        for L in (A, B):
+            half = L["ring_vert"][L["poly_ring"][n // 2]]
+            L["xy"][half:] = np.round(L["xy"][half:] * 3000) / 3000
+    ids = np.arange(n, dtype=np.int32)
+    got = prt.overlay(torch.from_numpy(np.stack([ids, ids], axis=1)).cuda(), prt.Layer.from_dict(A),
+                      prt.Layer.from_dict(B), op=OPS[op]).contours()
+    for i in range(n):
+        assert same_contours(got[i], oracle.gpc_clip(rings_of(A, i), rings_of(B, i), op)), f"pair {i}"
