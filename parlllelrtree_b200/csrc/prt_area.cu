@@ -506,196 +506,196 @@ __device__ inline bool pair_boundary(BwdPair<V> &W, const float4 *ext, int na, i
   bool exact = false;  // by the definition from here on (sticky)
   double area2 = 0.0, err = 0.0;
   for (int half = 0; half < 2; half++) {
-  const int side = half ? 1 - searcher : searcher;
-  const BwdPoly<V> &P = W.poly[side], &Q = W.poly[1 - side];
-  const int np = side ? nb : na, nq = side ? na : nb;
-  const int nwq = (nq + 31) >> 5;
-  bool carry = false;  // inside state after the last edge of the previous round
-  for (int e0 = 0; e0 < np; e0 += 32) {
-    const int i = e0 + lane;
-    const bool valid = i < np && P.sgn[i] != 0;
-    const int j = valid ? P.nxt[i] : 0;
-    double px = 0.0, py = 0.0, qx = 0.0, qy = 0.0;
-    float4 pb = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (valid) {
-      px = P.x[i];
-      py = P.y[i];
-      qx = P.x[j];
-      qy = P.y[j];
-      pb = P.bb[i];
-    }
-    const double rx = qx - px, ry = qy - py;
-    double c1 = 0.0, c2 = 0.0;  // sums of sign t and sign t^2 over the edge's clean crossings
-    int c0 = 0;                 // and of the signs
-    int m = 0;                  // their number
-    double tfirst = 1.0;        // the first one
-    if (half == 0 && !exact) {
-      bool unclean = false;
+    const int side = half ? 1 - searcher : searcher;
+    const BwdPoly<V> &P = W.poly[side], &Q = W.poly[1 - side];
+    const int np = side ? nb : na, nq = side ? na : nb;
+    const int nwq = (nq + 31) >> 5;
+    bool carry = false;  // inside state after the last edge of the previous round
+    for (int e0 = 0; e0 < np; e0 += 32) {
+      const int i = e0 + lane;
+      const bool valid = i < np && P.sgn[i] != 0;
+      const int j = valid ? P.nxt[i] : 0;
+      double px = 0.0, py = 0.0, qx = 0.0, qy = 0.0;
+      float4 pb = make_float4(0.f, 0.f, 0.f, 0.f);
       if (valid) {
-        const bool material_left = P.sgn[i] > 0;
-        const double rl = fabs(rx) + fabs(ry);
-        const int s0 = g(pb.y), s1 = g(pb.w), x0 = gx(pb.x), x1 = gx(pb.z);
-        for (int c = 0; c < nwq; c++) {
-          uint32_t bits = bwd_cands(W.slab, c, s0, s1, x0, x1);
-          while (bits) {
-            const int k = 32 * c + __ffs(bits) - 1;
-            bits &= bits - 1;
-            const float4 b = Q.bb[k];
-            if (b.w < pb.y || b.y > pb.w || b.z < pb.x || b.x > pb.z) continue;
+        px = P.x[i];
+        py = P.y[i];
+        qx = P.x[j];
+        qy = P.y[j];
+        pb = P.bb[i];
+      }
+      const double rx = qx - px, ry = qy - py;
+      double c1 = 0.0, c2 = 0.0;  // sums of sign t and sign t^2 over the edge's clean crossings
+      int c0 = 0;                 // and of the signs
+      int m = 0;                  // their number
+      double tfirst = 1.0;        // the first one
+      if (half == 0 && !exact) {
+        bool unclean = false;
+        if (valid) {
+          const bool material_left = P.sgn[i] > 0;
+          const double rl = fabs(rx) + fabs(ry);
+          const int s0 = g(pb.y), s1 = g(pb.w), x0 = gx(pb.x), x1 = gx(pb.z);
+          for (int c = 0; c < nwq; c++) {
+            uint32_t bits = bwd_cands(W.slab, c, s0, s1, x0, x1);
+            while (bits) {
+              const int k = 32 * c + __ffs(bits) - 1;
+              bits &= bits - 1;
+              const float4 b = Q.bb[k];
+              if (b.w < pb.y || b.y > pb.w || b.z < pb.x || b.x > pb.z) continue;
+              const int l = Q.nxt[k];
+              const double ax = Q.x[k], ay = Q.y[k], bx = Q.x[l], by = Q.y[l];
+              const double sx = bx - ax, sy = by - ay;
+              const double den = rx * sy - ry * sx;
+              const double apx = ax - px, apy = ay - py;
+              const double tn = apx * sy - apy * sx;
+              const double un = apx * ry - apy * rx;
+              if (den == 0.0) {
+                unclean |= tn == 0.0 || un == 0.0;  // collinear
+                continue;
+              }
+              // t = tn / den and u = un / den, with the signs of den folded in
+              const double d = fabs(den), tol = 1e-9 * d;
+              const double tt = den > 0.0 ? tn : -tn, uu = den > 0.0 ? un : -un;
+              if (tt < -tol || tt > d + tol || uu < -tol || uu > d + tol) continue;  // next_crossing rejects it
+              const double sl = fabs(sx) + fabs(sy);
+              if (!(tt > tol && tt < d - tol && uu > tol && uu < d - tol && d > 1e-6 * rl * sl)) {
+                unclean = true;
+                continue;
+              }
+              if constexpr (kArea) err += 2.0 * ((rl + sl) * rl * sl / d);  // seen from both edges
+              const double t = tn / den, u = un / den;  // next_crossing's t from either edge
+              // den > 0: P's edge goes from the left of Q's edge to its right,
+              // out of Q where Q's material is on the left, and Q's edge the
+              // other way
+              const bool leaves = (den > 0.0) == (Q.sgn[k] > 0);
+              const double st = leaves ? -t : t;
+              c0 += leaves ? -1 : 1;
+              c1 += st;
+              c2 += st * t;
+              tfirst = fmin(tfirst, t);
+              m++;
+              const uint32_t x = atomicAdd(&X.count, 1u);
+              if (x < (uint32_t)bwd_crossings(V)) {
+                X.u[x] = (den < 0.0) == material_left ? -u : u;
+                X.next[x] = (uint16_t)atomicExch(&X.head[k], x + 1);
+              } else {
+                unclean = true;
+              }
+            }
+          }
+        }
+        exact = __any_sync(kFullMask, unclean);
+        if constexpr (kArea) {
+          if (exact) return false;
+        }
+      } else if (half == 1 && !exact && valid) {
+        for (uint32_t x = X.head[i]; x;) {
+          const double st = X.u[x - 1], t = fabs(st);
+          c0 += st < 0.0 ? -1 : 1;
+          c1 += st;
+          c2 += st * t;
+          tfirst = fmin(tfirst, t);
+          m++;
+          x = X.next[x - 1];
+        }
+      }
+      double it = 0.0, i1 = 0.0;
+      if (!exact) {
+        const int rs = valid ? P.rst[i] : i;  // this edge's ring starts at edge rs
+        // the first interval of each ring starting in this round, by its
+        // midpoint: the whole warp tests it against all edges of the other polygon
+        const bool rstart = valid && rs == i;
+        double mx0 = 0.0, my0 = 0.0;
+        if (rstart) {
+          const double tm = 0.5 * tfirst;
+          mx0 = px + tm * rx;
+          my0 = py + tm * ry;
+        }
+        bool first = false;
+        for (unsigned q = __ballot_sync(kFullMask, rstart); q; q &= q - 1) {
+          const int L = __ffs(q) - 1;
+          const double mxl = __shfl_sync(kFullMask, mx0, L), myl = __shfl_sync(kFullMask, my0, L);
+          bool in = false;
+          for (int k = lane; k < nq; k += 32) {
             const int l = Q.nxt[k];
-            const double ax = Q.x[k], ay = Q.y[k], bx = Q.x[l], by = Q.y[l];
-            const double sx = bx - ax, sy = by - ay;
-            const double den = rx * sy - ry * sx;
-            const double apx = ax - px, apy = ay - py;
-            const double tn = apx * sy - apy * sx;
-            const double un = apx * ry - apy * rx;
-            if (den == 0.0) {
-              unclean |= tn == 0.0 || un == 0.0;  // collinear
-              continue;
-            }
-            // t = tn / den and u = un / den, with the signs of den folded in
-            const double d = fabs(den), tol = 1e-9 * d;
-            const double tt = den > 0.0 ? tn : -tn, uu = den > 0.0 ? un : -un;
-            if (tt < -tol || tt > d + tol || uu < -tol || uu > d + tol) continue;  // next_crossing rejects it
-            const double sl = fabs(sx) + fabs(sy);
-            if (!(tt > tol && tt < d - tol && uu > tol && uu < d - tol && d > 1e-6 * rl * sl)) {
-              unclean = true;
-              continue;
-            }
-            if constexpr (kArea) err += 2.0 * ((rl + sl) * rl * sl / d);  // seen from both edges
-            const double t = tn / den, u = un / den;  // next_crossing's t from either edge
-            // den > 0: P's edge goes from the left of Q's edge to its right,
-            // out of Q where Q's material is on the left, and Q's edge the
-            // other way
-            const bool leaves = (den > 0.0) == (Q.sgn[k] > 0);
-            const double st = leaves ? -t : t;
-            c0 += leaves ? -1 : 1;
-            c1 += st;
-            c2 += st * t;
-            tfirst = fmin(tfirst, t);
-            m++;
-            const uint32_t x = atomicAdd(&X.count, 1u);
-            if (x < (uint32_t)bwd_crossings(V)) {
-              X.u[x] = (den < 0.0) == material_left ? -u : u;
-              X.next[x] = (uint16_t)atomicExch(&X.head[k], x + 1);
-            } else {
-              unclean = true;
+            const double ay = Q.y[k], by = Q.y[l];
+            if ((ay > myl) != (by > myl)) {
+              const double ax = Q.x[k], bx = Q.x[l];
+              const double xi = ax + (myl - ay) * (bx - ax) / (by - ay);
+              if (mxl < xi) in = !in;
             }
           }
+          const bool inside = (__popc(__ballot_sync(kFullMask, in)) & 1) != 0;
+          if (lane == L) first = inside;
+        }
+        const unsigned odd = __ballot_sync(kFullMask, (m & 1) != 0);
+        const int from = rs > e0 ? rs - e0 : 0;
+        const int par = __popc(odd & lt & ~((1u << from) - 1u)) & 1;
+        const bool sf = __shfl_sync(kFullMask, first, from);
+        const bool st = (rs >= e0 ? sf : carry) != (par != 0);  // inside state at the edge's start
+        const bool end = st != ((m & 1) != 0);
+        carry = __shfl_sync(kFullMask, end, 31);
+        if (__any_sync(kFullMask, valid && (int)st + c0 != (int)end)) {
+          exact = true;
+          if constexpr (kArea) return false;
+        }
+        if (valid) {
+          const double s1 = end ? 1.0 : 0.0;
+          it = 0.5 * (s1 - c2);
+          i1 = (s1 - c1) - it;
         }
       }
-      exact = __any_sync(kFullMask, unclean);
+      if constexpr (!kArea) {
+        if (exact) {
+          if (masks != 1 - side) {
+            masks = 1 - side;
+            __syncwarp();
+            bwd_slabs(Q, nq, g, gx, W.slab);
+          }
+          if (valid)
+            bwd_edge_exact(Q, W.slab, nwq, ext[1 - side], g, gx, pb, px, py, rx, ry, side ? Ag : Bg, &it, &i1);
+        }
+      }
       if constexpr (kArea) {
-        if (exact) return false;
+        // it + i1 = sum (t1 - t0) over the inside intervals
+        if (valid) area2 += P.sgn[i] * (it + i1) * ((px - ox) * ry - (py - oy) * rx);
+        continue;
       }
-    } else if (half == 1 && !exact && valid) {
-      for (uint32_t x = X.head[i]; x;) {
-        const double st = X.u[x - 1], t = fabs(st);
-        c0 += st < 0.0 ? -1 : 1;
-        c1 += st;
-        c2 += st * t;
-        tfirst = fmin(tfirst, t);
-        m++;
-        x = X.next[x - 1];
-      }
-    }
-    double it = 0.0, i1 = 0.0;
-    if (!exact) {
-      const int rs = valid ? P.rst[i] : i;  // this edge's ring starts at edge rs
-      // the first interval of each ring starting in this round, by its
-      // midpoint: the whole warp tests it against all edges of the other polygon
-      const bool rstart = valid && rs == i;
-      double mx0 = 0.0, my0 = 0.0;
-      if (rstart) {
-        const double tm = 0.5 * tfirst;
-        mx0 = px + tm * rx;
-        my0 = py + tm * ry;
-      }
-      bool first = false;
-      for (unsigned q = __ballot_sync(kFullMask, rstart); q; q &= q - 1) {
-        const int L = __ffs(q) - 1;
-        const double mxl = __shfl_sync(kFullMask, mx0, L), myl = __shfl_sync(kFullMask, my0, L);
-        bool in = false;
-        for (int k = lane; k < nq; k += 32) {
-          const int l = Q.nxt[k];
-          const double ay = Q.y[k], by = Q.y[l];
-          if ((ay > myl) != (by > myl)) {
-            const double ax = Q.x[k], bx = Q.x[l];
-            const double xi = ax + (myl - ay) * (bx - ax) / (by - ay);
-            if (mxl < xi) in = !in;
-          }
-        }
-        const bool inside = (__popc(__ballot_sync(kFullMask, in)) & 1) != 0;
-        if (lane == L) first = inside;
-      }
-      const unsigned odd = __ballot_sync(kFullMask, (m & 1) != 0);
-      const int from = rs > e0 ? rs - e0 : 0;
-      const int par = __popc(odd & lt & ~((1u << from) - 1u)) & 1;
-      const bool sf = __shfl_sync(kFullMask, first, from);
-      const bool st = (rs >= e0 ? sf : carry) != (par != 0);  // inside state at the edge's start
-      const bool end = st != ((m & 1) != 0);
-      carry = __shfl_sync(kFullMask, end, 31);
-      if (__any_sync(kFullMask, valid && (int)st + c0 != (int)end)) {
-        exact = true;
-        if constexpr (kArea) return false;
-      }
+      // contributions: it to the end vertex j, i1 to the start vertex i; the
+      // lane of the next edge of the ring hands its start contribution over so
+      // the shared vertex takes one atomic per coordinate
+      double gxj = 0.0, gyj = 0.0, gxi = 0.0, gyi = 0.0;
       if (valid) {
-        const double s1 = end ? 1.0 : 0.0;
-        it = 0.5 * (s1 - c2);
-        i1 = (s1 - c1) - it;
+        const double s = P.sgn[i];
+        const double nx = w * s * ry, ny = -w * s * rx;
+        gxj = nx * it;
+        gyj = ny * it;
+        gxi = nx * i1;
+        gyi = ny * i1;
+      }
+      const int key = valid ? i : -1;                         // this edge's start vertex
+      const int kend = valid ? j : -2;                        // its end vertex
+      const int knext = __shfl_down_sync(kFullMask, key, 1);  // start vertex of the next lane's edge
+      const int kprev = __shfl_up_sync(kFullMask, kend, 1);   // end vertex of the previous lane's edge
+      const double hx = __shfl_down_sync(kFullMask, gxi, 1), hy = __shfl_down_sync(kFullMask, gyi, 1);
+      const bool take = lane < 31 && knext == kend;  // the next lane's i1 part goes with mine
+      const bool given = lane > 0 && kprev == key;   // mine went to the previous lane
+      if (take) {
+        gxj += hx;
+        gyj += hy;
+      }
+      double *gr = side ? gb : ga;
+      const int64_t vbase = side ? vb : va;
+      if (valid && (gxj != 0.0 || gyj != 0.0)) {
+        atomicAdd(&gr[2 * (vbase + j)], gxj);
+        atomicAdd(&gr[2 * (vbase + j) + 1], gyj);
+      }
+      if (valid && !given && (gxi != 0.0 || gyi != 0.0)) {
+        atomicAdd(&gr[2 * (vbase + i)], gxi);
+        atomicAdd(&gr[2 * (vbase + i) + 1], gyi);
       }
     }
-    if constexpr (!kArea) {
-      if (exact) {
-        if (masks != 1 - side) {
-          masks = 1 - side;
-          __syncwarp();
-          bwd_slabs(Q, nq, g, gx, W.slab);
-        }
-        if (valid)
-          bwd_edge_exact(Q, W.slab, nwq, ext[1 - side], g, gx, pb, px, py, rx, ry, side ? Ag : Bg, &it, &i1);
-      }
-    }
-    if constexpr (kArea) {
-      // it + i1 = sum (t1 - t0) over the inside intervals
-      if (valid) area2 += P.sgn[i] * (it + i1) * ((px - ox) * ry - (py - oy) * rx);
-      continue;
-    }
-    // contributions: it to the end vertex j, i1 to the start vertex i; the
-    // lane of the next edge of the ring hands its start contribution over so
-    // the shared vertex takes one atomic per coordinate
-    double gxj = 0.0, gyj = 0.0, gxi = 0.0, gyi = 0.0;
-    if (valid) {
-      const double s = P.sgn[i];
-      const double nx = w * s * ry, ny = -w * s * rx;
-      gxj = nx * it;
-      gyj = ny * it;
-      gxi = nx * i1;
-      gyi = ny * i1;
-    }
-    const int key = valid ? i : -1;                         // this edge's start vertex
-    const int kend = valid ? j : -2;                        // its end vertex
-    const int knext = __shfl_down_sync(kFullMask, key, 1);  // start vertex of the next lane's edge
-    const int kprev = __shfl_up_sync(kFullMask, kend, 1);   // end vertex of the previous lane's edge
-    const double hx = __shfl_down_sync(kFullMask, gxi, 1), hy = __shfl_down_sync(kFullMask, gyi, 1);
-    const bool take = lane < 31 && knext == kend;  // the next lane's i1 part goes with mine
-    const bool given = lane > 0 && kprev == key;   // mine went to the previous lane
-    if (take) {
-      gxj += hx;
-      gyj += hy;
-    }
-    double *gr = side ? gb : ga;
-    const int64_t vbase = side ? vb : va;
-    if (valid && (gxj != 0.0 || gyj != 0.0)) {
-      atomicAdd(&gr[2 * (vbase + j)], gxj);
-      atomicAdd(&gr[2 * (vbase + j) + 1], gyj);
-    }
-    if (valid && !given && (gxi != 0.0 || gyi != 0.0)) {
-      atomicAdd(&gr[2 * (vbase + i)], gxi);
-      atomicAdd(&gr[2 * (vbase + i) + 1], gyi);
-    }
-  }
-  __syncwarp();  // the crossings of the first half, for the second
+    __syncwarp();  // the crossings of the first half, for the second
   }
   if constexpr (kArea) {
     acc->area = area2;

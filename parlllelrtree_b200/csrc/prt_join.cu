@@ -13,9 +13,9 @@
 // first and written at their places by a second launch, so that frontiers and
 // pairs stay in (query, entry) order and need no sort (prt_join_begin).  Window
 // counts visit the tree depth first instead, a warp per query with the
-// counters in registers (counts_kernel).  The last two prune: a query
-// that contains the box of an entry intersects every record below it, so nothing
-// below is tested.
+// counters in registers (counts_kernel).  The last two prune: a query that
+// contains the box of an entry intersects every record below it, so nothing below
+// is tested.
 #include <cuda_runtime.h>
 
 #include <algorithm>

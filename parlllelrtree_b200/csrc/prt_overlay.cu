@@ -9,6 +9,8 @@
 //            into size bins; each bin is ONE persistent launch whose workers
 //            own a fixed arena slice and take the next 32 pairs per warp from
 //            an atomic ticket, so a warp's lanes clip pairs of similar cost.
+//            All operations but XOR first trace the pairs in general position
+//            (prt_trace.cuh); the bins then hold what that left.
 // Results go to shared pools through atomic bump reservations (contours and
 // vertices), the device analogue of the reference's per-pair device malloc
 // (GPC:703-718).  Pairs whose slice or pool reservation was too small are
@@ -747,8 +749,8 @@ static int run_batched(OverlayState &st, const int64_t *d_idx, int64_t count, in
   int64_t counts[PRT_MAX_BINS];
   for (int b = 0; b < nb; b++) counts[b] = hb[b + 1] - hb[b];
   // Too few pairs to keep the GPU busy one per thread (under half a wave of
-  // the thread-only launch, e.g. the 2 x 10,000-star overlay's ~21k pairs in
-  // ~650 warps): clip every pair with a whole warp instead, so there are as
+  // the thread-only launch, e.g. an exclusive or of 2 x 10,000 stars, ~21k pairs
+  // in ~650 warps): clip every pair with a whole warp instead, so there are as
   // many warps as pairs.  Both clippers give the same output.
   constexpr int64_t kFewWarps = (int64_t)kSMs * kLptThreadWarpsPerSM / 2;
   prt_schedule run_sc = sc, few_sc = sc;
