@@ -9,8 +9,8 @@
 //            into size bins; each bin is ONE persistent launch whose workers
 //            own a fixed arena slice and take the next 32 pairs per warp from
 //            an atomic ticket, so a warp's lanes clip pairs of similar cost.
-//            All operations but XOR first trace the pairs in general position
-//            (prt_trace.cuh); the bins then hold what that left.
+//            Pairs in general position are traced first (prt_trace.cuh); the
+//            bins then hold what that left.
 // Results go to shared pools through atomic bump reservations (contours and
 // vertices), the device analogue of the reference's per-pair device malloc
 // (GPC:703-718).  Pairs whose slice or pool reservation was too small are
@@ -21,6 +21,7 @@
 #include <vector>
 
 #include <mutex>
+#include <type_traits>
 
 #include "prt_gpc.cuh"
 #include "prt_internal.cuh"
@@ -282,7 +283,7 @@ __global__ void __launch_bounds__(32, kLptThreadWarpsPerSM)
   lpt_body<false>(S, O, order, plan, tickets, arena, scale, nullptr, rest);
 }
 
-// All operations but XOR by tracing (prt_trace.cuh): one block per pair of the sorted
+// Pairs by tracing (prt_trace.cuh): one block per pair of the sorted
 // positions [begin, end), largest pairs first, from one ticket.  A pair that is
 // not traced goes to its bin's part of left_order for the launch above.
 template <typename C>
@@ -700,9 +701,8 @@ static int run_batched(OverlayState &st, const int64_t *d_idx, int64_t count, in
     unsigned long long left[PRT_MAX_BINS];  // pairs of each bin that were not traced
   } h;
   static_assert(sizeof(Head) <= 512, "head block");
-  const bool trace_pairs = st.S.op != PRT_GPC_XOR;
   unsigned char *scr = nullptr;
-  int rc = dmalloc(reinterpret_cast<void **>(&scr), 512 + 20 * n + (trace_pairs ? 4 * n : 0), s);
+  int rc = dmalloc(reinterpret_cast<void **>(&scr), 512 + 24 * n, s);
   if (rc) return rc;
   Head *d = reinterpret_cast<Head *>(scr);
   uint32_t *k0 = reinterpret_cast<uint32_t *>(scr + 512);
@@ -710,10 +710,10 @@ static int run_batched(OverlayState &st, const int64_t *d_idx, int64_t count, in
   cudaMemsetAsync(scr, 0, 512, s);
   BinThresholds T;
   for (int b = 0; b < nb; b++) T.thr[b] = sc.bin_thresholds[b];
-  const int64_t cls_verts[trace::kClasses] = {trace::Class3::kVerts, trace::Class2::kVerts, trace::Class1::kVerts,
-                                              trace::Class0::kVerts};
+  const int64_t cls_verts[trace::kClasses] = {trace::Class3<0>::kVerts, trace::Class2<0>::kVerts,
+                                              trace::Class1<0>::kVerts, trace::Class0<0>::kVerts};
   for (int c = 0; c < trace::kClasses; c++) T.thr[nb + c] = cls_verts[c];
-  const int cuts = nb + (trace_pairs ? trace::kClasses : 0);
+  const int cuts = nb + trace::kClasses;
   const int g = grid_for(n, 256, 16);
   {
     PRT_PROF("size_key", s);
@@ -749,8 +749,8 @@ static int run_batched(OverlayState &st, const int64_t *d_idx, int64_t count, in
   int64_t counts[PRT_MAX_BINS];
   for (int b = 0; b < nb; b++) counts[b] = hb[b + 1] - hb[b];
   // Too few pairs to keep the GPU busy one per thread (under half a wave of
-  // the thread-only launch, e.g. an exclusive or of 2 x 10,000 stars, ~21k pairs
-  // in ~650 warps): clip every pair with a whole warp instead, so there are as
+  // the thread-only launch, e.g. the 2 x 10,000-star overlay's ~21k pairs in ~650
+  // warps): clip every pair with a whole warp instead, so there are as
   // many warps as pairs.  Both clippers give the same output.
   constexpr int64_t kFewWarps = (int64_t)kSMs * kLptThreadWarpsPerSM / 2;
   prt_schedule run_sc = sc, few_sc = sc;
@@ -769,7 +769,7 @@ static int run_batched(OverlayState &st, const int64_t *d_idx, int64_t count, in
   if (bytes > kArenaBudgetLeast) bytes = plan_bins(run_sc, counts, hm, arena_budget(), plan, &smem, scale, true);
   // What tracing leaves may be few pairs out of many: that is known on the device
   // alone, so both launches are made and one of them ends at once.
-  const bool both = trace_pairs && thread_warps >= kFewWarps;
+  const bool both = thread_warps >= kFewWarps;
   if (both) bytes = std::max(bytes, plan_bins(few_sc, counts, hm, bytes, few, &few_smem, scale, true));
   for (int p = 0; p < (both ? 2 : 1); p++) {
     BinPlan &pl = p ? few : plan;
@@ -784,31 +784,37 @@ static int run_batched(OverlayState &st, const int64_t *d_idx, int64_t count, in
   if (!rc) rc = prepare_lpt_launch(std::max(smem, few_smem));
   if (!rc && warps > 0) rc = dmalloc(reinterpret_cast<void **>(&arena), bytes, s);
   TraceRest rest = {nullptr, 0, 0, 0};
-  if (!rc && warps > 0 && trace_pairs) {
+  if (!rc && warps > 0) {
     PRT_PROF("trace", s);
     const int64_t *cut = h.bnd + nb;
-    rc = launch_trace<trace::Class3>(st.S, st.O, order, 0, cut[1], plan, &d->trace_tickets[0], left_order, d->left, s);
-    if (!rc)
-      rc = launch_trace<trace::Class2>(st.S, st.O, order, cut[1], cut[2], plan, &d->trace_tickets[1], left_order,
-                                       d->left, s);
-    if (!rc)
-      rc = launch_trace<trace::Class1>(st.S, st.O, order, cut[2], cut[3], plan, &d->trace_tickets[2], left_order,
-                                       d->left, s);
-    if (!rc)
-      rc = launch_trace<trace::Class0>(st.S, st.O, order, cut[3], n, plan, &d->trace_tickets[3], left_order, d->left, s);
+    auto go = [&](auto two) {
+      constexpr int kTwo = decltype(two)::value;
+      int e = launch_trace<trace::Class3<kTwo>>(st.S, st.O, order, 0, cut[1], plan, &d->trace_tickets[0], left_order,
+                                                d->left, s);
+      if (!e)
+        e = launch_trace<trace::Class2<kTwo>>(st.S, st.O, order, cut[1], cut[2], plan, &d->trace_tickets[1], left_order,
+                                              d->left, s);
+      if (!e)
+        e = launch_trace<trace::Class1<kTwo>>(st.S, st.O, order, cut[2], cut[3], plan, &d->trace_tickets[2], left_order,
+                                              d->left, s);
+      if (!e)
+        e = launch_trace<trace::Class0<kTwo>>(st.S, st.O, order, cut[3], n, plan, &d->trace_tickets[3], left_order,
+                                              d->left, s);
+      return e;
+    };
+    rc = st.S.op == PRT_GPC_XOR ? go(std::integral_constant<int, 1>{}) : go(std::integral_constant<int, 0>{});
     rest = {d->left, thread_bins, both ? kFewWarps : 0, INT64_MAX};
   }
   if (!rc && warps > 0) {
     PRT_PROF("clip_batched", s);
-    const uint32_t *todo = trace_pairs ? left_order : order;
     if (plan.thread_only)
-      clip_lpt_thread_kernel<<<(unsigned)warps, 32, 0, s>>>(st.S, st.O, todo, plan, d->tickets, arena, scale, rest);
+      clip_lpt_thread_kernel<<<(unsigned)warps, 32, 0, s>>>(st.S, st.O, left_order, plan, d->tickets, arena, scale, rest);
     else
-      clip_lpt_kernel<<<(unsigned)warps, 32, smem, s>>>(st.S, st.O, todo, plan, d->tickets, arena, scale, nullptr, rest);
+      clip_lpt_kernel<<<(unsigned)warps, 32, smem, s>>>(st.S, st.O, left_order, plan, d->tickets, arena, scale, nullptr, rest);
     if (both) {
       rest.min_warps = 0;
       rest.max_warps = kFewWarps;
-      clip_lpt_kernel<<<(unsigned)few.warp0[nb], 32, few_smem, s>>>(st.S, st.O, todo, few, d->rest_tickets, arena, scale,
+      clip_lpt_kernel<<<(unsigned)few.warp0[nb], 32, few_smem, s>>>(st.S, st.O, left_order, few, d->rest_tickets, arena, scale,
                                                                    nullptr, rest);
     }
   }

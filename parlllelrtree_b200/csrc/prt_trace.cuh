@@ -1,6 +1,5 @@
-// Intersection, difference and union of a pair in general position by tracing, with
-// the result that the scanbeam clippers (prt_gpc.cuh, prt_wgpc.cuh) give, bit for
-// bit.  (An exclusive or passes every crossing twice and stays with them.)
+// Overlay of a pair in general position by tracing, with the result that the scanbeam clippers (prt_gpc.cuh, prt_wgpc.cuh) give, bit for
+// bit.
 //
 // GPC sweeps the pair beam by beam (a beam: two neighbouring vertex ys), a chain
 // of dependent steps per beam however little happens in it.  When nothing
@@ -12,7 +11,8 @@
 //  * the boundary runs along A where A is inside B and along B where B is inside
 //    A (outside for a union, and of a difference along B backwards) and changes
 //    over at every crossing, so the contours are cycles of runs of consecutive
-//    vertices between crossings;
+//    vertices between crossings; an exclusive or keeps every run, and at a crossing
+//    one contour ends below and another starts above;
 //  * GPC's vertex lists grow to the left and right and are joined at maxima, so a
 //    contour comes out cut at its highest vertex: that vertex is the last one
 //    written of an outer contour and the first one of a hole;
@@ -69,10 +69,11 @@ __device__ __forceinline__ bool bany(bool v) {
 // Room for one class of pairs: NT threads per pair; at most kVerts vertices and
 // kCross crossings; 2^kSlabShift vertex ys per slab of the edge search; kList edges over
 // all slabs, and nodes over all contours.
-template <int NT_, int kVerts_, int kCross_, int kSlabShift_, int kList_, int kBlocks_>
+template <int NT_, int kVerts_, int kCross_, int kSlabShift_, int kList_, int kBlocks_, int kTwo_>
 struct Class {
   static constexpr int NT = NT_, kVerts = kVerts_, kCross = kCross_, kSlabShift = kSlabShift_, kList = kList_;
   static constexpr int kBlocks = kBlocks_;  // resident per SM
+  static constexpr int kTwo = kTwo_;        // 1: exclusive or (an instantiation of its own costs the others nothing)
   static constexpr int kSlabs = (kVerts >> kSlabShift) + 1;
   static constexpr int kContours = kCross / 2 + kMaxRings;
   static_assert(kList >= kVerts && kCross >= 2 * kMaxRings && kCross < 4095 && kVerts <= kLast &&
@@ -114,6 +115,11 @@ struct Pair {
   int n;
   double margin, least;
   bool convex;
+  // an exclusive or has two nodes per crossing: 2c where contours end below it,
+  // 2c + 1 where they start above
+  static constexpr int two = C::kTwo;
+  __device__ __forceinline__ int crossing(int node) const { return (node & 0x7fff) >> two; }
+  __device__ __forceinline__ bool up(int v) const { return S.rank[nxt(v)] > S.rank[v]; }
   __device__ __forceinline__ double x(int v) const { return S.vx[v]; }
   __device__ __forceinline__ double y(int v) const { return S.sy[S.rank[v]]; }
   __device__ __forceinline__ int nxt(int v) const {
@@ -252,18 +258,26 @@ __device__ __forceinline__ bool test_edges(const Pair<C> &P, const TEdge &a, con
 // Order of a node in GPC's sweep: vertices by their y, crossings after the
 // vertex below them by their y in the beam.
 template <typename C>
-__device__ __forceinline__ uint32_t node_key(const Smem<C> &S, int node) {
-  return node & 0x8000 ? ((uint32_t)S.beam[node & 0x7fff] << 12) + 1u + S.ord[node & 0x7fff]
-                       : (uint32_t)S.rank[node] << 12;
+__device__ __forceinline__ uint32_t node_key(const Pair<C> &P, int node) {
+  if (!(node & 0x8000)) return (uint32_t)P.S.rank[node] << 12;
+  const int c = P.crossing(node);
+  return ((uint32_t)P.S.beam[c] << 12) + 1u + ((uint32_t)P.S.ord[c] << P.two) + (node & P.two);
 }
 
-// Whether the material lies below a contour's local maximum (node m).
+// Whether the result lies below a contour's local maximum (node m, next: the node
+// that follows it).
 template <typename C>
-__device__ __forceinline__ bool max_is_outer(const Pair<C> &P, int m) {
-  if (m & 0x8000) return P.convex;  // one quadrant at a crossing belongs to the result, of a union three
+__device__ __forceinline__ bool max_is_outer(const Pair<C> &P, int m, int next) {
+  if (m & 0x8000) {
+    // one quadrant at a crossing belongs to the result, of a union three, of an
+    // exclusive or two: below it goes on along the left edge when they are the
+    // lower and the upper one
+    const int c = P.crossing(m);
+    return P.two ? P.S.out[c] == (P.S.aleft[c] ? 0 : 1) : P.convex;
+  }
   const TEdge e1 = edge_of(P, m), e0 = edge_of(P, P.prv(m));
-  const bool fwd = P.S.mat[P.S.ring[m]];
-  // material on the left: below when the boundary comes up the right edge (the
+  const bool fwd = next & 0x8000 ? P.S.ce[P.S.rside[P.S.ring[m]]][P.crossing(next)] == m : next == P.nxt(m);
+  // the result on the left: below when the boundary comes up the right edge (the
   // one with the smaller slope) and goes down the left one
   return fwd ? e0.dx < e1.dx : e1.dx < e0.dx;
 }
@@ -375,7 +389,7 @@ __device__ int trace_pair(Smem<C> &S, int op, const gpc::PolyView &A, const gpc:
   if (na + nb > kMaxRings) return kLeft;
   // ---- rings whose boxes meet a ring of the other polygon (minimax_test,
   // GPC:1656-1709); the others take no part (a difference keeps the subject's, a
-  // union all)
+  // union and an exclusive or keep all)
   for (int r = 0; r < na + nb; r++) {
     const gpc::PolyView &p = r < na ? A : B;
     const int64_t g = r < na ? A.r0 + r : B.r0 + (r - na);
@@ -399,7 +413,7 @@ __device__ int trace_pair(Smem<C> &S, int op, const gpc::PolyView &A, const gpc:
   double most = 0.0, most_x = 0.0, wide = 0.0, ymin = gpc::kDblMax, ymax = -gpc::kDblMax;
   int n = 0, nr = 0;
   for (int r = 0; r < na + nb; r++) {
-    bool meets = op == PRT_GPC_UNION || (op == PRT_GPC_DIFF && r < na);
+    bool meets = op == PRT_GPC_UNION || op == PRT_GPC_XOR || (op == PRT_GPC_DIFF && r < na);
     for (int q = r < na ? na : 0; q < (r < na ? na + nb : na); q++)
       meets |= r < na ? gpc::bbox_overlap(S.rbb[r], S.rbb[q]) : gpc::bbox_overlap(S.rbb[q], S.rbb[r]);
     if (!meets) continue;
@@ -633,14 +647,18 @@ __device__ int trace_pair(Smem<C> &S, int op, const gpc::PolyView &A, const gpc:
     // polygon 0's boundary enters polygon 1 here: the boundary of an intersection
     // goes on along polygon 0, else along polygon 1; of a union the other way round
     const bool same = (up[0] == (S.mat[ring[0]] != 0)) == (up[1] == (S.mat[ring[1]] != 0));
-    S.out[c] = ((same != (S.aleft[c] != 0)) != (op == PRT_GPC_UNION)) ? 0 : 1;
+    // of an exclusive or along the left edge, up and down, when the quadrant below
+    // belongs to the result, else along the right one
+    S.out[c] = ((same != (S.aleft[c] != 0)) != (op == PRT_GPC_UNION || op == PRT_GPC_XOR)) ? 0 : 1;
   }
   if (bany<NT>(bad)) return kLeft;
-  // the run that starts at each crossing: its vertices and the crossing at its end
-  for (int c = tid; c < nx; c += NT) {
-    const int s = S.out[c], e = S.ce[s][c], r = S.ring[e], p = S.pos[s][c];
+  // the run that starts at each crossing node: its vertices and the node at its end
+  const int nodes = nx << P.two;
+  if (nodes > C::kCross) return kLeft;
+  for (int t = tid; t < nodes; t += NT) {
+    const int c = t >> P.two, s = S.out[c], e = S.ce[s][c], r = S.ring[e], p = S.pos[s][c];
     const int len = S.rstart[r + 1] - S.rstart[r];
-    const bool fwd = S.mat[r];
+    const bool fwd = P.two ? (t & 1) == (int)P.up(e) : S.mat[r] != 0;
     int q = fwd ? p + 1 : p - 1;
     bool wrap = q < 0 || q >= nx || S.ring[S.ce[s][S.seq[s][q]]] != r;
     if (wrap) {  // the ring's first or last crossing
@@ -649,8 +667,8 @@ __device__ int trace_pair(Smem<C> &S, int op, const gpc::PolyView &A, const gpc:
         q += fwd ? -1 : 1;
     }
     const int d = S.seq[s][q], f = S.ce[s][d];
-    S.next[c] = (uint16_t)d;
-    S.cnt[c] = (uint16_t)((fwd ? f - e : e - f) + (wrap ? len : 0));
+    S.next[t] = (uint16_t)(d << P.two | (P.two && fwd != P.up(f)));
+    S.cnt[t] = (uint16_t)((fwd ? f - e : e - f) + (wrap ? len : 0));
     // the polygons' boundaries enter and leave each other in turn
     if (S.out[d] == s) bad = true;
   }
@@ -658,8 +676,8 @@ __device__ int trace_pair(Smem<C> &S, int op, const gpc::PolyView &A, const gpc:
   // ---- contours: cycles of runs, then whole rings inside the other polygon
   if (tid == 0) {
     int at = 0, nc = 0;
-    for (int c = 0; c < nx; c++) S.cyc[c] = 255;
-    for (int c = 0; c < nx && nc < C::kContours && nc < 250; c++) {
+    for (int c = 0; c < nodes; c++) S.cyc[c] = 255;
+    for (int c = 0; c < nodes && nc < C::kContours && nc < 250; c++) {
       if (S.cyc[c] != 255) continue;
       S.head[nc] = (uint16_t)at;
       for (int d = c; S.cyc[d] == 255; d = S.next[d]) {
@@ -670,7 +688,7 @@ __device__ int trace_pair(Smem<C> &S, int op, const gpc::PolyView &A, const gpc:
       S.len[nc] = (uint16_t)(at - S.head[nc]);
       nc++;
     }
-    for (int c = 0; c < nx; c++)
+    for (int c = 0; c < nodes; c++)
       bad |= S.cyc[c] == 255;
     S.ncont = nc;
     S.nodes = at;
@@ -682,24 +700,25 @@ __device__ int trace_pair(Smem<C> &S, int op, const gpc::PolyView &A, const gpc:
     if (S.hit[r]) continue;
     const int side = S.rside[r];
     const bool wanted = op != PRT_GPC_UNION && (op != PRT_GPC_DIFF || side == 1);  // inside, else outside
-    if (inside_rings(P, S.rstart[r], [&](int q) { return S.rside[q] != side; }) != wanted) continue;
+    const bool inside = inside_rings(P, S.rstart[r], [&](int q) { return S.rside[q] != side; });
+    if (!P.two && inside != wanted) continue;
     const int len = S.rstart[r + 1] - S.rstart[r];
     if (nc >= C::kContours || total + len > C::kList) return kLeft;
     if (tid == 0) {
       S.head[nc] = (uint16_t)total;
       S.len[nc] = (uint16_t)len;
     }
-    const bool fwd = S.mat[r];
+    const bool fwd = (S.mat[r] != 0) != (P.two && inside);
     for (int k = tid; k < len; k += NT)
       S.list[total + k] = (uint16_t)(fwd ? S.rstart[r] + k : S.rstart[r + 1] - 1 - k);
     total += len;
     nc++;
   }
-  for (int c = warp; c < nx; c += kWarps) {
-    const int s = S.out[c], e = S.ce[s][c], r = S.ring[e], r0 = S.rstart[r], r1 = S.rstart[r + 1];
-    const int at = S.runoff[c], m = S.cnt[c];
-    if (lane == 0) S.list[at] = (uint16_t)(0x8000 | c);
-    if (S.mat[r]) {
+  for (int t = warp; t < nodes; t += kWarps) {
+    const int c = t >> P.two, s = S.out[c], e = S.ce[s][c], r = S.ring[e], r0 = S.rstart[r], r1 = S.rstart[r + 1];
+    const int at = S.runoff[t], m = S.cnt[t];
+    if (lane == 0) S.list[at] = (uint16_t)(0x8000 | t);
+    if (P.two ? (t & 1) == (int)P.up(e) : S.mat[r] != 0) {
       for (int k = lane; k < m; k += 32) {
         const int v = e + 1 + k;
         S.list[at + 1 + k] = (uint16_t)(v < r1 ? v : v - (r1 - r0));
@@ -717,7 +736,7 @@ __device__ int trace_pair(Smem<C> &S, int op, const gpc::PolyView &A, const gpc:
   if (nc == 1) {  // the usual case, all threads on it
     uint32_t best = 0, at = 0;
     for (int k = tid; k < S.len[0]; k += NT) {
-      const uint32_t key = node_key(S, S.list[k]);
+      const uint32_t key = node_key(P, S.list[k]);
       if (key >= best) {
         best = key;
         at = k;
@@ -729,20 +748,20 @@ __device__ int trace_pair(Smem<C> &S, int op, const gpc::PolyView &A, const gpc:
     bsync<NT>();
     if (tid == 0) {
       S.top[0] = (uint16_t)S.best;
-      S.hole[0] = !max_is_outer(P, S.list[S.top[0]]);
+      S.hole[0] = !max_is_outer(P, S.list[S.top[0]], S.list[S.top[0] + 1 < S.len[0] ? S.top[0] + 1 : 0]);
       S.rep[0] = 0;
     }
   }
   for (int c = warp; c < nc && nc > 1; c += kWarps) {
     const int h = S.head[c], m = S.len[c];
     uint32_t best = 0;
-    for (int k = lane; k < m; k += 32) best = max(best, node_key(S, S.list[h + k]));
+    for (int k = lane; k < m; k += 32) best = max(best, node_key(P, S.list[h + k]));
     best = __reduce_max_sync(0xffffffffu, best);
     int at = 0;
     for (int k = lane; k < m; k += 32)
-      if (node_key(S, S.list[h + k]) == best) at = k;
+      if (node_key(P, S.list[h + k]) == best) at = k;
     at = __reduce_max_sync(0xffffffffu, at);
-    const bool outer = max_is_outer(P, S.list[h + at]);
+    const bool outer = max_is_outer(P, S.list[h + at], S.list[h + (at + 1 < m ? at + 1 : 0)]);
     uint32_t rep = 0;
     // the part of the cycle between two maxima that holds the minimum: at the
     // highest maximum inside it the side that survives the join
@@ -752,9 +771,9 @@ __device__ int trace_pair(Smem<C> &S, int op, const gpc::PolyView &A, const gpc:
       uint32_t bk = 0;
       uint32_t low = 0xffffffffu;
       for (int o = lo + lane; o <= hi; o += 32) {
-        const uint32_t k = node_key(S, node(o));
+        const uint32_t k = node_key(P, node(o));
         low = min(low, k);
-        if (o > lo && o < hi && k > node_key(S, node(o - 1)) && k > node_key(S, node(o + 1))) bk = max(bk, k);
+        if (o > lo && o < hi && k > node_key(P, node(o - 1)) && k > node_key(P, node(o + 1))) bk = max(bk, k);
       }
       bk = __reduce_max_sync(0xffffffffu, bk);
       if (bk == 0) {
@@ -763,9 +782,9 @@ __device__ int trace_pair(Smem<C> &S, int op, const gpc::PolyView &A, const gpc:
       }
       int q = 0;
       for (int o = lo + lane; o <= hi; o += 32)
-        if (node_key(S, node(o)) == bk) q = o;
+        if (node_key(P, node(o)) == bk) q = o;
       q = __reduce_max_sync(0xffffffffu, q);
-      if (max_is_outer(P, node(q))) hi = q - 1;
+      if (max_is_outer(P, node(q), node(q + 1))) hi = q - 1;
       else lo = q + 1;
     }
     if (lane == 0) {
@@ -797,8 +816,8 @@ __device__ int trace_pair(Smem<C> &S, int op, const gpc::PolyView &A, const gpc:
         const int o = S.top[c] + (S.hole[c] ? m - w : m - 1 - w);
         return (int)S.list[h + o % m];
       };
-      auto px = [&](int v) { return v & 0x8000 ? S.cx[v & 0x7fff] : P.x(v); };
-      auto py = [&](int v) { return v & 0x8000 ? S.cy[v & 0x7fff] : P.y(v); };
+      auto px = [&](int v) { return v & 0x8000 ? S.cx[P.crossing(v)] : P.x(v); };
+      auto py = [&](int v) { return v & 0x8000 ? S.cy[P.crossing(v)] : P.y(v); };
       const double x0 = px(node(0)), y0 = py(node(0));
       double a = 0.0;
       for (int w = tid; w < m; w += NT) {
@@ -858,8 +877,8 @@ __device__ int trace_pair(Smem<C> &S, int op, const gpc::PolyView &A, const gpc:
       if (o >= m) o -= m;
       const int v = S.list[h + o];
       double2 q;
-      q.x = v & 0x8000 ? S.cx[v & 0x7fff] : P.x(v);
-      q.y = v & 0x8000 ? S.cy[v & 0x7fff] : P.y(v);
+      q.x = v & 0x8000 ? S.cx[P.crossing(v)] : P.x(v);
+      q.y = v & 0x8000 ? S.cy[P.crossing(v)] : P.y(v);
       reinterpret_cast<double2 *>(O.xy)[v0 + w] = q;
     }
   }
@@ -868,10 +887,14 @@ __device__ int trace_pair(Smem<C> &S, int op, const gpc::PolyView &A, const gpc:
 
 // Pairs of up to 128 vertices in all (1,024; 4,160: one polygon of the 4,096 that
 // the uneven layers go up to with a small one; 8,448: two of them).
-using Class0 = Class<32, 128, 64, 3, 352, 20>;
-using Class1 = Class<128, 1024, 256, 3, 3 * 1024, 4>;
-using Class2 = Class<256, 4160, 256, 3, 4160 * 13 / 8, 2>;
-using Class3 = Class<512, 8448, 512, 3, 8448 * 3 / 2, 1>;
+template <int kTwo>
+using Class0 = Class<32, 128, 64, 3, 352, 20, kTwo>;
+template <int kTwo>
+using Class1 = Class<128, 1024, 256, 3, 3 * 1024, 4, kTwo>;
+template <int kTwo>
+using Class2 = Class<256, 4160, 256, 3, 4160 * 13 / 8, 2, kTwo>;
+template <int kTwo>
+using Class3 = Class<512, 8448, 512, 3, 8448 * 3 / 2, 1, kTwo>;
 constexpr int kClasses = 4;
 
 }  // namespace trace

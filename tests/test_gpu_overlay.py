@@ -275,11 +275,11 @@ def test_traced_on_a_grid(cuda):
         assert same_contours(got[i], oracle.gpc_clip(rings_of(A, i), rings_of(B, i), 1)), f"pair {i}"
 
 
-@pytest.mark.parametrize("op", [0, 3])
+@pytest.mark.parametrize("op", [0, 2, 3])
 @pytest.mark.parametrize("na,nb,hole_frac", [(3, 3, 0.0), (16, 15, 0.9), (64, 64, 0.9), (64, 65, 0.0), (512, 513, 0.9),
                                              (4096, 129, 0.9), (4352, 4096, 0.0)])
-def test_traced_difference_and_union(cuda, op, na, nb, hole_frac):
-    """The same pairs' difference and union, and polygons on a grid."""
+def test_traced_other_operations(cuda, op, na, nb, hole_frac):
+    """The same pairs' difference, exclusive or and union, and polygons on a grid."""
     import parlllelrtree_b200 as prt
 
     n = 64 if na + nb < 200 else 6
