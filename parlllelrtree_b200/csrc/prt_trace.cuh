@@ -229,6 +229,9 @@ __device__ __forceinline__ bool test_edges(const Pair<C> &P, const TEdge &a, con
   if (!(fabs(s0) > m && fabs(s1) > m)) return true;
   if ((s0 > 0.0) == (s1 > 0.0)) return false;
   if (S.rside[S.ring[a.v]] == S.rside[S.ring[b.v]]) return true;  // a polygon that crosses itself
+  // GPC takes edges of slopes within an epsilon for parallel (layers that are far
+  // taller than wide)
+  if (!(fabs(a.dx - b.dx) > 8.0 * gpc::kEps)) return true;
   // the beam of the crossing
   int k0 = lo, k1 = hi;
   double d0 = s0, d1 = s1;

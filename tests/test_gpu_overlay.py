@@ -298,3 +298,24 @@ def test_traced_other_operations(cuda, op, na, nb, hole_frac):
                       prt.Layer.from_dict(B), op=OPS[op]).contours()
     for i in range(n):
         assert same_contours(got[i], oracle.gpc_clip(rings_of(A, i), rings_of(B, i), op)), f"pair {i}"
+
+
+@pytest.mark.parametrize("op", [0, 1, 2, 3])
+@pytest.mark.parametrize("sx,sy", [(1.0, 1e9), (1e9, 1.0), (1e6, 1e6), (1e-9, 1.0), (1.0, 1e18), (1e-18, 1e-18)])
+def test_traced_scales(cuda, op, sx, sy):
+    """Polygons much wider or taller than the other way, very large and very small."""
+    import parlllelrtree_b200 as prt
+
+    n = 48
+    rng = np.random.default_rng(17)
+    c = rng.random((n, 2))
+    r = np.full(n, 0.01)
+    A = dg.star_layer(n, seed=3, nv_lo=4, nv_hi=30, centre_xy=c, radii=r, hole_frac=0.3)
+    B = dg.star_layer(n, seed=4, nv_lo=4, nv_hi=30, centre_xy=c + rng.uniform(-0.01, 0.01, (n, 2)), radii=r, hole_frac=0.3)
+    for L in (A, B):
+        L["xy"] = L["xy"] * np.array([sx, sy])
+    ids = np.arange(n, dtype=np.int32)
+    got = prt.overlay(torch.from_numpy(np.stack([ids, ids], axis=1)).cuda(), prt.Layer.from_dict(A),
+                      prt.Layer.from_dict(B), op=OPS[op]).contours()
+    for i in range(n):
+        assert same_contours(got[i], oracle.gpc_clip(rings_of(A, i), rings_of(B, i), op)), f"pair {i}"
