@@ -46,6 +46,10 @@ namespace trace {
 
 constexpr int kMaxRings = 32;
 constexpr int kLast = 0x8000;
+// Smallest |y| of a vertex that is not 0: two ys are then 1e-146 apart or equal, so
+// that neither the slopes nor the buckets per unit of y below overflow, and what a
+// product of an x and a y difference loses to underflow is far below the margin.
+constexpr double kLeastY = 1e-130;
 
 template <int NT>
 __device__ __forceinline__ void bsync() {
@@ -454,7 +458,7 @@ __device__ int trace_pair(Smem<C> &S, int op, const gpc::PolyView &A, const gpc:
       for (int v = v0 + tid; v < v1; v += NT) {
         const double x = S.rxy[r][2 * (v - v0)], y = S.rxy[r][2 * (v - v0) + 1];
         S.vx[v] = x;
-        bad |= !(fabs(x) <= most && fabs(y) <= most);  // NaN
+        bad |= !(fabs(x) <= most && fabs(y) <= most) || (y != 0.0 && fabs(y) < kLeastY);  // NaN; ys next to 0
         S.sy[v] = y;
         S.ring[v] = (uint8_t)r;
       }

@@ -319,3 +319,33 @@ def test_traced_scales(cuda, op, sx, sy):
                       prt.Layer.from_dict(B), op=OPS[op]).contours()
     for i in range(n):
         assert same_contours(got[i], oracle.gpc_clip(rings_of(A, i), rings_of(B, i), op)), f"pair {i}"
+
+
+def same_bits(a, b) -> bool:
+    return same_contours(a, b) and all(np.array_equal(np.signbit(v1), np.signbit(v2)) for (_, v1), (_, v2) in zip(a, b))
+
+
+def check_all(A, B, n, op):
+    import parlllelrtree_b200 as prt
+
+    ids = np.arange(n, dtype=np.int32)
+    got = prt.overlay(torch.from_numpy(np.stack([ids, ids], axis=1)).cuda(), prt.Layer.from_dict(A),
+                      prt.Layer.from_dict(B), op=OPS[op]).contours()
+    for i in range(n):
+        assert same_bits(got[i], oracle.gpc_clip(rings_of(A, i), rings_of(B, i), op)), f"pair {i}"
+
+
+@pytest.mark.parametrize("op", [0, 1, 2, 3])
+@pytest.mark.parametrize("na,nb,sx,sy", [(60, 40, 1e-9, 1e-307), (300, 40, 1e-9, 1e-307), (1500, 100, 1e-9, 1e-306),
+                                         (4500, 300, 1e-9, 1e-306), (30, 20, 1e140, 1e-150), (30, 20, 1.0, 1e-131)])
+def test_ys_next_to_zero(cuda, op, na, nb, sx, sy):
+    """Pairs of every tracing class whose y extent is next to nothing, where
+    vertices per unit of y are beyond the largest double."""
+    n = 24 if na < 100 else 4
+    rng = np.random.default_rng(na)
+    c = np.zeros((n, 2))
+    A = dg.star_layer(n, seed=na, nv_lo=na, nv_hi=na, centre_xy=c, radii=np.ones(n))
+    B = dg.star_layer(n, seed=nb, nv_lo=nb, nv_hi=nb, centre_xy=rng.uniform(-1, 1, (n, 2)), radii=np.ones(n))
+    for L in (A, B):
+        L["xy"] = L["xy"] * np.array([sx, sy])
+    check_all(A, B, n, op)
