@@ -16,6 +16,7 @@ import numpy as np
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 REF_DIR = os.path.join(HERE, "_ref")
+REF_FILES = ("BotomUp-rtree.cu", "TopDown-rtree.cu", "vector_map_overlay_gpc_kernel.cu")
 _LIB = None
 _REF = {}
 
@@ -30,7 +31,8 @@ def build(force: bool = False) -> None:
 
 def build_ref() -> bool:
     """Builds oracle/_ref from the reference sources; False if they are absent."""
-    if not os.path.isdir(os.environ.get("PRT_REFERENCE_DIR", "/root/reference")):
+    ref = os.environ.get("PRT_REFERENCE_DIR", "/root/reference")
+    if not all(os.path.exists(os.path.join(ref, f)) for f in REF_FILES):
         return False
     subprocess.run(["bash", os.path.join(HERE, "ref", "build_ref.sh")], check=True,
                    stdout=subprocess.DEVNULL)

@@ -62,3 +62,11 @@ def test_reference_arm_line():
     assert d["impl"] == "reference"
     if "unavailable" not in d:
         assert d["value"] > 0 and d["cpu_baseline"]["cores"] >= 1 and d["e2e"]["h2d_bytes_per_step"] == 0
+
+
+def test_empty_reference_folder_is_absent(tmp_path, monkeypatch):
+    """A folder without the reference's files counts as no reference."""
+    import oracle
+
+    monkeypatch.setenv("PRT_REFERENCE_DIR", str(tmp_path))
+    assert oracle.build_ref() is False
