@@ -26,10 +26,10 @@
 // with the same distance at the crossing's beam), edges that meet in a local
 // extremum included, at the vertex y next to it.  The distance between two edges is
 // linear in y, so that covers every beam.  No vertex lies on a horizontal edge, and
-// no two horizontal edges follow each other (GPC drops the vertex between them).  A
-// polygon that crosses or touches itself fails the check too.  A pair that fails
-// it, or that has more vertices, rings or crossings than there is room for, is left
-// to the scanbeam clippers.
+// no two horizontal edges follow each other (GPC drops the vertex between them).  No
+// scanline holds both +0 and -0.  A polygon that crosses or touches itself fails the
+// check too.  A pair that fails it, or that has more vertices, rings or crossings than
+// there is room for, is left to the scanbeam clippers.
 //
 // A block per pair, everything between the input and the result in shared memory,
 // vertices in 16-bit indices so that two pairs of 4,160 vertices share an SM.  What
@@ -158,7 +158,7 @@ __device__ __forceinline__ TEdge edge_of(const Pair<C> &P, int v) {
   e.tx = e.up ? x2 : x1;
   e.by = P.S.sy[e.rb];
   e.ty = P.S.sy[e.rt];
-  e.dx = (e.tx - e.bx) / (e.ty - e.by);  // horizontal: +inf, its left end is the lower one
+  e.dx = (e.tx - e.bx) / (e.ty - e.by);  // horizontal: +inf, its left end is the lower one and both ys the same zero
   return e;
 }
 
@@ -486,9 +486,11 @@ __device__ int trace_pair(Smem<C> &S, int op, const gpc::PolyView &A, const gpc:
           if (yw < y) {
             before++;
           } else if (yw == y && w != v) {
+            // +0 and -0 on one scanline: the clipper writes one of them for all, and
+            // the y difference of a horizontal edge between them is -0
             const double d = x - S.vx[w];
             before += d > 0.0;
-            bad |= !(fabs(d) > P.margin);
+            bad |= !(fabs(d) > P.margin) || signbit(y) != signbit(yw);
           }
         }
         S.rank[v] = (uint16_t)(start + before);

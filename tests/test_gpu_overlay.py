@@ -321,10 +321,6 @@ def test_traced_scales(cuda, op, sx, sy):
         assert same_contours(got[i], oracle.gpc_clip(rings_of(A, i), rings_of(B, i), op)), f"pair {i}"
 
 
-def same_bits(a, b) -> bool:
-    return same_contours(a, b) and all(np.array_equal(np.signbit(v1), np.signbit(v2)) for (_, v1), (_, v2) in zip(a, b))
-
-
 def check_all(A, B, n, op):
     import parlllelrtree_b200 as prt
 
@@ -332,7 +328,7 @@ def check_all(A, B, n, op):
     got = prt.overlay(torch.from_numpy(np.stack([ids, ids], axis=1)).cuda(), prt.Layer.from_dict(A),
                       prt.Layer.from_dict(B), op=OPS[op]).contours()
     for i in range(n):
-        assert same_bits(got[i], oracle.gpc_clip(rings_of(A, i), rings_of(B, i), op)), f"pair {i}"
+        assert same_contours(got[i], oracle.gpc_clip(rings_of(A, i), rings_of(B, i), op)), f"pair {i}"
 
 
 @pytest.mark.parametrize("op", [0, 1, 2, 3])
@@ -349,3 +345,25 @@ def test_ys_next_to_zero(cuda, op, na, nb, sx, sy):
     for L in (A, B):
         L["xy"] = L["xy"] * np.array([sx, sy])
     check_all(A, B, n, op)
+
+
+@pytest.mark.parametrize("op", [0, 1, 2, 3])
+def test_both_zeros_on_a_scanline(cuda, op):
+    """Horizontal edges between y = +0.0 and y = -0.0, as rounding to whole numbers
+    gives them, alone and in polygons on a grid around the origin."""
+    a = [(-1, 1), (2, 1), (2, -0.0), (-1, 0.0)]
+    cases = [([a], [[(0, -2), (1, -2), (0.5, 0.5)]]), ([a], [[(0, -2), (1, -2), (0.5, -0.5)]]),
+             ([a[::-1]], [[(0, -2), (1, -2), (0.5, 0.5)]]), ([[(x, -y) for x, y in a]], [[(0, -2), (1, -2), (0.5, 0.5)]]),
+             ([[(-1, 1), (2, 1), (2, 0.0), (-1, -0.0)]], [[(0, -2), (1, -2), (0.5, 0.5)]]),
+             ([[(-1, 1), (2, 1), (2, -0.0), (-1, -0.0)]], [[(0, -2), (1, -2), (0.5, 0.5)]]),
+             ([[(-1, 1), (2, 1), (2, 0.0), (-1, 0.0)]], [[(0.2, -0.0), (1, -2), (0.5, 0.5)]])]
+    rng = np.random.default_rng(31)
+
+    def star():
+        t = np.sort(rng.random(int(rng.integers(4, 17)))) * 2 * np.pi
+        r = rng.uniform(2, 6, len(t))
+        return np.round(np.stack([r * np.cos(t), r * np.sin(t)], 1) + rng.uniform(-2, 2, 2))
+
+    cases += [([star() for _ in range(1 + k % 2)], [star()]) for k in range(3000)]
+    assert any((np.signbit(p) & (p == 0)).any() for s, _ in cases[7:] for p in s)
+    check_all(layer_of([s for s, _ in cases]), layer_of([c for _, c in cases]), len(cases), op)
