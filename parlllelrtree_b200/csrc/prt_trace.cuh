@@ -50,6 +50,8 @@ constexpr int kLast = 0x8000;
 // that neither the slopes nor the buckets per unit of y below overflow, and what a
 // product of an x and a y difference loses to underflow is far below the margin.
 constexpr double kLeastY = 1e-130;
+// Coordinates stay below this: products of two differences do not overflow.
+constexpr double kMostXY = 1e150;
 
 template <int NT>
 __device__ __forceinline__ void bsync() {
@@ -442,7 +444,7 @@ __device__ int trace_pair(Smem<C> &S, int op, const gpc::PolyView &A, const gpc:
     n += (int)len;
     nr++;
   }
-  if (!(most < 1e300)) return kLeft;  // infinities and NaN
+  if (!(most < kMostXY)) return kLeft;  // infinities and NaN too
   bsync<NT>();
   // An edge's x at a y is off by at most u|x| for the last addition and 5u w for the
   // slope, the y difference and their product (u half an epsilon, w the x extent):

@@ -367,3 +367,20 @@ def test_both_zeros_on_a_scanline(cuda, op):
     cases += [([star() for _ in range(1 + k % 2)], [star()]) for k in range(3000)]
     assert any((np.signbit(p) & (p == 0)).any() for s, _ in cases[7:] for p in s)
     check_all(layer_of([s for s, _ in cases]), layer_of([c for _, c in cases]), len(cases), op)
+
+
+@pytest.mark.parametrize("op", [0, 1, 2, 3])
+@pytest.mark.parametrize("scale", [1e149, 1e155, 1e160, 1e290])
+def test_products_that_overflow(cuda, op, scale):
+    """Coordinates whose products of differences are within, and beyond, the
+    largest double; pairs with holes and inside each other, which are told apart
+    by such products."""
+    n = 300
+    rng = np.random.default_rng(23)
+    c, r = np.zeros((n, 2)), np.full(n, 1.0)
+    A = dg.star_layer(n, seed=5, nv_lo=4, nv_hi=12, centre_xy=c, radii=r, hole_frac=0.5)
+    B = dg.star_layer(n, seed=6, nv_lo=4, nv_hi=12, centre_xy=rng.uniform(-0.8, 0.8, (n, 2)),
+                      radii=rng.uniform(0.2, 1.2, n), hole_frac=0.3)
+    for L in (A, B):
+        L["xy"] = L["xy"] * scale
+    check_all(A, B, n, op)
