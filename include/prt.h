@@ -310,7 +310,10 @@ int prt_clip_pair_host(int op, int s_ncont, const int32_t *s_nverts, const doubl
  * mode) of the largest bin that still has pairs, so the largest pairs are
  * clipped first by all warps.  A launch whose thread-mode pairs would fill
  * less than half a wave of warps one pair per thread clips every pair in warp
- * mode instead (same output, more warps in flight). */
+ * mode instead (same output, more warps in flight).
+ * Pairs in general position are traced rather than clipped, with the same output,
+ * unless sweep_only is 1 (for timing and testing the clippers themselves); the
+ * graph pipeline clips every pair. */
 #define PRT_MAX_BINS 8
 typedef struct {
   int32_t nbins;
@@ -318,7 +321,7 @@ typedef struct {
   int64_t bin_thresholds[PRT_MAX_BINS];
   int32_t bin_warp_mode[PRT_MAX_BINS];
   int32_t warps_per_sm;
-  int32_t reserved;
+  int32_t sweep_only;  /* 1: prt_overlay_run clips every pair as above; else it traces pairs in general position first */
 } prt_schedule;
 
 /* Sets the schedule used by later calls of this process (NULL restores the

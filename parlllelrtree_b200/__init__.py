@@ -369,7 +369,7 @@ MAX_BINS = 8
 
 class _Schedule(C.Structure):
     _fields_ = [("nbins", C.c_int32), ("aet_slots", C.c_int32), ("bin_thresholds", C.c_int64 * MAX_BINS),
-                ("bin_warp_mode", C.c_int32 * MAX_BINS), ("warps_per_sm", C.c_int32), ("reserved", C.c_int32)]
+                ("bin_warp_mode", C.c_int32 * MAX_BINS), ("warps_per_sm", C.c_int32), ("sweep_only", C.c_int32)]
 
     @classmethod
     def from_dict(cls, d: dict) -> "_Schedule":
@@ -379,6 +379,7 @@ class _Schedule(C.Structure):
         s.aet_slots = int(d.get("aet_slots", 64))
         wm = list(d.get("warp_mode", [1] * len(thr)))
         s.warps_per_sm = int(d.get("warps_per_sm", 12))
+        s.sweep_only = int(d.get("sweep_only", 0))
         for b in range(len(thr)):
             s.bin_thresholds[b] = int(thr[b])
             s.bin_warp_mode[b] = int(wm[b])
@@ -386,16 +387,17 @@ class _Schedule(C.Structure):
 
     def to_dict(self) -> dict:
         n = self.nbins
-        return {"thresholds": [int(self.bin_thresholds[b]) for b in range(n)],
-                "warp_mode": [int(self.bin_warp_mode[b]) for b in range(n)],
-                "warps_per_sm": int(self.warps_per_sm), "aet_slots": int(self.aet_slots)}
+        d = {"thresholds": [int(self.bin_thresholds[b]) for b in range(n)],
+             "warp_mode": [int(self.bin_warp_mode[b]) for b in range(n)],
+             "warps_per_sm": int(self.warps_per_sm), "aet_slots": int(self.aet_slots)}
+        return dict(d, sweep_only=1) if self.sweep_only == 1 else d
 
 
 def get_schedule() -> dict:
     """The batched schedule in use (prt_schedule_get): size-bin thresholds
     (descending vertex-count upper bounds), per-bin warp mode (1 = one pair
-    per warp), persistent warps per SM, and the warp clipper's shared-memory
-    slots."""
+    per warp), persistent warps per SM, the warp clipper's shared-memory
+    slots, and sweep_only when it is 1 (no tracing)."""
     s = _Schedule()
     check(lib().prt_schedule_get(C.byref(s)))
     return s.to_dict()

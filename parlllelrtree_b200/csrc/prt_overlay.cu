@@ -769,7 +769,7 @@ static int run_batched(OverlayState &st, const int64_t *d_idx, int64_t count, in
   if (bytes > kArenaBudgetLeast) bytes = plan_bins(run_sc, counts, hm, arena_budget(), plan, &smem, scale, true);
   // What tracing leaves may be few pairs out of many: that is known on the device
   // alone, so both launches are made and one of them ends at once.
-  const bool both = thread_warps >= kFewWarps;
+  const bool traced = sc.sweep_only != 1, both = traced && thread_warps >= kFewWarps;
   if (both) bytes = std::max(bytes, plan_bins(few_sc, counts, hm, bytes, few, &few_smem, scale, true));
   for (int p = 0; p < (both ? 2 : 1); p++) {
     BinPlan &pl = p ? few : plan;
@@ -784,7 +784,8 @@ static int run_batched(OverlayState &st, const int64_t *d_idx, int64_t count, in
   if (!rc) rc = prepare_lpt_launch(std::max(smem, few_smem));
   if (!rc && warps > 0) rc = dmalloc(reinterpret_cast<void **>(&arena), bytes, s);
   TraceRest rest = {nullptr, 0, 0, 0};
-  if (!rc && warps > 0) {
+  const uint32_t *todo = traced ? left_order : order;
+  if (!rc && warps > 0 && traced) {
     PRT_PROF("trace", s);
     const int64_t *cut = h.bnd + nb;
     auto go = [&](auto two) {
@@ -808,13 +809,13 @@ static int run_batched(OverlayState &st, const int64_t *d_idx, int64_t count, in
   if (!rc && warps > 0) {
     PRT_PROF("clip_batched", s);
     if (plan.thread_only)
-      clip_lpt_thread_kernel<<<(unsigned)warps, 32, 0, s>>>(st.S, st.O, left_order, plan, d->tickets, arena, scale, rest);
+      clip_lpt_thread_kernel<<<(unsigned)warps, 32, 0, s>>>(st.S, st.O, todo, plan, d->tickets, arena, scale, rest);
     else
-      clip_lpt_kernel<<<(unsigned)warps, 32, smem, s>>>(st.S, st.O, left_order, plan, d->tickets, arena, scale, nullptr, rest);
+      clip_lpt_kernel<<<(unsigned)warps, 32, smem, s>>>(st.S, st.O, todo, plan, d->tickets, arena, scale, nullptr, rest);
     if (both) {
       rest.min_warps = 0;
       rest.max_warps = kFewWarps;
-      clip_lpt_kernel<<<(unsigned)few.warp0[nb], 32, few_smem, s>>>(st.S, st.O, left_order, few, d->rest_tickets, arena, scale,
+      clip_lpt_kernel<<<(unsigned)few.warp0[nb], 32, few_smem, s>>>(st.S, st.O, todo, few, d->rest_tickets, arena, scale,
                                                                    nullptr, rest);
     }
   }

@@ -240,3 +240,45 @@ def test_many_crossings_per_beam(cuda, sched):
         for k in range(0, n, 6):
             ref = oracle.gpc_clip(rings_of(A, k), rings_of(B, k), OPS.index(op))
             assert same_contours(plain[k], ref), (op, k)
+
+
+# The tests above with tracing off: as the schedule stands, pairs in general
+# position are traced, and the clippers see only the others.
+SWEPT = [(t, a) for t, args in ((test_golden_pairs_warp, [(op, s) for op in range(4) for s in ("warp", "warp32")]),
+                                (test_holes_and_uneven_sizes, [("warp",), ("warp32",), ("mixed",)]),
+                                (test_large_lobed_stars, [()]),
+                                (test_degenerate_and_bundled, [("warp",), ("warp32",)]),
+                                (test_shared_edge_tessellations, [()]),
+                                (test_many_crossings_per_beam, [("warp",), ("warp32",)])) for a in args]
+
+
+@pytest.mark.parametrize("test,args", SWEPT, ids=[f"{t.__name__[5:]}-{'-'.join(map(str, a))}" for t, a in SWEPT])
+def test_without_tracing(cuda, monkeypatch, test, args):
+    for k, v in SCHEDS.items():
+        monkeypatch.setitem(SCHEDS, k, dict(v, sweep_only=1))
+    names = [n for n in test.__code__.co_varnames[1:test.__code__.co_argcount]]
+    test(cuda, **dict(zip(sorted(names), args)))
+
+
+def test_area_mode_without_tracing(cuda):
+    """The clippers' areas of the pairs that the boundary integral leaves: a
+    thread's and a warp's are the same bits."""
+    import parlllelrtree_b200 as prt
+
+    A = dg.star_layer(200, seed=21, nv_lo=16, nv_hi=900, r_lo=0.02, r_hi=0.06, zipf=1.1)
+    B = dg.star_layer(200, seed=22, nv_lo=16, nv_hi=900, r_lo=0.02, r_hi=0.06, zipf=1.1)
+    LA, LB = prt.Layer.from_dict(A), prt.Layer.from_dict(B)
+    t = prt.build_bottomup(LA.mbr(), fanout=16)
+    pairs = t.join(LB.mbr(), sorted=True)
+    l2p = t.leaf_order().long()
+    pa = l2p[pairs[:, 0].long()].int()
+    pb = pairs[:, 1].int()
+    with prt.schedule(dict(MIXED, warp_mode=[1, 0, 0], sweep_only=1)):
+        a0 = prt.intersection_area(LA, LB, pa, pb)
+    with prt.schedule(dict(WARP, sweep_only=1)):
+        a1 = prt.intersection_area(LA, LB, pa, pb)
+    assert torch.equal(a0, a1)
+    with prt.schedule(WARP):  # traced: another order of the same sum
+        a2 = prt.intersection_area(LA, LB, pa, pb)
+    assert torch.allclose(a2, a1, rtol=1e-9, atol=1e-15)
+    assert prt.get_schedule().get("sweep_only", 0) == 0
