@@ -377,8 +377,8 @@ int prt_layer_mbr(const prt_layer *layer, double *d_out, void *stream);
 int prt_layer_mbr_i32(const prt_layer *layer, double scale, int32_t *d_out, void *stream);
 
 /* Autotuner (no reference counterpart): times the build + join for fanouts
- * 8..32 and the batched clip for candidate schedules (warp-mode threshold,
- * shared-memory slots, warps per SM) on an evenly strided sample of at most
+ * 8..32 and the batched clip, without tracing, for candidate schedules (warp-mode
+ * threshold, shared-memory slots, warps per SM) on an evenly strided sample of at most
  * max_sample_pairs candidate pairs (<= 0: 200,000), within about
  * time_budget_s seconds (<= 0: 30).  Installs the best schedule with
  * prt_schedule_set and returns the choice. */

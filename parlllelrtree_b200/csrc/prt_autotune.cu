@@ -147,7 +147,11 @@ int prt_autotune(const prt_layer *base, const prt_layer *overlay, int op, int64_
   // ---- 3. schedule: coordinate descent
   prt_schedule saved;
   prt_schedule_get(&saved);
-  auto time_sched = [&](const prt_schedule &sc, double *ms_out) -> int {
+  // the clippers' time: tracing goes by no schedule, and where it takes most
+  // pairs the candidates would differ by noise (the graph pipeline, which does not
+  // trace, then runs with the choice)
+  auto time_sched = [&](prt_schedule sc, double *ms_out) -> int {
+    sc.sweep_only = 1;
     int r = prt_schedule_set(&sc);
     if (r) return r;
     double best = 1e30;

@@ -132,3 +132,25 @@ def test_autotune_installs_a_valid_schedule(cuda, tmp_path):
         assert all(same_contours(x, y) for x, y in zip(tuned, plain))
     finally:
         prt.set_schedule(saved)
+
+
+def test_autotune_times_the_clippers(cuda):
+    """The candidates are timed without tracing, which goes by no schedule; the
+    installed schedule traces."""
+    import parlllelrtree_b200 as prt
+    from parlllelrtree_b200 import _lib
+
+    A, B = _layers(n=600, seed=11, zipf=1.2, nv_hi=400)
+    LA, LB = prt.Layer.from_dict(A), prt.Layer.from_dict(B)
+    saved = prt.get_schedule()
+    try:
+        _lib.profile_enable(2)
+        _lib.profile_reset()
+        r = prt.autotune(LA, LB, max_sample_pairs=2000, time_budget_s=20.0, use_cache=False)
+        seen = _lib.profile_read()
+        assert "clip_batched" in seen and "trace" not in seen
+        assert "sweep_only" not in r["schedule"] and "sweep_only" not in prt.get_schedule()
+    finally:
+        _lib.profile_enable(0)
+        _lib.profile_reset()
+        prt.set_schedule(saved)
