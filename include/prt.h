@@ -231,6 +231,9 @@ int prt_overlay_run_ref(const prt_pair *d_pairs, int64_t n_pairs, int32_t offset
 /* sizes[0] pairs, [1] contours, [2] vertices, [3] non-empty results,
  * [4] pairs retried with larger arenas. */
 int prt_results_sizes(const prt_results *r, int64_t *sizes);
+/* Pairs that the scanbeam clippers took: those that tracing left, or all of
+ * them (plain schedule, sweep_only). */
+int prt_results_left(const prt_results *r, int64_t *h_count);
 /* Device views of the result arrays (valid until prt_results_free).  Like the
  * reference's gpc_polygon array, each pair points at its own contours:
  * pair i owns contours [pair_cont_start[i], + pair_ncont[i]); contour c owns

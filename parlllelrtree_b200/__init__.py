@@ -260,6 +260,13 @@ class Results:
         except Exception:
             pass
 
+    @property
+    def left(self) -> int:
+        """Pairs that the scanbeam clippers took (prt_results_left)."""
+        n = C.c_int64(0)
+        check(lib().prt_results_left(self._h, C.byref(n)))
+        return int(n.value)
+
     def to_host(self):
         """(pair_cont_off [P+1], cont_nverts [C], cont_hole [C], xy [V, 2]) in pair order."""
         off = np.zeros(self.n_pairs + 1, np.int64)

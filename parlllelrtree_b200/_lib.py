@@ -51,6 +51,7 @@ _SIGS = {
     "prt_overlay_run_ref": (_I, [_P, _I64, C.c_int32, _P, _P, _P, _P, _P, _I64, _P, _P, _P, _P, _I64, _I, _I,
                                  _P, _P]),
     "prt_results_sizes": (_I, [_P, _P]),
+    "prt_results_left": (_I, [_P, _P]),
     "prt_results_device": (_I, [_P, _P, _P, _P, _P, _P, _P]),
     "prt_results_copy": (_I, [_P, _P, _P, _P, _P]),
     "prt_results_area": (_I, [_P, _P, _P]),

@@ -547,8 +547,12 @@ struct OverlayState {
   int64_t n;
   int sched = PRT_SCHED_PLAIN;
   int64_t retried = 0;
-  unsigned long long *words = nullptr;  // the block the pool counters are in: [2..5] result totals, [6] vertices in
+  bool traced = false;
+  // the block the pool counters are in: [2..5] result totals, [6] vertices in, then
+  // the pairs of each bin that were not traced
+  unsigned long long *words = nullptr;
 };
+constexpr int kTotalsWord = 2, kLeftWord = 8, kWords = kLeftWord + PRT_MAX_BINS;
 
 // Result pools for a first guess at the result size from the vertices that
 // went in (grown on demand): one contour per pair and one per 64 vertices;
@@ -698,7 +702,6 @@ static int run_batched(OverlayState &st, const int64_t *d_idx, int64_t count, in
     int64_t bnd[kCuts], mx[kCuts];
     unsigned long long tickets[PRT_MAX_BINS + 1];  // bins + fallbacks
     unsigned long long rest_tickets[PRT_MAX_BINS + 1], trace_tickets[trace::kClasses];
-    unsigned long long left[PRT_MAX_BINS];  // pairs of each bin that were not traced
   } h;
   static_assert(sizeof(Head) <= 512, "head block");
   unsigned char *scr = nullptr;
@@ -708,6 +711,8 @@ static int run_batched(OverlayState &st, const int64_t *d_idx, int64_t count, in
   uint32_t *k0 = reinterpret_cast<uint32_t *>(scr + 512);
   uint32_t *k1 = k0 + n, *v0 = k1 + n, *v1 = v0 + n, *order = v1 + n, *left_order = order + n;
   cudaMemsetAsync(scr, 0, 512, s);
+  unsigned long long *left = st.words + kLeftWord;
+  if (d_idx) cudaMemsetAsync(left, 0, 8 * PRT_MAX_BINS, s);  // again, for the pairs of this call
   BinThresholds T;
   for (int b = 0; b < nb; b++) T.thr[b] = sc.bin_thresholds[b];
   const int64_t cls_verts[trace::kClasses] = {trace::Class3<0>::kVerts, trace::Class2<0>::kVerts,
@@ -785,26 +790,27 @@ static int run_batched(OverlayState &st, const int64_t *d_idx, int64_t count, in
   if (!rc && warps > 0) rc = dmalloc(reinterpret_cast<void **>(&arena), bytes, s);
   TraceRest rest = {nullptr, 0, 0, 0};
   const uint32_t *todo = traced ? left_order : order;
+  st.traced = traced;
   if (!rc && warps > 0 && traced) {
     PRT_PROF("trace", s);
     const int64_t *cut = h.bnd + nb;
     auto go = [&](auto two) {
       constexpr int kTwo = decltype(two)::value;
       int e = launch_trace<trace::Class3<kTwo>>(st.S, st.O, order, 0, cut[1], plan, &d->trace_tickets[0], left_order,
-                                                d->left, s);
+                                                left, s);
       if (!e)
         e = launch_trace<trace::Class2<kTwo>>(st.S, st.O, order, cut[1], cut[2], plan, &d->trace_tickets[1], left_order,
-                                              d->left, s);
+                                              left, s);
       if (!e)
         e = launch_trace<trace::Class1<kTwo>>(st.S, st.O, order, cut[2], cut[3], plan, &d->trace_tickets[2], left_order,
-                                              d->left, s);
+                                              left, s);
       if (!e)
         e = launch_trace<trace::Class0<kTwo>>(st.S, st.O, order, cut[3], n, plan, &d->trace_tickets[3], left_order,
-                                              d->left, s);
+                                              left, s);
       return e;
     };
     rc = st.S.op == PRT_GPC_XOR ? go(std::integral_constant<int, 1>{}) : go(std::integral_constant<int, 0>{});
-    rest = {d->left, thread_bins, both ? kFewWarps : 0, INT64_MAX};
+    rest = {left, thread_bins, both ? kFewWarps : 0, INT64_MAX};
   }
   if (!rc && warps > 0) {
     PRT_PROF("clip_batched", s);
@@ -1047,31 +1053,36 @@ int overlay_impl(const PairSrc &S, int64_t n, int sched, double *d_area, cudaStr
   memset(&st.O, 0, sizeof st.O);
   st.O.area = d_area;
   int rc = dalloc(&st.O.status, std::max<int64_t>(n, 1), s);
-  if (!rc) rc = dalloc(&st.words, 8, s);
+  if (!rc) rc = dalloc(&st.words, kWords, s);
   st.O.pool = st.words;
   if (!rc && !d_area) rc = dalloc(&st.O.pair_cstart, std::max<int64_t>(n, 1), s);
   if (!rc && !d_area) rc = dalloc(&st.O.pair_ncont, std::max<int64_t>(n, 1), s);
   if (!rc) {
-    cudaError_t e = cudaMemsetAsync(st.words, 0, 64, s);
+    cudaError_t e = cudaMemsetAsync(st.words, 0, 8 * kWords, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(st.O.status, 0, 4 * std::max<int64_t>(n, 1), s);
     if (e != cudaSuccess) rc = cuda_status(e, "memset");
   }
   if (!rc && n == 0) rc = first_pools(st, 0, s);
   if (!rc && n > 0) rc = sched == PRT_SCHED_PLAIN ? run_plain(st, nullptr, n, 1, s) : run_batched(st, nullptr, n, 1, s);
-  // totals of the live results (pools may hold abandoned reservations) and
-  // the pairs to retry, read back together
-  unsigned long long tot[4] = {0, 0, 0, 0};
+  // totals of the live results (pools may hold abandoned reservations), the pairs
+  // to retry and those that were not traced, read back together
+  unsigned long long tot[kWords - kTotalsWord] = {0};
+  int64_t left = n;
   for (int pass = 0; pass < 2 && !rc && n > 0; pass++) {
-    cudaError_t e = pass ? cudaMemsetAsync(st.words + 2, 0, sizeof tot, s) : cudaSuccess;
+    cudaError_t e = pass ? cudaMemsetAsync(st.words + kTotalsWord, 0, 32, s) : cudaSuccess;
     if (e == cudaSuccess) {
       PRT_PROF("result_totals", s);
       result_totals_kernel<<<grid_for(n, 256, 8), 256, 0, s>>>(st.O.status, st.O.pair_cstart, st.O.pair_ncont,
-                                                               st.O.cont_nverts, n, st.words + 2);
+                                                               st.O.cont_nverts, n, st.words + kTotalsWord);
       e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(tot, st.words + 2, sizeof tot, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(tot, st.words + kTotalsWord, sizeof tot, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) rc = cuda_status(e, "overlay results");
+    if (pass == 0 && st.traced) {
+      left = 0;
+      for (int b = 0; b < PRT_MAX_BINS; b++) left += (int64_t)tot[kLeftWord - kTotalsWord + b];
+    }
     if (rc || tot[3] == 0) break;
     rc = retry_failed(st, s);
   }
@@ -1082,6 +1093,7 @@ int overlay_impl(const PairSrc &S, int64_t n, int sched, double *d_area, cudaStr
   prt_results *r = new prt_results();
   r->n_pairs = n;
   r->retried = st.retried;
+  r->left = left;
   r->pair_cstart = st.O.pair_cstart;
   r->pair_ncont = st.O.pair_ncont;
   r->status = st.O.status;
@@ -1224,6 +1236,12 @@ int prt_results_sizes(const prt_results *r, int64_t *sizes) {
   sizes[2] = r->n_vert;
   sizes[3] = r->nonempty;
   sizes[4] = r->retried;
+  return PRT_OK;
+}
+
+int prt_results_left(const prt_results *r, int64_t *h_count) {
+  PRT_CHECK(r && h_count, PRT_ERR_INVALID, "NULL argument");
+  *h_count = r->left;
   return PRT_OK;
 }
 

@@ -124,7 +124,7 @@ int overlay_graph_enqueue(const PairSrc &S, const unsigned long long *d_npairs, 
 // vertices [cont_vstart[c], + cont_nverts[c]) of xy.  Pools are filled by
 // atomic reservations, so they are not in pair order.
 struct prt_results {
-  int64_t n_pairs, n_cont, n_vert, nonempty, retried;
+  int64_t n_pairs, n_cont, n_vert, nonempty, retried, left;
   int64_t *pair_cstart;
   int32_t *pair_ncont;
   int32_t *status;

@@ -384,3 +384,87 @@ def test_products_that_overflow(cuda, op, scale):
     for L in (A, B):
         L["xy"] = L["xy"] * scale
     check_all(A, B, n, op)
+
+
+def stars_across(n, na, nb):
+    """Stars, each with a smaller one across its boundary: a few crossings, general
+    position."""
+    rng = np.random.default_rng(na * 31 + nb)
+    c = rng.random((n, 2))
+    A = dg.star_layer(n, seed=na, nv_lo=na, nv_hi=na, centre_xy=c, radii=np.full(n, 0.01))
+    B = dg.star_layer(n, seed=nb + 1, nv_lo=nb, nv_hi=nb, centre_xy=c + [0.006, 0.003], radii=np.full(n, 0.004))
+    return A, B
+
+
+def ids_of(n):
+    ids = np.arange(n, dtype=np.int32)
+    return torch.from_numpy(np.stack([ids, ids], axis=1)).cuda()
+
+
+@pytest.mark.parametrize("na,nb,left", [(64, 64, 0), (124, 5, 0), (1020, 4, 0), (1020, 5, 0), (4096, 64, 0), (4096, 65, 0),
+                                        (4352, 4096, 0), (4353, 4096, 4)])
+def test_class_limits(cuda, na, nb, left):
+    """Pairs at and one above the tracing classes' 128, 1,024, 4,160 and 8,448
+    vertices are traced, up to the last."""
+    import parlllelrtree_b200 as prt
+
+    A, B = stars_across(4, na, nb)
+    r = prt.overlay(ids_of(4), prt.Layer.from_dict(A), prt.Layer.from_dict(B))
+    assert r.left == left
+    for i, got in enumerate(r.contours()):
+        assert same_contours(got, oracle.gpc_clip(rings_of(A, i), rings_of(B, i), 1)), f"pair {i}"
+
+
+def test_pairs_left_are_counted(cuda):
+    """Equal polygons are left; every pair counts where nothing is traced."""
+    import parlllelrtree_b200 as prt
+
+    A, B = stars_across(40, 12, 9)
+    LA, LB = prt.Layer.from_dict(A), prt.Layer.from_dict(B)
+    for op in OPS:
+        assert prt.overlay(ids_of(40), LA, LB, op=op).left == 0
+        assert prt.overlay(ids_of(40), LA, LA, op=op).left == 40
+    assert prt.overlay(ids_of(40), LA, LB, sched="plain").left == 40
+    with prt.schedule(dict(prt.get_schedule(), sweep_only=1)):
+        assert prt.overlay(ids_of(40), LA, LB).left == 40
+    assert prt.overlay(ids_of(0), LA, LB).left == 0
+
+
+@pytest.mark.parametrize("op", ["int", "xor"])
+@pytest.mark.parametrize("equal", [0, 1000, 56_800, 56_832, 60_000])
+def test_many_small_pairs_left(cuda, op, equal):
+    """62,000 small pairs, too many for a warp each, of which tracing leaves a few, some
+    1,776 warps of one pair per thread (the line between the two launches), and most."""
+    import parlllelrtree_b200 as prt
+
+    n = 62_000
+    A, B = stars_across(n, 8, 8)
+    B["xy"][: 8 * equal] = A["xy"][: 8 * equal]
+    LA, LB = prt.Layer.from_dict(A), prt.Layer.from_dict(B)
+    r = prt.overlay(ids_of(n), LA, LB, op=op)
+    assert r.left == equal
+    got, ref = r.to_host(), prt.overlay(ids_of(n), LA, LB, op=op, sched="plain").to_host()
+    assert all(np.array_equal(g, e) for g, e in zip(got, ref))
+    c = r.contours_of(range(0, n, 500))
+    for k, i in enumerate(range(0, n, 500)):
+        assert same_contours(c[k], oracle.gpc_clip(rings_of(A, i), rings_of(B, i), OPS.index(op))), f"pair {i}"
+
+
+@pytest.mark.parametrize("op", OPS)
+def test_traced_bits(cuda, op):
+    """Traced results are those of the clippers bit for bit, zeros' signs too."""
+    import parlllelrtree_b200 as prt
+
+    rng = np.random.default_rng(41)
+    A = dg.star_layer(3000, seed=1, nv_lo=4, nv_hi=40, r_lo=2.0, r_hi=8.0, centre_xy=rng.uniform(-6, 6, (3000, 2)), hole_frac=0.2)
+    B = dg.star_layer(3000, seed=2, nv_lo=4, nv_hi=40, r_lo=2.0, r_hi=8.0, centre_xy=rng.uniform(-6, 6, (3000, 2)), hole_frac=0.2)
+    for L in (A, B):  # a third on whole numbers
+        v = L["ring_vert"][L["poly_ring"][1000]]
+        L["xy"][:v] = np.round(L["xy"][:v])
+    LA, LB = prt.Layer.from_dict(A), prt.Layer.from_dict(B)
+    r = prt.overlay(ids_of(3000), LA, LB, op=op)
+    assert 0 < r.left < 1000
+    with prt.schedule(dict(prt.get_schedule(), sweep_only=1)):
+        ref = prt.overlay(ids_of(3000), LA, LB, op=op).to_host()
+    assert all(np.array_equal(g.view(np.int64) if g.dtype == np.float64 else g,
+                              e.view(np.int64) if e.dtype == np.float64 else e) for g, e in zip(r.to_host(), ref))
