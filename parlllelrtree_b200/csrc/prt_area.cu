@@ -151,6 +151,7 @@ __device__ void pieces(const Poly &A, const Poly &B, double w, double *grad, int
 // a vertex receives (as the end of one edge, as the start of the next) are
 // summed across neighbouring lanes before the atomics.  Edges with more than
 // kBwdMaxT crossings take the global-memory path (next_crossing).
+constexpr int kBwdOneV = 32;  // both polygons' vertices together (gradients only)
 constexpr int kBwdSmallV = 64;
 constexpr int kBwdMidV = 128;
 constexpr int kBwdLargeV = 256;  // BwdPoly's 8-bit vertex indices hold no more
@@ -310,6 +311,27 @@ __device__ inline uint32_t bit_transpose(uint32_t x) {
     x = (lane & j) ? ((x & ~m) | ((t >> j) & m)) : ((x & m) | ((t << j) & ~m));
   }
   return x;
+}
+
+// y and x slab masks of two staged polygons of up to 32 edges each (four
+// independent transposes).
+template <int V>
+__device__ inline void bwd_slabs_both(const BwdPoly<V> *M, int na, int nb, const SlabGrid &gy, const SlabGrid &gx,
+                                      BwdSlabs<V> &SA, BwdSlabs<V> &SB) {
+  const int lane = threadIdx.x & 31;
+  uint32_t ry[2] = {0, 0}, rx[2] = {0, 0};
+#pragma unroll
+  for (int p = 0; p < 2; p++)
+    if (lane < (p ? nb : na)) {
+      const float4 b = M[p].bb[lane];
+      ry[p] = (kFullMask >> (31 - gy(b.w))) & (kFullMask << gy(b.y));
+      rx[p] = (kFullMask >> (31 - gx(b.z))) & (kFullMask << gx(b.x));
+    }
+  SA.y[0][lane] = bit_transpose(ry[0]);
+  SA.x[0][lane] = bit_transpose(rx[0]);
+  SB.y[0][lane] = bit_transpose(ry[1]);
+  SB.x[0][lane] = bit_transpose(rx[1]);
+  __syncwarp();
 }
 
 // y and x slab masks of a staged polygon (two independent transposes per word).
@@ -490,7 +512,10 @@ struct AreaSum {
 // Returns false in area mode as soon as any crossing of the pair is unclean
 // (the caller then clips the pair with GPC); in gradient mode it always runs
 // to the end, by the definition from the first unclean crossing on.
-template <bool kArea, int V>
+// kOne (na + nb <= kBwdOneV): both polygons' edges in one round, every edge searching for
+// itself: two half-empty rounds and the chains cost more than finding each crossing
+// twice.
+template <bool kArea, bool kOne, int V>
 __device__ inline bool pair_boundary(BwdPair<V> &W, const float4 *ext, int na, int nb, const SlabGrid &g,
                                      const SlabGrid &gx, double w, double *ga, double *gb, int64_t va, int64_t vb,
                                      const Poly &Ag, const Poly &Bg, double ox, double oy, AreaSum *acc) {
@@ -499,20 +524,28 @@ __device__ inline bool pair_boundary(BwdPair<V> &W, const float4 *ext, int na, i
   BwdCrossings<V> &X = W.cross;
   const int searcher = nb < na ? 1 : 0;
   int masks = 1 - searcher;  // the polygon W.slab belongs to
-  bwd_slabs(W.poly[masks], masks ? nb : na, g, gx, W.slab);
-  for (int k = lane; k < (masks ? nb : na); k += 32) X.head[k] = 0;
-  if (lane == 0) X.count = 0;
-  __syncwarp();
+  static_assert(!kOne || sizeof(BwdSlabs<V>) <= sizeof(BwdCrossings<V>), "A's masks in the place of the chains");
+  BwdSlabs<V> &SA = *reinterpret_cast<BwdSlabs<V> *>(&X);
+  if constexpr (kOne) {
+    bwd_slabs_both(W.poly, na, nb, g, gx, SA, W.slab);
+  } else {
+    bwd_slabs(W.poly[masks], masks ? nb : na, g, gx, W.slab);
+    for (int k = lane; k < (masks ? nb : na); k += 32) X.head[k] = 0;
+    if (lane == 0) X.count = 0;
+    __syncwarp();
+  }
   bool exact = false;  // by the definition from here on (sticky)
   double area2 = 0.0, err = 0.0;
-  for (int half = 0; half < 2; half++) {
-    const int side = half ? 1 - searcher : searcher;
+  for (int half = 0; half < (kOne ? 1 : 2); half++) {
+    // kOne: lanes [0, na) have A's edges, [na, na + nb) B's
+    const int side = kOne ? (lane < na ? 0 : 1) : half ? 1 - searcher : searcher;
+    const int lane0 = kOne && side ? na : 0;
     const BwdPoly<V> &P = W.poly[side], &Q = W.poly[1 - side];
     const int np = side ? nb : na, nq = side ? na : nb;
     const int nwq = (nq + 31) >> 5;
     bool carry = false;  // inside state after the last edge of the previous round
-    for (int e0 = 0; e0 < np; e0 += 32) {
-      const int i = e0 + lane;
+    for (int e0 = 0; e0 < (kOne ? 1 : np); e0 += 32) {
+      const int i = e0 + lane - lane0;
       const bool valid = i < np && P.sgn[i] != 0;
       const int j = valid ? P.nxt[i] : 0;
       double px = 0.0, py = 0.0, qx = 0.0, qy = 0.0;
@@ -535,8 +568,8 @@ __device__ inline bool pair_boundary(BwdPair<V> &W, const float4 *ext, int na, i
           const bool material_left = P.sgn[i] > 0;
           const double rl = fabs(rx) + fabs(ry);
           const int s0 = g(pb.y), s1 = g(pb.w), x0 = gx(pb.x), x1 = gx(pb.z);
-          for (int c = 0; c < nwq; c++) {
-            uint32_t bits = bwd_cands(W.slab, c, s0, s1, x0, x1);
+          for (int c = 0; c < (kOne ? 1 : nwq); c++) {
+            uint32_t bits = bwd_cands(kOne && side ? SA : W.slab, c, s0, s1, x0, x1);
             while (bits) {
               const int k = 32 * c + __ffs(bits) - 1;
               bits &= bits - 1;
@@ -562,8 +595,9 @@ __device__ inline bool pair_boundary(BwdPair<V> &W, const float4 *ext, int na, i
                 unclean = true;
                 continue;
               }
-              if constexpr (kArea) err += 2.0 * ((rl + sl) * rl * sl / d);  // seen from both edges
-              const double t = tn / den, u = un / den;  // next_crossing's t from either edge
+              // seen from both edges
+              if constexpr (kArea) err += (kOne ? 1.0 : 2.0) * ((rl + sl) * rl * sl / d);
+              const double t = tn / den;  // next_crossing's t
               // den > 0: P's edge goes from the left of Q's edge to its right,
               // out of Q where Q's material is on the left, and Q's edge the
               // other way
@@ -574,12 +608,15 @@ __device__ inline bool pair_boundary(BwdPair<V> &W, const float4 *ext, int na, i
               c2 += st * t;
               tfirst = fmin(tfirst, t);
               m++;
-              const uint32_t x = atomicAdd(&X.count, 1u);
-              if (x < (uint32_t)bwd_crossings(V)) {
-                X.u[x] = (den < 0.0) == material_left ? -u : u;
-                X.next[x] = (uint16_t)atomicExch(&X.head[k], x + 1);
-              } else {
-                unclean = true;
+              if constexpr (!kOne) {
+                const double u = un / den;  // and seen from the other edge
+                const uint32_t x = atomicAdd(&X.count, 1u);
+                if (x < (uint32_t)bwd_crossings(V)) {
+                  X.u[x] = (den < 0.0) == material_left ? -u : u;
+                  X.next[x] = (uint16_t)atomicExch(&X.head[k], x + 1);
+                } else {
+                  unclean = true;
+                }
               }
             }
           }
@@ -605,6 +642,7 @@ __device__ inline bool pair_boundary(BwdPair<V> &W, const float4 *ext, int na, i
         // the first interval of each ring starting in this round, by its
         // midpoint: the whole warp tests it against all edges of the other polygon
         const bool rstart = valid && rs == i;
+        const int rlane = rs + lane0;
         double mx0 = 0.0, my0 = 0.0;
         if (rstart) {
           const double tm = 0.5 * tfirst;
@@ -616,11 +654,13 @@ __device__ inline bool pair_boundary(BwdPair<V> &W, const float4 *ext, int na, i
           const int L = __ffs(q) - 1;
           const double mxl = __shfl_sync(kFullMask, mx0, L), myl = __shfl_sync(kFullMask, my0, L);
           bool in = false;
-          for (int k = lane; k < nq; k += 32) {
-            const int l = Q.nxt[k];
-            const double ay = Q.y[k], by = Q.y[l];
+          const int sl = kOne ? (L < na ? 0 : 1) : side;
+          const BwdPoly<V> &QL = W.poly[1 - sl];
+          for (int k = lane; k < (sl ? na : nb); k += 32) {
+            const int l = QL.nxt[k];
+            const double ay = QL.y[k], by = QL.y[l];
             if ((ay > myl) != (by > myl)) {
-              const double ax = Q.x[k], bx = Q.x[l];
+              const double ax = QL.x[k], bx = QL.x[l];
               const double xi = ax + (myl - ay) * (bx - ax) / (by - ay);
               if (mxl < xi) in = !in;
             }
@@ -629,7 +669,7 @@ __device__ inline bool pair_boundary(BwdPair<V> &W, const float4 *ext, int na, i
           if (lane == L) first = inside;
         }
         const unsigned odd = __ballot_sync(kFullMask, (m & 1) != 0);
-        const int from = rs > e0 ? rs - e0 : 0;
+        const int from = rlane > e0 ? rlane - e0 : 0;
         const int par = __popc(odd & lt & ~((1u << from) - 1u)) & 1;
         const bool sf = __shfl_sync(kFullMask, first, from);
         const bool st = (rs >= e0 ? sf : carry) != (par != 0);  // inside state at the edge's start
@@ -647,13 +687,14 @@ __device__ inline bool pair_boundary(BwdPair<V> &W, const float4 *ext, int na, i
       }
       if constexpr (!kArea) {
         if (exact) {
-          if (masks != 1 - side) {
+          if (!kOne && masks != 1 - side) {
             masks = 1 - side;
             __syncwarp();
             bwd_slabs(Q, nq, g, gx, W.slab);
           }
           if (valid)
-            bwd_edge_exact(Q, W.slab, nwq, ext[1 - side], g, gx, pb, px, py, rx, ry, side ? Ag : Bg, &it, &i1);
+            bwd_edge_exact(Q, kOne && side ? SA : W.slab, nwq, side ? ext[0] : ext[1], g, gx, pb, px, py, rx, ry,
+                           side ? Ag : Bg, &it, &i1);
         }
       }
       if constexpr (kArea) {
@@ -673,8 +714,8 @@ __device__ inline bool pair_boundary(BwdPair<V> &W, const float4 *ext, int na, i
         gxi = nx * i1;
         gyi = ny * i1;
       }
-      const int key = valid ? i : -1;                         // this edge's start vertex
-      const int kend = valid ? j : -2;                        // its end vertex
+      const int key = valid ? side << 8 | i : -1;             // this edge's start vertex
+      const int kend = valid ? side << 8 | j : -2;            // its end vertex
       const int knext = __shfl_down_sync(kFullMask, key, 1);  // start vertex of the next lane's edge
       const int kprev = __shfl_up_sync(kFullMask, kend, 1);   // end vertex of the previous lane's edge
       const double hx = __shfl_down_sync(kFullMask, gxi, 1), hy = __shfl_down_sync(kFullMask, gyi, 1);
@@ -732,6 +773,8 @@ __device__ __forceinline__ int64_t list_items(const PairList &L, int64_t n) {
 // of 2 warps.  Before it, 50k pairs of 4-160 vertices (a third of them above
 // 128) took 10.8 ms here on the global-memory path and 11.5 ms in the
 // forward's GPC clip.
+// The smallest stage is launched beside the 64-vertex one, in whose tail it runs:
+// both take what area_tiny_kernel lists.
 template <int V>
 __global__ void __launch_bounds__(32 * bwd_warps(V), V > kBwdMidV ? 5 : 4) area_bwd_kernel(
     const int32_t *__restrict__ pa, const int32_t *__restrict__ pb, int64_t n, LayerDev base, LayerDev over,
@@ -741,6 +784,8 @@ __global__ void __launch_bounds__(32 * bwd_warps(V), V > kBwdMidV ? 5 : 4) area_
   BwdPoly<V> *M = W.poly;
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  if constexpr (V != kBwdOneV) cudaGridDependencySynchronize();
+  if constexpr (V == kBwdSmallV) cudaTriggerProgrammaticLaunchCompletion();
   const int64_t items = list_items(PL, n);
   // a pair's ids are read one pair ahead and its ring ranges half a pair
   // ahead, so the staging of a pair waits only for its ring starts and
@@ -790,15 +835,19 @@ __global__ void __launch_bounds__(32 * bwd_warps(V), V > kBwdMidV ? 5 : 4) area_
         const float x0 = fmaxf(ext[0].x, ext[1].x), x1 = fminf(ext[0].z, ext[1].z);
         const float y0 = fmaxf(ext[0].y, ext[1].y), y1 = fminf(ext[0].w, ext[1].w);
         if (!(x0 > x1 || y0 > y1)) {
-          const SlabGrid gy = slab_grid(y0, y1), gx = slab_grid(x0, x1);
           Poly A{base.ring_vert, base.ring_hole, base.xy, rr[0], rr[1]};
           Poly B{over.ring_vert, over.ring_hole, over.xy, rr[2], rr[3]};
-          pair_boundary<false>(W, ext, nv[0], nv[1], gy, gx, w, grad_base, grad_over, vb[0], vb[1], A, B, 0.0,
-                               0.0, nullptr);
+          const SlabGrid gy = slab_grid(y0, y1), gx = slab_grid(x0, x1);
+          if constexpr (V == kBwdOneV)
+            pair_boundary<false, true>(W, ext, nv[0], nv[1], gy, gx, w, grad_base, grad_over, vb[0], vb[1], A, B, 0.0,
+                                       0.0, nullptr);
+          else
+            pair_boundary<false, false>(W, ext, nv[0], nv[1], gy, gx, w, grad_base, grad_over, vb[0], vb[1], A, B,
+                                        0.0, 0.0, nullptr);
         }
       } else if (PL.defer) {
         if ((threadIdx.x & 31) == 0) PL.defer[atomicAdd(PL.defer_count, 1ull)] = (int32_t)i;
-      } else {
+      } else if (V > kBwdOneV) {  // all that is listed for the smallest stage fits
         const double w = upstream ? upstream[i] : 1.0;
         Poly A{base.ring_vert, base.ring_hole, base.xy, rr[0], rr[1]};
         Poly B{over.ring_vert, over.ring_hole, over.xy, rr[2], rr[3]};
@@ -812,6 +861,7 @@ __global__ void __launch_bounds__(32 * bwd_warps(V), V > kBwdMidV ? 5 : 4) area_
     for (int q = 0; q < 4; q++) rr[q] = rn[q];
     __syncwarp();
   }
+  if constexpr (V == kBwdOneV) cudaGridDependencySynchronize();  // the next stage waits for this one alone
 }
 
 // Forward: one warp per pair, staged as in the backward.  A pair gets its
@@ -843,7 +893,10 @@ std::atomic<int64_t> g_fwd_fallbacks{0};
 // per-edge sums stay in registers, A's vertices (and in gradient mode its
 // gradient, until the pair is known to be clean) in shared memory.  The other
 // pairs are listed for the staged kernels, the unclean ones too in gradient
-// mode; in area mode those go to the GPC clip like theirs.
+// mode; in area mode those go to the GPC clip like theirs.  Of the pairs that are
+// left, those of up to kBwdOneV vertices together have a stage of their own in
+// gradient mode (100k pairs of 9-16 vertices: 364 us -> 295 us; 20k of equal
+// 4-6-vertex parcels, all unclean, 180 -> 120).
 constexpr int kTinyV = 8;
 constexpr int kTinyBlock = 128;
 
@@ -867,15 +920,15 @@ __device__ __forceinline__ void append_pair(bool ask, int64_t i, int32_t *list, 
   __syncthreads();
 }
 
-// The ring of a polygon that a thread can take: first vertex, vertices and
-// orientation sign flip of a hole; false for the others.
-__device__ __forceinline__ bool tiny_ring(const LayerDev &L, int64_t poly, int64_t *v0, int *nv, bool *hole) {
-  const int64_t r = L.poly_ring[poly];
-  if (L.poly_ring[poly + 1] != r + 1) return false;
+// A polygon's rings, first vertex and vertices; whether a thread can take it, and
+// then its ring's hole flag.
+__device__ __forceinline__ bool tiny_ring(const LayerDev &L, int64_t poly, int64_t *rings, int64_t *v0, int64_t *nv,
+                                          bool *hole) {
+  const int64_t r = L.poly_ring[poly], e = L.poly_ring[poly + 1];
+  *rings = e - r;
   *v0 = L.ring_vert[r];
-  const int64_t n = L.ring_vert[r + 1] - *v0;
-  if (n < 3 || n > kTinyV) return false;
-  *nv = (int)n;
+  *nv = L.ring_vert[e] - *v0;
+  if (e != r + 1 || *nv < 3 || *nv > kTinyV) return false;
   *hole = L.ring_hole && L.ring_hole[r];
   return true;
 }
@@ -894,7 +947,7 @@ __global__ void __launch_bounds__(kTinyBlock, kArea ? 4 : 3) area_tiny_kernel(
     const int32_t *__restrict__ pa, const int32_t *__restrict__ pb, int64_t n, LayerDev base, LayerDev over,
     const double *__restrict__ upstream, double *grad_base, double *grad_over, double *__restrict__ area,
     int32_t *__restrict__ fb, unsigned long long *__restrict__ fb_count, int32_t *__restrict__ defer,
-    unsigned long long *__restrict__ defer_count) {
+    unsigned long long *__restrict__ defer_count, int32_t *__restrict__ one, unsigned long long *__restrict__ one_count) {
   __shared__ TinySmem<kArea> S;
   __shared__ unsigned s_count[kTinyBlock / 32];
   __shared__ unsigned long long s_base;
@@ -903,11 +956,17 @@ __global__ void __launch_bounds__(kTinyBlock, kArea ? 4 : 3) area_tiny_kernel(
   int64_t va = 0, vb = 0;
   int na = 0, nb = 0;
   bool ha = false, hb = false;
-  bool mine = false;  // this thread takes the pair
+  bool mine = false, few = false;  // this thread takes the pair; the smallest stage can
   if (i < n) {
     const int64_t a = pa[i], b = pb[i];
-    if (a >= 0 && a < base.n_poly && b >= 0 && b < over.n_poly)
-      mine = tiny_ring(base, a, &va, &na, &ha) && tiny_ring(over, b, &vb, &nb, &hb);
+    if (a >= 0 && a < base.n_poly && b >= 0 && b < over.n_poly) {
+      int64_t ra, rb, ma, mb;
+      const bool ta = tiny_ring(base, a, &ra, &va, &ma, &ha), tb = tiny_ring(over, b, &rb, &vb, &mb, &hb);
+      mine = ta && tb;
+      few = ra <= 31 && rb <= 31 && ma + mb <= kBwdOneV;
+      na = (int)ma;
+      nb = (int)mb;
+    }
   }
   bool clean = true;
   double bound = 0.0, area2 = 0.0;
@@ -1130,7 +1189,9 @@ __global__ void __launch_bounds__(kTinyBlock, kArea ? 4 : 3) area_tiny_kernel(
     append_pair(mine && !keep, i, fb, fb_count, s_count, &s_base);
     append_pair(i < n && !mine, i, defer, defer_count, s_count, &s_base);
   } else {
-    append_pair(i < n && !(mine && clean), i, defer, defer_count, s_count, &s_base);
+    const bool left = i < n && !(mine && clean);
+    append_pair(left && few, i, one, one_count, s_count, &s_base);
+    append_pair(left && !few, i, defer, defer_count, s_count, &s_base);
   }
 }
 
@@ -1146,6 +1207,7 @@ __global__ void __launch_bounds__(32 * bwd_warps(V), V <= kBwdSmallV || V > kBwd
   const int lane = threadIdx.x & 31;
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  cudaGridDependencySynchronize();
   const int64_t items = list_items(PL, n);
   auto fallback = [&](int64_t i) {
     if (lane == 0) fb[atomicAdd(fb_count, 1ull)] = (int32_t)i;
@@ -1186,8 +1248,8 @@ __global__ void __launch_bounds__(32 * bwd_warps(V), V <= kBwdSmallV || V > kBwd
     Poly B{over.ring_vert, over.ring_hole, over.xy, rb0, rb1};
     AreaSum acc{0.0, 0.0};
     const double ox = M[0].x[0], oy = M[0].y[0];  // the pair-local origin
-    const bool ok = pair_boundary<true>(W, ext, nv[0], nv[1], gy, gx, 1.0, nullptr, nullptr, vb[0], vb[1], A, B,
-                                        ox, oy, &acc);
+    const bool ok = pair_boundary<true, false>(W, ext, nv[0], nv[1], gy, gx, 1.0, nullptr, nullptr, vb[0], vb[1], A, B,
+                                               ox, oy, &acc);
     if (ok) {
       double a2 = acc.area, er = acc.err;
       for (int o = 16; o; o >>= 1) {
@@ -1235,20 +1297,36 @@ int area_blocks(int64_t n_pairs, int threads, const void *kernel) {
   return grid_for(n_pairs * 32, threads, b);
 }
 
-template <int V>
-void launch_area_fwd(const int32_t *pa, const int32_t *pb, int64_t n, const LayerDev &base, const LayerDev &over,
-                     double *area, int32_t *fb, unsigned long long *fb_count, const PairList &PL, cudaStream_t s) {
-  const int threads = 32 * bwd_warps(V);
-  area_fwd_kernel<V><<<area_blocks(n, threads, (const void *)area_fwd_kernel<V>), threads, 0, s>>>(
-      pa, pb, n, base, over, area, fb, fb_count, PL);
+// A launch that starts when the kernel before it on the stream lets it
+// (cudaGridDependencySynchronize waits for that kernel's end).
+template <typename... K, typename... A>
+cudaError_t launch_dependent(void (*kernel)(K...), int blocks, int threads, cudaStream_t s, A... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3((unsigned)blocks);
+  c.blockDim = dim3((unsigned)threads);
+  c.stream = s;
+  c.attrs = &attr;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, static_cast<K>(args)...);
 }
 
 template <int V>
-void launch_area_bwd(const int32_t *pa, const int32_t *pb, int64_t n, const LayerDev &base, const LayerDev &over,
-                     const double *up, double *gb, double *go, const PairList &PL, cudaStream_t s) {
+cudaError_t launch_area_fwd(const int32_t *pa, const int32_t *pb, int64_t n, const LayerDev &base, const LayerDev &over,
+                            double *area, int32_t *fb, unsigned long long *fb_count, const PairList &PL, cudaStream_t s) {
   const int threads = 32 * bwd_warps(V);
-  area_bwd_kernel<V><<<area_blocks(n, threads, (const void *)area_bwd_kernel<V>), threads, 0, s>>>(pa, pb, n, base,
-                                                                                                  over, up, gb, go, PL);
+  return launch_dependent(area_fwd_kernel<V>, area_blocks(n, threads, (const void *)area_fwd_kernel<V>), threads, s, pa,
+                          pb, n, base, over, area, fb, fb_count, PL);
+}
+
+template <int V>
+cudaError_t launch_area_bwd(const int32_t *pa, const int32_t *pb, int64_t n, const LayerDev &base, const LayerDev &over,
+                            const double *up, double *gb, double *go, const PairList &PL, cudaStream_t s) {
+  const int threads = 32 * bwd_warps(V);
+  return launch_dependent(area_bwd_kernel<V>, area_blocks(n, threads, (const void *)area_bwd_kernel<V>), threads, s, pa,
+                          pb, n, base, over, up, gb, go, PL);
 }
 
 }  // namespace
@@ -1278,14 +1356,18 @@ int prt_area_fwd(const int32_t *d_pair_a, const int32_t *d_pair_b, int64_t n_pai
     PRT_PROF("area_fwd", s);
     const LayerDev A = layer_dev(base), B = layer_dev(overlay);
     area_tiny_kernel<true><<<(unsigned)((n_pairs + kTinyBlock - 1) / kTinyBlock), kTinyBlock, 0, s>>>(
-        d_pair_a, d_pair_b, n_pairs, A, B, nullptr, nullptr, nullptr, d_area, fb, cnt, small, cnt + 1);
-    launch_area_fwd<kBwdSmallV>(d_pair_a, d_pair_b, n_pairs, A, B, d_area, fb, cnt,
-                                PairList{small, cnt + 1, mid, cnt + 2}, s);
-    launch_area_fwd<kBwdMidV>(d_pair_a, d_pair_b, n_pairs, A, B, d_area, fb, cnt,
-                              PairList{mid, cnt + 2, large, cnt + 3}, s);
-    launch_area_fwd<kBwdLargeV>(d_pair_a, d_pair_b, n_pairs, A, B, d_area, fb, cnt,
-                                PairList{large, cnt + 3, nullptr, nullptr}, s);
+        d_pair_a, d_pair_b, n_pairs, A, B, nullptr, nullptr, nullptr, d_area, fb, cnt, small, cnt + 1, nullptr,
+        nullptr);
     e = cudaGetLastError();
+    if (e == cudaSuccess)
+      e = launch_area_fwd<kBwdSmallV>(d_pair_a, d_pair_b, n_pairs, A, B, d_area, fb, cnt,
+                                      PairList{small, cnt + 1, mid, cnt + 2}, s);
+    if (e == cudaSuccess)
+      e = launch_area_fwd<kBwdMidV>(d_pair_a, d_pair_b, n_pairs, A, B, d_area, fb, cnt,
+                                    PairList{mid, cnt + 2, large, cnt + 3}, s);
+    if (e == cudaSuccess)
+      e = launch_area_fwd<kBwdLargeV>(d_pair_a, d_pair_b, n_pairs, A, B, d_area, fb, cnt,
+                                      PairList{large, cnt + 3, nullptr, nullptr}, s);
   }
   unsigned long long m = 0;
   if (e == cudaSuccess) e = cudaMemcpyAsync(&m, cnt, 8, cudaMemcpyDeviceToHost, s);
@@ -1342,27 +1424,35 @@ int prt_area_bwd(const int32_t *d_pair_a, const int32_t *d_pair_b, int64_t n_pai
             PRT_ERR_INVALID, "NULL argument");
   if (n_pairs == 0) return PRT_OK;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  // pairs with a polygon too large for one stage's staging: listed by it,
-  // taken by the next
+  // pairs that tiny polygons' threads leave, of few vertices together or more;
+  // pairs with a polygon too large for one stage's staging: listed by it, taken by
+  // the next
   unsigned char *scr = nullptr;
-  int rc = dmalloc(reinterpret_cast<void **>(&scr), 64 + 12 * (size_t)n_pairs, s);
+  int rc = dmalloc(reinterpret_cast<void **>(&scr), 64 + 16 * (size_t)n_pairs, s);
   if (rc) return rc;
-  unsigned long long *cnt = reinterpret_cast<unsigned long long *>(scr);  // the three stage lists
-  int32_t *small = reinterpret_cast<int32_t *>(scr + 64), *mid = small + n_pairs, *large = mid + n_pairs;
-  cudaError_t e = cudaMemsetAsync(cnt, 0, 24, s);
+  unsigned long long *cnt = reinterpret_cast<unsigned long long *>(scr);  // the stages' lists
+  int32_t *one = reinterpret_cast<int32_t *>(scr + 64);
+  int32_t *small = one + n_pairs, *mid = small + n_pairs, *large = mid + n_pairs;
+  cudaError_t e = cudaMemsetAsync(cnt, 0, 32, s);
   if (e == cudaSuccess) {
     PRT_PROF("area_bwd", s);
     const LayerDev A = layer_dev(base), B = layer_dev(overlay);
     area_tiny_kernel<false><<<(unsigned)((n_pairs + kTinyBlock - 1) / kTinyBlock), kTinyBlock, 0, s>>>(
         d_pair_a, d_pair_b, n_pairs, A, B, d_upstream, d_grad_base, d_grad_overlay, nullptr, nullptr, nullptr, small,
-        cnt);
-    launch_area_bwd<kBwdSmallV>(d_pair_a, d_pair_b, n_pairs, A, B, d_upstream, d_grad_base, d_grad_overlay,
-                                PairList{small, cnt, mid, cnt + 1}, s);
-    launch_area_bwd<kBwdMidV>(d_pair_a, d_pair_b, n_pairs, A, B, d_upstream, d_grad_base, d_grad_overlay,
-                              PairList{mid, cnt + 1, large, cnt + 2}, s);
-    launch_area_bwd<kBwdLargeV>(d_pair_a, d_pair_b, n_pairs, A, B, d_upstream, d_grad_base, d_grad_overlay,
-                                PairList{large, cnt + 2, nullptr, nullptr}, s);
+        cnt, one, cnt + 3);
     e = cudaGetLastError();
+    if (e == cudaSuccess)
+      e = launch_area_bwd<kBwdSmallV>(d_pair_a, d_pair_b, n_pairs, A, B, d_upstream, d_grad_base, d_grad_overlay,
+                                      PairList{small, cnt, mid, cnt + 1}, s);
+    if (e == cudaSuccess)
+      e = launch_area_bwd<kBwdOneV>(d_pair_a, d_pair_b, n_pairs, A, B, d_upstream, d_grad_base, d_grad_overlay,
+                                    PairList{one, cnt + 3, nullptr, nullptr}, s);
+    if (e == cudaSuccess)
+      e = launch_area_bwd<kBwdMidV>(d_pair_a, d_pair_b, n_pairs, A, B, d_upstream, d_grad_base, d_grad_overlay,
+                                    PairList{mid, cnt + 1, large, cnt + 2}, s);
+    if (e == cudaSuccess)
+      e = launch_area_bwd<kBwdLargeV>(d_pair_a, d_pair_b, n_pairs, A, B, d_upstream, d_grad_base, d_grad_overlay,
+                                      PairList{large, cnt + 2, nullptr, nullptr}, s);
   }
   dfree(scr, s);
   if (e != cudaSuccess) return cuda_status(e, "area backward");

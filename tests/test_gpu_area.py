@@ -273,3 +273,42 @@ def test_tiny_polygons(cuda, nv):
         scale = wn[i] * max(np.abs(rs).max(), np.abs(rc).max(), 1e-30)
         assert np.abs(ga[i] - wn[i] * rs).max() <= 1e-9 * scale, i
         assert np.abs(gb[i] - wn[i] * rc).max() <= 1e-9 * scale, i
+
+
+def check_pairs(A, B, area, ga, gb, which):
+    """Areas and gradients of the sum against the oracle's, pair i of A's and B's
+    polygons i (the tolerances of test_forward_and_adjoint_match_oracle)."""
+    for i in which:
+        s, q = rings_of(A, i), rings_of(B, i)
+        ref = oracle.result_area(oracle.gpc_clip(s, q, 1))
+        assert abs(area[i] - ref) <= 1e-9 * abs(ref) + 1e-22, i
+        ra, rb = (slice(L["poly_ring"][i], L["poly_ring"][i + 1]) for L in (A, B))
+        _, rs, rc = oracle.area_grad(s, q, A["ring_hole"][ra], B["ring_hole"][rb])
+        va, vb = (slice(L["ring_vert"][r.start], L["ring_vert"][r.stop]) for L, r in ((A, ra), (B, rb)))
+        scale = max(np.abs(rs).max(), np.abs(rc).max(), 1e-30)
+        assert np.abs(ga[va] - rs).max() <= 1e-9 * scale, i
+        assert np.abs(gb[vb] - rc).max() <= 1e-9 * scale, i
+
+
+@pytest.mark.parametrize("na,nb,hole_frac", [(3, 3, 0.0), (8, 8, 0.0), (8, 9, 0.0), (9, 23, 0.0), (16, 16, 0.0),
+                                             (16, 17, 0.0), (29, 3, 0.0), (29, 4, 0.0), (10, 8, 0.9)])
+def test_many_small_pairs(cuda, na, nb, hole_frac):
+    """9,000 pairs around the sizes of the thread per pair (8 vertices each) and of
+    the one-round stage (32 together, holes included), some of equal polygons."""
+    import parlllelrtree_b200 as prt
+
+    n = 9000
+    rng = np.random.default_rng(na * 100 + nb)
+    c, r = rng.random((n, 2)), np.full(n, 0.01)
+    A = dg.star_layer(n, seed=3, nv_lo=na, nv_hi=na, centre_xy=c, radii=r, hole_frac=hole_frac)
+    B = dg.star_layer(n, seed=4, nv_lo=nb, nv_hi=nb, centre_xy=c + rng.uniform(-0.012, 0.012, (n, 2)),
+                      radii=r * rng.uniform(0.3, 1.5, n), hole_frac=hole_frac)
+    if na == nb:
+        B["xy"][:20 * nb] = A["xy"][:20 * na]
+    LA, LB = prt.Layer.from_dict(A), prt.Layer.from_dict(B)
+    idx = torch.arange(n, dtype=torch.int32, device="cuda")
+    xa, xb = LA.xy.clone().requires_grad_(True), LB.xy.clone().requires_grad_(True)
+    area = prt.intersection_area(LA, LB, idx, idx, xa, xb)
+    area.sum().backward()
+    check_pairs(A, B, area.detach().cpu().numpy(), xa.grad.cpu().numpy(), xb.grad.cpu().numpy(),
+                list(range(200)) + list(range(200, n, 30)))
