@@ -775,7 +775,8 @@ __device__ __forceinline__ int64_t list_items(const PairList &L, int64_t n) {
 // forward's GPC clip.
 // The smallest stage is launched beside the 64-vertex one, in whose tail it runs:
 // both take what area_tiny_kernel lists.
-template <int V>
+// kMixed: pairs of few vertices are taken here too, in one round.
+template <int V, bool kMixed>
 __global__ void __launch_bounds__(32 * bwd_warps(V), V > kBwdMidV ? 5 : 4) area_bwd_kernel(
     const int32_t *__restrict__ pa, const int32_t *__restrict__ pb, int64_t n, LayerDev base, LayerDev over,
     const double *__restrict__ upstream, double *grad_base, double *grad_over, PairList PL) {
@@ -838,7 +839,7 @@ __global__ void __launch_bounds__(32 * bwd_warps(V), V > kBwdMidV ? 5 : 4) area_
           Poly A{base.ring_vert, base.ring_hole, base.xy, rr[0], rr[1]};
           Poly B{over.ring_vert, over.ring_hole, over.xy, rr[2], rr[3]};
           const SlabGrid gy = slab_grid(y0, y1), gx = slab_grid(x0, x1);
-          if constexpr (V == kBwdOneV)
+          if (V == kBwdOneV || (kMixed && nv[0] + nv[1] <= kBwdOneV))
             pair_boundary<false, true>(W, ext, nv[0], nv[1], gy, gx, w, grad_base, grad_over, vb[0], vb[1], A, B, 0.0,
                                        0.0, nullptr);
           else
@@ -899,6 +900,12 @@ std::atomic<int64_t> g_fwd_fallbacks{0};
 // 4-6-vertex parcels, all unclean, 180 -> 120).
 constexpr int kTinyV = 8;
 constexpr int kTinyBlock = 128;
+// A thread takes 15-25 us for its pair however few there are.  Up to kFewPairs
+// pairs, two or three waves of warps, every pair starts in the 64-vertex stage (1,000
+// pairs of 4-6 vertices: backward 44 -> 31 us; from some 10,000 on the threads are as
+// fast), and up to kOnePairWave, one wave of the 256-vertex stage, what does not
+// fit goes straight to that.
+constexpr int64_t kFewPairs = 8192, kOnePairWave = (int64_t)kSMs * 10;
 
 // Appends i to a list for the threads of the block that ask (one atomic per
 // block: when no pair is tiny, every one of them is listed).
@@ -1287,13 +1294,16 @@ __global__ void scatter_area_kernel(const int32_t *__restrict__ fb, int64_t m, c
     area[fb[k]] = src[k];
 }
 
-int area_blocks(int64_t n_pairs, int threads, const void *kernel) {
-  int b = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, threads, 0) != cudaSuccess || b < 1) {
-    cudaGetLastError();
-    b = 4;
+// Exactly the resident blocks (each warp loops over pairs): no tail wave.
+int area_blocks(int64_t n_pairs, int threads, const void *kernel, std::atomic<int> &per_sm) {
+  int b = per_sm.load(std::memory_order_relaxed);
+  if (b == 0) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, threads, 0) != cudaSuccess || b < 1) {
+      cudaGetLastError();
+      b = 4;
+    }
+    per_sm.store(b, std::memory_order_relaxed);
   }
-  // exactly the resident blocks (each warp loops over pairs): no tail wave
   return grid_for(n_pairs * 32, threads, b);
 }
 
@@ -1317,16 +1327,19 @@ template <int V>
 cudaError_t launch_area_fwd(const int32_t *pa, const int32_t *pb, int64_t n, const LayerDev &base, const LayerDev &over,
                             double *area, int32_t *fb, unsigned long long *fb_count, const PairList &PL, cudaStream_t s) {
   const int threads = 32 * bwd_warps(V);
-  return launch_dependent(area_fwd_kernel<V>, area_blocks(n, threads, (const void *)area_fwd_kernel<V>), threads, s, pa,
-                          pb, n, base, over, area, fb, fb_count, PL);
+  static std::atomic<int> per_sm{0};
+  return launch_dependent(area_fwd_kernel<V>, area_blocks(n, threads, (const void *)area_fwd_kernel<V>, per_sm), threads,
+                          s, pa, pb, n, base, over, area, fb, fb_count, PL);
 }
 
-template <int V>
+template <int V, bool kMixed = false>
 cudaError_t launch_area_bwd(const int32_t *pa, const int32_t *pb, int64_t n, const LayerDev &base, const LayerDev &over,
                             const double *up, double *gb, double *go, const PairList &PL, cudaStream_t s) {
   const int threads = 32 * bwd_warps(V);
-  return launch_dependent(area_bwd_kernel<V>, area_blocks(n, threads, (const void *)area_bwd_kernel<V>), threads, s, pa,
-                          pb, n, base, over, up, gb, go, PL);
+  static std::atomic<int> per_sm{0};
+  return launch_dependent(area_bwd_kernel<V, kMixed>,
+                          area_blocks(n, threads, (const void *)area_bwd_kernel<V, kMixed>, per_sm), threads, s, pa, pb,
+                          n, base, over, up, gb, go, PL);
 }
 
 }  // namespace
@@ -1355,19 +1368,20 @@ int prt_area_fwd(const int32_t *d_pair_a, const int32_t *d_pair_b, int64_t n_pai
   if (e == cudaSuccess) {
     PRT_PROF("area_fwd", s);
     const LayerDev A = layer_dev(base), B = layer_dev(overlay);
-    area_tiny_kernel<true><<<(unsigned)((n_pairs + kTinyBlock - 1) / kTinyBlock), kTinyBlock, 0, s>>>(
-        d_pair_a, d_pair_b, n_pairs, A, B, nullptr, nullptr, nullptr, d_area, fb, cnt, small, cnt + 1, nullptr,
-        nullptr);
-    e = cudaGetLastError();
-    if (e == cudaSuccess)
-      e = launch_area_fwd<kBwdSmallV>(d_pair_a, d_pair_b, n_pairs, A, B, d_area, fb, cnt,
-                                      PairList{small, cnt + 1, mid, cnt + 2}, s);
-    if (e == cudaSuccess)
+    if (n_pairs > kFewPairs) {
+      area_tiny_kernel<true><<<(unsigned)((n_pairs + kTinyBlock - 1) / kTinyBlock), kTinyBlock, 0, s>>>(
+          d_pair_a, d_pair_b, n_pairs, A, B, nullptr, nullptr, nullptr, d_area, fb, cnt, small, cnt + 1, nullptr,
+          nullptr);
+      e = cudaGetLastError();
+    }
+    PairList first = {nullptr, nullptr, mid, cnt + 2}, last = {mid, cnt + 2, nullptr, nullptr};
+    if (n_pairs > kFewPairs) first = {small, cnt + 1, mid, cnt + 2};
+    if (n_pairs > kOnePairWave) last = {large, cnt + 3, nullptr, nullptr};
+    if (e == cudaSuccess) e = launch_area_fwd<kBwdSmallV>(d_pair_a, d_pair_b, n_pairs, A, B, d_area, fb, cnt, first, s);
+    if (e == cudaSuccess && n_pairs > kOnePairWave)
       e = launch_area_fwd<kBwdMidV>(d_pair_a, d_pair_b, n_pairs, A, B, d_area, fb, cnt,
                                     PairList{mid, cnt + 2, large, cnt + 3}, s);
-    if (e == cudaSuccess)
-      e = launch_area_fwd<kBwdLargeV>(d_pair_a, d_pair_b, n_pairs, A, B, d_area, fb, cnt,
-                                      PairList{large, cnt + 3, nullptr, nullptr}, s);
+    if (e == cudaSuccess) e = launch_area_fwd<kBwdLargeV>(d_pair_a, d_pair_b, n_pairs, A, B, d_area, fb, cnt, last, s);
   }
   unsigned long long m = 0;
   if (e == cudaSuccess) e = cudaMemcpyAsync(&m, cnt, 8, cudaMemcpyDeviceToHost, s);
@@ -1437,22 +1451,29 @@ int prt_area_bwd(const int32_t *d_pair_a, const int32_t *d_pair_b, int64_t n_pai
   if (e == cudaSuccess) {
     PRT_PROF("area_bwd", s);
     const LayerDev A = layer_dev(base), B = layer_dev(overlay);
-    area_tiny_kernel<false><<<(unsigned)((n_pairs + kTinyBlock - 1) / kTinyBlock), kTinyBlock, 0, s>>>(
-        d_pair_a, d_pair_b, n_pairs, A, B, d_upstream, d_grad_base, d_grad_overlay, nullptr, nullptr, nullptr, small,
-        cnt, one, cnt + 3);
-    e = cudaGetLastError();
-    if (e == cudaSuccess)
-      e = launch_area_bwd<kBwdSmallV>(d_pair_a, d_pair_b, n_pairs, A, B, d_upstream, d_grad_base, d_grad_overlay,
-                                      PairList{small, cnt, mid, cnt + 1}, s);
-    if (e == cudaSuccess)
-      e = launch_area_bwd<kBwdOneV>(d_pair_a, d_pair_b, n_pairs, A, B, d_upstream, d_grad_base, d_grad_overlay,
-                                    PairList{one, cnt + 3, nullptr, nullptr}, s);
-    if (e == cudaSuccess)
+    PairList last = {mid, cnt + 1, nullptr, nullptr};
+    if (n_pairs > kOnePairWave) last = {large, cnt + 2, nullptr, nullptr};
+    if (n_pairs > kFewPairs) {
+      area_tiny_kernel<false><<<(unsigned)((n_pairs + kTinyBlock - 1) / kTinyBlock), kTinyBlock, 0, s>>>(
+          d_pair_a, d_pair_b, n_pairs, A, B, d_upstream, d_grad_base, d_grad_overlay, nullptr, nullptr, nullptr, small,
+          cnt, one, cnt + 3);
+      e = cudaGetLastError();
+      if (e == cudaSuccess)
+        e = launch_area_bwd<kBwdSmallV>(d_pair_a, d_pair_b, n_pairs, A, B, d_upstream, d_grad_base, d_grad_overlay,
+                                        PairList{small, cnt, mid, cnt + 1}, s);
+      if (e == cudaSuccess)
+        e = launch_area_bwd<kBwdOneV>(d_pair_a, d_pair_b, n_pairs, A, B, d_upstream, d_grad_base, d_grad_overlay,
+                                      PairList{one, cnt + 3, nullptr, nullptr}, s);
+    } else {
+      e = launch_area_bwd<kBwdSmallV, true>(d_pair_a, d_pair_b, n_pairs, A, B, d_upstream, d_grad_base, d_grad_overlay,
+                                            PairList{nullptr, nullptr, mid, cnt + 1}, s);
+    }
+    if (e == cudaSuccess && n_pairs > kOnePairWave)
       e = launch_area_bwd<kBwdMidV>(d_pair_a, d_pair_b, n_pairs, A, B, d_upstream, d_grad_base, d_grad_overlay,
                                     PairList{mid, cnt + 1, large, cnt + 2}, s);
     if (e == cudaSuccess)
-      e = launch_area_bwd<kBwdLargeV>(d_pair_a, d_pair_b, n_pairs, A, B, d_upstream, d_grad_base, d_grad_overlay,
-                                      PairList{large, cnt + 2, nullptr, nullptr}, s);
+      e = launch_area_bwd<kBwdLargeV>(d_pair_a, d_pair_b, n_pairs, A, B, d_upstream, d_grad_base, d_grad_overlay, last,
+                                      s);
   }
   dfree(scr, s);
   if (e != cudaSuccess) return cuda_status(e, "area backward");

@@ -312,3 +312,30 @@ def test_many_small_pairs(cuda, na, nb, hole_frac):
     area.sum().backward()
     check_pairs(A, B, area.detach().cpu().numpy(), xa.grad.cpu().numpy(), xb.grad.cpu().numpy(),
                 list(range(200)) + list(range(200, n, 30)))
+
+
+@pytest.mark.parametrize("n", [1, 1480, 1481, 8192, 8193])
+def test_stages_by_the_number_of_pairs(cuda, n):
+    """Polygons of all stages' sizes around the numbers of pairs at which the
+    one-thread kernel and the 128-vertex stage come in."""
+    import parlllelrtree_b200 as prt
+
+    rng = np.random.default_rng(n)
+    sizes = np.array([4, 6, 11, 16, 30, 64, 65, 128, 129, 256, 257])
+    p = np.array([20, 20, 20, 10, 10, 8, 4, 4, 2, 1, 1]) / 100
+
+    def layer(seed, c, r):
+        nv = rng.choice(sizes, n, p=p) if n > 1 else np.array([129])
+        ring_vert, xy = dg._star_rings(np.random.default_rng(seed), c, r, nv)
+        return {"poly_ring": np.arange(n + 1), "ring_vert": ring_vert, "ring_hole": np.zeros(n, np.int32), "xy": xy}
+
+    c, r = rng.random((n, 2)), np.full(n, 0.01)
+    A = layer(1, c, r)
+    B = layer(2, c + rng.uniform(-0.01, 0.01, (n, 2)), r * rng.uniform(0.3, 1.5, n))
+    LA, LB = prt.Layer.from_dict(A), prt.Layer.from_dict(B)
+    idx = torch.arange(n, dtype=torch.int32, device="cuda")
+    xa, xb = LA.xy.clone().requires_grad_(True), LB.xy.clone().requires_grad_(True)
+    area = prt.intersection_area(LA, LB, idx, idx, xa, xb)
+    area.sum().backward()
+    check_pairs(A, B, area.detach().cpu().numpy(), xa.grad.cpu().numpy(), xb.grad.cpu().numpy(),
+                range(0, n, max(1, n // 400)))
