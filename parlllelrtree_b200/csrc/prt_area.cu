@@ -32,6 +32,7 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <climits>
 
 #include "prt_internal.cuh"
 #include "prt_overlay.cuh"
@@ -230,6 +231,7 @@ __device__ inline bool bwd_load_pair(const LayerDev &LA, int64_t ra0, int64_t ra
                                      int64_t rb1, BwdPoly<V> *M, int *nv, int64_t *vb, float4 *ext) {
   const int lane = threadIdx.x & 31;
   const int nr[2] = {(int)(ra1 - ra0), (int)(rb1 - rb0)};
+  nv[0] = nv[1] = INT_MAX;
   if (nr[0] > 31 || nr[1] > 31) return false;
   int64_t rv[2] = {0, 0};
   int hl[2] = {0, 0};
@@ -755,7 +757,9 @@ __device__ __noinline__ void bwd_pair_global(const Poly &A, const Poly &B, doubl
 // Pair lists of the staged launches: the first stage (V = kBwdSmallV) takes
 // every pair and lists those with a polygon above V vertices (or 31 rings) in
 // `defer`; the next stages (V = kBwdMidV, kBwdLargeV) take only the pairs the
-// one before listed (`sel`, *sel_count of them).
+// one before listed (`sel`, *sel_count of them).  The gradients of pairs too large for
+// the last stage are taken on the global-memory path by the one before it, which has 16
+// warps per SM for its 10 (10k pairs of 257-400 vertices: 28.5 ms against 40.9).
 struct PairList {
   const int32_t *sel;                   // items of this launch (nullptr: pairs 0 .. n-1)
   const unsigned long long *sel_count;  // how many (device)
@@ -846,7 +850,7 @@ __global__ void __launch_bounds__(32 * bwd_warps(V), V > kBwdMidV ? 5 : 4) area_
             pair_boundary<false, false>(W, ext, nv[0], nv[1], gy, gx, w, grad_base, grad_over, vb[0], vb[1], A, B,
                                         0.0, 0.0, nullptr);
         }
-      } else if (PL.defer) {
+      } else if (PL.defer && (V != kBwdMidV || max(nv[0], nv[1]) <= kBwdLargeV)) {
         if ((threadIdx.x & 31) == 0) PL.defer[atomicAdd(PL.defer_count, 1ull)] = (int32_t)i;
       } else if (V > kBwdOneV) {  // all that is listed for the smallest stage fits
         const double w = upstream ? upstream[i] : 1.0;

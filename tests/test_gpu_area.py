@@ -339,3 +339,29 @@ def test_stages_by_the_number_of_pairs(cuda, n):
     area.sum().backward()
     check_pairs(A, B, area.detach().cpu().numpy(), xa.grad.cpu().numpy(), xb.grad.cpu().numpy(),
                 range(0, n, max(1, n // 400)))
+
+
+@pytest.mark.parametrize("n", [6, 1500])
+def test_pairs_above_every_stage(cuda, n):
+    """Polygons of 300 vertices and of 33 rings (a square with a grid of square holes)
+    in calls that take one and both of the larger stages."""
+    import parlllelrtree_b200 as prt
+
+    rng = np.random.default_rng(n)
+    sq = lambda x, y, s: np.array([[x, y], [x + s, y], [x + s, y + s], [x, y + s]])
+    holes = [sq(0.1 + 0.11 * (k % 8), 0.2 + 0.17 * (k // 8), 0.05)[::-1] for k in range(32)]
+    big = dg.star_layer(3, seed=9, nv_lo=300, nv_hi=300, centre_xy=np.full((3, 2), 0.5), radii=np.full(3, 0.6))
+    polys_a, polys_b = [], []
+    for i in range(n):
+        move = rng.uniform(-0.2, 0.2, 2)
+        polys_a.append([sq(0, 0, 1.0)] + holes if i % 3 == 0 else [rings_of(big, i % 3)[0]] if i < 30 else [sq(0, 0, 1.0)])
+        polys_b.append([rings_of(big, 0)[0] + move] if i < 30 else [sq(0.3, 0.2, 0.9) + move])
+    layers = [dg.layer_from_rings([r for p in polys for r in p], [int(k > 0) for p in polys for k in range(len(p))],
+                                  [len(p) for p in polys]) for polys in (polys_a, polys_b)]
+    A, B = layers
+    LA, LB = prt.Layer.from_dict(A), prt.Layer.from_dict(B)
+    idx = torch.arange(n, dtype=torch.int32, device="cuda")
+    xa, xb = LA.xy.clone().requires_grad_(True), LB.xy.clone().requires_grad_(True)
+    area = prt.intersection_area(LA, LB, idx, idx, xa, xb)
+    area.sum().backward()
+    check_pairs(A, B, area.detach().cpu().numpy(), xa.grad.cpu().numpy(), xb.grad.cpu().numpy(), range(min(n, 60)))
