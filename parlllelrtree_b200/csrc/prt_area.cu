@@ -1039,7 +1039,7 @@ __global__ void __launch_bounds__(kTinyBlock, kArea ? 4 : 3) area_tiny_kernel(
       double err = 0.0;
       bool st = false;  // inside state at the start of A's edge k
       double cx = 0.0, cy = 0.0;  // what the edge before gives to A's vertex k
-      for (int k = 0; k < na; k++) {
+      for (int k = 0; k < na && clean; k++) {
         const int l = k + 1 == na ? 0 : k + 1;
         const double px = S.x[k][tid], py = S.y[k][tid], qx = S.x[l][tid], qy = S.y[l][tid];
         const double rx = qx - px, ry = qy - py;
