@@ -1009,8 +1009,9 @@ __global__ void __launch_bounds__(kTinyBlock, kArea ? 4 : 3) area_tiny_kernel(
       }
     }
     cmax = fmax(cmax, fmax(fmax(fabs(blx), fabs(bly)), fmax(fabs(bhx), fabs(bhy))));
-    // boxes apart: no crossing, no point of one inside the other (a NaN
-    // coordinate is not apart, and not clean below)
+    // boxes apart: no crossing, no point of one inside the other (the boxes leave
+    // NaN coordinates out, as the staged kernels' do; of a pair that is not apart
+    // they are not clean below)
     const bool apart = lox > bhx || hix < blx || loy > bhy || hiy < bly;
     if (!apart) {
       for (int k = 0; k < na; k++) {

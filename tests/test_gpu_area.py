@@ -365,3 +365,29 @@ def test_pairs_above_every_stage(cuda, n):
     area = prt.intersection_area(LA, LB, idx, idx, xa, xb)
     area.sum().backward()
     check_pairs(A, B, area.detach().cpu().numpy(), xa.grad.cpu().numpy(), xb.grad.cpu().numpy(), range(min(n, 60)))
+
+
+@pytest.mark.parametrize("n", [24, 9000])
+def test_nan_vertex_of_a_polygon_apart(cuda, n):
+    """Polygons of 3 to 8 vertices, one of them NaN (any place, either polygon), whose
+    other vertices are apart from the other polygon: no area, no gradient, staged
+    (24 pairs) or one thread per pair."""
+    import parlllelrtree_b200 as prt
+
+    nv = 3 + np.arange(n) % 6
+    c = np.random.default_rng(2).random((n, 2))
+
+    def layer(seed, c):
+        ring_vert, xy = dg._star_rings(np.random.default_rng(seed), c, np.full(n, 0.01), nv)
+        return {"poly_ring": np.arange(n + 1), "ring_vert": ring_vert, "ring_hole": np.zeros(n, np.int32), "xy": xy}
+
+    A, B = layer(1, c), layer(2, c + [0.03, 0.0])
+    for i in range(n):
+        L = (A, B)[i % 2]
+        L["xy"][L["ring_vert"][i] + (i // 6) % nv[i], i // 12 % 2] = np.nan
+    LA, LB = prt.Layer.from_dict(A), prt.Layer.from_dict(B)
+    idx = torch.arange(n, dtype=torch.int32, device="cuda")
+    xa, xb = LA.xy.clone().requires_grad_(True), LB.xy.clone().requires_grad_(True)
+    area = prt.intersection_area(LA, LB, idx, idx, xa, xb)
+    area.sum().backward()
+    assert (area == 0).all() and (xa.grad == 0).all() and (xb.grad == 0).all()
