@@ -68,46 +68,54 @@ __device__ __forceinline__ void store_extent(const double *b, double scale, int 
 constexpr int kMbrGroup = 4, kMbrSmall = 64;
 constexpr int64_t kMbrGrouped = (int64_t)kSMs * 64 * kMbrGroup;
 
-template <typename Out, bool kAligned>
+template <typename Out, bool kAligned, int kGroup>
 __device__ __forceinline__ void poly_mbr_body(const LayerDev &L, double scale, Out *__restrict__ out) {
   const int lane = threadIdx.x & 31, g = lane >> 3;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const int64_t w0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   constexpr double kMax = 1.7976931348623157e308;
-  const int group = L.n_poly >= kMbrGrouped ? kMbrGroup : 1;
-  for (int64_t p0 = w0 * group; p0 < L.n_poly; p0 += nw * group) {
+  for (int64_t p0 = w0 * kGroup; p0 < L.n_poly; p0 += nw * kGroup) {
     // lanes 8 g .. 8 g + 7: polygon p0 + g (one polygon: all lanes)
-    const int64_t p = group > 1 ? p0 + g : p0;
+    const int64_t p = kGroup > 1 ? p0 + g : p0;
     int64_t v0 = 0, v1 = 0;
     if (p < L.n_poly) {
       v0 = L.ring_vert[L.poly_ring[p]];
       v1 = L.ring_vert[L.poly_ring[p + 1]];
     }
-    if (group > 1 && !__any_sync(0xffffffffu, v1 - v0 > kMbrSmall)) {
-      double b[4] = {kMax, kMax, -kMax, -kMax};
-      extend<kAligned, 8>(L.xy, v0, v1, lane & 7, b);
-      reduce_extent(b, 8);
-      if (p < L.n_poly && (lane & 7) < 4) store_extent(b, scale, lane & 7, p, out);
-      continue;
+    if constexpr (kGroup > 1) {
+      if (!__any_sync(0xffffffffu, v1 - v0 > kMbrSmall)) {
+        double b[4] = {kMax, kMax, -kMax, -kMax};
+        extend<kAligned, 8>(L.xy, v0, v1, lane & 7, b);
+        reduce_extent(b, 8);
+        if (p < L.n_poly && (lane & 7) < 4) store_extent(b, scale, lane & 7, p, out);
+        continue;
+      }
     }
-    for (int k = 0; k < group && p0 + k < L.n_poly; k++) {
+#pragma unroll 1
+    for (int k = 0; k < kGroup && p0 + k < L.n_poly; k++) {
+      const int64_t from = kGroup > 1 ? __shfl_sync(0xffffffffu, v0, 8 * k) : v0;
+      const int64_t to = kGroup > 1 ? __shfl_sync(0xffffffffu, v1, 8 * k) : v1;
       double b[4] = {kMax, kMax, -kMax, -kMax};
-      extend<kAligned, 32>(L.xy, __shfl_sync(0xffffffffu, v0, 8 * k), __shfl_sync(0xffffffffu, v1, 8 * k), lane, b);
+      extend<kAligned, 32>(L.xy, from, to, lane, b);
       reduce_extent(b, 32);
       if (lane < 4) store_extent(b, scale, lane, p0 + k, out);
     }
   }
 }
 
-template <typename Out>
+template <typename Out, int kGroup>
 __global__ void poly_mbr_kernel(LayerDev L, double scale, Out *__restrict__ out) {
-  if ((reinterpret_cast<uintptr_t>(L.xy) & 15) == 0) poly_mbr_body<Out, true>(L, scale, out);
-  else poly_mbr_body<Out, false>(L, scale, out);
+  if ((reinterpret_cast<uintptr_t>(L.xy) & 15) == 0) poly_mbr_body<Out, true, kGroup>(L, scale, out);
+  else poly_mbr_body<Out, false, kGroup>(L, scale, out);
 }
 
-inline int poly_mbr_grid(int64_t n_poly) {
-  const int64_t group = n_poly >= kMbrGrouped ? kMbrGroup : 1;
-  return grid_for((n_poly + group - 1) / group * 32, 256, 8);
+template <typename Out>
+void launch_poly_mbr(const LayerDev &L, double scale, Out *out, cudaStream_t s) {
+  if (L.n_poly >= kMbrGrouped)
+    poly_mbr_kernel<Out, kMbrGroup>
+        <<<grid_for((L.n_poly + kMbrGroup - 1) / kMbrGroup * 32, 256, 8), 256, 0, s>>>(L, scale, out);
+  else
+    poly_mbr_kernel<Out, 1><<<grid_for(L.n_poly * 32, 256, 8), 256, 0, s>>>(L, scale, out);
 }
 
 // Largest vertex count of a polygon of the layer (sizes the biggest arenas).
@@ -177,8 +185,8 @@ int enqueue_run(prt_pipeline *p, cudaStream_t s) {
   PRT_CUDA(cudaMemsetAsync(p->counters, 0, sizeof(unsigned long long) * (PRT_MAX_LEVELS + 2), s));
   {
     PRT_PROF("poly_mbr", s);
-    poly_mbr_kernel<double><<<poly_mbr_grid(p->base.n_poly), 256, 0, s>>>(p->base, 1.0, p->base_mbr);
-    poly_mbr_kernel<double><<<poly_mbr_grid(p->over.n_poly), 256, 0, s>>>(p->over, 1.0, p->over_mbr);
+    launch_poly_mbr<double>(p->base, 1.0, p->base_mbr, s);
+    launch_poly_mbr<double>(p->over, 1.0, p->over_mbr, s);
   }
   int rc = bu_enqueue(p->tree, p->base_mbr, nullptr, p->build_err, s);
   if (!rc)
@@ -330,7 +338,7 @@ int prt_layer_mbr(const prt_layer *layer, double *d_out, void *stream) {
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   {
     PRT_PROF("poly_mbr", s);
-    poly_mbr_kernel<double><<<poly_mbr_grid(layer->n_poly), 256, 0, s>>>(layer_dev(layer), 1.0, d_out);
+    launch_poly_mbr<double>(layer_dev(layer), 1.0, d_out, s);
   }
   PRT_CUDA(cudaGetLastError());
   return PRT_OK;
@@ -344,7 +352,7 @@ int prt_layer_mbr_i32(const prt_layer *layer, double scale, int32_t *d_out, void
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   {
     PRT_PROF("poly_mbr", s);
-    poly_mbr_kernel<int32_t><<<poly_mbr_grid(layer->n_poly), 256, 0, s>>>(layer_dev(layer), scale, d_out);
+    launch_poly_mbr<int32_t>(layer_dev(layer), scale, d_out, s);
   }
   PRT_CUDA(cudaGetLastError());
   return PRT_OK;
