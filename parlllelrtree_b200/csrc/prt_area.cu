@@ -1312,29 +1312,13 @@ int area_blocks(int64_t n_pairs, int threads, const void *kernel, std::atomic<in
   return grid_for(n_pairs * 32, threads, b);
 }
 
-// A launch that starts when the kernel before it on the stream lets it
-// (cudaGridDependencySynchronize waits for that kernel's end).
-template <typename... K, typename... A>
-cudaError_t launch_dependent(void (*kernel)(K...), int blocks, int threads, cudaStream_t s, A... args) {
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t c = {};
-  c.gridDim = dim3((unsigned)blocks);
-  c.blockDim = dim3((unsigned)threads);
-  c.stream = s;
-  c.attrs = &attr;
-  c.numAttrs = 1;
-  return cudaLaunchKernelEx(&c, kernel, static_cast<K>(args)...);
-}
-
 template <int V>
 cudaError_t launch_area_fwd(const int32_t *pa, const int32_t *pb, int64_t n, const LayerDev &base, const LayerDev &over,
                             double *area, int32_t *fb, unsigned long long *fb_count, const PairList &PL, cudaStream_t s) {
   const int threads = 32 * bwd_warps(V);
   static std::atomic<int> per_sm{0};
   return launch_dependent(area_fwd_kernel<V>, area_blocks(n, threads, (const void *)area_fwd_kernel<V>, per_sm), threads,
-                          s, pa, pb, n, base, over, area, fb, fb_count, PL);
+                          0, s, pa, pb, n, base, over, area, fb, fb_count, PL);
 }
 
 template <int V, bool kMixed = false>
@@ -1343,8 +1327,8 @@ cudaError_t launch_area_bwd(const int32_t *pa, const int32_t *pb, int64_t n, con
   const int threads = 32 * bwd_warps(V);
   static std::atomic<int> per_sm{0};
   return launch_dependent(area_bwd_kernel<V, kMixed>,
-                          area_blocks(n, threads, (const void *)area_bwd_kernel<V, kMixed>, per_sm), threads, s, pa, pb,
-                          n, base, over, up, gb, go, PL);
+                          area_blocks(n, threads, (const void *)area_bwd_kernel<V, kMixed>, per_sm), threads, 0, s, pa,
+                          pb, n, base, over, up, gb, go, PL);
 }
 
 }  // namespace

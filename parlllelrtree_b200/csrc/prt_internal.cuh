@@ -69,6 +69,24 @@ struct ProfScope {
 #define PRT_PROF_CAT(a, b) PRT_PROF_CAT2(a, b)
 #define PRT_PROF(name, s) ::prt::ProfScope PRT_PROF_CAT(prt_prof_, __LINE__)(name, s)
 
+// ---- launches ----------------------------------------------------------------
+// A launch that starts when the kernel before it on the stream lets it
+// (cudaGridDependencySynchronize waits for that kernel's end).
+template <typename... K, typename... A>
+cudaError_t launch_dependent(void (*kernel)(K...), int blocks, int threads, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3((unsigned)blocks);
+  c.blockDim = dim3((unsigned)threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  c.attrs = &attr;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, static_cast<K>(args)...);
+}
+
 // ---- stream-ordered scratch ------------------------------------------------
 int dmalloc(void **p, size_t bytes, cudaStream_t s);
 void dfree(void *p, cudaStream_t s);

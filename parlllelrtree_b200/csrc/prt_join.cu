@@ -706,7 +706,7 @@ struct CountsItem {
 
 struct CountsQueue {
   const CountsItem *in;          // work of this launch (nullptr: the root for every query)
-  int64_t n_in;
+  const unsigned long long *n_in;
   CountsItem *out;               // work left over
   unsigned long long *out_count;
   int64_t out_cap;
@@ -723,15 +723,23 @@ struct CountsQueue {
 // A query that is not done after kCountsSteps steps (a long thin window, a tree
 // that cannot be pruned) leaves what is on its stack to the next launch, where
 // every node is a work item of its own.
-// Bound by instruction issue (0.66 per cycle and scheduler; DRAM and L2 under
-// 10%): 1M windows of 1e-4..1e-2 on 10M boxes, 2.15 ms at F = 16 and 2.21 at
-// F = 32, breadth first 3.55 and 4.24.  1 and 3 rounds at F = 16: 2.67 and 2.10
-// ms; 5 blocks per SM: 2.42.  Nodes of 8 entries and fewer keep the warp too
-// little to do per round (313k windows on 740k boxes, F = 8: 409 us against
+// Bound by instruction issue (0.77 per cycle and scheduler): some 110 instructions a
+// step and 60 a query.  From kCountsBatched queries on a warp therefore takes several
+// and tests them against the root a lane each: 1M windows of 1e-4..1e-2 on 10M boxes
+// 2.17 -> 2.06 ms at F = 16 (breadth first 3.55), on 10k and 100k boxes 0.62 -> 0.52 and
+// 0.83 -> 0.73 ms (breadth first 0.50 and 0.74; 100k windows are the same either
+// way).  Without batches, 10M boxes: 1 and 3 rounds at F = 16 2.67 and 2.10 ms, 5
+// blocks per SM 2.42; two walks per warp 2.71.  Nodes of 8 entries and fewer keep the
+// warp too little to do per round (313k windows on 740k boxes, F = 8: 409 us against
 // 325): they go breadth first (kCountsWideFanout).
 constexpr int kCountsBlock = 256;
 constexpr int kCountsSteps = 256;
 constexpr int kCountsWideFanout = 9;  // fanouts from here on go depth first
+// Calls of so many queries batch them, so that a warp gets kCountsBatches batches or
+// more of 8 to 32 queries.
+constexpr int64_t kCountsBatched = 1 << 17;
+constexpr int kCountsBatches = 3;
+constexpr int kCountsChain = 1;  // launches until the host looks at what is left
 
 template <int G>
 constexpr int counts_rounds() { return G == 32 ? 4 : G == 16 ? 2 : 1; }
@@ -742,120 +750,184 @@ constexpr int counts_pop() { return counts_rounds<G>() * (32 / G); }
 // walk that takes one at a time (fanout - 1 more per level).
 inline int counts_stack(int levels, int fanout, int pop) { return (2 * levels + pop) * (fanout - 1) + 1; }
 
-template <typename T, int G>
+// Shared memory of a block's warps with kBatch: a batch's queries, the root's
+// entries that each hits and contains, and the root's entries.
+template <typename T>
+struct CountsBatch {
+  Box<T> query[kCountsBlock / 32][32];
+  uint2 hits[kCountsBlock / 32][32];
+  Box<T> root[32];
+};
+
+// kBatch: a warp takes `batch` queries at a time, a lane of it testing each against
+// the root, and then walks for those that hit something there (trees of two
+// levels and more, not for left-over work).
+template <typename T, int G, bool kBatch>
 __global__ void __launch_bounds__(kCountsBlock, sizeof(T) == 4 ? 4 : 3)
-    counts_kernel(CountsTree t, const Box<T> *__restrict__ queries, int64_t nq, int fanout, int td_slots,
-                  int stack_cap, const unsigned *__restrict__ flags, long long *__restrict__ counts, CountsQueue Q) {
-  extern __shared__ __align__(16) unsigned char s_raw[];
+    counts_kernel(CountsTree t, const Box<T> *__restrict__ queries, int64_t nq, int batch, int max_steps, int fanout,
+                  int td_slots, int stack_cap, const unsigned *__restrict__ flags, long long *__restrict__ counts, CountsQueue Q) {
+  extern __shared__ __align__(32) unsigned char s_raw[];
   constexpr int kNodes = 32 / G, kRounds = counts_rounds<G>(), kPop = counts_pop<G>();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane / G, e = lane % G;
   const uint32_t gmask = (G == 32 ? 0xffffffffu : (1u << G) - 1u) << (lane - e);
   const uint32_t lt = lanemask_lt();
   const bool on = e < fanout;
-  CountsLevel *s_lv = reinterpret_cast<CountsLevel *>(s_raw);
+  cudaGridDependencySynchronize();
+  const int64_t work = !kBatch && Q.in ? (int64_t)min(*Q.n_in, (unsigned long long)Q.out_cap) : nq;
+  if (work == 0) return;
+  CountsBatch<T> &B = *reinterpret_cast<CountsBatch<T> *>(s_raw);
+  CountsLevel *s_lv = reinterpret_cast<CountsLevel *>(s_raw + (kBatch ? sizeof(CountsBatch<T>) : 0));
   uint2 *stack = reinterpret_cast<uint2 *>(s_lv + t.levels) + warp * stack_cap;  // (node, level)
-  for (int l = threadIdx.x; l < t.levels; l += kCountsBlock) s_lv[l] = t.lv[l];
-  __syncthreads();
   const Box<T> *mbr = reinterpret_cast<const Box<T> *>(t.mbr) + e;
+  for (int l = threadIdx.x; l < t.levels; l += kCountsBlock) s_lv[l] = t.lv[l];
+  if (kBatch && threadIdx.x < fanout)
+    B.root[threadIdx.x] = load_box(reinterpret_cast<const Box<T> *>(t.mbr), (int64_t)t.lv[t.levels - 1].first + threadIdx.x);
+  __syncthreads();
   const bool prune = all_proper(flags);
   const int room = stack_cap - (t.levels + kPop) * (fanout - 1);  // most entries a kPop step may start from
   const uint32_t leaf_last = s_lv[0].last, leaf_lack = fanout - s_lv[0].fill;
-  const int64_t work = Q.in ? Q.n_in : nq;
-  const int64_t stride = (int64_t)gridDim.x * (kCountsBlock / 32);
-  for (int64_t w = blockIdx.x * (int64_t)(kCountsBlock / 32) + warp; w < work; w += stride) {
+  const int64_t step = kBatch ? batch : 1, stride = (int64_t)gridDim.x * (kCountsBlock / 32) * step;
+  for (int64_t w = (blockIdx.x * (int64_t)(kCountsBlock / 32) + warp) * step; w < work; w += stride) {
+    uint32_t todo = 1u;  // queries of the batch to walk for
     CountsItem it{(uint32_t)w, s_lv[t.levels - 1].first, t.levels - 1};
-    if (Q.in) it = Q.in[w];
-    const Box<T> qb = load_box(queries, it.q);
-    __syncwarp();
-    if (lane == 0) stack[0] = make_uint2(it.node, (uint32_t)it.level);
-    __syncwarp();
-    int sp = 1, steps = 0;
-    // the group's nodes, the same on its lanes: visited, entries that levels'
-    // last nodes lack, sum of max(hits, 1), leaf hits
-    uint32_t visits = 0, lack = 0, c1 = 0, c2 = 0;
-    // this lane's contained subtrees: nodes, entries, leaf entries (a tree has
-    // fewer than 2^32 entries)
-    uint32_t d_nodes = 0, d_entries = 0, d_leaf = 0;
-    while (sp > 0) {
-      const int pop = sp <= room ? min(sp, kPop) : 1;
-      uint2 nd[kRounds];
-      Box<T> b[kRounds];
-#pragma unroll
-      for (int r = 0; r < kRounds; r++) {
-        nd[r] = make_uint2(0u, 0xffffffffu);
-        if (r * kNodes + g < pop) {
-          nd[r] = stack[sp - 1 - r * kNodes - g];
-          if (on) b[r] = load_box(mbr, nd[r].x);
+    if constexpr (kBatch) {
+      const uint32_t fill = s_lv[t.levels - 1].fill;
+      uint32_t hits = 0, conts = 0;
+      __syncwarp();
+      if (lane < batch && w + lane < nq) {
+        const Box<T> q = load_box(queries, w + lane);
+        for (uint32_t j = 0; j < fill; j++) {
+          const Box<T> r = B.root[j];
+          hits |= (overlaps(r, q) ? 1u : 0u) << j;
+          conts |= (prune && contains(q, r) ? 1u : 0u) << j;
+        }
+        B.query[warp][lane] = q;
+        B.hits[warp][lane] = make_uint2(hits, conts & hits);
+        if (hits == 0) {
+          long long *out = &counts[3 * (w + lane)];
+          out[0] = td_slots ? fanout : fill;
+          out[1] = out[2] = 0;
         }
       }
-      sp -= pop;
+      todo = __ballot_sync(0xffffffffu, hits != 0);
       __syncwarp();
+    } else if (Q.in) {
+      it = Q.in[w];
+    }
+    for (; todo; todo &= todo - 1) {
+      Box<T> qb;
+      int sp, steps = 0;
+      // the group's nodes, the same on its lanes: visited, entries that levels'
+      // last nodes lack, sum of max(hits, 1), leaf hits
+      uint32_t visits = 0, lack = 0, c1 = 0, c2 = 0;
+      // this lane's contained subtrees: nodes, entries, leaf entries (a tree has
+      // fewer than 2^32 entries)
+      uint32_t d_nodes = 0, d_entries = 0, d_leaf = 0;
+      // adds the subtree below an entry whose child starts at x, of level m
+      auto add_subtree = [&](uint32_t x, uint32_t m) {
+        uint32_t n = 1;  // its nodes of level m, [x, end)
+        for (;; m--) {
+          const CountsLevel M = s_lv[m];
+          const uint32_t end = min(x + n * (uint32_t)fanout, M.last + M.fill);  // all n nodes are in the tree
+          d_nodes += n;
+          n = end - x;
+          d_entries += n;
+          if (m == 0) break;
+          x = x * (uint32_t)fanout + M.child;
+        }
+        d_leaf += n;
+      };
+      if constexpr (kBatch) {
+        const int j = __ffs(todo) - 1;
+        it.q = (uint32_t)w + j;
+        qb = B.query[warp][j];
+        const uint2 h = B.hits[warp][j];
+        const CountsLevel L = s_lv[t.levels - 1];
+        if (g == 0) {
+          visits = 1;
+          c1 = __popc(h.x);
+          lack = fanout - L.fill;
+        }
+        const uint32_t x = (L.first + e) * (uint32_t)fanout + L.child;
+        const uint32_t pb = h.x & ~h.y;
+        if (g == 0 && (pb >> e & 1u)) stack[__popc(pb & lt)] = make_uint2(x, t.levels - 2);
+        if (g == 0 && (h.y >> e & 1u)) add_subtree(x, t.levels - 2);
+        sp = __popc(pb);
+      } else {
+        qb = load_box(queries, it.q);
+        __syncwarp();
+        if (lane == 0) stack[0] = make_uint2(it.node, (uint32_t)it.level);
+        sp = 1;
+      }
+      __syncwarp();
+      while (sp > 0) {
+        const int pop = sp <= room ? min(sp, kPop) : 1;
+        uint2 nd[kRounds];
+        Box<T> b[kRounds];
 #pragma unroll
-      for (int r = 0; r < kRounds; r++) {
-        if (r * kNodes >= pop) break;
-        const bool live = nd[r].y != 0xffffffffu;
-        const bool hit = live && on && overlaps(b[r], qb);
-        const int k = __popc(__ballot_sync(0xffffffffu, hit) & gmask);
-        const bool inner = live && nd[r].y != 0;
-        if (live) {
-          visits++;
-          c1 += max(k, 1);
-          if (!inner) {
-            c2 += k;
-            if (nd[r].x == leaf_last) lack += leaf_lack;
+        for (int r = 0; r < kRounds; r++) {
+          nd[r] = make_uint2(0u, 0xffffffffu);
+          if (r * kNodes + g < pop) {
+            nd[r] = stack[sp - 1 - r * kNodes - g];
+            if (on) b[r] = load_box(mbr, nd[r].x);
           }
         }
-        if (__any_sync(0xffffffffu, inner)) {
-          const bool in = hit && inner && prune && contains(qb, b[r]);
-          const bool push = hit && inner && !in;
-          const uint32_t pb = __ballot_sync(0xffffffffu, push);
-          if (inner) {
-            const CountsLevel L = s_lv[nd[r].y];
-            if (nd[r].x == L.last) lack += fanout - L.fill;
-            uint32_t x = (nd[r].x + e) * (uint32_t)fanout + L.child;  // the entry's child
-            if (push) stack[sp + __popc(pb & lt)] = make_uint2(x, nd[r].y - 1u);
-            if (in) {
-              // the subtree below: [x, end) of every level
-              uint32_t n = 1;  // its nodes of level m
-              for (uint32_t m = nd[r].y - 1u;; m--) {
-                const CountsLevel M = s_lv[m];
-                const uint64_t end = min((uint64_t)x + (uint64_t)n * fanout, (uint64_t)M.last + M.fill);
-                d_nodes += n;
-                n = (uint32_t)(end - x);
-                d_entries += n;
-                if (m == 0) break;
-                x = x * (uint32_t)fanout + M.child;
-              }
-              d_leaf += n;
+        sp -= pop;
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < kRounds; r++) {
+          if (r * kNodes >= pop) break;
+          const bool live = nd[r].y != 0xffffffffu;
+          const bool hit = live && on && overlaps(b[r], qb);
+          const int k = __popc(__ballot_sync(0xffffffffu, hit) & gmask);
+          const bool inner = live && nd[r].y != 0;
+          if (live) {
+            visits++;
+            c1 += max(k, 1);
+            if (!inner) {
+              c2 += k;
+              if (nd[r].x == leaf_last) lack += leaf_lack;
             }
           }
-          sp += __popc(pb);
+          if (__any_sync(0xffffffffu, inner)) {
+            const bool in = hit && inner && prune && contains(qb, b[r]);
+            const bool push = hit && inner && !in;
+            const uint32_t pb = __ballot_sync(0xffffffffu, push);
+            if (inner) {
+              const CountsLevel L = s_lv[nd[r].y];
+              if (nd[r].x == L.last) lack += fanout - L.fill;
+              const uint32_t x = (nd[r].x + e) * (uint32_t)fanout + L.child;  // the entry's child
+              if (push) stack[sp + __popc(pb & lt)] = make_uint2(x, nd[r].y - 1u);
+              if (in) add_subtree(x, nd[r].y - 1u);
+            }
+            sp += __popc(pb);
+          }
+        }
+        __syncwarp();
+        if (++steps >= (kBatch ? kCountsSteps : max_steps) && sp > 0) {
+          // too long a walk: the rest of it to the next launch, if that has room
+          unsigned long long at = 0;
+          if (lane == 0) at = atomicAdd(Q.out_count, (unsigned long long)sp);
+          at = __shfl_sync(0xffffffffu, at, 0);
+          const int fits = (int)min((long long)sp, max(0ll, (long long)Q.out_cap - (long long)at));
+          for (int k = lane; k < fits; k += 32) Q.out[at + k] = CountsItem{it.q, stack[sp - 1 - k].x, (int32_t)stack[sp - 1 - k].y};
+          sp -= fits;
+          steps = 0;
+          __syncwarp();
         }
       }
-      __syncwarp();
-      if (++steps >= kCountsSteps && sp > 0) {
-        // too long a walk: the rest of it to the next launch, if that has room
-        unsigned long long at = 0;
-        if (lane == 0) at = atomicAdd(Q.out_count, (unsigned long long)sp);
-        at = __shfl_sync(0xffffffffu, at, 0);
-        const int fits = (int)min((long long)sp, max(0ll, (long long)Q.out_cap - (long long)at));
-        for (int k = lane; k < fits; k += 32) Q.out[at + k] = CountsItem{it.q, stack[sp - 1 - k].x, (int32_t)stack[sp - 1 - k].y};
-        sp -= fits;
-        steps = 0;
-        __syncwarp();
+      if (e != 0) visits = lack = c1 = c2 = 0;
+      const uint32_t r0 = __reduce_add_sync(
+          0xffffffffu, td_slots ? (visits + d_nodes) * (uint32_t)fanout : visits * (uint32_t)fanout - lack + d_entries);
+      const uint32_t r1 = __reduce_add_sync(0xffffffffu, c1 - visits + (d_entries - d_nodes));
+      const uint32_t r2 = __reduce_add_sync(0xffffffffu, c2 + d_leaf);
+      if (lane < 3) {
+        unsigned long long *out = reinterpret_cast<unsigned long long *>(&counts[3 * (int64_t)it.q + lane]);
+        const unsigned long long v = lane == 0 ? r0 : lane == 1 ? r1 : r2;
+        if (!kBatch && Q.in) atomicAdd(out, v);
+        else *out = v;
       }
-    }
-    if (e != 0) visits = lack = c1 = c2 = 0;
-    const uint32_t r0 = __reduce_add_sync(
-        0xffffffffu, td_slots ? (visits + d_nodes) * (uint32_t)fanout : visits * (uint32_t)fanout - lack + d_entries);
-    const uint32_t r1 = __reduce_add_sync(0xffffffffu, c1 - visits + (d_entries - d_nodes));
-    const uint32_t r2 = __reduce_add_sync(0xffffffffu, c2 + d_leaf);
-    if (lane < 3) {
-      unsigned long long *out = reinterpret_cast<unsigned long long *>(&counts[3 * (int64_t)it.q + lane]);
-      const unsigned long long v = lane == 0 ? r0 : lane == 1 ? r1 : r2;
-      if (Q.in) atomicAdd(out, v);
-      else *out = v;
     }
   }
 }
@@ -980,43 +1052,56 @@ int prt_query_counts(const prt_tree *t, const void *d_queries, int coord_type, i
     c.lv[l].fill = (uint32_t)(t->lv.count[l] - (nodes - 1) * t->fanout);
     c.lv[l].child = l > 0 ? (uint32_t)(t->lv.offset[l - 1] - first * t->fanout) : 0u;
   }
-  // two work queues for the walks that are left over, and their counts
+  // two work queues for the walks that are left over, and the counts of what the
+  // launches leave
   constexpr int64_t kQueue = 1 << 20;
   CountsItem *queue = nullptr;
   unsigned long long *left = nullptr;
   rc = dalloc(&queue, 2 * kQueue, s);
-  if (!rc) rc = dalloc(&left, 1, s);
-  CountsQueue Q;
-  memset(&Q, 0, sizeof Q);
-  Q.out_count = left;
-  Q.out_cap = kQueue;
-  for (int round = 0; !rc; round++) {
-    Q.out = queue + (round & 1) * kQueue;
-    cudaError_t e = cudaMemsetAsync(left, 0, 8, s);
-    if (e == cudaSuccess)
+  if (!rc) rc = dalloc(&left, kCountsChain + 1, s);
+  int chain = kCountsChain, round = 0;
+  unsigned long long n_left = 1;
+  while (!rc && n_left > 0) {
+    cudaError_t e = cudaMemsetAsync(left, 0, 8 * kCountsChain, s);
+    int last = 0;
+    for (int i = 0; i < chain && e == cudaSuccess && !rc; i++, round++) {
+      CountsQueue Q;
+      Q.in = round ? queue + ((round - 1) & 1) * kQueue : nullptr;
+      Q.n_in = i ? &left[i - 1] : left + kCountsChain;
+      Q.out = queue + (round & 1) * kQueue;
+      Q.out_count = &left[last = i];
+      Q.out_cap = kQueue;
       rc = dispatch_group(t->coord, t->fanout, [&](auto tag, auto g) {
         using T = decltype(tag);
-        constexpr int G = decltype(g)::value, kWarps = kCountsBlock / 32;
+        constexpr int G = std::max(decltype(g)::value, 16), kWarps = kCountsBlock / 32;  // smaller ones went above
         const int cap = counts_stack(c.levels, t->fanout, counts_pop<G>());
-        const size_t smem = sizeof(CountsLevel) * c.levels + sizeof(uint2) * (size_t)kWarps * cap;
-        int b = 0;
-        PRT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, counts_kernel<T, G>, kCountsBlock, smem));
-        const int64_t work = Q.in ? Q.n_in : nq;
-        const int64_t blocks = std::min<int64_t>((work + kWarps - 1) / kWarps, (int64_t)kSMs * std::max(b, 1));
-        PRT_PROF("counts", s);
-        counts_kernel<T, G><<<(unsigned)blocks, kCountsBlock, smem, s>>>(
-            c, reinterpret_cast<const Box<T> *>(d_queries), nq, t->fanout, td_slots, cap, t->d_flags,
-            reinterpret_cast<long long *>(d_counts), Q);
-        return PRT_OK;
+        auto launch = [&](auto kernel, size_t smem, int batch) {
+          smem += sizeof(CountsLevel) * c.levels + sizeof(uint2) * (size_t)kWarps * cap;
+          int b = 0;
+          PRT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, kCountsBlock, smem));
+          const int64_t resident = (int64_t)kSMs * std::max(b, 1);
+          if (batch) batch = (int)std::min<int64_t>(32, nq / (resident * kWarps * kCountsBatches));
+          const int64_t per = (int64_t)kWarps * std::max(batch, 1);
+          const int64_t blocks = Q.in ? resident : std::min<int64_t>((nq + per - 1) / per, resident);
+          const int steps = kCountsSteps;
+          PRT_PROF("counts", s);
+          PRT_CUDA(launch_dependent(kernel, (int)blocks, kCountsBlock, smem, s, c,
+                                    reinterpret_cast<const Box<T> *>(d_queries), nq, batch, steps, t->fanout, td_slots,
+                                    cap, t->d_flags, reinterpret_cast<long long *>(d_counts), Q));
+          return PRT_OK;
+        };
+        if (!Q.in && c.levels > 1 && nq >= kCountsBatched) return launch(counts_kernel<T, G, true>, sizeof(CountsBatch<T>), 1);
+        return launch(counts_kernel<T, G, false>, 0, 0);
       });
-    unsigned long long n_left = 0;
-    if (!rc && e == cudaSuccess) e = cudaGetLastError();
-    if (!rc && e == cudaSuccess) e = cudaMemcpyAsync(&n_left, left, 8, cudaMemcpyDeviceToHost, s);
+    }
+    if (!rc && e == cudaSuccess) e = cudaMemcpyAsync(&n_left, &left[last], 8, cudaMemcpyDeviceToHost, s);
     if (!rc && e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (!rc && e != cudaSuccess) rc = cuda_status(e, "query counts");
     if (rc || n_left == 0) break;
-    Q.in = Q.out;
-    Q.n_in = std::min<int64_t>((int64_t)n_left, kQueue);
+    chain = 1;
+    // the count of what this round left, where the next one's first launch reads it
+    e = cudaMemcpyAsync(left + kCountsChain, &left[last], 8, cudaMemcpyDeviceToDevice, s);
+    if (e != cudaSuccess) rc = cuda_status(e, "query counts");
   }
   dfree(queue, s);
   dfree(left, s);

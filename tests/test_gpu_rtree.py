@@ -316,3 +316,38 @@ def test_one_block_buckets(cuda, kind, equal, n):
     perm = oracle.stable_argsort(oracle.keys_morton32(b)[0])
     assert np.array_equal(t.leaf_order().cpu().numpy(), perm)
     check_levels(t, oracle.pack(b, 16, perm))
+
+
+def windows(kind, n, seed):
+    """Small windows, some points, a hundred large ones and one around everything."""
+    rng = np.random.default_rng(seed)
+    c, half = rng.random((n, 2)), 10.0 ** rng.uniform(-5, -2, (n, 1))
+    half[: n // 100] = 0.0
+    half[n // 100: n // 100 + 100] = 0.2
+    half[n // 2] = 2.0
+    q = np.concatenate([c - half, c + half], 1)
+    return q.astype(np.float32) if kind == "f32" else q if kind == "f64" else np.rint(q * 1e6).astype(
+        np.int64 if kind == "i64" else np.int32)
+
+
+@pytest.mark.parametrize("kind", ["f32", "f64", "i64", "i32"])
+@pytest.mark.parametrize("F,n", [(9, 9), (9, 10), (10, 5000), (16, 16), (16, 17), (16, 4097), (17, 3000), (32, 33),
+                                 (32, 20000)])
+def test_counts_of_many_windows(cuda, kind, F, n):
+    """Just under and just over the number of windows from which warps take batches of
+    them, trees of one level and more, with and without a record that intersects
+    nothing, against the oracle."""
+    import parlllelrtree_b200 as prt
+
+    q = windows(kind, 131_072 + 77, F)
+    b = boxes_of(kind, n, seed=F + n, side=3e-3)
+    for improper in (False, True):
+        if improper:
+            b[n // 2, 0], b[n // 2, 2] = b[n // 2, 2] + 1, b[n // 2, 0] - 1
+        t = prt.build_bottomup(torch.from_numpy(b).cuda(), fanout=F)
+        lv = t.levels_mbr()
+        for td in (False, True):
+            ref = oracle.query_counts(lv, F, q, td_slots=td)
+            for m in (131_071, 131_072, len(q)):
+                got = t.query_counts(torch.from_numpy(q[:m]).cuda(), td_slots=td).cpu().numpy()
+                assert np.array_equal(got, ref[:m]), (improper, td, m)
