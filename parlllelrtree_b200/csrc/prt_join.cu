@@ -739,7 +739,13 @@ constexpr int kCountsWideFanout = 9;  // fanouts from here on go depth first
 // more of 8 to 32 queries.
 constexpr int64_t kCountsBatched = 1 << 17;
 constexpr int kCountsBatches = 3;
-constexpr int kCountsChain = 1;  // launches until the host looks at what is left
+// Queries that leave most warps idle (kCountsFew times as many could be resident)
+// hand what is left of a walk on after kCountsFewSteps, to launches that are made at
+// once, kCountsChain in all, as a wait for each would cost more than they do.  2M
+// boxes, F = 16: 100 windows across the whole extent 139 -> 83 us (breadth first 80), 100
+// of 0.1 by 0.1 where nothing can be pruned 359 -> 112 (128); 100 small windows, for
+// which there is nothing left, 53 -> 58 (66).
+constexpr int kCountsFew = 8, kCountsFewSteps = 24, kCountsChain = 3;
 
 template <int G>
 constexpr int counts_rounds() { return G == 32 ? 4 : G == 16 ? 2 : 1; }
@@ -1059,7 +1065,7 @@ int prt_query_counts(const prt_tree *t, const void *d_queries, int coord_type, i
   unsigned long long *left = nullptr;
   rc = dalloc(&queue, 2 * kQueue, s);
   if (!rc) rc = dalloc(&left, kCountsChain + 1, s);
-  int chain = kCountsChain, round = 0;
+  int chain = 1, round = 0;  // launches until the host looks
   unsigned long long n_left = 1;
   while (!rc && n_left > 0) {
     cudaError_t e = cudaMemsetAsync(left, 0, 8 * kCountsChain, s);
@@ -1080,10 +1086,11 @@ int prt_query_counts(const prt_tree *t, const void *d_queries, int coord_type, i
           int b = 0;
           PRT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, kCountsBlock, smem));
           const int64_t resident = (int64_t)kSMs * std::max(b, 1);
+          if (!Q.in && nq * kCountsFew < resident * kWarps) chain = kCountsChain;
           if (batch) batch = (int)std::min<int64_t>(32, nq / (resident * kWarps * kCountsBatches));
           const int64_t per = (int64_t)kWarps * std::max(batch, 1);
           const int64_t blocks = Q.in ? resident : std::min<int64_t>((nq + per - 1) / per, resident);
-          const int steps = kCountsSteps;
+          const int steps = i + 1 < chain ? kCountsFewSteps : kCountsSteps;
           PRT_PROF("counts", s);
           PRT_CUDA(launch_dependent(kernel, (int)blocks, kCountsBlock, smem, s, c,
                                     reinterpret_cast<const Box<T> *>(d_queries), nq, batch, steps, t->fanout, td_slots,

@@ -351,3 +351,30 @@ def test_counts_of_many_windows(cuda, kind, F, n):
             for m in (131_071, 131_072, len(q)):
                 got = t.query_counts(torch.from_numpy(q[:m]).cuda(), td_slots=td).cpu().numpy()
                 assert np.array_equal(got, ref[:m]), (improper, td, m)
+
+
+@pytest.mark.parametrize("kind", ["f32", "i64"])
+@pytest.mark.parametrize("F", [10, 16, 32])
+@pytest.mark.parametrize("nq", [1, 300, 443, 444, 591, 592, 700])
+def test_counts_of_few_long_windows(cuda, kind, F, nq):
+    """Windows across the whole extent and around everything, on a tree that cannot be
+    pruned and on one that can, around the numbers of windows up to which long walks
+    are handed on early: what a launch leaves, once and again."""
+    import parlllelrtree_b200 as prt
+
+    n = 60_000
+    rng = np.random.default_rng(nq)
+    y = rng.random(nq)
+    q = np.stack([np.full(nq, -1.0), y, np.full(nq, 2.0), y + 1e-3], 1)
+    q[nq // 2] = [-1, -1, 2, 2]
+    q[:: 7, 3] += 0.05
+    q = q.astype(np.float32) if kind == "f32" else np.rint(q * 1e6).astype(np.int64)
+    b = boxes_of(kind, n, seed=F, side=1e-3)
+    for improper in (True, False):
+        if not improper:
+            b[n // 2] = b[0]
+        else:
+            b[n // 2, 0], b[n // 2, 2] = b[n // 2, 2] + 1, b[n // 2, 0] - 1
+        t = prt.build_bottomup(torch.from_numpy(b).cuda(), fanout=F)
+        got = t.query_counts(torch.from_numpy(q).cuda()).cpu().numpy()
+        assert np.array_equal(got, oracle.query_counts(t.levels_mbr(), F, q)), improper
