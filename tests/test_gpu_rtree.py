@@ -378,3 +378,23 @@ def test_counts_of_few_long_windows(cuda, kind, F, nq):
         t = prt.build_bottomup(torch.from_numpy(b).cuda(), fanout=F)
         got = t.query_counts(torch.from_numpy(q).cuda()).cpu().numpy()
         assert np.array_equal(got, oracle.query_counts(t.levels_mbr(), F, q)), improper
+
+
+@pytest.mark.parametrize("F", [2, 4, 5])
+@pytest.mark.parametrize("nq", [65_535, 65_536])
+def test_unsorted_joins_of_small_nodes(cuda, F, nq):
+    """The line between one traversal in order and two in none, with and without
+    pairs, against the oracle."""
+    import parlllelrtree_b200 as prt
+
+    b = boxes_of("f32", 3000, seed=F, side=3e-3)
+    q = windows("f32", nq, 3)
+    t = prt.build_bottomup(torch.from_numpy(b).cuda(), fanout=F)
+    ref = oracle.join_pairs(t.levels_mbr(), F, q)
+    ref = ref[np.lexsort((ref[:, 0], ref[:, 1]))]
+    for srt in (False, True):
+        got = t.join(torch.from_numpy(q).cuda(), sorted=srt).cpu().numpy().astype(np.int64)
+        if not srt:
+            got = got[np.lexsort((got[:, 0], got[:, 1]))]
+        assert np.array_equal(got, ref), srt
+    assert len(t.join(torch.from_numpy(q + np.float32(9)).cuda())) == 0
