@@ -25,11 +25,11 @@
 // further apart at both ends of it than rounding can move them (or cross properly,
 // with the same distance at the crossing's beam), edges that meet in a local
 // extremum included, at the vertex y next to it.  The distance between two edges is
-// linear in y, so that covers every beam.  No vertex lies on a horizontal edge, and
-// no two horizontal edges follow each other (GPC drops the vertex between them).  No
-// scanline holds both +0 and -0.  A polygon that crosses or touches itself fails the
-// check too.  A pair that fails it, or that has more vertices, rings or crossings than
-// there is room for, is left to the scanbeam clippers.
+// linear in y, so that covers every beam.  No vertex lies on a horizontal edge, no
+// two horizontal edges follow each other (GPC drops the vertex between them), and no y
+// is -0.  A polygon that crosses or touches itself fails the check too.  A pair that
+// fails it, or that has more vertices, rings or crossings than there is room for, is
+// left to the scanbeam clippers.
 //
 // A block per pair, everything between the input and the result in shared memory,
 // vertices in 16-bit indices so that two pairs of 4,160 vertices share an SM.  What
@@ -46,10 +46,18 @@ namespace trace {
 
 constexpr int kMaxRings = 32;
 constexpr int kLast = 0x8000;
-// Smallest |y| of a vertex that is not 0: two ys are then 1e-146 apart or equal, so
-// that neither the slopes nor the buckets per unit of y below overflow, and what a
-// product of an x and a y difference loses to underflow is far below the margin.
-constexpr double kLeastY = 1e-130;
+// Smallest |y| of a vertex that is not 0, 2^-432 or 1e-130: two ys are then 1e-146
+// apart or equal, so that neither the slopes nor the buckets per unit of y below
+// overflow, and what a product of an x and a y difference loses to underflow is far
+// below the margin.  -0 is no y either: of two zeros on a scanline the clipper writes
+// one for all, and the y difference of a horizontal edge between them may be -0, its
+// slope then -inf.  (In integers: two comparisons of doubles per vertex, and one of
+// signs per tie, cost the 60,000 stars' 2.19 ms 4%.)
+constexpr int kLeastY = (1023 - 432) << 20;  // a double's high word
+__device__ __forceinline__ bool y_allowed(double y) {
+  const int hi = __double2hiint(y);
+  return (hi & 0x7fffffff) >= kLeastY || (hi | __double2loint(y)) == 0;
+}
 // Coordinates stay below this: products of two differences do not overflow.
 constexpr double kMostXY = 1e150;
 
@@ -160,7 +168,7 @@ __device__ __forceinline__ TEdge edge_of(const Pair<C> &P, int v) {
   e.tx = e.up ? x2 : x1;
   e.by = P.S.sy[e.rb];
   e.ty = P.S.sy[e.rt];
-  e.dx = (e.tx - e.bx) / (e.ty - e.by);  // horizontal: +inf, its left end is the lower one and both ys the same zero
+  e.dx = (e.tx - e.bx) / (e.ty - e.by);  // horizontal: +inf, its left end is the lower one
   return e;
 }
 
@@ -460,7 +468,7 @@ __device__ int trace_pair(Smem<C> &S, int op, const gpc::PolyView &A, const gpc:
       for (int v = v0 + tid; v < v1; v += NT) {
         const double x = S.rxy[r][2 * (v - v0)], y = S.rxy[r][2 * (v - v0) + 1];
         S.vx[v] = x;
-        bad |= !(fabs(x) <= most && fabs(y) <= most) || (y != 0.0 && fabs(y) < kLeastY);  // NaN; ys next to 0
+        bad |= !(fabs(x) <= most && fabs(y) <= most) || !y_allowed(y);  // NaN; ys next to 0
         S.sy[v] = y;
         S.ring[v] = (uint8_t)r;
       }
@@ -488,11 +496,9 @@ __device__ int trace_pair(Smem<C> &S, int op, const gpc::PolyView &A, const gpc:
           if (yw < y) {
             before++;
           } else if (yw == y && w != v) {
-            // +0 and -0 on one scanline: the clipper writes one of them for all, and
-            // the y difference of a horizontal edge between them is -0
             const double d = x - S.vx[w];
             before += d > 0.0;
-            bad |= !(fabs(d) > P.margin) || signbit(y) != signbit(yw);
+            bad |= !(fabs(d) > P.margin);
           }
         }
         S.rank[v] = (uint16_t)(start + before);
