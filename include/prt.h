@@ -474,6 +474,11 @@ int prt_write_polygon_file(const char *path, const int32_t *h_num, const int32_t
  * the default. */
 int prt_debug_wait_limit(int polls, int never_published);
 
+/* Test hook for the paths without device memory (no reference counterpart): single
+ * allocations of the library above `bytes` fail (PRT_ERR_NOMEM) in the calls that
+ * follow, process-wide; <= 0: none do. */
+int prt_debug_alloc_limit(int64_t bytes);
+
 #ifdef __cplusplus
 }
 #endif

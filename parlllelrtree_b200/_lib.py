@@ -72,6 +72,7 @@ _SIGS = {
     "prt_area_fwd": (_I, [_P, _P, _I64, _P, _P, _P, _P]),
     "prt_area_bwd": (_I, [_P, _P, _I64, _P, _P, _P, _P, _P, _P]),
     "prt_area_fwd_fallbacks": (_I, [_P]),
+    "prt_debug_alloc_limit": (_I, [_I64]),
     "prt_debug_wait_limit": (_I, [_I, _I]),
     "prt_overlay_stream": (_I, [_P, _I64, C.c_int32, _P, _P, _P, _I, _I, _I64, _P, _P, _P]),
     "prt_rect_file_count": (_I, [C.c_char_p, _P]),

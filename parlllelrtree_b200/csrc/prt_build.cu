@@ -11,6 +11,7 @@
 #include <type_traits>
 
 #include <algorithm>
+#include <atomic>
 #include <vector>
 #include <cstdarg>
 #include <cstring>
@@ -62,8 +63,16 @@ static void keep_pool_memory() {
   cudaGetLastError();
 }
 
+static std::atomic<int64_t> g_alloc_limit{0};  // test hook: 0 none
+
 int dmalloc(void **p, size_t bytes, cudaStream_t s) {
   if (bytes == 0) bytes = 16;
+  const int64_t limit = g_alloc_limit.load(std::memory_order_relaxed);
+  if (limit > 0 && bytes > (size_t)limit) {
+    *p = nullptr;
+    set_error("%zu bytes asked for, limited to %lld", bytes, (long long)limit);
+    return PRT_ERR_NOMEM;
+  }
   keep_pool_memory();
   cudaError_t e = cudaMallocAsync(p, bytes, s);
   if (e != cudaSuccess) {
@@ -1391,6 +1400,11 @@ int tree_alloc(const void *d_boxes, int coord, int64_t n, int fanout, int kind, 
 }  // namespace prt
 
 using namespace prt;
+
+extern "C" int prt_debug_alloc_limit(int64_t bytes) {
+  g_alloc_limit.store(bytes > 0 ? bytes : 0);
+  return PRT_OK;
+}
 
 extern "C" {
 

@@ -1125,6 +1125,12 @@ __global__ void ring_vert_from_ref_kernel(const int32_t *num, const int64_t *pre
 
 using namespace prt;
 
+namespace {
+// 64 MiB of vertices: device memory that a copy-out takes stays with the process, and
+// a copy of this size takes 8 ms (250 MB in one piece and in four: the same time).
+constexpr int64_t kCopyPiece = 1 << 22;
+}  // namespace
+
 extern "C" {
 
 int prt_schedule_set(const prt_schedule *sched) {
@@ -1263,31 +1269,46 @@ int prt_results_copy(const prt_results *r, int64_t *h_pair_cont_off, int32_t *h_
   PRT_CHECK(r && h_pair_cont_off && h_cont_nverts && h_cont_hole && h_xy, PRT_ERR_INVALID, "NULL argument");
   const int64_t n = r->n_pairs;
   PRT_CUDA(cudaDeviceSynchronize());
-  // put into pair order on the device, so that each array leaves it in one
-  // copy straight into the caller's memory
+  // put into pair order on the device, a piece of at most kCopyPiece vertices at a
+  // time, and copied from there straight into the caller's memory
   {
-    void *block = nullptr;
-    int64_t *off = nullptr;
-    int32_t *nv = nullptr, *hole = nullptr;
-    double *xy = nullptr;
-    int rc = results_compact(r, nullptr, &block, &off, &nv, &hole, &xy);
+    CompactResults c;
+    int rc = results_compact(r, kCopyPiece, nullptr, c);
     if (!rc) {
-      cudaError_t e = cudaMemcpyAsync(h_pair_cont_off, off, 8 * (size_t)(n + 1), cudaMemcpyDeviceToHost, nullptr);
-      if (e == cudaSuccess && r->n_cont > 0) {
-        e = cudaMemcpyAsync(h_cont_nverts, nv, 4 * (size_t)r->n_cont, cudaMemcpyDeviceToHost, nullptr);
-        if (e == cudaSuccess)
-          e = cudaMemcpyAsync(h_cont_hole, hole, 4 * (size_t)r->n_cont, cudaMemcpyDeviceToHost, nullptr);
-        if (e == cudaSuccess)
-          e = cudaMemcpyAsync(h_xy, xy, 16 * (size_t)r->n_vert, cudaMemcpyDeviceToHost, nullptr);
+      const int64_t nc = r->n_cont;
+      cudaError_t e = cudaMemcpyAsync(h_pair_cont_off, c.pair_off, 8 * (size_t)(n + 1), cudaMemcpyDeviceToHost, nullptr);
+      if (e == cudaSuccess && nc > 0) {
+        e = cudaMemcpyAsync(h_cont_nverts, c.nverts, 4 * (size_t)nc, cudaMemcpyDeviceToHost, nullptr);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(h_cont_hole, c.hole, 4 * (size_t)nc, cudaMemcpyDeviceToHost, nullptr);
+        if (e == cudaSuccess && r->n_vert <= kCopyPiece)
+          e = cudaMemcpyAsync(h_xy, c.xy, 16 * (size_t)r->n_vert, cudaMemcpyDeviceToHost, nullptr);
       }
       if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
-      dfree(block, nullptr);
+      int64_t v = 0;
+      for (int64_t c0 = 0, c1; r->n_vert > kCopyPiece && c0 < nc && e == cudaSuccess && !rc; c0 = c1) {
+        int64_t m = h_cont_nverts[c0];
+        for (c1 = c0 + 1; c1 < nc && m + h_cont_nverts[c1] <= kCopyPiece; c1++) m += h_cont_nverts[c1];
+        const double *from = c.xy;
+        if (m > kCopyPiece) {  // one contour, as it lies in the pool
+          int64_t src = 0;
+          e = cudaMemcpy(&src, c.src + c0, 8, cudaMemcpyDeviceToHost);
+          from = r->xy + 2 * src;
+        } else {
+          rc = results_compact_vertices(r, c, c0, c1, nullptr);
+        }
+        if (e == cudaSuccess && !rc)
+          e = cudaMemcpyAsync(h_xy + 2 * v, from, 16 * (size_t)m, cudaMemcpyDeviceToHost, nullptr);
+        v += m;
+      }
+      if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+      dfree(c.block, nullptr);
+      if (rc) return rc;
       return e == cudaSuccess ? PRT_OK : cuda_status(e, "results copy");
     }
     if (rc != PRT_ERR_NOMEM) return rc;
   }
-  // no room on the device for a second copy of the results: the pools as
-  // they are, put into pair order on the host
+  // no room on the device for that: the pools as they are, put into pair order on
+  // the host
   unsigned long long used[2];
   PRT_CUDA(cudaMemcpy(used, r->pool, sizeof used, cudaMemcpyDeviceToHost));
   std::vector<int64_t> cs(n), cvs(used[0]);

@@ -137,10 +137,19 @@ struct prt_results {
 
 namespace prt {
 
-// Compacts a result set into pair order in device buffers allocated on s:
-// pair_off [n+1], nverts / hole [n_cont], xy [2 n_vert] (all in one block
-// returned in *block, to be released with dfree).
-int results_compact(const prt_results *r, cudaStream_t s, void **block, int64_t **pair_off, int32_t **nverts,
-                    int32_t **hole, double **xy);
+// A result set in pair order, in device buffers of one block (to be released with
+// dfree): pair_off [n+1], nverts / hole [n_cont]; per contour the first vertex in
+// the pools (src) and in pair order (vert_off [n_cont+1]); xy, `room` vertices or all.
+struct CompactResults {
+  void *block = nullptr;
+  int64_t *pair_off = nullptr, *src = nullptr, *vert_off = nullptr;
+  int32_t *nverts = nullptr, *hole = nullptr;
+  double *xy = nullptr;
+};
+
+// Fills c on s, the vertices where they fit in the room; else they are put there
+// contours [c0, c1) at a time.
+int results_compact(const prt_results *r, int64_t room, cudaStream_t s, CompactResults &c);
+int results_compact_vertices(const prt_results *r, const CompactResults &c, int64_t c0, int64_t c1, cudaStream_t s);
 
 }  // namespace prt

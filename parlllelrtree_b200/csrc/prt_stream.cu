@@ -52,14 +52,16 @@ __global__ void compact_headers_kernel(const int64_t *__restrict__ pair_cstart, 
   }
 }
 
-// Vertices in pair order: one warp per output contour, 16-byte (x, y) moves.
+// Vertices in pair order, from the first contour's on: one warp per output contour,
+// 16-byte (x, y) moves.
 __global__ void compact_vertices_kernel(const int64_t *__restrict__ src, const int32_t *__restrict__ nverts,
                                         const int64_t *__restrict__ vert_off, int64_t n_cont,
                                         const double2 *__restrict__ xy, double2 *__restrict__ out) {
   const int lane = threadIdx.x & 31;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  const int64_t first = vert_off[0];
   for (int64_t c = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; c < n_cont; c += nw) {
-    const int64_t s0 = src[c], d0 = vert_off[c];
+    const int64_t s0 = src[c], d0 = vert_off[c] - first;
     const int m = nverts[c];
     for (int j = lane; j < m; j += 32) out[d0 + j] = xy[s0 + j];
   }
@@ -67,9 +69,17 @@ __global__ void compact_vertices_kernel(const int64_t *__restrict__ src, const i
 
 }  // namespace
 
-int results_compact(const prt_results *r, cudaStream_t s, void **block, int64_t **pair_off, int32_t **nverts,
-                    int32_t **hole, double **xy) {
-  const int64_t n = r->n_pairs, nc = r->n_cont, nv = r->n_vert;
+int results_compact_vertices(const prt_results *r, const CompactResults &c, int64_t c0, int64_t c1, cudaStream_t s) {
+  PRT_PROF("compact_vertices", s);
+  compact_vertices_kernel<<<grid_for((c1 - c0) * 32, 256, 8), 256, 0, s>>>(
+      c.src + c0, c.nverts + c0, c.vert_off + c0, c1 - c0, reinterpret_cast<const double2 *>(r->xy),
+      reinterpret_cast<double2 *>(c.xy));
+  PRT_CUDA(cudaGetLastError());
+  return PRT_OK;
+}
+
+int results_compact(const prt_results *r, int64_t room, cudaStream_t s, CompactResults &c) {
+  const int64_t n = r->n_pairs, nc = r->n_cont, nv = std::min(r->n_vert, room);
   // layout: pair_off (n+1) | src (nc) | vert_off (nc+1) | xy (2 nv) | nverts (nc) | hole (nc),
   // each part starting on a 256-byte boundary (xy is moved as 16-byte pairs)
   auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
@@ -78,30 +88,28 @@ int results_compact(const prt_results *r, cudaStream_t s, void **block, int64_t 
   unsigned char *p = nullptr;
   int rc = dmalloc(reinterpret_cast<void **>(&p), b_off + b_src + b_voff + b_xy + 2 * b_nv, s);
   if (rc) return rc;
-  int64_t *off = reinterpret_cast<int64_t *>(p);
-  int64_t *src = reinterpret_cast<int64_t *>(p + b_off);
-  int64_t *voff = reinterpret_cast<int64_t *>(p + b_off + b_src);
-  double *oxy = reinterpret_cast<double *>(p + b_off + b_src + b_voff);
-  int32_t *onv = reinterpret_cast<int32_t *>(p + b_off + b_src + b_voff + b_xy);
-  int32_t *oh = reinterpret_cast<int32_t *>(p + b_off + b_src + b_voff + b_xy + b_nv);
+  c.block = p;
+  c.pair_off = reinterpret_cast<int64_t *>(p);
+  c.src = reinterpret_cast<int64_t *>(p + b_off);
+  c.vert_off = reinterpret_cast<int64_t *>(p + b_off + b_src);
+  c.xy = reinterpret_cast<double *>(p + b_off + b_src + b_voff);
+  c.nverts = reinterpret_cast<int32_t *>(p + b_off + b_src + b_voff + b_xy);
+  c.hole = reinterpret_cast<int32_t *>(p + b_off + b_src + b_voff + b_xy + b_nv);
   if (n > 0) {
-    rc = exclusive_scan<int32_t>(r->pair_ncont, n, off, off + n, s);
+    rc = exclusive_scan<int32_t>(r->pair_ncont, n, c.pair_off, c.pair_off + n, s);
   } else {
-    cudaError_t e = cudaMemsetAsync(off, 0, 8, s);
+    cudaError_t e = cudaMemsetAsync(c.pair_off, 0, 8, s);
     if (e != cudaSuccess) rc = cuda_status(e, "memset");
   }
   if (!rc && nc > 0) {
     {
       PRT_PROF("compact_headers", s);
-      compact_headers_kernel<<<grid_for(n, 256, 8), 256, 0, s>>>(r->pair_cstart, r->pair_ncont, off, n, r->cont_nverts,
-                                                                 r->cont_hole, r->cont_vstart, onv, oh, src);
+      compact_headers_kernel<<<grid_for(n, 256, 8), 256, 0, s>>>(r->pair_cstart, r->pair_ncont, c.pair_off, n,
+                                                                 r->cont_nverts, r->cont_hole, r->cont_vstart, c.nverts,
+                                                                 c.hole, c.src);
     }
-    rc = exclusive_scan<int32_t>(onv, nc, voff, voff + nc, s);
-    if (!rc) {
-      PRT_PROF("compact_vertices", s);
-      compact_vertices_kernel<<<grid_for(nc * 32, 256, 8), 256, 0, s>>>(
-        src, onv, voff, nc, reinterpret_cast<const double2 *>(r->xy), reinterpret_cast<double2 *>(oxy));
-    }
+    rc = exclusive_scan<int32_t>(c.nverts, nc, c.vert_off, c.vert_off + nc, s);
+    if (!rc && r->n_vert <= room) rc = results_compact_vertices(r, c, 0, nc, s);
   }
   if (!rc) {
     cudaError_t e = cudaGetLastError();
@@ -109,14 +117,9 @@ int results_compact(const prt_results *r, cudaStream_t s, void **block, int64_t 
   }
   if (rc) {
     dfree(p, s);
-    return rc;
+    c.block = nullptr;
   }
-  *block = p;
-  *pair_off = off;
-  *nverts = onv;
-  *hole = oh;
-  *xy = oxy;
-  return PRT_OK;
+  return rc;
 }
 
 }  // namespace prt
@@ -296,10 +299,9 @@ extern "C" int prt_overlay_stream(const prt_pair *d_pairs, int64_t n_pairs, int3
     S.over = layer_dev(overlay);
     S.op = op;
     rc = overlay_impl(S, c.n, sched, nullptr, s, &c.res);
-    int64_t *off = nullptr;
-    int32_t *nv = nullptr, *hole = nullptr;
-    double *xy = nullptr;
-    if (!rc) rc = results_compact(c.res, s, &c.block, &off, &nv, &hole, &xy);
+    CompactResults d;
+    if (!rc) rc = results_compact(c.res, c.res->n_vert, s, d);
+    c.block = d.block;
     // the previous chunk's copy overlapped this chunk's clip
     bool landed = false;
     if (pending) {
@@ -311,10 +313,10 @@ extern "C" int prt_overlay_stream(const prt_pair *d_pairs, int64_t n_pairs, int3
     if (!rc) {
       c.nc = c.res->n_cont;
       c.nv = c.res->n_vert;
-      c.d_off = off;
-      c.d_nv = nv;
-      c.d_hole = hole;
-      c.d_xy = xy;
+      c.d_off = d.pair_off;
+      c.d_nv = d.nverts;
+      c.d_hole = d.hole;
+      c.d_xy = d.xy;
       // buf[cur] held the chunk before the previous one, delivered already
       const size_t bytes = 8 * (size_t)(c.n + 1) + 8 * (size_t)c.nc + 16 * (size_t)c.nv + 64;
       rc = ensure_host(buf[cur], bytes);

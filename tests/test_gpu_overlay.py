@@ -468,3 +468,32 @@ def test_traced_bits(cuda, op):
         ref = prt.overlay(ids_of(3000), LA, LB, op=op).to_host()
     assert all(np.array_equal(g.view(np.int64) if g.dtype == np.float64 else g,
                               e.view(np.int64) if e.dtype == np.float64 else e) for g, e in zip(r.to_host(), ref))
+
+
+def test_large_results_leave_in_pieces(cuda):
+    """Results above the 64 MiB of vertices that a copy-out puts into order at a time,
+    and the same without device memory to do it in."""
+    import parlllelrtree_b200 as prt
+    from parlllelrtree_b200 import _lib
+
+    n = 12_000
+    A, B = stars_across(n, 500, 400)
+    B["xy"] = A["xy"][np.arange(n * 500).reshape(n, 500)[:, :400].reshape(-1)] + [0.0004, 0.0003]
+    r = prt.overlay(ids_of(n), prt.Layer.from_dict(A), prt.Layer.from_dict(B), op="union")
+    assert r.n_vertices * 16 > 64 << 20
+    off, nv, hole, xy = r.to_host()
+    assert off[-1] == len(nv) == r.n_contours and nv.sum() == len(xy) == r.n_vertices
+    L = _lib.lib()
+    try:
+        L.prt_debug_alloc_limit(1 << 16)
+        host = r.to_host()
+        with pytest.raises(prt.PrtError) as e:
+            prt.overlay(ids_of(n), prt.Layer.from_dict(A), prt.Layer.from_dict(B))
+        assert e.value.code == _lib.PRT_ERR_NOMEM
+    finally:
+        L.prt_debug_alloc_limit(0)
+    assert all(np.array_equal(a, b) for a, b in zip((off, nv, hole, xy), host))
+    vo = np.concatenate([[0], np.cumsum(nv)])
+    for i in range(0, n, 600):
+        got = [(int(hole[c]), xy[vo[c]:vo[c + 1]]) for c in range(off[i], off[i + 1])]
+        assert same_contours(got, oracle.gpc_clip(rings_of(A, i), rings_of(B, i), 3)), f"pair {i}"
