@@ -21,6 +21,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <new>
 #include <type_traits>
 #include <vector>
 
@@ -1005,7 +1006,8 @@ int prt_join_begin(const prt_tree *t, const void *d_queries, int coord_type, int
   int rc = check_join(t, d_queries, coord_type, nq, nullptr, 0);
   if (rc) return rc;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  prt_join_state *st = new prt_join_state();
+  prt_join_state *st = new (std::nothrow) prt_join_state();
+  PRT_CHECK(st != nullptr, PRT_ERR_NOMEM, "no host memory");
   st->stream = s;
   if (nq > 0) rc = run_ordered(t, d_queries, nq, st->o, s);
   if (rc) {
