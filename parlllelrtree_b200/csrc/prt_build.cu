@@ -625,9 +625,10 @@ __global__ void __launch_bounds__(kTdThreads, kTdThreads == 256 ? (sizeof(T) == 
     // proportion to key - lo, about as many buckets as records, and a record's
     // place in its bucket is counted like the last level's, instead of three radix
     // passes or more; with 64-bit coordinates and one block of them per SM four or
-    // more (300k 64-bit boxes on a 1e6 grid, three passes: 37 us against 39).  The counting grows with the largest bucket: with one above kTdCrowd
-    // the passes below sort the level (tiles of equal keys; without the limit 720
-    // us where it takes 444 with one of 32, 453 with 12).
+    // more (300k 64-bit boxes on a 1e6 grid, three passes: 37 us against 39).  The
+    // counting grows with the largest bucket: with one above kTdCrowd the passes below
+    // sort the level (tiles of equal keys; without the limit 720 us where it takes 444
+    // with one of 32, 453 with 12).
     if (total_bits > (sizeof(T) == 4 ? 16 : 24)) {
       constexpr int kPer = kTdWarps * 256 / kTdThreads;  // counters per thread
       uint32_t *cnt = &S.wh[0][0];
@@ -1338,51 +1339,46 @@ int bu_enqueue(prt_tree *t, const void *d_boxes, const int32_t *d_ids, unsigned 
   void *keys0 = kp, *keys1 = kp + kb * n;
   uint32_t *vals0 = reinterpret_cast<uint32_t *>(kp + 2 * kb * n);
   uint32_t *vals1 = vals0 + n;
-  cudaError_t e = cudaSuccess;
-  int g = grid_for(n, 256, 16);
-  if (e == cudaSuccess) {
-    if (t->key_mode == PRT_KEY_MORTON32) {
-      {
-        PRT_PROF("extent_init", s);
-        extent_init_kernel<<<1, 256, 0, s>>>(ext, t->d_flags, hist);
-      }
-      rc = dispatch_coord(t->coord, [&](auto tag) {
-        using T = decltype(tag);
-        const Box<T> *b = reinterpret_cast<const Box<T> *>(d_boxes);
-        {
-          PRT_PROF("extent_f64", s);
-          // 16 blocks per SM: enough loads in flight to stream the boxes
-          extent_f64_kernel<T><<<grid_for(n, 256, 16), 256, 0, s>>>(b, n, ext);
-        }
-        {
-          PRT_PROF("morton32", s);
-          morton32_kernel<T><<<g, 256, 0, s>>>(b, n, ext, reinterpret_cast<uint32_t *>(keys0), vals0, hist);
-        }
-        return PRT_OK;
-      });
-      if (!rc)
-        rc = radix_sort_pairs<uint32_t>(reinterpret_cast<uint32_t *>(keys0), vals0,
-                                        reinterpret_cast<uint32_t *>(keys1), vals1, n, 32, sel, err, s, hist);
-    } else {
-      long long *ei = reinterpret_cast<long long *>(ext);
-      const Box<int64_t> *b = reinterpret_cast<const Box<int64_t> *>(d_boxes);
-      {
-        PRT_PROF("extent_i64_init", s);
-        extent_i64_init_kernel<<<1, 1, 0, s>>>(ei, t->d_flags);
-      }
-      {
-        PRT_PROF("extent_i64", s);
-        extent_i64_kernel<<<grid_for(n, 256, 4), 256, 0, s>>>(b, n, ei);
-      }
-      {
-        PRT_PROF("ref64", s);
-        ref64_kernel<<<g, 256, 0, s>>>(b, n, ei, reinterpret_cast<uint64_t *>(keys0), vals0);
-      }
-      rc = radix_sort_pairs<uint64_t>(reinterpret_cast<uint64_t *>(keys0), vals0,
-                                      reinterpret_cast<uint64_t *>(keys1), vals1, n, 64, sel, err, s);
+  const int g = grid_for(n, 256, 16);
+  if (t->key_mode == PRT_KEY_MORTON32) {
+    {
+      PRT_PROF("extent_init", s);
+      extent_init_kernel<<<1, 256, 0, s>>>(ext, t->d_flags, hist);
     }
+    rc = dispatch_coord(t->coord, [&](auto tag) {
+      using T = decltype(tag);
+      const Box<T> *b = reinterpret_cast<const Box<T> *>(d_boxes);
+      {
+        PRT_PROF("extent_f64", s);
+        // 16 blocks per SM: enough loads in flight to stream the boxes
+        extent_f64_kernel<T><<<grid_for(n, 256, 16), 256, 0, s>>>(b, n, ext);
+      }
+      {
+        PRT_PROF("morton32", s);
+        morton32_kernel<T><<<g, 256, 0, s>>>(b, n, ext, reinterpret_cast<uint32_t *>(keys0), vals0, hist);
+      }
+      return PRT_OK;
+    });
+    if (!rc)
+      rc = radix_sort_pairs<uint32_t>(reinterpret_cast<uint32_t *>(keys0), vals0,
+                                      reinterpret_cast<uint32_t *>(keys1), vals1, n, 32, sel, err, s, hist);
   } else {
-    rc = cuda_status(e, "memset");
+    long long *ei = reinterpret_cast<long long *>(ext);
+    const Box<int64_t> *b = reinterpret_cast<const Box<int64_t> *>(d_boxes);
+    {
+      PRT_PROF("extent_i64_init", s);
+      extent_i64_init_kernel<<<1, 1, 0, s>>>(ei, t->d_flags);
+    }
+    {
+      PRT_PROF("extent_i64", s);
+      extent_i64_kernel<<<grid_for(n, 256, 4), 256, 0, s>>>(b, n, ei);
+    }
+    {
+      PRT_PROF("ref64", s);
+      ref64_kernel<<<g, 256, 0, s>>>(b, n, ei, reinterpret_cast<uint64_t *>(keys0), vals0);
+    }
+    rc = radix_sort_pairs<uint64_t>(reinterpret_cast<uint64_t *>(keys0), vals0,
+                                    reinterpret_cast<uint64_t *>(keys1), vals1, n, 64, sel, err, s);
   }
   if (!rc) rc = dispatch_coord(t->coord, [&](auto tag) {
     using T = decltype(tag);

@@ -753,10 +753,10 @@ static int run_batched(OverlayState &st, const int64_t *d_idx, int64_t count, in
   BinPlan plan, few;
   int64_t counts[PRT_MAX_BINS];
   for (int b = 0; b < nb; b++) counts[b] = hb[b + 1] - hb[b];
-  // Too few pairs to keep the GPU busy one per thread (under half a wave of
-  // the thread-only launch, e.g. the 2 x 10,000-star overlay's ~21k pairs in ~650
-  // warps): clip every pair with a whole warp instead, so there are as
-  // many warps as pairs.  Both clippers give the same output.
+  // Too few pairs to keep the GPU busy one per thread (under half a wave of the
+  // thread-only launch, e.g. the 2 x 10,000-star overlay's ~21k pairs in ~650
+  // warps): clip every pair with a whole warp instead, so that there are as many
+  // warps as pairs.  Both clippers give the same output.
   constexpr int64_t kFewWarps = (int64_t)kSMs * kLptThreadWarpsPerSM / 2;
   prt_schedule run_sc = sc, few_sc = sc;
   unsigned thread_bins = 0;

@@ -6,11 +6,10 @@
 // sort can be captured in a CUDA graph).  Each remaining pass is ONE kernel:
 // a CTA takes the next tile in launch order (atomic ticket), ranks its keys
 // with a warp-level multisplit (lanes with the same digit found by one ballot
-// per digit bit), learns its global digit
-// offsets by decoupled look-back over the preceding tiles (bounded spin, an
-// error flag instead of a hang), stages the tile in shared memory in digit
-// order and writes it out in coalesced runs.  Stable: ranks follow the
-// original order within a warp, then warp order, then tile order.
+// per digit bit), learns its global digit offsets by decoupled look-back over the
+// preceding tiles (bounded spin, an error flag instead of a hang), stages the tile
+// in shared memory in digit order and writes it out in coalesced runs.  Stable:
+// ranks follow the original order within a warp, then warp order, then tile order.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -195,12 +194,12 @@ __global__ void __launch_bounds__(kSortBlock, sizeof(KeyT) == 4 ? PRT_SORT_MIN_B
       }
     }
   }
-  // 1. stable ranks and the warps' digit histograms in one sweep: lanes with
-  //    the same digit are found by one ballot per digit bit; all of
-  //    them read the warp's counter and the lowest bumps it.  Items are ranked in index order (item slot i of lane l is
-  //    tile position wb + 32 i + l), which makes the pass stable.
-  //    Full tiles, all but one per run, go without the checks per item (10M
-  //    32-bit keys: 86 -> 82 us a pass).
+  // 1. stable ranks and the warps' digit histograms in one sweep: lanes with the
+  //    same digit are found by one ballot per digit bit; all of them read the
+  //    warp's counter and the lowest bumps it.  Items are ranked in index order
+  //    (item slot i of lane l is tile position wb + 32 i + l), which makes the pass
+  //    stable.  Full tiles, all but one per run, go without the checks per item
+  //    (10M 32-bit keys: 86 -> 82 us a pass).
   const uint32_t lt = lanemask_lt();
   uint32_t *wh = S.warp_hist[warp];
   uint32_t dr[kItems];  // rank << 9 | digit (256 + lane: no item)

@@ -1,5 +1,5 @@
-// Overlay of a pair in general position by tracing, with the result that the scanbeam clippers (prt_gpc.cuh, prt_wgpc.cuh) give, bit for
-// bit.
+// Overlay of a pair in general position by tracing, with the result that the
+// scanbeam clippers (prt_gpc.cuh, prt_wgpc.cuh) give, bit for bit.
 //
 // GPC sweeps the pair beam by beam (a beam: two neighbouring vertex ys), a chain
 // of dependent steps per beam however little happens in it.  When nothing
@@ -90,8 +90,7 @@ struct Class {
   static constexpr int kTwo = kTwo_;        // 1: exclusive or (an instantiation of its own costs the others nothing)
   static constexpr int kSlabs = (kVerts >> kSlabShift) + 1;
   static constexpr int kContours = kCross / 2 + kMaxRings;
-  static_assert(kList >= kVerts && kCross >= 2 * kMaxRings && kCross < 4095 && kVerts <= kLast &&
-                kList >= kVerts, "limits");
+  static_assert(kList >= kVerts && kCross >= 2 * kMaxRings && kCross < 4095 && kVerts <= kLast, "limits");
 };
 
 template <typename C>
