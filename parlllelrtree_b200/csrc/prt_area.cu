@@ -157,8 +157,8 @@ constexpr int kBwdSmallV = 64;
 constexpr int kBwdMidV = 128;
 constexpr int kBwdLargeV = 256;  // BwdPoly's 8-bit vertex indices hold no more
 constexpr int kBwdMaxT = 16;
-// Warps (pairs) per block of the V-vertex stage: the 256-vertex staging takes
-// 22 KB a pair, so blocks of 2 warps fit 10 pairs an SM where blocks of 4 fit 8.
+// Warps (pairs) per block of the V-vertex stage: the 256-vertex staging takes 23 KB a
+// pair, 8 pairs an SM.
 constexpr int bwd_warps(int V) { return V > kBwdMidV ? 2 : 4; }
 constexpr int kSlabs = 32;
 constexpr unsigned kFullMask = 0xffffffffu;
@@ -759,7 +759,7 @@ __device__ __noinline__ void bwd_pair_global(const Poly &A, const Poly &B, doubl
 // `defer`; the next stages (V = kBwdMidV, kBwdLargeV) take only the pairs the
 // one before listed (`sel`, *sel_count of them).  The gradients of pairs too large for
 // the last stage are taken on the global-memory path by the one before it, which has 16
-// warps per SM for its 10 (10k pairs of 257-400 vertices: 28.5 ms against 40.9).
+// warps per SM for its 8 (10k pairs of 257-400 vertices: 28.5 ms against 40.9).
 struct PairList {
   const int32_t *sel;                   // items of this launch (nullptr: pairs 0 .. n-1)
   const unsigned long long *sel_count;  // how many (device)
@@ -771,9 +771,9 @@ __device__ __forceinline__ int64_t list_items(const PairList &L, int64_t n) {
   return L.sel ? (int64_t)min((unsigned long long)n, *L.sel_count) : n;
 }
 
-// 4 blocks of 4 warps per SM (118-120 registers, no spills; measured at 1M
+// 4 blocks of 4 warps per SM (up to 128 registers, no spills; measured at 1M
 // pairs of 16-64-vertex stars, 5 blocks of the V = 64 kernel spill and run
-// 10% slower).  The 256-vertex stage is bound by its shared memory: 5 blocks
+// 10% slower).  The 256-vertex stage is bound by its shared memory: 4 blocks
 // of 2 warps.  Before it, 50k pairs of 4-160 vertices (a third of them above
 // 128) took 10.8 ms here on the global-memory path and 11.5 ms in the
 // forward's GPC clip.
@@ -909,7 +909,7 @@ constexpr int kTinyBlock = 128;
 // pairs of 4-6 vertices: backward 44 -> 31 us; from some 10,000 on the threads are as
 // fast), and up to kOnePairWave, one wave of the 256-vertex stage, what does not
 // fit goes straight to that.
-constexpr int64_t kFewPairs = 8192, kOnePairWave = (int64_t)kSMs * 10;
+constexpr int64_t kFewPairs = 8192, kOnePairWave = (int64_t)kSMs * 8;
 
 // Appends i to a list for the threads of the block that ask (one atomic per
 // block: when no pair is tiny, every one of them is listed).
@@ -950,9 +950,9 @@ struct TinySmem {
   double gx[kArea ? 1 : kTinyV][kTinyBlock], gy[kArea ? 1 : kTinyV][kTinyBlock];
 };
 
-// 200k parcels (471k pairs): forward 85 us, backward 105 against 535 and 604 with
-// a warp each; 3 blocks per SM for the gradients (120 us against 132 with 4, and
-// 186 with 5), 4 for the areas (103; 107 and 123 with 3 and 5).
+// 200k parcels (471k pairs), the kernel alone: forward 85 us, backward 105 against 535
+// and 604 with a warp each.  The whole call: 120 us backward with 3 blocks per SM, 132
+// with 4 and 186 with 5; 103 us forward with 4, 107 and 123 with 3 and 5.
 template <bool kArea>
 __global__ void __launch_bounds__(kTinyBlock, kArea ? 4 : 3) area_tiny_kernel(
     const int32_t *__restrict__ pa, const int32_t *__restrict__ pb, int64_t n, LayerDev base, LayerDev over,

@@ -314,7 +314,7 @@ def test_many_small_pairs(cuda, na, nb, hole_frac):
                 list(range(200)) + list(range(200, n, 30)))
 
 
-@pytest.mark.parametrize("n", [1, 1480, 1481, 8192, 8193])
+@pytest.mark.parametrize("n", [1, 1184, 1185, 8192, 8193])
 def test_stages_by_the_number_of_pairs(cuda, n):
     """Polygons of all stages' sizes around the numbers of pairs at which the
     one-thread kernel and the 128-vertex stage come in."""
