@@ -745,8 +745,11 @@ constexpr int kCountsBatches = 3;
 // once, kCountsChain in all, as a wait for each would cost more than they do.  2M
 // boxes, F = 16: 100 windows across the whole extent 139 -> 83 us (breadth first 80), 100
 // of 0.1 by 0.1 where nothing can be pruned 359 -> 112 (128); 100 small windows, for
-// which there is nothing left, 53 -> 58 (66).
+// which there is nothing left, 53 -> 58 (66).  Not on trees of under kCountsLong nodes,
+// where walks are short.  With a look at what is left before the later launches small
+// windows stay at 53, and long ones take 126 and 157.
 constexpr int kCountsFew = 8, kCountsFewSteps = 24, kCountsChain = 3;
+constexpr int64_t kCountsLong = 1024;
 
 template <int G>
 constexpr int counts_rounds() { return G == 32 ? 4 : G == 16 ? 2 : 1; }
@@ -1053,8 +1056,10 @@ int prt_query_counts(const prt_tree *t, const void *d_queries, int coord_type, i
   CountsTree c;
   c.mbr = t->d_mbr;
   c.levels = t->lv.levels;
+  int64_t all_nodes = 0;
   for (int l = 0; l < c.levels; l++) {
     const int64_t nodes = t->lv.padded[l] / t->fanout, first = t->lv.offset[l];
+    all_nodes += nodes;
     c.lv[l].first = (uint32_t)first;
     c.lv[l].last = (uint32_t)(first + (nodes - 1) * t->fanout);
     c.lv[l].fill = (uint32_t)(t->lv.count[l] - (nodes - 1) * t->fanout);
@@ -1088,7 +1093,7 @@ int prt_query_counts(const prt_tree *t, const void *d_queries, int coord_type, i
           int b = 0;
           PRT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, kCountsBlock, smem));
           const int64_t resident = (int64_t)kSMs * std::max(b, 1);
-          if (!Q.in && nq * kCountsFew < resident * kWarps) chain = kCountsChain;
+          if (!Q.in && nq * kCountsFew < resident * kWarps && all_nodes >= kCountsLong) chain = kCountsChain;
           if (batch) batch = (int)std::min<int64_t>(32, nq / (resident * kWarps * kCountsBatches));
           const int64_t per = (int64_t)kWarps * std::max(batch, 1);
           const int64_t blocks = Q.in ? resident : std::min<int64_t>((nq + per - 1) / per, resident);
