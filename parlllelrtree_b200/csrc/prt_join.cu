@@ -711,6 +711,7 @@ struct CountsQueue {
   CountsItem *out;               // work left over
   unsigned long long *out_count;
   int64_t out_cap;
+  unsigned *ticket;              // batches taken beyond the warps' first ones
 };
 
 // Per-query counters (entries examined, sum of max(0, hits - 1) per visited
@@ -727,19 +728,23 @@ struct CountsQueue {
 // Bound by instruction issue (0.77 per cycle and scheduler): some 110 instructions a
 // step and 60 a query.  From kCountsBatched queries on a warp therefore takes several
 // and tests them against the root a lane each: 1M windows of 1e-4..1e-2 on 10M boxes
-// 2.17 -> 2.06 ms at F = 16 (breadth first 3.55), on 10k and 100k boxes 0.62 -> 0.52 and
-// 0.83 -> 0.73 ms (breadth first 0.50 and 0.74; 100k windows are the same either
-// way).  Without batches, 10M boxes: 1 and 3 rounds at F = 16 2.67 and 2.10 ms, 5
+// 2.32 -> 1.82 ms at F = 16 (breadth first 3.55), on 10k and 100k boxes 0.62 -> 0.49 and
+// 0.82 -> 0.68 ms (breadth first 0.50 and 0.74).
+// Without batches, 10M boxes: 1 and 3 rounds at F = 16 2.67 and 2.10 ms, 5
 // blocks per SM 2.42; two walks per warp 2.71.  Nodes of 8 entries and fewer keep the
 // warp too little to do per round (313k windows on 740k boxes, F = 8: 409 us against
 // 325): they go breadth first (kCountsWideFanout).
 constexpr int kCountsBlock = 256;
 constexpr int kCountsSteps = 256;
 constexpr int kCountsWideFanout = 9;  // fanouts from here on go depth first
-// Calls of so many queries batch them, so that a warp gets kCountsBatches batches or
-// more of 8 to 32 queries.
+// Calls of so many queries batch them, kCountsBatch at a time, a warp's first batch by
+// its index and the next ones from a counter.  Batches dealt out in advance differ in
+// what their walks cost and in how many a warp gets: 1M windows on 10M boxes 2.08 ms,
+// 1.82 from the counter, 300k 0.79 and 0.68, 131k 0.45 and 0.41 (batches of 16 1.85,
+// 0.73 and 0.46; of 4 1.82, 0.66 and 0.38, but 3 to 6% slower on 10k and 1M boxes, where
+// a walk is short and the root's share in it large).
 constexpr int64_t kCountsBatched = 1 << 17;
-constexpr int kCountsBatches = 3;
+constexpr int kCountsBatch = 8;
 // Queries that leave most warps idle (kCountsFew times as many could be resident)
 // hand what is left of a walk on after kCountsFewSteps, to launches that are made at
 // once, kCountsChain in all, as a wait for each would cost more than they do.  2M
@@ -764,17 +769,17 @@ inline int counts_stack(int levels, int fanout, int pop) { return (2 * levels + 
 // entries that each hits and contains, and the root's entries.
 template <typename T>
 struct CountsBatch {
-  Box<T> query[kCountsBlock / 32][32];
-  uint2 hits[kCountsBlock / 32][32];
+  Box<T> query[kCountsBlock / 32][kCountsBatch];
+  uint2 hits[kCountsBlock / 32][kCountsBatch];
   Box<T> root[32];
 };
 
-// kBatch: a warp takes `batch` queries at a time, a lane of it testing each against
+// kBatch: a warp takes kCountsBatch queries at a time, a lane of it testing each against
 // the root, and then walks for those that hit something there (trees of two
 // levels and more, not for left-over work).
 template <typename T, int G, bool kBatch>
 __global__ void __launch_bounds__(kCountsBlock, sizeof(T) == 4 ? 4 : 3)
-    counts_kernel(CountsTree t, const Box<T> *__restrict__ queries, int64_t nq, int batch, int max_steps, int fanout,
+    counts_kernel(CountsTree t, const Box<T> *__restrict__ queries, int64_t nq, int max_steps, int fanout,
                   int td_slots, int stack_cap, const unsigned *__restrict__ flags, long long *__restrict__ counts, CountsQueue Q) {
   extern __shared__ __align__(32) unsigned char s_raw[];
   constexpr int kNodes = 32 / G, kRounds = counts_rounds<G>(), kPop = counts_pop<G>();
@@ -797,15 +802,18 @@ __global__ void __launch_bounds__(kCountsBlock, sizeof(T) == 4 ? 4 : 3)
   const bool prune = all_proper(flags);
   const int room = stack_cap - (t.levels + kPop) * (fanout - 1);  // most entries a kPop step may start from
   const uint32_t leaf_last = s_lv[0].last, leaf_lack = fanout - s_lv[0].fill;
-  const int64_t step = kBatch ? batch : 1, stride = (int64_t)gridDim.x * (kCountsBlock / 32) * step;
-  for (int64_t w = (blockIdx.x * (int64_t)(kCountsBlock / 32) + warp) * step; w < work; w += stride) {
+  const uint32_t warps = gridDim.x * (kCountsBlock / 32);
+  constexpr int step = kBatch ? kCountsBatch : 1;
+  for (int64_t w = (int64_t)(blockIdx.x * (kCountsBlock / 32) + warp) * step; w < work;) {
+    uint32_t next = 0;
+    if (kBatch && lane == 0) next = atomicAdd(Q.ticket, 1u);
     uint32_t todo = 1u;  // queries of the batch to walk for
     CountsItem it{(uint32_t)w, s_lv[t.levels - 1].first, t.levels - 1};
     if constexpr (kBatch) {
       const uint32_t fill = s_lv[t.levels - 1].fill;
       uint32_t hits = 0, conts = 0;
       __syncwarp();
-      if (lane < batch && w + lane < nq) {
+      if (lane < step && w + lane < nq) {
         const Box<T> q = load_box(queries, w + lane);
         for (uint32_t j = 0; j < fill; j++) {
           const Box<T> r = B.root[j];
@@ -939,6 +947,7 @@ __global__ void __launch_bounds__(kCountsBlock, sizeof(T) == 4 ? 4 : 3)
         else *out = v;
       }
     }
+    w = kBatch ? (int64_t)(warps + __shfl_sync(0xffffffffu, next, 0)) * step : w + warps;
   }
 }
 
@@ -1071,16 +1080,17 @@ int prt_query_counts(const prt_tree *t, const void *d_queries, int coord_type, i
   CountsItem *queue = nullptr;
   unsigned long long *left = nullptr;
   rc = dalloc(&queue, 2 * kQueue, s);
-  if (!rc) rc = dalloc(&left, kCountsChain + 1, s);
+  if (!rc) rc = dalloc(&left, kCountsChain + 2, s);
   int chain = 1, round = 0;  // launches until the host looks
   unsigned long long n_left = 1;
   while (!rc && n_left > 0) {
-    cudaError_t e = cudaMemsetAsync(left, 0, 8 * kCountsChain, s);
+    cudaError_t e = cudaMemsetAsync(left, 0, 8 * (kCountsChain + 1), s);
     int last = 0;
     for (int i = 0; i < chain && e == cudaSuccess && !rc; i++, round++) {
       CountsQueue Q;
       Q.in = round ? queue + ((round - 1) & 1) * kQueue : nullptr;
-      Q.n_in = i ? &left[i - 1] : left + kCountsChain;
+      Q.n_in = i ? &left[i - 1] : left + kCountsChain + 1;
+      Q.ticket = reinterpret_cast<unsigned *>(left + kCountsChain);
       Q.out = queue + (round & 1) * kQueue;
       Q.out_count = &left[last = i];
       Q.out_cap = kQueue;
@@ -1094,18 +1104,17 @@ int prt_query_counts(const prt_tree *t, const void *d_queries, int coord_type, i
           PRT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, kCountsBlock, smem));
           const int64_t resident = (int64_t)kSMs * std::max(b, 1);
           if (!Q.in && nq * kCountsFew < resident * kWarps && all_nodes >= kCountsLong) chain = kCountsChain;
-          if (batch) batch = (int)std::min<int64_t>(32, nq / (resident * kWarps * kCountsBatches));
-          const int64_t per = (int64_t)kWarps * std::max(batch, 1);
+          const int64_t per = (int64_t)kWarps * batch;
           const int64_t blocks = Q.in ? resident : std::min<int64_t>((nq + per - 1) / per, resident);
           const int steps = i + 1 < chain ? kCountsFewSteps : kCountsSteps;
           PRT_PROF("counts", s);
           PRT_CUDA(launch_dependent(kernel, (int)blocks, kCountsBlock, smem, s, c,
-                                    reinterpret_cast<const Box<T> *>(d_queries), nq, batch, steps, t->fanout, td_slots,
+                                    reinterpret_cast<const Box<T> *>(d_queries), nq, steps, t->fanout, td_slots,
                                     cap, t->d_flags, reinterpret_cast<long long *>(d_counts), Q));
           return PRT_OK;
         };
-        if (!Q.in && c.levels > 1 && nq >= kCountsBatched) return launch(counts_kernel<T, G, true>, sizeof(CountsBatch<T>), 1);
-        return launch(counts_kernel<T, G, false>, 0, 0);
+        if (!Q.in && c.levels > 1 && nq >= kCountsBatched) return launch(counts_kernel<T, G, true>, sizeof(CountsBatch<T>), kCountsBatch);
+        return launch(counts_kernel<T, G, false>, 0, 1);
       });
     }
     if (!rc && e == cudaSuccess) e = cudaMemcpyAsync(&n_left, &left[last], 8, cudaMemcpyDeviceToHost, s);
@@ -1114,7 +1123,7 @@ int prt_query_counts(const prt_tree *t, const void *d_queries, int coord_type, i
     if (rc || n_left == 0) break;
     chain = 1;
     // the count of what this round left, where the next one's first launch reads it
-    e = cudaMemcpyAsync(left + kCountsChain, &left[last], 8, cudaMemcpyDeviceToDevice, s);
+    e = cudaMemcpyAsync(left + kCountsChain + 1, &left[last], 8, cudaMemcpyDeviceToDevice, s);
     if (e != cudaSuccess) rc = cuda_status(e, "query counts");
   }
   dfree(queue, s);
