@@ -242,7 +242,8 @@ int prt_results_device(const prt_results *r, const int64_t **pair_cont_start,
                        const int32_t **pair_ncont, const int64_t **cont_vert_start,
                        const int32_t **cont_nverts, const int32_t **cont_hole, const double **xy);
 /* Copies the results to host buffers in pair order (CSR): h_pair_cont_off
- * [pairs+1], h_cont_nverts / h_cont_hole [contours], h_xy [2*vertices]. */
+ * [pairs+1], h_cont_nverts / h_cont_hole [contours], h_xy [2*vertices].  Takes
+ * device memory for the contours' headers and at most 64 MiB of vertices. */
 int prt_results_copy(const prt_results *r, int64_t *h_pair_cont_off, int32_t *h_cont_nverts,
                      int32_t *h_cont_hole, double *h_xy);
 /* Copies the results of the k pairs listed in h_pairs (pair indices) to host

@@ -25,10 +25,12 @@
 // even-odd test of each midpoint when a crossing is not clean; see
 // pair_boundary).  Contributions are scaled by the upstream gradient and
 // accumulated with atomicAdd, since a polygon may appear in many pairs.  Both
-// directions run in stages: polygons of up to 64 vertices staged in shared
-// memory first, the pairs that do not fit listed for a 128-vertex staging,
-// then a 256-vertex one, and larger ones on a global-memory path (backward)
-// or the GPC clip (forward).
+// directions run in stages: pairs of one-ring polygons of at most 8 vertices a
+// thread each (area_tiny_kernel; with few pairs the next stage does them too),
+// polygons of up to 64 vertices staged in shared memory (backward: pairs of 32
+// together in a form of their own), the pairs that do not fit listed for a
+// 128-vertex staging, then a 256-vertex one, and larger ones on a global-memory
+// path (backward, on the 128-vertex stage) or the GPC clip (forward).
 #include <cuda_runtime.h>
 
 #include <atomic>
